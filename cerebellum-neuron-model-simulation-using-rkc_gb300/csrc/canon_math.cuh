@@ -33,19 +33,20 @@
 #include <math.h>
 #include <stdint.h>
 
+#include "fp_int.cuh"
+
 #define CM_LN2_HI 0x1.62e42fefa2000p-1
 #define CM_LN2_LO 0x1.9ef35793c7673p-41
 #define CM_INV_LN2 0x1.71547652b82fep+0
-#define CM_SQRT2 0x1.6a09e667f3bcdp+0
 
-__host__ __device__ static inline uint64_t cm_bits(double x) {
+GB_HD uint64_t cm_bits(double x) {
 #ifdef __CUDA_ARCH__
   return (uint64_t)__double_as_longlong(x);
 #else
   uint64_t u; __builtin_memcpy(&u, &x, 8); return u;
 #endif
 }
-__host__ __device__ static inline double cm_from_bits(uint64_t u) {
+GB_HD double cm_from_bits(uint64_t u) {
 #ifdef __CUDA_ARCH__
   return __longlong_as_double((long long)u);
 #else
@@ -53,11 +54,16 @@ __host__ __device__ static inline double cm_from_bits(uint64_t u) {
 #endif
 }
 
-__host__ __device__ static inline double cm_exp(double x) {
-  if (x != x) return x;
-  if (x > 709.782712893384) return HUGE_VAL;
-  if (x < -745.1332191019412) return 0.0;
-  double kd = rint(x * CM_INV_LN2);
+GB_HD double cm_exp(double x) {
+  /* range checks on the bits: |x| < 704 (0x40860000...) needs none */
+  if ((uint32_t)(cm_bits(x) >> 32 & 0x7fffffff) >= 0x40860000u) {
+    if (x != x) return x;
+    if (x > 709.782712893384) return HUGE_VAL;
+    if (x < -745.1332191019412) return 0.0;
+  }
+  /* rint and its integer by adding and subtracting 1.5 2^52 (|x / ln2| < 2^11) */
+  const double sh = x * CM_INV_LN2 + 0x1.8p52;
+  const double kd = sh - 0x1.8p52;
   double r = fma(-kd, CM_LN2_HI, x);
   r = fma(-kd, CM_LN2_LO, r);
   double p = 0x1.6124613a86d09p-33;          /* 1/13! */
@@ -74,23 +80,28 @@ __host__ __device__ static inline double cm_exp(double x) {
   p = fma(p, r, 0x1.0000000000000p-1);       /* 1/2!  */
   p = fma(p, r, 1.0);
   p = fma(p, r, 1.0);
-  int k = (int)kd;
+  int k = (int)(uint32_t)cm_bits(sh);
   if (k > 1023) { p *= 2.0; k -= 1; }
   if (k < -1022) { p *= 0x1p-54; k += 54; }
   return p * cm_from_bits((uint64_t)(k + 1023) << 52);
 }
 
-__host__ __device__ static inline double cm_log(double x) {
-  if (!(x > 0.0)) return (x == 0.0) ? -HUGE_VAL : (x - x) / (x - x);
-  if (x == HUGE_VAL) return x;
+GB_HD double cm_log(double x) {
   int e = 0;
-  if (x < 0x1p-1022) { x *= 0x1p54; e = -54; }
   uint64_t u = cm_bits(x);
+  if (u - (1ULL << 52) >= 0x7ff0000000000000ULL - (1ULL << 52)) {  /* not a positive normal number */
+    if (!(x > 0.0)) return (x == 0.0) ? -HUGE_VAL : (x - x) / (x - x);
+    if (x == HUGE_VAL) return x;
+    x *= 0x1p54;
+    e = -54;
+    u = cm_bits(x);
+  }
   e += (int)((u >> 52) & 0x7ff) - 1023;
-  double m = cm_from_bits((u & 0x000fffffffffffffULL) | 0x3ff0000000000000ULL);
-  if (m > CM_SQRT2) { m *= 0.5; e += 1; }
+  const int up = (u & 0x000fffffffffffffULL) > 0x6a09e667f3bcdULL;   /* m > sqrt 2: halve it */
+  e += up;
+  double m = cm_from_bits((u & 0x000fffffffffffffULL) | ((uint64_t)(1023 - up) << 52));
   double f = m - 1.0;
-  double s = f / (2.0 + f);
+  double s = gbrkc::mdiv(f, 2.0 + f);
   double z = s * s;
   double R = 0x1.642c8590b2164p-4;           /* 2/23 */
   R = fma(R, z, 0x1.8618618618618p-4);       /* 2/21 */
@@ -105,13 +116,13 @@ __host__ __device__ static inline double cm_log(double x) {
   R = fma(R, z, 0x1.5555555555555p-1);       /* 2/3  */
   R = R * z;
   double lm = fma(s, R, 2.0 * s);
-  double ed = (double)e;
+  double ed = cm_from_bits(0x4338000000000000ULL + (uint64_t)(int64_t)e) - 0x1.8p52;   /* (double)e */
   return fma(ed, CM_LN2_HI, fma(ed, CM_LN2_LO, lm));
 }
 
-__host__ __device__ static inline double cm_pow(double x, double y) { return cm_exp(y * cm_log(x)); }
+GB_HD double cm_pow(double x, double y) { return cm_exp(y * cm_log(x)); }
 
-#define CM_FN __host__ __device__ static inline
+#define CM_FN GB_HD
 /* Cube root for the step-size controller's err^(1/3), err >= 0.
  * x = 2^e m with m in [1, 2); e = 3q + r (r = 0, 1, 2) and z = 2^r m in
  * [1, 8), so cbrt(x) = 2^q cbrt(z).  The reciprocal cube root y = z^(-1/3)
@@ -125,15 +136,19 @@ __host__ __device__ static inline double cm_pow(double x, double y) { return cm_
  * arithmetic: within 4 ulp, 0.7 ulp on average (tests/test_canon_math.py).  0, +inf and NaN
  * return themselves. */
 CM_FN double cm_cbrt(double x) {
-  if (!(x > 0.0) || x == HUGE_VAL) return x;
   int e = 0;
-  if (x < 0x1p-1022) { x *= 0x1p54; e = -54; }
-  const uint64_t u = cm_bits(x);
+  uint64_t u = cm_bits(x);
+  if (u - (1ULL << 52) >= 0x7ff0000000000000ULL - (1ULL << 52)) {  /* not a positive normal number */
+    if (!(x > 0.0) || x == HUGE_VAL) return x;
+    x *= 0x1p54;
+    e = -54;
+    u = cm_bits(x);
+  }
   e += (int)((u >> 52) & 0x7ff) - 1023;
   const int q = (e >= 0) ? e / 3 : -((2 - e) / 3);
   const int r = e - 3 * q;
   const double Z = cm_from_bits((u & 0x000fffffffffffffULL) | ((uint64_t)(1023 + r) << 52));
-  const float zf = (float)Z;
+  const float zf = gbrkc::d2f(Z);
   float y = 0x1.0b5c7ap+0f;
   y = y + (-0x1.1bfbb8p-3f) * zf;
   y = y + (0x1.2a6c02p-7f) * zf * zf;
@@ -142,7 +157,7 @@ CM_FN double cm_cbrt(double x) {
     const float t = 4.0f - zf * y3;
     y = (y * t) * 0x1.555556p-2f;
   }
-  double Y = (double)y;
+  double Y = gbrkc::f2d(y);
   for (int k = 0; k < 2; k++) {
     const double Y3 = (Y * Y) * Y;
     const double d = fma(-Z, Y3, 1.0);

@@ -472,7 +472,7 @@ struct gbrkc_engine {
   int gr_warps = 0;             // granule warps of the next launch (32 lanes each)
   int gr_warps_need = 0;        // granule warps that would give every granule system with work its own lane
   int gr_warps_max = 0;         // granule warps the CTAs can hold beside the other roles
-  int lanes = 16;               // lanes of a warp that take single-lane systems
+  int lanes = 16;               // lanes of a warp in use by granule systems (one each, or four: TEAM_LANE4)
   long gr_active = -1;          // granule systems with work (-1: not known yet)
   double role_work[NTYPES] = {};  // smoothed CTA-ms per role
   int *d_queue = nullptr;
@@ -513,7 +513,8 @@ extern "C" int gbrkc_engine_create(int precision, gbrkc_engine **out) {
   std::unique_ptr<gbrkc_engine> E(new gbrkc_engine());
   E->precision = precision;
   E->gr_f64 = precision == GBRKC_MIXED && mixed_granules_fp64();
-  // lanes per warp that take single-lane systems: fewer systems in a warp
+  // lanes per warp that take single-lane systems (granule cells of other than
+  // four compartments; for those see build_impl): fewer systems in a warp
   // diverge less but need more warps (measured on the GB300: 1024 granule
   // cells on 32 SMs took 115 / 103 / 95 ms per simulated ms with 32 / 16 / 8
   // lanes; the mixed workload's persistent launch 596 / 574 / 628 / 1135 ms
@@ -755,6 +756,11 @@ void fill_state(gbrkc_engine *E, PoolHost &P, const HostSystem &S, long off, int
   }
 }
 
+// granule systems a warp takes with `lanes` of its lanes in use
+int systems_per_warp(const PoolHost &P, int lanes) {
+  return P.team == TEAM_LANE4 ? quads_per_warp(lanes) : lanes;
+}
+
 int assemble_pool(gbrkc_engine *E, PoolHost &P) {
   const int type = P.type;
   const int nion = NION[type], ncond = NCOND[type];
@@ -871,9 +877,8 @@ int assemble_pool(gbrkc_engine *E, PoolHost &P) {
   P.ws_total = ws;
   // launch configuration: team shape by system size, workspace in shared
   // memory when it fits
-  // tiny cells: one system per thread, the block's first warps spread over
-  // the SMs (a warp's FP64 instructions cost the same for 1 or 32 lanes, so
-  // 32 systems side by side beat one system over 4 lanes)
+  // tiny cells: one system per thread (or per four, one compartment a lane),
+  // the block's first warps spread over the SMs
   const int nsys = (int)P.systems.size();
   if (P.max_nc <= LANE_MAX_NC) {
     P.team = (P.type == GR && P.min_nc == 4 && P.max_nc == 4 && P.max_ncell == 1) ? TEAM_LANE4 : TEAM_THREAD;
@@ -988,7 +993,8 @@ int assemble_pool(gbrkc_engine *E, PoolHost &P) {
     int dev = 0, sms = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    P.grid = std::max(1, std::min((nsys + 31) / 32, sms));
+    const int per = systems_per_warp(P, 32);
+    P.grid = std::max(1, std::min((nsys + per - 1) / per, sms));
   } else {
     P.grid = (nsys + teams - 1) / teams;
   }
@@ -1097,6 +1103,7 @@ int upload_pool(gbrkc_engine *E, PoolHost &P, PoolView<R> &V) {
   }
   V.soma_out = nullptr;
   V.lanes = E->lanes;
+  V.per_warp = systems_per_warp(P, E->lanes);
   V.rec_w = P.rec_w;
   P.d_cell_soma = const_cast<int *>(V.cell_soma);
   V.ncell_pool = P.ncell;
@@ -1126,8 +1133,8 @@ bool granules_all_in_flight(const gbrkc_engine *E, long warps) {
   return (warps + MEGA_BLOCK / 32 - 1) / (MEGA_BLOCK / 32) <= (E->mega_grid - nother) / 2;
 }
 
-// Granule warps for the next persistent launch: one lane per granule system
-// with work (parked slots, finished budgets and stopped systems need none).
+// Granule warps for the next persistent launch: a place (one lane, or four)
+// per granule system with work (parked slots, finished budgets and stopped systems need none).
 // When they are all in flight (granules_all_in_flight) the granule CTAs are
 // re-fitted to them at once, the other roles giving the difference; else
 // the warps fill the granule role's CTAs (at most 8 a CTA) and lanes take
@@ -1140,10 +1147,15 @@ void fit_granule_warps(gbrkc_engine *E) {
   // the preferred lanes per warp, doubled while the warps would need more
   // than half of the CTAs' warp slots (the other roles need the rest)
   int lanes = E->lanes;
-  while (lanes < 32 && (active + lanes - 1) / lanes > E->gr_warps_max / 2) lanes = std::min(32, 2 * lanes);
+  auto warps_for = [&](int l) {
+    const int k = systems_per_warp(G, l);
+    return (active + k - 1) / k;
+  };
+  while (lanes < 32 && warps_for(lanes) > E->gr_warps_max / 2) lanes = std::min(32, 2 * lanes);
   G.vd.lanes = G.vf.lanes = lanes;
+  G.vd.per_warp = G.vf.per_warp = systems_per_warp(G, lanes);
   const int per = MEGA_BLOCK / 32;
-  const long need = std::max(1L, std::min((long)E->gr_warps_max, (active + lanes - 1) / lanes));
+  const long need = std::max(1L, std::min((long)E->gr_warps_max, warps_for(lanes)));
   E->gr_warps_need = (int)need;
   const bool all_in = granules_all_in_flight(E, need);
   const int want = all_in ? (int)need : (int)std::min(need, (long)per * E->role_ctas[GR]);
@@ -1438,7 +1450,8 @@ int setup_mega(gbrkc_engine *E) {
     int others_n = 0;
     for (int t = 1; t < NTYPES; t++) others_n += !E->pools[t].systems.empty();
     E->gr_warps_max = (E->mega_grid - others_n) * (MEGA_BLOCK / 32);
-    const long need = ((long)E->pools[GR].systems.size() + 31) / 32;
+    const int k = systems_per_warp(E->pools[GR], 32);
+    const long need = ((long)E->pools[GR].systems.size() + k - 1) / k;
     E->gr_warps = (int)std::min<long>(need, E->gr_warps_max);
     E->gr_warps_need = E->gr_warps;
   }
@@ -1454,13 +1467,13 @@ int setup_mega(gbrkc_engine *E) {
   if (E->role_ctas[GR] > 0) {
     // two granule warps to a CTA beside other roles, else spread over all;
     // beside other roles at most the granule share of the estimated work (a
-    // granule compartment costs about 29 Golgi compartments: the granule
+    // granule compartment costs about ten Golgi compartments: the granule
     // controller's tolerance of 1e-9 keeps its steps short)
     E->role_ctas[GR] = others ? (E->gr_warps + 1) / 2 : std::min(E->gr_warps, E->mega_grid);
     if (others) {
       double wo = 0.0;
       for (int t = 1; t < NTYPES; t++) wo += w[t] * (double)E->pools[t].nc;
-      const double wg = 29.0 * (double)E->pools[GR].nc;
+      const double wg = 10.0 * (double)E->pools[GR].nc;
       E->role_ctas[GR] = std::min(E->role_ctas[GR], std::max(1, (int)(E->mega_grid * wg / (wg + wo))));
     }
     E->role_ctas[GR] = std::max(1, std::min(E->role_ctas[GR], E->mega_grid - others));
@@ -1672,6 +1685,10 @@ static int build_impl(gbrkc_engine *E) {
     int rc = assemble_pool(E, P);
     if (rc) return rc;
   }
+  // granule cells of four compartments start from two to a warp (8 lanes): the
+  // fewer share a warp the less it diverges, and fit_granule_warps doubles
+  // the count while the warps would not fit
+  if (E->pools[GR].team == TEAM_LANE4 && !getenv("GBRKC_LANES")) E->lanes = 8;
   {
     int rc = setup_mega(E);
     if (rc) return rc;
@@ -1771,7 +1788,8 @@ extern "C" int gbrkc_advance(gbrkc_engine *E, double t0, int n_iv) {
 extern "C" int gbrkc_retired_systems(gbrkc_engine *E) { return E ? E->n_retired : 0; }
 
 // ------------------------------------------------------- gbrkc_autotune
-// Granule systems run one per lane; how many lanes of a warp take systems
+// Granule systems run one per lane, or one per four lanes where they have
+// four compartments (quad_sys.cuh); how many lanes of a warp are in use
 // (cells per warp, hence per CTA) trades divergence -- a warp runs the union
 // of its lanes' step-attempt paths -- against warps, i.e. CTAs taken from the
 // other roles.  The best count depends on the workload's dynamics and mix,

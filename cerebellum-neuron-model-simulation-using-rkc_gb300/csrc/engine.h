@@ -109,7 +109,8 @@ struct PoolView {
   int *spk_count;
   int spk_cap;
   double spk_th;
-  int lanes;                          // single-lane pools: lanes of each warp that take systems
+  int lanes;                          // granule pools: lanes of each warp in use, one system a lane or (TEAM_LANE4) per four
+  int per_warp;                       // granule pools: systems a warp takes (lanes, or lanes / 4)
   int ws_in_smem;                     // stage the workspace in shared memory
   long ws_tile_doubles;               // shared-memory workspace per team
   // chemical synapses onto this pool (network mode; syn_mode 0 = none)
@@ -171,8 +172,8 @@ int launch_syn_update(const SynView &S, void *stream, double t, long long interv
 // Team shapes the kernels are instantiated for: one thread (tiny cells, 32
 // systems per warp, blocks of MEGA_BLOCK threads with interleaved shared
 // workspaces), 4 or 32 lanes per system, or a whole block per system.
-// TEAM_LANE4: one thread per system for pools whose systems all have exactly
-// 4 compartments (loops unrolled at compile time).
+// TEAM_LANE4: four lanes per system for pools whose systems all have exactly
+// 4 compartments, one compartment a lane (quad_sys.cuh).
 // TEAM_CLUSTER8 / TEAM_CLUSTER16: one system per cluster of 8 / 16 CTAs
 // (very large systems; 16 is a non-portable cluster size, used where the
 // device can co-schedule it).
@@ -182,12 +183,14 @@ enum TeamKind {
   TEAM_THREAD = 1, TEAM_LANE4 = 2, TEAM_TILE4 = 4, TEAM_WARP = 32, TEAM_BLOCK = 0,
   TEAM_CLUSTER8 = 108, TEAM_CLUSTER16 = 116, TEAM_GRID = 200
 };
+// systems a warp takes when `lanes` of its lanes are in use, four lanes each
+constexpr int quads_per_warp(int lanes) { return lanes < 8 ? 1 : lanes / 4; }
 constexpr int team_cluster_size(int team) {
   return team == TEAM_CLUSTER8 ? 8 : team == TEAM_CLUSTER16 ? 16 : 0;
 }
 
 // All pools in one persistent launch: CTA b < role_end[0] integrates granule
-// systems (one per lane, on the CTA's first warps), then Golgi
+// systems (one per lane or per four, on the CTA's first warps), then Golgi
 // (32-lane warps), Purkinje and olive (whole blocks).  Each role pulls
 // systems from its own atomic queue.
 template <typename R>

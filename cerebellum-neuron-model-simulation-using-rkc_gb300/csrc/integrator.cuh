@@ -369,6 +369,20 @@ __device__ __forceinline__ void log_spike(const PoolView<R> &P, int pc, double t
   P.spk_prev[pc] = x;
 }
 
+// The stage count 1 + (int)sqrt(x) of a step (solve_rkc.cu:954-961), the root
+// rounded to FP64 first; false where it is NaN or 10^9 and above.
+__device__ __forceinline__ bool stage_count(double x, int &m) {
+  bool ok;
+  int r = int_sqrt(x, ok);
+  if (!ok) {
+    const double marg = sqrt(x);
+    if (!(marg < 1.0e9)) return false;
+    r = (int)marg;
+  }
+  m = 1 + r;
+  return true;
+}
+
 template <int CT, typename R, class Team>
 struct Sys {
   static constexpr int LS = Team::LS, NCF = Team::NCF;
@@ -386,6 +400,8 @@ struct Sys {
   // flat driver state
   double t0;
   int k_iv, n_iv, iv0, rej_run;
+  int mmax;                    // c.mmax, an integer
+  Recip rnc;                   // 1 / nc
   long long attempts0;
   mutable int red_buf = 0;     // cluster reductions: block-sum buffer in use
 
@@ -689,22 +705,23 @@ struct Sys {
     const double ynrm = sqrt(sumsq(yn));
     const double vnrm = sqrt(sumsq(ede));
     double dynrm;
-    if (ynrm != 0.0 && vnrm != 0.0) {
+    if (!fpi_is_zero(ynrm) && !fpi_is_zero(vnrm)) {
       dynrm = ynrm * sqrtu;
-      const double al = dynrm / vnrm;
+      const double al = mdiv(dynrm, vnrm);
       for (int i = tm.rank(); i < nc; i += tm.size()) v1[i] = fma(al, ede[i], yn[i]);
-    } else if (ynrm != 0.0) {
+    } else if (!fpi_is_zero(ynrm)) {
       dynrm = ynrm * sqrtu;
       for (int i = tm.rank(); i < nc; i += tm.size()) v1[i] = fma(sqrtu, yn[i], yn[i]);
-    } else if (vnrm != 0.0) {
+    } else if (!fpi_is_zero(vnrm)) {
       dynrm = uround;
-      const double al = dynrm / vnrm;
+      const double al = mdiv(dynrm, vnrm);
       for (int i = tm.rank(); i < nc; i += tm.size()) v1[i] = al * ede[i];
     } else {
       dynrm = uround;
       for (int i = tm.rank(); i < nc; i += tm.size()) v1[i] = dynrm;
     }
     tm.sync();
+    const Recip rdyn = recip(dynrm);
     double sigma = 0.0, sigmal;
     for (int iter = 0; iter < RHO_ITMAX; iter++) {
       c.n_rho_iter++;
@@ -732,12 +749,12 @@ struct Sys {
       }
       const double dfnrm = sqrt(dfsq);
       sigmal = sigma;
-      sigma = dfnrm / dynrm;
+      sigma = div_by(dfnrm, rdyn);
       sprad_old[0] = sprad_old[1];
       sprad_old[1] = sprad_old[2];
       sprad_old[2] = c.sprad;
       c.sprad = 1.2 * sigma;
-      if (iter >= 1 && fabs(sigma - sigmal) <= ((sigma > small) ? sigma : small) * 0.001) {
+      if (iter >= 1 && nn_le(fpi_abs(sigma - sigmal), (nn_lt(small, sigma) ? sigma : small) * 0.001)) {
         for (int i = tm.rank(); i < nc; i += tm.size()) ede[i] = -1.0 * yn[i] + v1[i];
         tm.sync();
         return;
@@ -750,8 +767,8 @@ struct Sys {
           return;
         }
       }
-      if (dfnrm != 0.0) {
-        const double al = dynrm / dfnrm;
+      if (!fpi_is_zero(dfnrm)) {
+        const double al = mdiv(dynrm, dfnrm);
         if constexpr (NCF > 0) {
           double w[NR];
 #pragma unroll
@@ -865,23 +882,23 @@ struct Sys {
       c.jacatt = 1;
     }
     c.last = 0;
-    if (1.1 * c.absh >= fabs(c.tend - c.lt)) {
-      c.absh = fabs(c.tend - c.lt);
+    const double left = fpi_abs(c.tend - c.lt);
+    if (nn_le(left, 1.1 * c.absh)) {
+      c.absh = left;
       c.last = 1;
     }
-    const double marg = sqrt(1.54 * c.absh * c.sprad + 1.0);
-    if (!(marg < 1.0e9)) {
+    int m;
+    if (!stage_count(1.54 * c.absh * c.sprad + 1.0, m)) {
       c.status |= ST_NAN;
       return ATT_FAIL;
     }
-    int m = 1 + (int)(marg);
-    if (m > c.mmax) {
-      m = (int)c.mmax;
+    if (m > mmax) {
+      m = mmax;
       c.absh = (m * m - 1) / (1.54 * c.sprad);
       c.last = 0;
     }
     double h = 1.0 * c.absh;
-    if (h <= hmin) h = hmin;
+    if (nn_le(h, hmin)) h = hmin;
     if (!step(h, m)) return ATT_FAIL;
     c.n_steps++;
     // F(y) into vtemp1 and the error terms, fused
@@ -894,10 +911,9 @@ struct Sys {
 #pragma unroll
         for (int i = 0; i < NCF; i++) {
           f[i] = rhs(y, i);
-          const double ay = fabs(y[i]), ayn = fabs(yn[i]);
-          const double wt = fma(c.tol, (ay > ayn) ? ay : ayn, c.tol);
+          const double wt = fma(c.tol, abs_max(y[i], yn[i]), c.tol);
           const double est = fma(h04, fn[i] + f[i], 0.8 * (yn[i] - y[i]));
-          const double qv = est / wt;
+          const double qv = mdiv(est, wt);
           q[i] = qv * qv;
         }
 #pragma unroll
@@ -907,10 +923,9 @@ struct Sys {
         for (int i = tm.rank(); i < nc; i += tm.size()) {
           const double f = rhs(y, i);
           v1[i] = f;
-          const double ay = fabs(y[i]), ayn = fabs(yn[i]);
-          const double wt = fma(c.tol, (ay > ayn) ? ay : ayn, c.tol);
+          const double wt = fma(c.tol, abs_max(y[i], yn[i]), c.tol);
           const double est = fma(h04, fn[i] + f, 0.8 * (yn[i] - y[i]));
-          const double qv = est / wt;
+          const double qv = mdiv(est, wt);
           sc[i] = qv * qv;
         }
         err = tree_sum(sc, nc);
@@ -921,18 +936,18 @@ struct Sys {
     if ((nc & (nc - 1)) == 0)
       err = sqrt(err * __longlong_as_double((long long)(1023 - (__ffs(nc) - 1)) << 52));  // 2^-log2(nc)
     else
-      err = sqrt(err / (double)nc);
-    if (!(err == err)) {
+      err = sqrt(div_by(err, rnc));
+    if (fpi_isnan(err)) {
       c.status |= ST_NAN;
       return ATT_FAIL;
     }
     // err^(1/3), shared by the reject and accept paths (one evaluation per
     // attempt whichever way the lanes of a warp go)
     const double cr = cm_cbrt(err);
-    if (err > 1.0) {
-      c.absh = 0.8 * c.absh / cr;
+    if (nn_lt(1.0, err)) {
+      c.absh = mdiv(0.8 * c.absh, cr);
       c.n_rej++;
-      if (c.absh < hmin) {
+      if (nn_lt(c.absh, hmin)) {
         c.idid = 4;
       } else {
         c.newspc = !c.jacatt;
@@ -961,19 +976,19 @@ struct Sys {
     }
     // err^(2/3) as the square of err^(1/3); errold^(1/3) carried over
     double fac = 10.0, temp1, temp2;
-    if (c.naccpt == 1) {
+    if (fpi_bits(c.naccpt) == fpi_bits(1.0)) {
       temp2 = cr;
-      if (0.8 < fac * temp2) fac = 0.8 / temp2;
+      if (nn_lt(0.8, fac * temp2)) fac = mdiv(0.8, temp2);
     } else {
       temp1 = 0.8 * c.absh * c.cbrt_errold;
-      temp2 = fabs(c.hold) * (cr * cr);
-      if (temp1 < fac * temp2) fac = temp1 / temp2;
+      temp2 = fpi_abs(c.hold) * (cr * cr);
+      if (nn_lt(temp1, fac * temp2)) fac = mdiv(temp1, temp2);
     }
     c.cbrt_errold = cr;
-    c.absh = ((0.1 > fac) ? 0.1 : fac) * c.absh;
+    c.absh = (nn_lt(fac, 0.1) ? 0.1 : fac) * c.absh;
     {
-      const double mn = fmin(hmax, c.absh);
-      c.absh = (hmin > mn) ? hmin : mn;
+      const double mn = nn_lt(c.absh, hmax) ? c.absh : hmax;
+      c.absh = nn_lt(mn, hmin) ? hmin : mn;
     }
     c.errold = err;
     c.hold = h;
@@ -1103,7 +1118,7 @@ struct Sys {
     }
     attempts0 = c.n_steps;
     rej_run = 0;
-    return (c.sum_dt != 0.0) ? TICK_ION : TICK_MORE;
+    return fpi_is_zero(c.sum_dt) ? TICK_MORE : TICK_ION;
   }
 
   // the ion update and new current vector a TICK_ION asked for
@@ -1147,6 +1162,8 @@ struct Sys {
     n_iv = n;
     iv0 = iv0_global;
     k_iv = 0;
+    mmax = (int)c.mmax;
+    rnc = recip((double)nc);
     if (c.status != 0 || n <= 0) return TICK_DONE;
     return begin_interval(t0);
   }
@@ -1165,8 +1182,8 @@ struct Sys {
     c.sum_dt += c.gt - c.gt_old;
     c.gt_old = c.gt;
     const bool ge = (CT == GO || CT == PKJ);
-    const bool trig = ge ? (c.sum_dt >= c.integ) : (c.sum_dt > c.integ);
-    if (c.idid == 2.0) return trig ? TICK_ION : TICK_MORE;
+    const bool trig = ge ? nn_le(c.integ, c.sum_dt) : nn_lt(c.integ, c.sum_dt);
+    if (!c.last) return trig ? TICK_ION : TICK_MORE;
     if (c.idid != 1.0) {
       c.status |= ST_IDID;
       return TICK_DONE;

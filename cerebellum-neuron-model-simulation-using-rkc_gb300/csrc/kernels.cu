@@ -13,7 +13,7 @@
 #include <cuda_runtime.h>
 
 #include "integrator.cuh"
-#include "lane_sys.cuh"
+#include "quad_sys.cuh"
 
 namespace gbrkc {
 
@@ -22,15 +22,21 @@ __global__ void __launch_bounds__(256, 1) k_advance(const __grid_constant__ Pool
                                                  int iv0, int init) {
   extern __shared__ __align__(16) double smem[];
   if (TS == TEAM_THREAD || TS == TEAM_LANE4) {
-    // the first P.lanes lanes of warp w of block b start at system
-    // P.lanes (w * grid + b) + lane: the first warps of every block are
-    // filled before any block's later warps
-    const int first = (((int)threadIdx.x >> 5) * (int)gridDim.x + (int)blockIdx.x) * P.lanes + ((int)threadIdx.x & 31);
-    const int stride = (int)gridDim.x * (MEGA_BLOCK / 32) * P.lanes;
-    if (TS == TEAM_LANE4)
-      run_lanes_regs<CT, R, MEGA_BLOCK, 4>(P, nullptr, first, stride, smem, t0, n_iv, iv0, init != 0);
-    else
+    // the first `per` systems of warp w of block b start at system
+    // per (w * grid + b): the first warps of every block are filled before
+    // any block's later warps
+    const bool quads = TS == TEAM_LANE4 && !init && n_iv > 0;
+    const int per = quads ? P.per_warp : P.lanes, lane = (int)threadIdx.x & 31;
+    const int first = (((int)threadIdx.x >> 5) * (int)gridDim.x + (int)blockIdx.x) * per + (quads ? lane >> 2 : lane);
+    const int stride = (int)gridDim.x * (MEGA_BLOCK / 32) * per;
+    if constexpr (TS == TEAM_LANE4) {
+      if (quads)
+        run_quads<CT, R>(P, nullptr, first, stride, per, t0, n_iv, iv0);
+      else
+        run_lanes<CT, R, MEGA_BLOCK, 4>(P, nullptr, first, stride, smem, t0, n_iv, iv0, init != 0);
+    } else {
       run_lanes<CT, R, MEGA_BLOCK>(P, nullptr, first, stride, smem, t0, n_iv, iv0, init != 0);
+    }
   } else if (TS == TEAM_BLOCK) {
     BlockTeam tm;
     for (int s = blockIdx.x; s < P.nsys; s += gridDim.x) {
@@ -137,10 +143,12 @@ __global__ void __launch_bounds__(MEGA_BLOCK, 1) k_mega(const __grid_constant__ 
   while (role < NTYPES - 1 && (int)blockIdx.x >= M.role_end[role]) role++;
   switch (role) {
     case GR:
-      // single-lane granule systems on the CTA's first warps
+      // granule systems on the CTA's first warps
       if ((int)(threadIdx.x >> 5) < M.lane_warps + ((int)blockIdx.x < M.lane_extra ? 1 : 0)) {
-        if (M.gr_nc4)
-          run_lanes_regs<GR, R, MEGA_BLOCK, 4>(M.pool[GR], M.queue + GR, 0, 0, smem, t0, n_iv, iv0, init != 0);
+        if (M.gr_nc4 && !init && n_iv > 0)
+          run_quads<GR, R>(M.pool[GR], M.queue + GR, 0, 0, M.pool[GR].per_warp, t0, n_iv, iv0);
+        else if (M.gr_nc4)
+          run_lanes<GR, R, MEGA_BLOCK, 4>(M.pool[GR], M.queue + GR, 0, 0, smem, t0, n_iv, iv0, init != 0);
         else
           run_lanes<GR, R, MEGA_BLOCK>(M.pool[GR], M.queue + GR, 0, 0, smem, t0, n_iv, iv0, init != 0);
       }

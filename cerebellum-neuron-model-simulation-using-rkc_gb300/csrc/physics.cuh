@@ -40,13 +40,21 @@ __device__ __forceinline__ R hh_xr(R c, R x, R k) {
     const R u = x / k;
     if (mabs(u) < R(1e-3)) return c * k * (R(1) + u * (R(0.5) + u * R(1.0 / 12.0)));
   }
-  return c * x / (R(1) - mexp(-x / k));
+  return mdiv(c * x, R(1) - mexp(cdiv(-x, k)));
 }
 
 // trapezoid gate step of every RKC ion kernel: (2 dt x_inf + (2 tau - dt) x) / (2 tau + dt)
 template <typename R>
 __device__ __forceinline__ R trap(R dt, R inf, R tau, R x) {
-  return (R(2.0) * dt * inf + (R(2.0) * tau - dt) * x) / (R(2.0) * tau + dt);
+  return mdiv(R(2.0) * dt * inf + (R(2.0) * tau - dt) * x, R(2.0) * tau + dt);
+}
+
+// the same for an alpha / beta gate: inf = a / (a + b), tau = k / (a + b), by
+// one reciprocal
+template <typename R>
+__device__ __forceinline__ R ab_trap(R dt, R a, R b, R k, R x) {
+  const auto r = mrecip(a + b);
+  return trap(dt, div_by(a, r), div_by(k, r), x);
 }
 
 // View of one compartment's gate and conductance slots in a pool (SoA).
@@ -62,7 +70,7 @@ struct Slots {
 
 // ---------------------------------------------------------------- Purkinje
 template <typename R> struct Pkj {
-  __device__ static R l(R v, R A, R B, R C, R D) { return A / (B + mexp((v + C) / D)); }
+  __device__ static R l(R v, R A, R B, R C, R D) { return mdiv(A, B + mexp(cdiv(v + C, D))); }
   __device__ static R am_NaF(R v) { return l(v, R(35.0), R(0.0), R(5.0), R(-10.0)); }
   __device__ static R ah_NaF(R v) { return l(v, R(0.225), R(1.0), R(80.0), R(10.0)); }
   __device__ static R am_NaP(R v) { return l(v, R(200.0), R(1.0), R(-18.0), R(-16.0)); }
@@ -88,8 +96,7 @@ template <typename R> struct Pkj {
 #define GB_AB(K, A, B)                                                                  \
   {                                                                                      \
     R a_ = A(v), b_ = B(v);                                                              \
-    R inf_ = a_ / (a_ + b_), tau_ = R(1.0) / (a_ + b_);                                  \
-    s.x(K) = trap(dt, inf_, tau_, s.x(K));                                               \
+    s.x(K) = ab_trap(dt, a_, b_, R(1.0), s.x(K));                                        \
   }
 
   // pkj_update_ion_RKC (pkj_ion.cu:304-358); returns nothing, updates state
@@ -99,21 +106,21 @@ template <typename R> struct Pkj {
     const double v_val = 0.5 * (vnew + v_old);
     double Ca_val = ca;
     double I = 1e-3 * (v_old - rev) *
-               ((double)s.g(PK_g_CaP) * (double)s.x(PK_m_CaP) * (double)s.x(PK_h_CaP) +
-                (double)s.g(PK_g_CaT) * (double)s.x(PK_m_CaT) * (double)s.x(PK_h_CaT));
+               (up(s.g(PK_g_CaP)) * up(s.x(PK_m_CaP)) * up(s.x(PK_h_CaP)) +
+                up(s.g(PK_g_CaT)) * up(s.x(PK_m_CaT)) * up(s.x(PK_h_CaT)));
     if (I > 0.0) I = 0.0;
-    else I = -I / (2.0 * F_PKJ * shell);
+    else I = mdiv(-I, 2.0 * F_PKJ * shell);
     double k1 = DT * (I - B_Ca1_PKJ * (Ca_val - Ca1_0_PKJ));
     double k2 = DT * (I - B_Ca1_PKJ * (Ca_val + k1 / 2.0 - Ca1_0_PKJ));
     double k3 = DT * (I - B_Ca1_PKJ * (Ca_val + k2 / 2.0 - Ca1_0_PKJ));
     double k4 = DT * (I - B_Ca1_PKJ * (Ca_val + k3 - Ca1_0_PKJ));
-    k1 = Ca_val + (k1 + k2 * 2.0 + k3 * 2.0 + k4) / 6.0;
+    k1 = Ca_val + cdiv(k1 + k2 * 2.0 + k3 * 2.0 + k4, 6.0);
     ca = k1;
     Ca_val = 0.5 * (Ca_val + k1);
     if (rev_fixed) rev = 12.5 * cm_log(Ca1OUT_PKJ / Ca1_0_PKJ);
-    else rev = 13.361624877 * cm_log(Ca1OUT_PKJ / Ca_val);
-    Ca_val = floor((Ca_val * 1000 - 0.04) / 0.099986667) * 0.099986667 + 0.04;
-    const R v = (R)v_val, dt = (R)DT;
+    else rev = 13.361624877 * cm_log(mdiv(Ca1OUT_PKJ, Ca_val));
+    Ca_val = floor(cdiv(Ca_val * 1000 - 0.04, 0.099986667)) * 0.099986667 + 0.04;
+    const R v = to<R>(v_val), dt = to<R>(DT);
     GB_AB(PK_m_NaF, am_NaF, bm_NaF);
     GB_AB(PK_h_NaF, ah_NaF, bh_NaF);
     GB_AB(PK_m_NaP, am_NaP, bm_NaP);
@@ -122,47 +129,47 @@ template <typename R> struct Pkj {
     GB_AB(PK_m_CaT, am_CaT, bm_CaT);
     GB_AB(PK_h_CaT, ah_CaT, bh_CaT);
     {
-      R e = mexp((v + R(82.0)) / R(7.0));
-      s.x(PK_m_Kh1) = trap(dt, R(0.8) / (R(1.0) + e), R(7.6), s.x(PK_m_Kh1));
-      s.x(PK_m_Kh2) = trap(dt, R(0.2) / (R(1.0) + e), R(36.8), s.x(PK_m_Kh2));
+      R e = mexp(cdiv(v + R(82.0), R(7.0)));
+      s.x(PK_m_Kh1) = trap(dt, mdiv(R(0.8), R(1.0) + e), R(7.6), s.x(PK_m_Kh1));
+      s.x(PK_m_Kh2) = trap(dt, mdiv(R(0.2), R(1.0) + e), R(36.8), s.x(PK_m_Kh2));
     }
     {
       R a, b;
-      if (mabs(v + R(12.0)) > R(1e-6)) a = R(-0.0235) * (v + R(12.0)) / (mexp(-(v + R(12.0)) / R(12.0)) - R(1.0));
+      if (mag_gt(mabs(v + R(12.0)), R(1e-6))) a = mdiv(R(-0.0235) * (v + R(12.0)), mexp(cdiv(-(v + R(12.0)), R(12.0))) - R(1.0));
       else a = R(0.0235) * R(12.0);
-      b = R(5.0) * mexp(-(v + R(147.0)) / R(30.0));
-      R tau = R(1.0) / (a + b);
-      if (mabs(v - R(8.0)) > R(1e-6)) a = R(-0.0235) * (v - R(8.0)) / (mexp(-(v - R(8.0)) / R(12.0)) - R(1.0));
+      b = R(5.0) * mexp(cdiv(-(v + R(147.0)), R(30.0)));
+      R tau = mdiv(R(1.0), a + b);
+      if (mag_gt(mabs(v - R(8.0)), R(1e-6))) a = mdiv(R(-0.0235) * (v - R(8.0)), mexp(cdiv(-(v - R(8.0)), R(12.0))) - R(1.0));
       else a = R(0.0235) * R(12.0);
-      b = R(5.0) * mexp(-(v + R(127.0)) / R(30.0));
-      R inf = a / (a + b);
+      b = R(5.0) * mexp(cdiv(-(v + R(127.0)), R(30.0)));
+      R inf = mdiv(a, a + b);
       s.x(PK_m_Kdr) = trap(dt, inf, tau, s.x(PK_m_Kdr));
     }
-    s.x(PK_h_Kdr) = trap(dt, R(1.0) / (R(1.0) + mexp((v + R(25.0)) / R(4.0))),
+    s.x(PK_h_Kdr) = trap(dt, mdiv(R(1.0), R(1.0) + mexp(cdiv(v + R(25.0), R(4.0)))),
                          (v_val < -25.0) ? R(1200.0) : R(10.0), s.x(PK_h_Kdr));
-    s.x(PK_m_KM) = trap(dt, R(1.0) / (R(1.0) + mexp(-(v + R(35.0)) / R(10.0))),
-                        R(200.0) / (R(3.3) * (mexp((v + R(35.0)) / R(20.0))) + mexp(-(v + R(35.0)) / R(20.0))),
+    s.x(PK_m_KM) = trap(dt, mdiv(R(1.0), R(1.0) + mexp(cdiv(-(v + R(35.0)), R(10.0)))),
+                        mdiv(R(200.0), R(3.3) * (mexp(cdiv(v + R(35.0), R(20.0)))) + mexp(cdiv(-(v + R(35.0)), R(20.0)))),
                         s.x(PK_m_KM));
     GB_AB(PK_m_KA, am_KA, bm_KA);
     GB_AB(PK_h_KA, ah_KA, bh_KA);
     {
       R b_ = bm_KC(v);
-      s.x(PK_m_KC) = trap(dt, R(7.5) / (R(7.5) + b_), R(1.0) / (R(7.5) + b_), s.x(PK_m_KC));
+      s.x(PK_m_KC) = ab_trap(dt, R(7.5), b_, R(1.0), s.x(PK_m_KC));
     }
-    const R caq = (R)Ca_val;
-    s.x(PK_z_KC) = trap(dt, R(1.0) / (R(1.0) + R(4.00) / caq), R(10.0), s.x(PK_z_KC));
+    const R caq = to<R>(Ca_val);
+    s.x(PK_z_KC) = trap(dt, mdiv(R(1.0), R(1.0) + mdiv(R(4.00), caq)), R(10.0), s.x(PK_z_KC));
     {
       R b_ = bm_K2(v);
-      s.x(PK_m_K2) = trap(dt, R(25.0) / (R(25.0) + b_), R(1.0) / (R(25.0) + b_), s.x(PK_m_K2));
+      s.x(PK_m_K2) = ab_trap(dt, R(25.0), b_, R(1.0), s.x(PK_m_K2));
     }
-    s.x(PK_z_K2) = trap(dt, R(1.0) / (R(1.0) + R(0.20) / caq), R(10.0), s.x(PK_z_K2));
+    s.x(PK_z_K2) = trap(dt, mdiv(R(1.0), R(1.0) + mdiv(R(0.20), caq)), R(10.0), s.x(PK_z_K2));
     v_elem = vnew;
   }
 
   // pkj_update_matrix (solve_rkc.cu:370-398)
   __device__ static R b(const Slots<R> &s, double vy, double iext, double rev) {
-    const R lv = (R)vy, vca = (R)rev;
-    return (-(R)iext + s.g(PK_g_leak) * (lv - R(V_LEAK_PKJ)) +
+    const R lv = to<R>(vy), vca = to<R>(rev);
+    return (-to<R>(iext) + s.g(PK_g_leak) * (lv - R(V_LEAK_PKJ)) +
             s.g(PK_g_NaF) * s.x(PK_m_NaF) * s.x(PK_m_NaF) * s.x(PK_m_NaF) * s.x(PK_h_NaF) * (lv - R(V_Na_PKJ)) +
             s.g(PK_g_NaP) * s.x(PK_m_NaP) * s.x(PK_m_NaP) * s.x(PK_m_NaP) * (lv - R(V_Na_PKJ)) +
             s.g(PK_g_CaP) * s.x(PK_m_CaP) * s.x(PK_h_CaP) * (lv - vca) +
@@ -179,13 +186,13 @@ template <typename R> struct Pkj {
 
 // ---------------------------------------------------------- inferior olive
 template <typename R> struct Io {
-  __device__ static R ar(R v) { return (R(1.7)) / (R(1.0) + mexp((-(v - R(5.0))) / R(13.9))); }
+  __device__ static R ar(R v) { return mdiv(R(1.7), R(1.0) + mexp(cdiv(-(v - R(5.0)), R(13.9)))); }
   __device__ static R as(R x) { return mmin(R(0.00002) * x, R(0.01)); }
   // 0.13 (v + 25) / (1 - exp(-(v + 25) / 10)) and 0.02 (v + 8.5) / (exp((v + 8.5) / 5) - 1)
   __device__ static R ax(R v) { return hh_xr(R(0.13), v + R(25.0), R(10.0)); }
   __device__ static R br(R v) { return -hh_xr(R(0.02), v + R(8.5), R(-5.0)); }
   __device__ static R bx(R v) { return R(1.69) * mexp(R(-0.0125) * (v + R(35.0))); }
-  __device__ static R n_tau(R v) { return R(47.0) * mexp((-(-v - R(50.0))) / R(900.0)) + R(5.0); }
+  __device__ static R n_tau(R v) { return R(47.0) * mexp(cdiv(-(-v - R(50.0)), R(900.0))) + R(5.0); }
 
   // io_update_ion_RKC (io_ion.cu:91-126)
   __device__ static void ion(const Slots<R> &s, double &v_elem, double &ca, int comp_type,
@@ -193,46 +200,46 @@ template <typename R> struct Io {
     const double v_old = v_elem;
     const double v_val = 0.5 * (vnew + v_old);
     double Ca_val = ca;
-    const double rr = (double)s.x(IO_r);
-    double I = (double)s.g(IO_g_CaH) * rr * rr * (v_old - V_Ca_IO);
+    const double rr = up(s.x(IO_r));
+    double I = up(s.g(IO_g_CaH)) * rr * rr * (v_old - V_Ca_IO);
     double k1 = DT * (-I * CA_PH_IO - BETA_CA_IO * (Ca_val));
     double k2 = DT * (-I * CA_PH_IO - BETA_CA_IO * (Ca_val + k1 / 2.0));
     double k3 = DT * (-I * CA_PH_IO - BETA_CA_IO * (Ca_val + k2 / 2.0));
     double k4 = DT * (-I * CA_PH_IO - BETA_CA_IO * (Ca_val + k3));
-    ca += (k1 + k2 * 2.0 + k3 * 2.0 + k4) / 6.0;
+    ca += cdiv(k1 + k2 * 2.0 + k3 * 2.0 + k4, 6.0);
     Ca_val = (Ca_val + ca) / 2.0;
-    const R v = (R)v_val, dt = (R)DT, c = (R)Ca_val;
-    s.x(IO_k) = trap(dt, R(1.0) / (R(1.0) + mexp((-v - R(61.0)) / R(4.2))), R(1.0), s.x(IO_k));
-    s.x(IO_l) = trap(dt, R(1.0) / (R(1.0) + mexp((v + R(85.5)) / (R(8.5)))),
-                     ((R(20.0) * mexp((v + R(160.0)) / R(30.0))) / (R(1.0) + mexp((v + R(84.0)) / R(7.3)))) + R(35.0),
+    const R v = to<R>(v_val), dt = to<R>(DT), c = to<R>(Ca_val);
+    s.x(IO_k) = trap(dt, mdiv(R(1.0), R(1.0) + mexp(cdiv(-v - R(61.0), R(4.2)))), R(1.0), s.x(IO_k));
+    s.x(IO_l) = trap(dt, mdiv(R(1.0), R(1.0) + mexp(cdiv(v + R(85.5), R(8.5)))),
+                     (mdiv(R(20.0) * mexp(cdiv(v + R(160.0), R(30.0))), R(1.0) + mexp(cdiv(v + R(84.0), R(7.3))))) + R(35.0),
                      s.x(IO_l));
     const R ntau = n_tau(v);
-    s.x(IO_n) = trap(dt, R(1.0) / (R(1.0) + mexp((-v - R(3.0)) / (R(10.0)))), ntau, s.x(IO_n));
-    s.x(IO_p) = trap(dt, R(1.0) / (R(1.0) + mexp((-v - R(51.0)) / (R(-12.0)))), ntau, s.x(IO_p));
+    s.x(IO_n) = trap(dt, mdiv(R(1.0), R(1.0) + mexp(cdiv(-v - R(3.0), R(10.0)))), ntau, s.x(IO_n));
+    s.x(IO_p) = trap(dt, mdiv(R(1.0), R(1.0) + mexp(cdiv(-v - R(51.0), R(-12.0)))), ntau, s.x(IO_p));
     {
       R a = ax(v), b = bx(v);
-      s.x(IO_x) = trap(dt, a / (a + b), R(1.0) / (a + b), s.x(IO_x));
+      s.x(IO_x) = ab_trap(dt, a, b, R(1.0), s.x(IO_x));
     }
     {
       R a = ar(v), b = br(v);
-      s.x(IO_r) = trap(dt, a / (a + b), R(5.0) / (a + b), s.x(IO_r));
+      s.x(IO_r) = ab_trap(dt, a, b, R(5.0), s.x(IO_r));
     }
-    s.x(IO_q) = trap(dt, R(1.0) / (R(1.0) + mexp((v + R(80.0)) / R(4.0))),
-                     R(1.0) / (mexp(R(-0.086) * v - R(14.6)) + mexp(R(0.07) * v - R(1.87))), s.x(IO_q));
+    s.x(IO_q) = trap(dt, mdiv(R(1.0), R(1.0) + mexp(cdiv(v + R(80.0), R(4.0)))),
+                     mdiv(R(1.0), mexp(R(-0.086) * v - R(14.6)) + mexp(R(0.07) * v - R(1.87))), s.x(IO_q));
     {
       R a = as(c);
-      s.x(IO_s) = trap(dt, a / (a + R(0.015)), R(1.0) / (a + R(0.015)), s.x(IO_s));
+      s.x(IO_s) = ab_trap(dt, a, R(0.015), R(1.0), s.x(IO_s));
     }
-    s.x(IO_m) = R(1.0) / (R(1.0) + mexp((-v - R(30.0)) / (R(5.5))));
+    s.x(IO_m) = mdiv(R(1.0), R(1.0) + mexp(cdiv(-v - R(30.0), R(5.5))));
     {
       R hi = R(1.0), ht = R(1.0);
       if (comp_type == 1) {
-        hi = R(1.0) / (R(1.0) + mexp((-v - R(70.0)) / (R(-5.8))));
-        ht = R(3.0) * mexp((-v - R(40.0)) / R(33.0));
+        hi = mdiv(R(1.0), R(1.0) + mexp(cdiv(-v - R(70.0), R(-5.8))));
+        ht = R(3.0) * mexp(cdiv(-v - R(40.0), R(33.0)));
       }
       if (comp_type == 2) {
-        hi = R(1.0) / (R(1.0) + mexp((-v - R(60.0)) / (R(-5.8))));
-        ht = R(1.5) * mexp((-v - R(40.0)) / R(33.0));
+        hi = mdiv(R(1.0), R(1.0) + mexp(cdiv(-v - R(60.0), R(-5.8))));
+        ht = R(1.5) * mexp(cdiv(-v - R(40.0), R(33.0)));
       }
       s.x(IO_h) = trap(dt, hi, ht, s.x(IO_h));
     }
@@ -241,8 +248,8 @@ template <typename R> struct Io {
 
   // io_update_matrix (solve_rkc.cu:413-435)
   __device__ static R b(const Slots<R> &s, double vy, double iext) {
-    const R lv = (R)vy;
-    return (-(R)iext + s.g(IO_g_leak) * (lv - R(V_LEAK_IO)) +
+    const R lv = to<R>(vy);
+    return (-to<R>(iext) + s.g(IO_g_leak) * (lv - R(V_LEAK_IO)) +
             s.g(IO_g_CaL) * (lv - R(V_Ca_IO)) * s.x(IO_k) * s.x(IO_k) * s.x(IO_k) * s.x(IO_l) +
             s.g(IO_g_Na) * (lv - R(V_Na_IO)) * s.x(IO_m) * s.x(IO_m) * s.x(IO_m) * s.x(IO_h) +
             s.g(IO_g_Kdr) * (lv - R(V_K_IO)) * s.x(IO_n) * s.x(IO_p) +
@@ -261,52 +268,52 @@ __device__ __forceinline__ double io_gap_current(double g, double diff) {
 // ------------------------------------------------------------------ granule
 template <typename R> struct Gr {
   __device__ static R a_nKV(R v) {
-    return (mabs(v + R(25.0)) > R(1.0e-6)) ? R(-0.017) * ((v + R(25.0)) / (mexp(-(v + R(25.0)) / R(10.0)) - R(1.0)))
-                                            : R(-0.17) * (R(1.0) + (v + R(25.0)) / R(20.0));
+    return (mag_gt(mabs(v + R(25.0)), R(1.0e-6))) ? R(-0.017) * (mdiv(v + R(25.0), mexp(cdiv(-(v + R(25.0)), R(10.0))) - R(1.0)))
+                                            : R(-0.17) * (R(1.0) + cdiv(v + R(25.0), R(20.0)));
   }
-  __device__ static R b_nKV(R v) { return R(0.2223) * mexp(-(v + R(35.0)) / R(80.0)); }
+  __device__ static R b_nKV(R v) { return R(0.2223) * mexp(cdiv(-(v + R(35.0)), R(80.0))); }
 
   // gr_update_ion_RKC_exp_imp (gr_ion.cu:461-480): Ca is never advanced
   __device__ static void ion(const Slots<R> &s, double &v_elem, double ca, double vnew, double DT) {
     const double v_val = (v_elem + vnew) / 2.0;
-    const R v = (R)v_val, dt = (R)DT, c = (R)ca;
+    const R v = to<R>(v_val), dt = to<R>(DT), c = to<R>(ca);
     {
       R a = a_nKV(v), b = b_nKV(v);
-      s.x(GR_n_KV) = trap(dt, a / (a + b), R(1.0) / (a + b), s.x(GR_n_KV));
+      s.x(GR_n_KV) = ab_trap(dt, a, b, R(1.0), s.x(GR_n_KV));
     }
     {
-      R a = R(0.771) / (R(1.0) + mexp(-(v + R(9.17203)) / R(23.32708)));
-      R b = R(0.1567) / mexp((v + R(18.27914)) / R(19.47175));
-      s.x(GR_a_KA) = trap(dt, R(1.0) / (R(1.0) + mexp(-(v + R(38.0)) / R(17.0))), (R(1.0) / (a + b)), s.x(GR_a_KA));
+      R a = mdiv(R(0.771), R(1.0) + mexp(cdiv(-(v + R(9.17203)), R(23.32708))));
+      R b = mdiv(R(0.1567), mexp(cdiv(v + R(18.27914), R(19.47175))));
+      s.x(GR_a_KA) = trap(dt, mdiv(R(1.0), R(1.0) + mexp(cdiv(-(v + R(38.0)), R(17.0)))), (mdiv(R(1.0), a + b)), s.x(GR_a_KA));
     }
     {
-      R a = R(0.0348) / (R(1.0) + mexp((v + R(111.33208)) / R(12.8433)));
-      R b = R(0.0327) / (R(1.0) + mexp(-(v + R(49.9537)) / R(8.90123)));
-      s.x(GR_b_KA) = trap(dt, R(1.0) / (R(1.0) + mexp((v + R(78.8)) / R(8.4))), (R(1.0) / (a + b)), s.x(GR_b_KA));
+      R a = mdiv(R(0.0348), R(1.0) + mexp(cdiv(v + R(111.33208), R(12.8433))));
+      R b = mdiv(R(0.0327), R(1.0) + mexp(cdiv(-(v + R(49.9537)), R(8.90123))));
+      s.x(GR_b_KA) = trap(dt, mdiv(R(1.0), R(1.0) + mexp(cdiv(v + R(78.8), R(8.4)))), (mdiv(R(1.0), a + b)), s.x(GR_b_KA));
     }
     {
-      R a = R(0.2302) * mexp(-(v + R(83.94)) / R(24.3902));
-      R b = R(0.2943) * mexp((v + R(83.94)) / R(35.714));
-      s.x(GR_ir_KIR) = trap(dt, a / (a + b), R(1.0) / (a + b), s.x(GR_ir_KIR));
+      R a = R(0.2302) * mexp(cdiv(-(v + R(83.94)), R(24.3902)));
+      R b = R(0.2943) * mexp(cdiv(v + R(83.94), R(35.714)));
+      s.x(GR_ir_KIR) = ab_trap(dt, a, b, R(1.0), s.x(GR_ir_KIR));
     }
     {
-      R a = R(0.0046) * mexp((v + R(30.0)) / R(40.0));
-      R b = R(0.0046) * mexp(-(v + R(30.0)) / R(20.0));
-      s.x(GR_s_KM) = trap(dt, R(1.0) / (R(1.0) + mexp(-(v + R(35.0)) / R(6.0))), (R(1.0) / (a + b)), s.x(GR_s_KM));
+      R a = R(0.0046) * mexp(cdiv(v + R(30.0), R(40.0)));
+      R b = R(0.0046) * mexp(cdiv(-(v + R(30.0)), R(20.0)));
+      s.x(GR_s_KM) = trap(dt, mdiv(R(1.0), R(1.0) + mexp(cdiv(-(v + R(35.0)), R(6.0)))), (mdiv(R(1.0), a + b)), s.x(GR_s_KM));
     }
     {
-      R a = R(1.4433) / (R(1.0) + (R(1.5e-3) * mexp(-v / R(11.765))) / c);
-      R b = R(0.8660) / (R(1.0) + c / (R(1.5e-4) * mexp(-v / R(11.765))));
-      s.x(GR_c_KCa) = trap(dt, a / (a + b), (R(1.0) / (a + b)), s.x(GR_c_KCa));
+      R a = mdiv(R(1.4433), R(1.0) + mdiv(R(1.5e-3) * mexp(cdiv(-v, R(11.765))), c));
+      R b = mdiv(R(0.8660), R(1.0) + mdiv(c, R(1.5e-4) * mexp(cdiv(-v, R(11.765)))));
+      s.x(GR_c_KCa) = ab_trap(dt, a, b, R(1.0), s.x(GR_c_KCa));
     }
     v_elem = vnew;
   }
 
   // gr_update_matrix (solve_rkc.cu:227-250)
   __device__ static R b(const Slots<R> &s, double vy, double iext) {
-    const R lv = (R)vy;
+    const R lv = to<R>(vy);
     return (+s.g(GR_g_leak1) * (lv - R(V_LEAK1_GR)) + s.g(GR_g_leak2) * (lv - R(V_LEAK2_GR)) +
-            s.g(GR_g_leak3) * (lv - R(V_LEAK3_GR)) - (R)iext +
+            s.g(GR_g_leak3) * (lv - R(V_LEAK3_GR)) - to<R>(iext) +
             +s.g(GR_g_Na) * (lv - R(V_Na_GR)) * s.x(GR_o_Na) +
             s.g(GR_g_Ca) * (lv - R(V_Ca_GR)) * s.x(GR_ch_Ca) * s.x(GR_ch_Ca) * s.x(GR_ci_Ca) +
             s.g(GR_g_KV) * (lv - R(V_K_GR)) * s.x(GR_n_KV) * s.x(GR_n_KV) * s.x(GR_n_KV) * s.x(GR_n_KV) +
@@ -426,19 +433,21 @@ template <typename R, class PAT>
 __device__ __forceinline__ int dd_solve(R (&A)[PAT::N][PAT::N], R (&b)[PAT::N]) {
   constexpr int N = PAT::N;
   constexpr Fill<N> F = PAT::fill;
+  decltype(mrecip(R())) piv[N];   // each pivot's reciprocal serves its column and the back substitution
 #pragma unroll
   for (int i = 0; i < N - 1; i++) {
     const R d = mabs(A[i][i]);
 #pragma unroll
     for (int j = i + 1; j < N; j++)
       if ((F.r[j] >> i) & 1u)
-        if (mabs(A[j][i]) > d) return DD_PIVOT;
-    if (d < R(1.0e-12)) return DD_SINGULAR;
+        if (mag_gt(mabs(A[j][i]), d)) return DD_PIVOT;
+    if (mag_lt(d, R(1.0e-12))) return DD_SINGULAR;
+    piv[i] = mrecip(A[i][i]);
 #pragma unroll
     for (int j = i + 1; j < N; j++) {
       if (!((F.r[j] >> i) & 1u)) continue;
-      if (A[j][i] == R(0.0)) continue;
-      const R w = A[j][i] / A[i][i];
+      if (is_zero(A[j][i])) continue;
+      const R w = div_by(A[j][i], piv[i]);
       A[j][i] = R(0.0);
 #pragma unroll
       for (int k = i + 1; k < N; k++)
@@ -446,12 +455,13 @@ __device__ __forceinline__ int dd_solve(R (&A)[PAT::N][PAT::N], R (&b)[PAT::N]) 
       b[j] = b[j] - b[i] * w;
     }
   }
+  piv[N - 1] = mrecip(A[N - 1][N - 1]);
 #pragma unroll
   for (int i = N - 1; i >= 0; i--) {
 #pragma unroll
     for (int j = i + 1; j < N; j++)
       if ((F.r[i] >> j) & 1u) b[i] = b[i] - A[i][j] * b[j];
-    b[i] = b[i] / A[i][i];
+    b[i] = div_by(b[i], piv[i]);
   }
   return DD_OK;
 }
@@ -476,9 +486,9 @@ __device__ __forceinline__ void dd_neg_matvec(const R (&M)[PAT::N][PAT::N], cons
 // a^4, b^4 come precomputed from the host (NaPar).
 template <typename R>
 __device__ void gr_na_fill(R (&M)[12][12], const NaPar &p, R alpha, R beta, R tdt, bool implicit_half) {
-  const R n1 = (R)p.n1, n2 = (R)p.n2, n3 = (R)p.n3, n4 = (R)p.n4;
-  const R Con = (R)p.Con, Coff = (R)p.Coff, Oon = (R)p.Oon, Ooff = (R)p.Ooff;
-  const R a = (R)p.a, b = (R)p.b, a4 = (R)p.a4, b4 = (R)p.b4;
+  const R n1 = to<R>(p.n1), n2 = to<R>(p.n2), n3 = to<R>(p.n3), n4 = to<R>(p.n4);
+  const R Con = to<R>(p.Con), Coff = to<R>(p.Coff), Oon = to<R>(p.Oon), Ooff = to<R>(p.Ooff);
+  const R a = to<R>(p.a), b = to<R>(p.b), a4 = to<R>(p.a4), b4 = to<R>(p.b4);
 #pragma unroll
   for (int i = 0; i < 12; i++)
 #pragma unroll
@@ -528,17 +538,17 @@ template <typename R>
 __device__ void gr_na(const Slots<R> &s, const NaPar &p, double v_new, double v_old, double DT) {
   // state order {c1..c5, i1..i6, o} (gr_ion.cu:104-105)
   const int slot[12] = {GR_c1, GR_c2, GR_c3, GR_c4, GR_c5, GR_i1, GR_i2, GR_i3, GR_i4, GR_i5, GR_i6, GR_o_Na};
-  const R vs = (R)p.vshift, tdt = R(2.0) / (R)DT;
+  const R vs = to<R>(p.vshift), tdt = mdiv(R(2.0), to<R>(DT));
   R M[12][12], vc[12], vcb[12];
-  const R vo = (R)v_old, vn = (R)v_new;
-  const R alpha0 = (R)p.Aa * mexp((vo - vs) / R(10.0));
-  const R beta0 = (R)p.Ab * mexp(-(vo - vs) / R(10.0));
+  const R vo = to<R>(v_old), vn = to<R>(v_new);
+  const R alpha0 = to<R>(p.Aa) * mexp(cdiv(vo - vs, R(10.0)));
+  const R beta0 = to<R>(p.Ab) * mexp(cdiv(-(vo - vs), R(10.0)));
   gr_na_fill(M, p, alpha0, beta0, tdt, false);
 #pragma unroll
   for (int k = 0; k < 12; k++) vc[k] = s.x(slot[k]);
   dd_neg_matvec<R, NaPattern>(M, vc, vcb);
-  const R alpha = (R)p.Aa * mexp((vn - vs) / R(10.0));
-  const R beta = (R)p.Ab * mexp(-(vn - vs) / R(10.0));
+  const R alpha = to<R>(p.Aa) * mexp(cdiv(vn - vs, R(10.0)));
+  const R beta = to<R>(p.Ab) * mexp(cdiv(-(vn - vs), R(10.0)));
   gr_na_fill(M, p, alpha, beta, tdt, true);
   const int rc = dd_solve<R, NaPattern>(M, vcb);
   if (rc == DD_SINGULAR) return;
@@ -566,104 +576,104 @@ template <typename R> struct Go {
     const double v_val = (v_old + vnew) / 2.0;
     double Ca_val = ca;
     const double Ca2_val = ca2;
-    const double ch = (double)s.x(GO_ch), ci = (double)s.x(GO_ci);
-    const double cl = (double)s.x(GO_cl), cmv = (double)s.x(GO_cm);
-    double I1 = 1e-3 * (double)s.g(GO_g_CaHVA) / area * ch * ch * ci * (v_old - V_Ca_GO);
-    double I2 = 1e-3 * (double)s.g(GO_g_CaLVA) / area * cl * cl * cmv * (v_old - (rev));
-    double k1 = DT * (-I1 / (2.0 * F_GO * SHELL1_D_GO) - B_Ca1_GO * (Ca_val - Ca1_0_GO));
-    double k2 = DT * (-I1 / (2.0 * F_GO * SHELL1_D_GO) - B_Ca1_GO * (Ca_val + k1 / 2.0 - Ca1_0_GO));
-    double k3 = DT * (-I1 / (2.0 * F_GO * SHELL1_D_GO) - B_Ca1_GO * (Ca_val + k2 / 2.0 - Ca1_0_GO));
-    double k4 = DT * (-I1 / (2.0 * F_GO * SHELL1_D_GO) - B_Ca1_GO * (Ca_val + k3 - Ca1_0_GO));
-    ca += (k1 + k2 * 2.0 + k3 * 2.0 + k4) / 6.0;
-    k1 = DT * (-I2 / (2.0 * F_GO * SHELL1_D_GO) - B_Ca1_GO * (Ca2_val - Ca1_0_GO));
-    k2 = DT * (-I2 / (2.0 * F_GO * SHELL1_D_GO) - B_Ca1_GO * (Ca2_val + k1 / 2.0 - Ca1_0_GO));
-    k3 = DT * (-I2 / (2.0 * F_GO * SHELL1_D_GO) - B_Ca1_GO * (Ca2_val + k2 / 2.0 - Ca1_0_GO));
-    k4 = DT * (-I2 / (2.0 * F_GO * SHELL1_D_GO) - B_Ca1_GO * (Ca2_val + k3 - Ca1_0_GO));
-    ca2 += (k1 + k2 * 2.0 + k3 * 2.0 + k4) / 6.0;
-    rev = (1e3) * (8.313424 * (23.0 + 273.15)) / (2 * F_GO) * cm_log(Ca1OUT_GO / ca2);
+    const double ch = up(s.x(GO_ch)), ci = up(s.x(GO_ci));
+    const double cl = up(s.x(GO_cl)), cmv = up(s.x(GO_cm));
+    double I1 = mdiv(1e-3 * up(s.g(GO_g_CaHVA)), area) * ch * ch * ci * (v_old - V_Ca_GO);
+    double I2 = mdiv(1e-3 * up(s.g(GO_g_CaLVA)), area) * cl * cl * cmv * (v_old - (rev));
+    double k1 = DT * (cdiv(-I1, 2.0 * F_GO * SHELL1_D_GO) - B_Ca1_GO * (Ca_val - Ca1_0_GO));
+    double k2 = DT * (cdiv(-I1, 2.0 * F_GO * SHELL1_D_GO) - B_Ca1_GO * (Ca_val + k1 / 2.0 - Ca1_0_GO));
+    double k3 = DT * (cdiv(-I1, 2.0 * F_GO * SHELL1_D_GO) - B_Ca1_GO * (Ca_val + k2 / 2.0 - Ca1_0_GO));
+    double k4 = DT * (cdiv(-I1, 2.0 * F_GO * SHELL1_D_GO) - B_Ca1_GO * (Ca_val + k3 - Ca1_0_GO));
+    ca += cdiv(k1 + k2 * 2.0 + k3 * 2.0 + k4, 6.0);
+    k1 = DT * (cdiv(-I2, 2.0 * F_GO * SHELL1_D_GO) - B_Ca1_GO * (Ca2_val - Ca1_0_GO));
+    k2 = DT * (cdiv(-I2, 2.0 * F_GO * SHELL1_D_GO) - B_Ca1_GO * (Ca2_val + k1 / 2.0 - Ca1_0_GO));
+    k3 = DT * (cdiv(-I2, 2.0 * F_GO * SHELL1_D_GO) - B_Ca1_GO * (Ca2_val + k2 / 2.0 - Ca1_0_GO));
+    k4 = DT * (cdiv(-I2, 2.0 * F_GO * SHELL1_D_GO) - B_Ca1_GO * (Ca2_val + k3 - Ca1_0_GO));
+    ca2 += cdiv(k1 + k2 * 2.0 + k3 * 2.0 + k4, 6.0);
+    rev = (1e3) * (8.313424 * (23.0 + 273.15)) / (2 * F_GO) * cm_log(mdiv(Ca1OUT_GO, ca2));
     Ca_val = (Ca_val + ca) / 2.0;
-    const R v = (R)v_val, dt = (R)DT, c = (R)Ca_val;
+    const R v = to<R>(v_val), dt = to<R>(DT), c = to<R>(Ca_val);
     {  // m_NaT
       R a = hh_xr(R(0.417), v + R(25.0), R(10.0));
       R b = R(16.68) * mexp(R(-0.055) * (v + R(50.0)));
-      s.x(GO_m_NaT) = trap(dt, a / (a + b), R(1.0) / (a + b), s.x(GO_m_NaT));
+      s.x(GO_m_NaT) = ab_trap(dt, a, b, R(1.0), s.x(GO_m_NaT));
     }
     {  // h_NaT
       R a = R(0.292) * mexp(R(-0.3) * (v + R(50.0)));
-      R b = R(4.17) / (R(1) + mexp(-(v + R(17.0)) / R(5.0)));
-      s.x(GO_h_NaT) = trap(dt, a / (a + b), R(1.0) / (a + b), s.x(GO_h_NaT));
+      R b = mdiv(R(4.17), R(1) + mexp(cdiv(-(v + R(17.0)), R(5.0))));
+      s.x(GO_h_NaT) = ab_trap(dt, a, b, R(1.0), s.x(GO_h_NaT));
     }
     {  // r_NaR
       // (1.11 - 68.5 (v - 4.48) / (exp(-(v - 4.48) / 6.8) - 1)) 1e-4
       R a = ((R(1.11) + hh_xr(R(68.5), v - R(4.48), R(6.8))) * R(1.0e-4));
-      R x = (v + R(44.0)) / R(0.11);
+      R x = cdiv(v + R(44.0), R(0.11));
       if (x > R(200.0)) x = R(200.0);
       R b;
       if (sizeof(R) == 4 && mabs(x) < R(1e-3))  // the same guard: 21.7 (v + 44) / (e^x - 1) -> 21.7 * 0.11
         b = (R(66.0) + R(21.7) * R(0.11) * (R(1) - x * (R(0.5) - x * R(1.0 / 12.0)))) * R(1.0e-3);
       else
-        b = ((R(66.0) + R(21.7) * (v + R(44)) / (mexp(x) - R(1.0))) * R(1.0e-3));
-      s.x(GO_r_NaR) = trap(dt, a / (a + b), R(1.0) / (a + b), s.x(GO_r_NaR));
+        b = ((R(66.0) + mdiv(R(21.7) * (v + R(44)), mexp(x) - R(1.0))) * R(1.0e-3));
+      s.x(GO_r_NaR) = ab_trap(dt, a, b, R(1.0), s.x(GO_r_NaR));
     }
     {  // s_NaR
-      R a = (R(0.443) * mexp(-(v + R(80.0)) / R(62.5)));
-      R b = (R(0.014) * mexp((v + R(83.3)) / R(16.1)));
-      s.x(GO_s_NaR) = trap(dt, a / (a + b), R(1.0) / (a + b), s.x(GO_s_NaR));
+      R a = (R(0.443) * mexp(cdiv(-(v + R(80.0)), R(62.5))));
+      R b = (R(0.014) * mexp(cdiv(v + R(83.3), R(16.1))));
+      s.x(GO_s_NaR) = ab_trap(dt, a, b, R(1.0), s.x(GO_s_NaR));
     }
     {  // p_NaP
       R a = hh_xr(R(0.421), v + R(40.0), R(5.0));
       R b = hh_xr(R(-0.287), v + R(40.0), R(-5.0));  // -0.287 (v + 40) / (1 - exp((v + 40) / 5))
-      s.x(GO_p_NaP) = trap(dt, (R(1) / (R(1.0) + mexp(-(v + R(43.0)) / R(5.0)))), (R(5.0) / (a + b)), s.x(GO_p_NaP));
+      s.x(GO_p_NaP) = trap(dt, (mdiv(R(1), R(1.0) + mexp(cdiv(-(v + R(43.0)), R(5.0))))), (mdiv(R(5.0), a + b)), s.x(GO_p_NaP));
     }
     {  // n_KV
       R a = hh_xr(R(0.062), v + R(26.0), R(10.0));
-      R b = R(0.78) * mexp(-(v + R(36.0)) / R(80.0));
-      s.x(GO_n_KV) = trap(dt, a / (a + b), R(1.0) / (a + b), s.x(GO_n_KV));
+      R b = R(0.78) * mexp(cdiv(-(v + R(36.0)), R(80.0)));
+      s.x(GO_n_KV) = ab_trap(dt, a, b, R(1.0), s.x(GO_n_KV));
     }
     {  // a_KA
-      R a = (R(0.62) / (R(1.0) + mexp(-(v + R(9.17)) / R(23.32))));
-      R b = (R(0.126) / (mexp((v + R(18.28)) / R(19.47))));
-      s.x(GO_a_KA) = trap(dt, (R(1.0) / (R(1.0) + mexp(-(v + R(38.0)) / R(17.0)))), (R(1.0) / (a + b)), s.x(GO_a_KA));
+      R a = (mdiv(R(0.62), R(1.0) + mexp(cdiv(-(v + R(9.17)), R(23.32)))));
+      R b = (mdiv(R(0.126), mexp(cdiv(v + R(18.28), R(19.47)))));
+      s.x(GO_a_KA) = trap(dt, (mdiv(R(1.0), R(1.0) + mexp(cdiv(-(v + R(38.0)), R(17.0))))), (mdiv(R(1.0), a + b)), s.x(GO_a_KA));
     }
     {  // b_KA
-      R a = (R(0.028) / (R(1.0) + mexp((v + R(111.0)) / R(12.84))));
-      R b = (R(0.026) / (R(1.0) + mexp(-(v + R(49.95)) / R(8.9))));
-      s.x(GO_b_KA) = trap(dt, (R(1.0) / (R(1.0) + mexp((v + R(78.8)) / R(8.4)))), (R(1.0) / (a + b)), s.x(GO_b_KA));
+      R a = (mdiv(R(0.028), R(1.0) + mexp(cdiv(v + R(111.0), R(12.84)))));
+      R b = (mdiv(R(0.026), R(1.0) + mexp(cdiv(-(v + R(49.95)), R(8.9)))));
+      s.x(GO_b_KA) = trap(dt, (mdiv(R(1.0), R(1.0) + mexp(cdiv(v + R(78.8), R(8.4))))), (mdiv(R(1.0), a + b)), s.x(GO_b_KA));
     }
     {  // sl_Kslow
-      R a = (R(0.0037) * mexp((v + R(30.0)) / R(40.0)));
-      R b = (R(0.0037) * mexp(-(v + R(30.0)) / R(20.0)));
-      s.x(GO_sl) = trap(dt, (R(1.0) / (R(1.0) + mexp(-(v + R(35.0)) / R(6.0)))), (R(1.0) / (a + b)), s.x(GO_sl));
+      R a = (R(0.0037) * mexp(cdiv(v + R(30.0), R(40.0))));
+      R b = (R(0.0037) * mexp(cdiv(-(v + R(30.0)), R(20.0))));
+      s.x(GO_sl) = trap(dt, (mdiv(R(1.0), R(1.0) + mexp(cdiv(-(v + R(35.0)), R(6.0))))), (mdiv(R(1.0), a + b)), s.x(GO_sl));
     }
     {  // c_KC (Ca-dependent)
-      R a = (R(3.2) / (R(1.0) + R(0.0015) * mexp(-(v) / R(11.7)) / c));
-      R b = (R(0.46) / (R(1.0) + c / (R(1.5e-4) * mexp(-(v) / R(11.7)))));
-      s.x(GO_c_KC) = trap(dt, (a / (a + b)), (R(1.0) / (a + b)), s.x(GO_c_KC));
+      R a = (mdiv(R(3.2), R(1.0) + mdiv(R(0.0015) * mexp(cdiv(-(v), R(11.7))), c)));
+      R b = (mdiv(R(0.46), R(1.0) + mdiv(c, R(1.5e-4) * mexp(cdiv(-(v), R(11.7))))));
+      s.x(GO_c_KC) = ab_trap(dt, a, b, R(1.0), s.x(GO_c_KC));
     }
     {  // ch_CaHVA
       R a = (R(0.0687) * mexp(R(0.063) * (v + R(29.0))));
       R b = (R(0.115) * mexp(R(-0.039) * (v + R(18.66))));
-      s.x(GO_ch) = trap(dt, (a / (a + b)), (R(1.0) / (a + b)), s.x(GO_ch));
+      s.x(GO_ch) = ab_trap(dt, a, b, R(1.0), s.x(GO_ch));
     }
     {  // ci_CaHVA
-      R a = (R(1.8e-3) * mexp(-(v + R(48.0)) / R(18.0)));
-      R b = (R(1.8e-3) * mexp((v + R(48.0)) / R(83.0)));
-      s.x(GO_ci) = trap(dt, (a / (a + b)), (R(1.0) / (a + b)), s.x(GO_ci));
+      R a = (R(1.8e-3) * mexp(cdiv(-(v + R(48.0)), R(18.0))));
+      R b = (R(1.8e-3) * mexp(cdiv(v + R(48.0), R(83.0))));
+      s.x(GO_ci) = ab_trap(dt, a, b, R(1.0), s.x(GO_ci));
     }
-    s.x(GO_cl) = trap(dt, (R(1.0) / (R(1.0) + mexp(-(v + R(52.0)) / R(7.4)))),
-                      ((R(3.0) + R(1.0) / (mexp((v + R(27.0)) / R(10.0)) + mexp(-(v + R(102.0)) / R(15.0)))) / R(0.85)),
+    s.x(GO_cl) = trap(dt, (mdiv(R(1.0), R(1.0) + mexp(cdiv(-(v + R(52.0)), R(7.4))))),
+                      (cdiv(R(3.0) + mdiv(R(1.0), mexp(cdiv(v + R(27.0), R(10.0))) + mexp(cdiv(-(v + R(102.0)), R(15.0)))), R(0.85))),
                       s.x(GO_cl));
-    s.x(GO_cm) = trap(dt, (R(1.0) / (R(1.0) + mexp((v + R(80.0)) / R(5.0)))),
-                      ((R(85.0) + R(1.0) / (mexp((v + R(48.0)) / R(4.0)) + mexp(-(v + R(407.0)) / R(50.0)))) / R(0.9)),
+    s.x(GO_cm) = trap(dt, (mdiv(R(1.0), R(1.0) + mexp(cdiv(v + R(80.0), R(5.0))))),
+                      (cdiv(R(85.0) + mdiv(R(1.0), mexp(cdiv(v + R(48.0), R(4.0))) + mexp(cdiv(-(v + R(407.0)), R(50.0)))), R(0.9))),
                       s.x(GO_cm));
     {  // HCN1 / HCN2 (r_HCN2 ramp decided on the FP64 voltage)
       const R r1 = (R(0.0021) * (v) + R(0.97));
-      const R s1 = (R(1.0) / (R(1.0) + mexp((v + R(72.5)) * R(0.11))));
+      const R s1 = (mdiv(R(1.0), R(1.0) + mexp((v + R(72.5)) * R(0.11))));
       R r2;
       if (v_val >= -64.70) r2 = R(0.0);
       else if (v_val <= -108.70) r2 = R(1.0);
       else r2 = (R(-0.0227) * (v) - R(1.47));
-      const R s2 = (R(1.0) / (R(1.0) + mexp((v + R(81.9)) * R(0.16))));
+      const R s2 = (mdiv(R(1.0), R(1.0) + mexp((v + R(81.9)) * R(0.16))));
       s.x(GO_hf1) = trap(dt, (r1 * s1), (mexp((R(0.0137) * v + R(3.37)) * R(2.3))), s.x(GO_hf1));
       s.x(GO_hf2) = trap(dt, (r2 * s2), (mexp((R(0.027) * v + R(5.6)) * R(2.3))), s.x(GO_hf2));
       s.x(GO_hs1) = trap(dt, ((R(1.0) - r1) * s1), (mexp((R(0.0145) * v + R(4.06)) * R(2.3))), s.x(GO_hs1));
@@ -675,10 +685,10 @@ template <typename R> struct Go {
   // go_KAHP_update_2order (go_ion.cu:88-213)
   __device__ static void kahp(const Slots<R> &s, double ca_new, double &ca_old, double DT) {
     const R i1 = R(80e-3), i2 = R(80e-3), i3 = R(200e-3), a1 = R(1.0), a2 = R(100e-3), b1 = R(160e-3), b2 = R(1.2);
-    R l_ca = (R)ca_old;
+    R l_ca = to<R>(ca_old);
     ca_old = ca_new;
-    const R l_dt = R(2.0) / (R)DT;
-    R d1 = R(200) * l_ca / R(3.0), d2 = R(160) * l_ca / R(3.0), d3 = R(80) * l_ca / R(3.0);
+    const R l_dt = mdiv(R(2.0), to<R>(DT));
+    R d1 = cdiv(R(200) * l_ca, R(3.0)), d2 = cdiv(R(160) * l_ca, R(3.0)), d3 = cdiv(R(80) * l_ca, R(3.0));
     const int slot[6] = {GO_c1, GO_c2, GO_c3, GO_c4, GO_o1, GO_o2};
     R vc[6], vcb[6];
 #pragma unroll
@@ -690,8 +700,8 @@ template <typename R> struct Go {
                  {R(0), R(0), b1, R(0), -a1 + l_dt, R(0)},
                  {R(0), R(0), R(0), b2, R(0), -a2 + l_dt}};
     dd_neg_matvec<R, KahpPattern>(E, vc, vcb);
-    l_ca = (R)ca_new;
-    d1 = R(200) * l_ca / R(3.0); d2 = R(160) * l_ca / R(3.0); d3 = R(80) * l_ca / R(3.0);
+    l_ca = to<R>(ca_new);
+    d1 = cdiv(R(200) * l_ca, R(3.0)); d2 = cdiv(R(160) * l_ca, R(3.0)); d3 = cdiv(R(80) * l_ca, R(3.0));
     R M[6][6] = {{-d1 - l_dt, i1, R(0), R(0), R(0), R(0)},
                  {d1, -d2 - i1 - l_dt, i2, R(0), R(0), R(0)},
                  {R(0), d2, -(d3 + i2 + b1) - l_dt, i3, a1, R(0)},
@@ -720,13 +730,13 @@ template <typename R> struct Go {
 
   // go_update_matrix (solve_rkc.cu:289-312)
   __device__ static R b(const Slots<R> &s, double vy, double iext, double rev) {
-    const R lv = (R)vy;
-    return (-(R)iext + s.g(GO_g_leak) * (lv - R(V_LEAK_GO)) +
+    const R lv = to<R>(vy);
+    return (-to<R>(iext) + s.g(GO_g_leak) * (lv - R(V_LEAK_GO)) +
             s.g(GO_g_NaT) * (lv - R(V_Na_GO)) * s.x(GO_m_NaT) * s.x(GO_m_NaT) * s.x(GO_m_NaT) * s.x(GO_h_NaT) +
             s.g(GO_g_NaR) * (lv - R(V_Na_GO)) * s.x(GO_r_NaR) * s.x(GO_s_NaR) +
             s.g(GO_g_NaP) * (lv - R(V_Na_GO)) * s.x(GO_p_NaP) +
             s.g(GO_g_CaHVA) * (lv - R(V_Ca_GO)) * s.x(GO_ch) * s.x(GO_ch) * s.x(GO_ci) +
-            s.g(GO_g_CaLVA) * (lv - (R)rev) * s.x(GO_cl) * s.x(GO_cl) * s.x(GO_cm) +
+            s.g(GO_g_CaLVA) * (lv - to<R>(rev)) * s.x(GO_cl) * s.x(GO_cl) * s.x(GO_cm) +
             s.g(GO_g_KAHP) * (lv - R(V_K_GO)) * (s.x(GO_o1) + s.x(GO_o2)) +
             s.g(GO_g_KV) * (lv - R(V_K_GO)) * s.x(GO_n_KV) * s.x(GO_n_KV) * s.x(GO_n_KV) * s.x(GO_n_KV) +
             s.g(GO_g_KA) * (lv - R(V_K_GO)) * s.x(GO_a_KA) * s.x(GO_a_KA) * s.x(GO_a_KA) * s.x(GO_b_KA) +
