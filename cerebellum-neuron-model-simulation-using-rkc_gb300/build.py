@@ -32,9 +32,12 @@ CXX = os.environ.get("CXX", "g++")
 CXXFLAGS = ["-O2", "-std=c++17", "-fPIC", "-ffp-contract=off", "-Wall", "-Wno-unused-function",
             f"-I{CUDA_HOME}/include", f"-I{os.path.join(ROOT, 'include')}"]
 
-KERNEL_TUS = ["kernels_fp64.cu", "kernels_fp32.cu", "compat.cu", "noalloc.cu", "synapse.cu"]
-TU_FLAGS = {"kernels_fp32.cu": ["-prec-div=false"]}
-HOST_TUS = ["engine.cpp", "host_init.cpp", "server.cpp"]
+# (source, object name, extra flags); the per-pool kernels once per cell type
+# and precision
+TUS = [("kernels_fp64.cu", "", []), ("kernels_fp32.cu", "", ["-prec-div=false"])]
+TUS += [("kernels_pool.cu", f"_{t}_{r}", [f"-DGBRKC_CT={t}", f"-DGBRKC_REAL={r}"]
+         + (["-prec-div=false"] if r == "float" else [])) for r in ("double", "float") for t in ("GR", "GO", "PKJ", "IO")]
+TUS += [(s, "", []) for s in ("compat.cu", "noalloc.cu", "synapse.cu", "engine.cpp", "host_init.cpp", "server.cpp")]
 
 
 def _newer(target: str, deps) -> bool:
@@ -49,21 +52,19 @@ def build(verbose: bool = False) -> str:
     headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh", ".cu"))]
     headers.append(os.path.join(ROOT, "include", "gbrkc.h"))
     procs, objs = [], []
-    for tu in KERNEL_TUS + HOST_TUS:
+    for tu, name, flags in TUS:
         src = os.path.join(CSRC, tu)
-        if not os.path.exists(src):
-            continue
-        obj = os.path.join(BUILD, tu + ".o")
+        obj = os.path.join(BUILD, tu + name + ".o")
         objs.append(obj)
         if not _newer(obj, [src, os.path.abspath(__file__)] + headers):
             continue
         if tu.endswith(".cu"):
-            cmd = [NVCC] + NVFLAGS + TU_FLAGS.get(tu, []) + ["-c", src, "-o", obj]
+            cmd = [NVCC] + NVFLAGS + flags + ["-c", src, "-o", obj]
         else:
             cmd = [CXX] + CXXFLAGS + ["-c", src, "-o", obj]
         if verbose:
             print(" ".join(cmd))
-        procs.append((tu, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT)))
+        procs.append((tu + name, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT)))
     failed = []
     for tu, p in procs:
         out, _ = p.communicate()

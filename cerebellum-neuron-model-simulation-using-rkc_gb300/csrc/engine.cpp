@@ -413,9 +413,14 @@ struct PoolHost {
   // launch configuration
   int team = TEAM_BLOCK, block = 256, grid = 1;
   int grid_bw = GRID_BLOCK;                 // grid team: threads of each CTA that own elements
-  int grid_rl = 0, grid_maxdeg = 0;         // grid team: row slots per CTA, entries per slot (0: no copy)
-  std::vector<int> grid_nbr;                // grid team: neighbour CTAs per CTA (empty: grid barriers only)
-  unsigned long long *d_grid_flags = nullptr;
+  // grid team (engine.h, PoolView): the longest row, the fullest CTA's
+  // elements, the most values a CTA receives, and the hand-over tables
+  int grid_maxdeg = 0, grp_ld = 0, grp_recv_max = 0, grp_nslots = 0;
+  int grp_ctas = 1;
+  std::vector<GroupTab> grp_tab;
+  std::vector<int> grp_chunk0, grp_col, grp_slot, grp_sptr, grp_send, grp_rptr, grp_rslot, grp_gap;
+  unsigned long long *d_grp_words = nullptr;   // published values, chunk sums and the abort flag
+  size_t grp_bytes = 0;
   size_t smem = 0;
   int ws_in_smem = 0;
   long ws_tile = 0;
@@ -432,7 +437,6 @@ struct PoolHost {
   double *d_spk_prev = nullptr;
   SpikeRec *d_spk_log = nullptr;         // owned here (re-sized by gbrkc_record_spikes)
   int *d_spk_count = nullptr;
-  unsigned *d_grid_bar = nullptr;        // grid team: the barrier's words (zeroed before each launch)
   int spk_cap = 0;
   std::vector<char> retired;
 };
@@ -638,24 +642,6 @@ int cluster_min_nc() {
   return 4096;
 }
 
-// Whether pool P is one system of at least cluster_min_nc() compartments
-// (GBRKC_GRID_MIN_NC overrides) and the engine's only one: such a system
-// runs on every SM of the device as one grid team, where a cluster would
-// give it 16 SMs.  GBRKC_GRID=0, or a forced cluster size
-// (GBRKC_CLUSTER_SIZE), keeps it on a cluster.
-bool grid_team_fits(const gbrkc_engine *E, const PoolHost &P) {
-  const char *g = getenv("GBRKC_GRID");
-  if (g && g[0] == '0') return false;
-  const char *cs = getenv("GBRKC_CLUSTER_SIZE");
-  if (cs && cs[0]) return false;
-  const char *m = getenv("GBRKC_GRID_MIN_NC");
-  const long min_nc = (m && m[0]) ? atol(m) : cluster_min_nc();
-  if (P.systems.size() != 1 || P.max_nc < min_nc) return false;
-  for (const HostSystem &S : E->systems)
-    if (S.type != P.type) return false;
-  return true;
-}
-
 // The grid team's shape for a system of nc compartments on at most cap
 // co-resident CTAs: the threads per CTA (bw, a power of two from 32 to
 // GRID_BLOCK, every one owning elements) and the CTA count.  It minimises the
@@ -754,6 +740,225 @@ void fill_state(gbrkc_engine *E, PoolHost &P, const HostSystem &S, long off, int
     P.stim_t0[cell0 + c] = S.stim_t0[c];
     P.stim_t1[cell0 + c] = S.stim_t1[c];
   }
+}
+
+// The group team's tables for the pool's systems on groups of `ctas` CTAs of
+// bw threads (group_sys.cuh); ctas 1 is the one-CTA team, which needs none.
+// CTA c owns the chunks of bw elements from c chunks / ctas on; every operator
+// entry's column becomes its place in the row's CTA, among the CTA's own
+// elements or behind them among the values it receives.  In the grid team an
+// element that another CTA reads gets a publishing slot; in a cluster its
+// thread gets the list of the CTAs to store it to.  False (the pool
+// unchanged) when shared memory does not hold a CTA's part, or when some CTA
+// reads from one that does not read from it, which the hand-over's double
+// buffering relies on.
+bool group_tables(PoolHost &P, int bw, int ctas, bool grid) {
+  const int nsys = (int)P.systems.size();
+  std::vector<GroupTab> tab(nsys);
+  std::vector<int> t_chunk0, t_col, t_slot, t_sptr, t_send, t_rptr, t_rslot, t_gap(std::max<size_t>(1, P.gap_pre.size()), -1);
+  std::map<std::pair<int, int>, int> seen;      // (own operator, index) of cells alike: their tables
+  int maxdeg = 0, most = 0, rows = 0, nslots = 0;
+  for (int k = 0; k < nsys; k++) {
+    const int nc = P.sys_nc[k], ncomp = P.sys_ncomp[k];
+    const bool own = P.sys_csr[k] >= 0;
+    const int *r = own ? P.s_row.data() + P.s_row0[P.sys_csr[k]] : P.t_row.data() + P.t_row0[P.sys_tmpl[k]];
+    const int *cl = own ? P.s_col.data() + P.s_nz0[P.sys_csr[k]] : P.t_col.data() + P.t_nz0[P.sys_tmpl[k]];
+    const int chunks = (nc + bw - 1) / bw;
+    for (int i = 0; i < (own ? nc : ncomp); i++) maxdeg = std::max(maxdeg, r[i + 1] - r[i]);
+    if (ctas == 1) {
+      rows = std::max(rows, chunks);
+      continue;
+    }
+    if (!own && P.sys_ncell[k] != 1) return false;
+    if (chunks < ctas) return false;
+    if (!own) {
+      auto it = seen.find({0, P.sys_tmpl[k]});
+      if (it != seen.end()) {
+        tab[k] = tab[it->second];
+        continue;
+      }
+      seen[{0, P.sys_tmpl[k]}] = k;
+    }
+    std::vector<int> chunk0(ctas + 1), owner(chunks);
+    for (int c = 0; c <= ctas; c++) chunk0[c] = (int)((long long)c * chunks / ctas);
+    for (int c = 0; c < ctas; c++) {
+      rows = std::max(rows, chunk0[c + 1] - chunk0[c]);
+      for (int q = chunk0[c]; q < chunk0[c + 1]; q++) owner[q] = c;
+    }
+    if (rows > GRID_MAX_ROWS || chunks > GRID_MAX_BLOCKS) return false;
+    auto cta_of = [&](int i) { return owner[i / bw]; };
+    // what each CTA reads of others: its rows' columns, and in an olive
+    // network the sending dendrites of its cells' gap junctions
+    std::vector<std::vector<int>> recv(ctas);
+    for (int i = 0; i < nc; i++)
+      for (int e = r[i]; e < r[i + 1]; e++)
+        if (cta_of(cl[e]) != cta_of(i)) recv[cta_of(i)].push_back(cl[e]);
+    const int g0 = P.sys_gap0[k], ng = P.sys_ngap[k];
+    for (int e = g0; e < g0 + ng; e++)
+      if (P.gap_pre[e] >= 0 && cta_of(P.gap_pre[e]) != cta_of(P.gap_post[e]))
+        recv[cta_of(P.gap_post[e])].push_back(P.gap_pre[e]);
+    GroupTab &T = tab[k];
+    T = GroupTab{(int)t_chunk0.size(), (int)t_col.size(), (int)t_slot.size(), (int)t_sptr.size(), (int)t_send.size(),
+                 (int)t_rptr.size(), (int)t_rslot.size()};
+    t_chunk0.insert(t_chunk0.end(), chunk0.begin(), chunk0.end());
+    std::vector<int> slot(nc, -1);
+    std::vector<std::vector<int>> send((size_t)ctas * bw);
+    std::vector<char> reads((size_t)ctas * ctas, 0);
+    t_rptr.push_back(0);
+    int taken = 0;
+    for (int c = 0; c < ctas; c++) {
+      std::sort(recv[c].begin(), recv[c].end());
+      recv[c].erase(std::unique(recv[c].begin(), recv[c].end()), recv[c].end());
+      for (size_t j = 0; j < recv[c].size(); j++) {
+        const int i = recv[c][j], from = cta_of(i), at = i - chunk0[from] * bw;
+        if (slot[i] < 0) slot[i] = nslots++;
+        t_rslot.push_back(slot[i]);
+        // row of the thread, reading CTA, its slot
+        send[(size_t)from * bw + at % bw].push_back((at / bw) << 24 | c << 16 | (int)j);
+        reads[(size_t)c * ctas + from] = 1;
+      }
+      taken += (int)recv[c].size();
+      t_rptr.push_back(taken);
+      most = std::max(most, (int)recv[c].size());
+    }
+    if (most > 0xffff) return false;
+    for (int a = 0; a < ctas; a++)
+      for (int b = 0; b < a; b++)
+        if (reads[(size_t)a * ctas + b] != reads[(size_t)b * ctas + a]) return false;
+    int n = 0;
+    t_sptr.push_back(0);
+    for (auto &v : send) {
+      t_send.insert(t_send.end(), v.begin(), v.end());
+      t_sptr.push_back(n += (int)v.size());
+    }
+    t_slot.insert(t_slot.end(), slot.begin(), slot.end());
+    auto place = [&](int c, int i) {
+      if (cta_of(i) == c) return i - chunk0[c] * bw;
+      const int j = (int)(std::lower_bound(recv[c].begin(), recv[c].end(), i) - recv[c].begin());
+      return (chunk0[c + 1] - chunk0[c]) * bw + j;
+    };
+    for (int i = 0; i < nc; i++)
+      for (int e = r[i]; e < r[i + 1]; e++) t_col.push_back(place(cta_of(i), cl[e]));
+    for (int e = g0; e < g0 + ng; e++)
+      if (P.gap_pre[e] >= 0) t_gap[e] = place(cta_of(P.gap_post[e]), P.gap_pre[e]);
+  }
+  if (rows > (grid ? GRID_MAX_ROWS : 2)) return false;
+  const int ld = rows * bw;
+  const size_t smem = grid_smem(ld, most, maxdeg, (grid || ctas == 1) ? 0 : ctas);
+  if (smem > GRID_SMEM_MAX) return false;
+  P.grp_tab = tab;
+  for (auto *v : {&t_chunk0, &t_col, &t_slot, &t_sptr, &t_send, &t_rptr, &t_rslot})
+    if (v->empty()) v->push_back(0);
+  P.grp_chunk0 = t_chunk0; P.grp_col = t_col; P.grp_slot = t_slot; P.grp_sptr = t_sptr; P.grp_send = t_send;
+  P.grp_rptr = t_rptr; P.grp_rslot = t_rslot; P.grp_gap = t_gap;
+  P.grid_maxdeg = maxdeg;
+  P.grp_ctas = ctas;
+  P.grp_ld = ld;
+  P.grp_recv_max = most;
+  P.grp_nslots = nslots;
+  P.team = (grid ? TEAM_GRID1 : ctas > 1 ? TEAM_CLU1 : TEAM_CTA1) + (rows == 1 ? 0 : rows == 2 ? 1 : 7);
+  P.block = bw;
+  P.grid = ctas;
+  P.grid_bw = bw;
+  P.ws_tile = (long)WS_VECS * ((P.max_nc + 1) & ~1);
+  P.ws_in_smem = 0;
+  P.smem = smem;
+  return true;
+}
+
+// A group team (group_sys.cuh) for a pool alone in its engine, where it
+// shortens the launch: the shape is the one of least estimated time, and the
+// pool keeps its other teams (a warp, a block or an old-style cluster per
+// system, inside the persistent launch) where theirs is less.  The estimate
+// counts FP64 warp instructions of a step attempt, 64 cycles each on an SM
+// with up to three warps and 19 per warp beyond (measured): 17 stages of 12
+// per element row, 22 for the error norm, the row's share of the ion updates
+// (FP64 gating: 0.15 to 0.5 updates of 1200 to 2300 an attempt), and 90 of the
+// controller, which every warp repeats; and the latency of handing over the
+// stage vector and the sums (CTA 60 and 500 cycles, cluster 400 and 1200,
+// grid 1400 and 4000).  A warp per system thus stays the better team once a
+// pool fills the GPU (77 Golgi cells: one CTA of 160 threads each; 2048: a
+// warp each).  A lone system of GRID_MIN_NC compartments always takes the
+// grid.  GBRKC_GROUP=0 and GBRKC_GRID=0 switch the teams off, a forced cluster
+// size (GBRKC_CLUSTER_SIZE) too; GBRKC_GRID_MIN_NC sends a lone system of that
+// size to the grid.
+constexpr long GRID_MIN_NC = 8192;
+bool group_team(const gbrkc_engine *E, PoolHost &P) {
+  const char *cs = getenv("GBRKC_CLUSTER_SIZE"), *gr = getenv("GBRKC_GROUP"), *gd = getenv("GBRKC_GRID");
+  const char *mn = getenv("GBRKC_GRID_MIN_NC");
+  if ((cs && cs[0]) || (gr && gr[0] == '0')) return false;
+  for (const HostSystem &S : E->systems)
+    if (S.type != P.type) return false;
+  const int nsys = (int)P.systems.size();
+  const long nc = P.max_nc, grid_nc = (mn && mn[0]) ? atol(mn) : GRID_MIN_NC;
+  const bool grid_ok = nsys == 1 && !(gd && gd[0] == '0');
+  auto to_grid = [&] {
+    const int g = P.f64 ? grid_capacity<double>(P.type) : grid_capacity<float>(P.type);
+    int bw = 0, ctas = 0;
+    return g > 0 && grid_shape(nc, g, &bw, &ctas) &&
+           group_tables(P, bw, (int)std::min<long>(ctas, (nc + bw - 1) / bw), true);
+  };
+  if (grid_ok && nc >= grid_nc) return to_grid();
+  if (nc >= GRID_MIN_NC) return false;
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (sms < 1) return false;
+  static const double ion[NTYPES] = {350.0, 860.0, 840.0, 170.0};
+  const double stages = 17.0, row = stages * 12.0 + 22.0 + (P.f64 ? ion[P.type] : 40.0), ctl = 90.0;
+  auto time = [&](double rows, double warps, double rounds, double hand, double sum) {
+    return rounds * ((rows * row + ctl) * std::max(64.0, 19.0 * warps) + (stages + 1) * hand + 1.3 * sum);
+  };
+  auto up = [](long a, long b) { return (a + b - 1) / b; };
+  // the persistent launch's teams: Golgi cells a warp each, others a block each
+  const double other = (P.type == GO && nc <= 320)
+                           ? time((double)up(nc, 32), (double)std::min(8L, up(nsys, sms)), (double)up(nsys, 8L * sms), 30, 700)
+                           : time((double)up(nc, 256), 8, (double)up(nsys, sms), 150, 1000);
+  double best = 0.9 * other;
+  int kind = 0, bbw = 0, bctas = 1;
+  for (int bw = 32; bw <= GRID_BLOCK; bw += 32) {
+    const long rows = up(nc, bw), fit = std::max(1, 65536 / (256 * bw));   // CTAs an SM's registers hold
+    if (rows <= 2) {
+      const long per = std::min(fit, up(nsys, sms));
+      const double t = time((double)rows, (double)(per * (bw / 32)), (double)up(nsys, per * sms), 60, 500);
+      if (t < best) { best = t; kind = 1; bbw = bw; bctas = 1; }
+    }
+    if (bw & (bw - 1)) continue;
+    for (long r = 1; r <= 2; r++) {
+      const long ctas = up(rows, r);
+      if (ctas < 2 || ctas > 16 || up(rows, ctas) != r) continue;
+      const long per = std::min(fit, up((long)nsys * ctas, sms));
+      const long at_once = std::max(1L, per * sms / ctas);
+      const double t = time((double)r, (double)(per * (bw / 32)), (double)up(nsys, at_once), 400, 1200);
+      if (t < best) { best = t; kind = 2; bbw = bw; bctas = (int)ctas; }
+    }
+  }
+  if (grid_ok) {
+    int bw = 0, ctas = 0;
+    if (grid_shape(nc, sms, &bw, &ctas)) {
+      const double t = time((double)up(nc, (long)bw * ctas), bw / 32.0, 1, 1400, 4000);
+      if (t < best && to_grid()) return true;
+    }
+  }
+  if (kind == 0) return false;
+  PoolHost before = P;
+  if (!group_tables(P, bbw, bctas, false)) return false;
+  int groups = nsys;
+  if (kind == 2) {
+    const int cap = P.f64 ? group_capacity<double>(P.type, P.team, bctas, bbw, P.smem)
+                          : group_capacity<float>(P.type, P.team, bctas, bbw, P.smem);
+    if (cap < 1) {
+      P = before;
+      return false;
+    }
+    groups = std::min(nsys, cap);
+  } else {
+    // as many CTAs as are resident at once share the systems out
+    const long per = std::min<long>(std::max(1, 65536 / (256 * bbw)), up(nsys, sms));
+    groups = (int)std::min<long>(nsys, per * sms);
+  }
+  P.grid = groups * bctas;
+  return true;
 }
 
 // granule systems a warp takes with `lanes` of its lanes in use
@@ -884,76 +1089,8 @@ int assemble_pool(gbrkc_engine *E, PoolHost &P) {
     P.team = (P.type == GR && P.min_nc == 4 && P.max_nc == 4 && P.max_ncell == 1) ? TEAM_LANE4 : TEAM_THREAD;
     P.block = MEGA_BLOCK;
   }
+  else if (group_team(E, P)) return 0;
   else if (P.max_nc <= 320) { P.team = TEAM_WARP; P.block = 128; }
-  else if (grid_team_fits(E, P)) {
-    // a lone large system: every SM of the device on it
-    const int g = P.f64 ? grid_capacity<double>(P.type) : grid_capacity<float>(P.type);
-    int bw = 0, ctas = 0;
-    if (g > 0 && grid_shape(P.max_nc, g, &bw, &ctas)) {
-      // CTAs of exactly the owning threads: every warp of a CTA repeats the
-      // controller's scalar FP64 work, so a warp without elements only
-      // costs FP64 issue slots
-      P.team = TEAM_GRID;
-      P.block = bw;
-      P.grid = ctas;
-      P.grid_bw = bw;
-      P.ws_tile = (long)WS_VECS * ((P.max_nc + 1) & ~1);
-      P.ws_in_smem = 0;
-      // each CTA's operator rows in shared memory when they fit: row slots
-      // of the widest row (diagonal dropped) of any of the pool's systems
-      int maxdeg = 0;
-      for (size_t k = 0; k < P.systems.size(); k++) {
-        const bool own = P.sys_csr[k] >= 0;
-        const int *r = own ? P.s_row.data() + P.s_row0[P.sys_csr[k]] : P.t_row.data() + P.t_row0[P.sys_tmpl[k]];
-        const int nr = own ? P.sys_nc[k] : P.sys_ncomp[k];
-        for (int j = 0; j < nr; j++) maxdeg = std::max(maxdeg, r[j + 1] - r[j]);
-      }
-      const long rl = (P.max_nc + (long)ctas * bw - 1) / ((long)ctas * bw) * bw;
-      const bool fits = maxdeg > 0 && grid_rows_smem(rl, maxdeg) <= GRID_ROWS_SMEM_MAX;
-      const char *ec = getenv("GBRKC_GRID_ROWS_SMEM");
-      const bool want = !(ec && ec[0] == '0');
-      P.grid_rl = (int)rl;
-      P.grid_maxdeg = (fits && want) ? maxdeg : 0;
-      P.smem = P.grid_maxdeg ? grid_rows_smem(rl, maxdeg) : 0;
-      // each CTA's neighbours: the owners of its rows' columns and the CTAs
-      // whose rows reach its elements (element i: CTA (i mod ctas*bw) / bw)
-      P.grid_nbr.clear();
-      const char *el = getenv("GBRKC_GRID_LOCAL");
-      if (!(el && el[0] == '0')) {
-        const long size = (long)ctas * bw;
-        std::vector<std::vector<char>> adj(ctas, std::vector<char>(ctas, 0));
-        for (size_t k = 0; k < P.systems.size(); k++) {
-          const bool own = P.sys_csr[k] >= 0;
-          const int nc = P.sys_nc[k], ncomp = P.sys_ncomp[k];
-          const int *r = own ? P.s_row.data() + P.s_row0[P.sys_csr[k]] : P.t_row.data() + P.t_row0[P.sys_tmpl[k]];
-          const int *cl = own ? P.s_col.data() + P.s_nz0[P.sys_csr[k]] : P.t_col.data() + P.t_nz0[P.sys_tmpl[k]];
-          for (int i = 0; i < nc; i++) {
-            const int j = (own || P.sys_ncell[k] == 1) ? i : i % ncomp, base = i - j;
-            const int a = (int)((i % size) / bw);
-            for (int e = r[j]; e < r[j + 1]; e++) {
-              const int b = (int)(((base + cl[e]) % size) / bw);
-              if (a != b) adj[a][b] = adj[b][a] = 1;
-            }
-          }
-        }
-        bool fit = true;
-        std::vector<int> nb((size_t)ctas * (GRID_MAX_NBR + 1), 0);
-        for (int a = 0; a < ctas && fit; a++) {
-          int n = 0;
-          for (int b = 0; b < ctas; b++)
-            if (adj[a][b]) {
-              if (n == GRID_MAX_NBR) { fit = false; break; }
-              nb[(size_t)a * (GRID_MAX_NBR + 1) + 1 + n++] = b;
-            }
-          nb[(size_t)a * (GRID_MAX_NBR + 1)] = n;
-        }
-        if (fit) P.grid_nbr = std::move(nb);
-      }
-      return 0;
-    }
-    P.team = TEAM_CLUSTER16;
-    P.block = 256;
-  }
   else if (P.max_nc >= cluster_min_nc()) { P.team = TEAM_CLUSTER16; P.block = 256; }
   else { P.team = TEAM_BLOCK; P.block = 256; }
   if (P.team == TEAM_CLUSTER16) {
@@ -1020,31 +1157,25 @@ int upload_pool(gbrkc_engine *E, PoolHost &P, PoolView<R> &V) {
   UP(P.sys_ncomp, V.sys_ncomp); UP(P.sys_tmpl, V.sys_tmpl); UP(P.sys_csr, V.sys_csr);
   UP(P.sys_cell0, V.sys_cell0); UP(P.sys_gap0, V.sys_gap0); UP(P.sys_ngap, V.sys_ngap);
   UP(P.sys_ws, V.sys_ws); UP(P.ctl, V.ctl);
-  V.grid_red = nullptr;
-  V.grid_bar = nullptr;
-  V.grid_nbr = nullptr;
-  V.grid_flags = nullptr;
-  V.grid_bw = P.grid_bw;
-  {
-    // fence.acq_rel + acquire polls; GBRKC_GRID_FENCE=sc for __threadfence
-    // on both sides of the wait (8% slower on the Purkinje 3x3 system)
-    const char *f = getenv("GBRKC_GRID_FENCE");
-    V.grid_light = (f && strcmp(f, "sc") == 0) ? 0 : 1;
-  }
-  V.grid_rl = P.grid_rl;
-  V.grid_maxdeg = P.grid_maxdeg;
-  if (P.team == TEAM_GRID) {
-    const std::vector<double> red(2 * GRID_MAX_BLOCKS, 0.0);
-    const std::vector<unsigned> bar(sizeof(GridBarrier) / sizeof(unsigned), 0u);
-    UP(red, V.grid_red);
-    UP(bar, V.grid_bar);
-    P.d_grid_bar = V.grid_bar;
-    if (!P.grid_nbr.empty()) {
-      const std::vector<unsigned long long> fl((size_t)P.grid * 16, 0ull);
-      UP(P.grid_nbr, V.grid_nbr);
-      UP(fl, V.grid_flags);
-      P.d_grid_flags = V.grid_flags;
-    }
+  if (team_is_group(P.team)) {
+    V.grid_bw = P.grid_bw;
+    V.grid_maxdeg = P.grid_maxdeg;
+    V.grp_ctas = P.grp_ctas;
+    V.grp_ld = P.grp_ld;
+    V.grp_recv_max = P.grp_recv_max;
+    V.grp_nslots = P.grp_nslots;
+    UP(P.grp_tab, V.grp_tab); UP(P.grp_chunk0, V.grp_chunk0); UP(P.grp_col, V.grp_col); UP(P.grp_slot, V.grp_slot);
+    UP(P.grp_sptr, V.grp_sptr); UP(P.grp_send, V.grp_send);
+    UP(P.grp_rptr, V.grp_rptr); UP(P.grp_rslot, V.grp_rslot); UP(P.grp_gap, V.grp_gap);
+    // one block, zeroed before each launch: the abort flag, and in the grid
+    // team the published values and chunk sums
+    const size_t n = team_is_grid(P.team) ? 4 * (size_t)P.grp_nslots + 4 * GRID_MAX_BLOCKS : 0;
+    const std::vector<unsigned long long> words(2 + n, 0ull);
+    UP(words, P.d_grp_words);
+    P.grp_bytes = words.size() * sizeof(unsigned long long);
+    V.grp_abort = (int *)P.d_grp_words;
+    V.grp_halo = P.d_grp_words + 2;
+    V.grp_red = V.grp_halo + 4 * (size_t)P.grp_nslots;
   }
   std::vector<double> zws(P.ws_total, 0.0);
   UP(zws, V.ws);
@@ -1265,11 +1396,7 @@ int launch_all(gbrkc_engine *E, double t0, int n_iv, int iv0, int init) {
         (P.block != MEGA_BLOCK || !P.ws_in_smem ||
          P.smem < (size_t)MEGA_BLOCK * (size_t)P.ws_tile * sizeof(double)))
       return fail(GBRKC_ESTATE, "single-lane pool %d: launch shape does not cover its workspaces", t);
-    if (P.team == TEAM_GRID) {
-      CUDA_TRY(cudaMemsetAsync(P.d_grid_bar, 0, sizeof(GridBarrier), E->streams[t]));
-      if (P.d_grid_flags)
-        CUDA_TRY(cudaMemsetAsync(P.d_grid_flags, 0, (size_t)P.grid * 16 * sizeof(unsigned long long), E->streams[t]));
-    }
+    if (team_is_group(P.team)) CUDA_TRY(cudaMemsetAsync(P.d_grp_words, 0, P.grp_bytes, E->streams[t]));
     CUDA_TRY(cudaEventRecord(E->ev_k0[t], E->streams[t]));
     if (P.f64)
       rc = launch_pool<double>(t, P.vd, P.team, P.grid, P.block, P.smem, E->streams[t], t0, n_iv, iv0, init);
@@ -1286,11 +1413,11 @@ int launch_all(gbrkc_engine *E, double t0, int n_iv, int iv0, int init) {
   for (int t = 0; t < NTYPES; t++) {
     E->last_kernel_ms[t] = 0.0f;
     if (!E->pools[t].systems.empty()) CUDA_TRY(cudaEventElapsedTime(&E->last_kernel_ms[t], E->ev_k0[t], E->ev_k1[t]));
-    if (E->pools[t].team == TEAM_GRID && !E->pools[t].systems.empty()) {
-      GridBarrier gb{};
-      CUDA_TRY(cudaMemcpy(&gb, E->pools[t].d_grid_bar, sizeof gb, cudaMemcpyDeviceToHost));
-      if (gb.abort)
-        return fail(GBRKC_ECUDA, "grid team (type %d): a barrier gave up waiting; the system is stopped", t);
+    if (team_is_group(E->pools[t].team) && E->pools[t].grp_ctas > 1 && !E->pools[t].systems.empty()) {
+      int gave_up = 0;
+      CUDA_TRY(cudaMemcpy(&gave_up, E->pools[t].d_grp_words, sizeof gave_up, cudaMemcpyDeviceToHost));
+      if (gave_up)
+        return fail(GBRKC_ECUDA, "group team (type %d): a wait gave up; the system is stopped", t);
     }
   }
   return 0;
@@ -1406,7 +1533,7 @@ int setup_mega(gbrkc_engine *E) {
   // pools of very large systems run on clusters, one launch per pool
   for (int t = 0; t < NTYPES; t++)
     if (!E->pools[t].systems.empty() &&
-        (team_cluster_size(E->pools[t].team) > 0 || E->pools[t].team == TEAM_GRID)) return 0;
+        (team_cluster_size(E->pools[t].team) > 0 || team_is_group(E->pools[t].team))) return 0;
   const PoolHost &G = E->pools[GR], &O = E->pools[GO];
   if (!G.systems.empty() && G.max_nc > LANE_MAX_NC) return 0;
   if (!O.systems.empty() && O.max_nc > 320) return 0;
@@ -2081,8 +2208,8 @@ extern "C" int gbrkc_type_team(gbrkc_engine *E, int type) {
   const PoolHost &P = E->pools[type];
   if (P.systems.empty()) return 0;
   if (E->mega) return GBRKC_TEAM_MEGA;
-  if (P.team == TEAM_GRID) return GBRKC_TEAM_GRID;
-  if (team_cluster_size(P.team) > 0) return GBRKC_TEAM_CLUSTER;
+  if (team_is_grid(P.team)) return GBRKC_TEAM_GRID;
+  if (team_cluster_size(P.team) > 0 || team_is_clu(P.team)) return GBRKC_TEAM_CLUSTER;
   return GBRKC_TEAM_POOL;
 }
 extern "C" float gbrkc_last_kernel_ms(gbrkc_engine *E, int type) {

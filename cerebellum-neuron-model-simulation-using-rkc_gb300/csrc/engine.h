@@ -56,6 +56,11 @@ struct Ctl {
   long long n_steps, n_rej, n_stage, n_rho, n_rho_iter, n_ion;
 };
 
+// Where a system's group tables begin (PoolView::grp_*).
+struct GroupTab {
+  int chunk0, col, slot, sptr, send, rptr, rslot;
+};
+
 // Everything a kernel needs for one pool (passed by value).
 template <typename R>
 struct PoolView {
@@ -120,21 +125,24 @@ struct PoolView {
   const double *syn_val;              // per synapse: conductance value (engine-wide table)
   const double *syn_e;                // per synapse: reversal potential
   double *syn_buf;                    // [stride] synaptic current taken at interval start
-  // grid team (one system over every CTA of a cooperative launch): block
-  // sums of the reductions, double-buffered, and the grid barrier's words
-  double *grid_red;                   // [2][GRID_MAX_BLOCKS]
-  unsigned *grid_bar;                 // GridBarrier
-  int grid_bw;                        // threads of each CTA that own elements (a power of two, 32..GRID_BLOCK)
-  int grid_light;                     // grid barrier: acq_rel fence + acquire polls (1) or sc fences (0)
-  // grid team: each CTA's rows of the operator in shared memory (grid_rl
-  // row slots of grid_maxdeg entries each); grid_maxdeg 0 = read the rows
-  // from global memory
-  int grid_rl, grid_maxdeg;
-  // grid team: per CTA its neighbour CTAs ([ctas][GRID_MAX_NBR + 1]: count,
-  // then the list) and the stage-count flags ([ctas * 16]); grid_nbr null:
-  // every stage barrier is the grid barrier
-  const int *grid_nbr;
-  unsigned long long *grid_flags;
+  // group teams (group_sys.cuh): one system over a CTA, a cluster, or every
+  // CTA of a cooperative launch
+  int grid_bw;                        // threads of a CTA, elements of a chunk
+  int grid_maxdeg;                    // the operator's longest row
+  int grp_ctas;                       // CTAs of a group
+  int grp_ld;                         // elements of the fullest CTA
+  int grp_recv_max;                   // most values a CTA receives
+  int grp_nslots;                     // grid: values that more than their own CTA reads
+  const GroupTab *grp_tab;            // per system: where its tables begin
+  const int *grp_chunk0;              // [ctas + 1] first chunk of each CTA
+  const int *grp_col;                 // per operator entry: the column's place in the row's CTA (own places, then received)
+  const int *grp_slot;                // grid, [nc]: the element's publishing slot, or -1
+  const int *grp_sptr, *grp_send;     // cluster, per thread: its hand-overs (row of the thread, reading CTA, its slot)
+  const int *grp_rptr, *grp_rslot;    // per CTA: the values it receives (grid: their slots)
+  const int *grp_gap;                 // olive, per gap edge: the sending dendrite's place, or -1
+  unsigned long long *grp_halo;       // grid: [2][nslots][2] published values
+  unsigned long long *grp_red;        // grid: [2][GRID_MAX_BLOCKS][2] published chunk sums
+  int *grp_abort;                     // a wait gave up
 };
 
 // How a pool takes its synaptic current (solve_rkc.cu): granule cells add
@@ -177,11 +185,14 @@ int launch_syn_update(const SynView &S, void *stream, double t, long long interv
 // TEAM_CLUSTER8 / TEAM_CLUSTER16: one system per cluster of 8 / 16 CTAs
 // (very large systems; 16 is a non-portable cluster size, used where the
 // device can co-schedule it).
-// TEAM_GRID: one system over every CTA of a cooperative launch (a system
-// that is alone in its engine and larger than a cluster holds efficiently).
+// Group teams (group_sys.cuh), at most one, two or eight elements a thread:
+// TEAM_CTA1..: one system per CTA of exactly its threads; TEAM_CLU1..: per
+// cluster of P.grp_ctas CTAs; TEAM_GRID1..: one system over every CTA of a
+// cooperative launch (a system that is alone in its engine).
 enum TeamKind {
   TEAM_THREAD = 1, TEAM_LANE4 = 2, TEAM_TILE4 = 4, TEAM_WARP = 32, TEAM_BLOCK = 0,
-  TEAM_CLUSTER8 = 108, TEAM_CLUSTER16 = 116, TEAM_GRID = 200
+  TEAM_CLUSTER8 = 108, TEAM_CLUSTER16 = 116, TEAM_CTA1 = 201, TEAM_CTA2 = 202, TEAM_CLU1 = 301, TEAM_CLU2 = 302,
+  TEAM_GRID1 = 401, TEAM_GRID2 = 402, TEAM_GRID8 = 408
 };
 // systems a warp takes when `lanes` of its lanes are in use, four lanes each
 constexpr int quads_per_warp(int lanes) { return lanes < 8 ? 1 : lanes / 4; }
@@ -213,34 +224,34 @@ constexpr int CLUSTER_BLOCK = 256;
 constexpr int CLUSTER_MAX_ROWS = 14;
 constexpr int CLUSTER_RED_DOUBLES = 2 * CLUSTER_MAX_ROWS + 8 * CLUSTER_MAX_ROWS + 2;
 constexpr int LANE_MAX_NC = 8;   // largest system integrated by a single lane
-// Grid team: CTAs of GRID_BLOCK threads, of which the first grid_bw (a power
-// of two) own elements: element i of a workspace vector is owned by thread
-// (i mod gridDim * grid_bw) of that numbering; a reduction covers at most
-// GRID_MAX_BLOCKS chunks of grid_bw elements and GRID_MAX_ROWS rows of
-// gridDim * grid_bw elements.
+constexpr bool team_is_grid(int team) { return team >= TEAM_GRID1; }
+constexpr bool team_is_clu(int team) { return team > 300 && team < 400; }
+constexpr bool team_is_group(int team) { return team > 200; }
+// Group teams: CTAs of grid_bw threads (at most GRID_BLOCK; a power of two
+// where a group has several CTAs); the elements go to the CTAs in runs of
+// whole chunks of grid_bw, at most GRID_MAX_ROWS chunks a CTA and
+// GRID_MAX_BLOCKS in all.
 constexpr int GRID_BLOCK = 256;
 constexpr int GRID_MAX_BLOCKS = 256;
 constexpr int GRID_MAX_ROWS = 8;
-constexpr int GRID_MAX_NBR = 32;   // neighbour CTAs a CTA's stage barrier can wait for (one a lane)
-constexpr size_t GRID_ROWS_SMEM_MAX = 160 * 1024;   // shared memory for a CTA's operator rows
-// bytes of that copy: per row slot its entry count, 1/Cm, and maxdeg
-// (column, conductance) pairs
-constexpr size_t grid_rows_smem(long rl, long maxdeg) { return (size_t)rl * (12 + 12 * (size_t)maxdeg); }
-// The grid barrier's words, each on its own 128-byte line: the count of
-// arrivals since the launch began (a CTA's k-th barrier ends when it reaches
-// k * gridDim) and the abort flag.
-struct GridBarrier {
-  unsigned long long count;
-  unsigned long long pad0[15];
-  int abort;
-  int pad1[31];
-};
+constexpr size_t GRID_SMEM_MAX = 200 * 1024;   // shared memory of a CTA
+// bytes of it: two stage buffers, per element its row (conductances, columns,
+// count, 1/Cm, row sum), and in a cluster of `ctas` the slots of hand-overs
+// and sums
+constexpr size_t grid_smem(long ld, long recv, long maxdeg, int ctas) {
+  return 16 * (size_t)(ld + recv) + (size_t)ld * (20 + 12 * (size_t)maxdeg) +
+         (ctas > 0 ? 16 + 32 * (size_t)recv + 32 * (size_t)GRID_MAX_ROWS * ctas : 0);
+}
 
 template <typename R>
 int launch_mega(const MegaView<R> &M, int grid, size_t smem, void *stream, double t0, int n_iv, int iv0,
                 int init);
 template <typename R>
 int prepare_mega_kernel(size_t smem, int *blocks_per_sm);
+
+// The kernel of a team for one cell type and precision (kernels_pool.cu).
+template <int CT, typename R>
+const void *pool_kernel(int team);
 
 // Launch the advance / initialise kernel of one pool (kernels.cu).
 template <typename R>
@@ -252,6 +263,9 @@ int prepare_pool_kernel(int type, int team, size_t smem);
 // with this shared memory (0: the shape does not fit).
 template <typename R>
 int cluster_capacity(int type, int team, size_t smem);
+// The same of a cluster group team's kernel, with `ctas` CTAs of `block` threads.
+template <typename R>
+int group_capacity(int type, int team, int ctas, int block, size_t smem);
 // CTAs of the grid team's cooperative launch (0: the device cannot launch it).
 template <typename R>
 int grid_capacity(int type);

@@ -1,0 +1,793 @@
+// RKC integrator for one system spread over the threads of a CTA, of a
+// cluster of CTAs, or (the grid team: a system alone in its engine, too large
+// for a cluster) of every CTA of a cooperative launch; its five RKC vectors
+// and its current b in registers, at most K elements a thread.
+//
+// What bounds it: an FP64 warp instruction costs 64 cycles on its SM
+// sub-partition whatever its lanes do, so a stage is about 12 of them per
+// element row, and the rest of a stage is the latency of handing the stage
+// vector's values to the threads that read them.  So:
+//  * Elements go to CTAs in runs of whole chunks of bw consecutive elements
+//    (a power of two where there are several CTAs): in a tree numbered along
+//    its branches most neighbours are then in the same CTA, read from shared
+//    memory.
+//  * A value that another CTA reads is handed over as two 64-bit words, each
+//    half of the value beside the evaluation's number: one store and one load
+//    that polls for that number, no fence, no flag, no barrier over the CTAs.
+//    In a cluster the writer stores into the reader's shared memory (about
+//    200 cycles), in the grid team into a slot of global memory that its
+//    readers poll in the L2 (about 1500).  Slots are double-buffered.  A CTA
+//    cannot overwrite a slot that its reader still polls: it writes
+//    evaluation k + 2 only after evaluation k + 1 has reached it from every
+//    CTA it reads from, the CTAs that read from it are the same ones (the
+//    host checks that), and each of them had taken evaluation k before it
+//    handed over k + 1.
+//  * Sums are the pairwise tree: warp shuffles, the chunk's warp partials,
+//    then every chunk's sum handed to every CTA the same way, one warp of
+//    which combines them in the tree's order.  A sum thus also separates
+//    everything before it from everything after it in all CTAs, so one
+//    system's slots serve the next one.
+// Every poll is bounded (GRID_SPIN_LIMIT) and raises the abort flag, after
+// which no wait waits and the CTAs leave the system at the next attempt
+// (status ST_BARRIER); a cluster, and a cooperative launch, make every CTA
+// resident, so the bound is a guard, not a schedule.
+//
+// Measured against the block, warp and old grid teams (a launch per pass, in
+// ms): full granule cell, FP64, one interval 39.5 -> 12.2 (a cluster of
+// 10 CTAs of 64 threads; one CTA before); 77 Golgi cells, FP64, five
+// intervals 45.5 -> 10.7 (clusters of 5 x 32); 16x16 olive network, mixed, 16
+// intervals 26.9 -> 10.8 (12 x 64); Purkinje 3x3, FP64, eight intervals 23.6
+// -> 20.3 (grid, 113 x 128: two fifths of it the FP64 ion updates).
+//
+// The arithmetic is Sys's (integrator.cuh) operation for operation.
+#pragma once
+#include "step_ctl.cuh"
+
+namespace gbrkc {
+
+constexpr long GRID_SPIN_LIMIT = 1L << 22;
+
+enum GroupComm { GRP_CTA, GRP_CLUSTER, GRP_GRID };
+
+// a value and its evaluation's number in one slot: {low half, number}, {high
+// half, number}, each word written and read whole
+template <int COMM>
+__device__ __forceinline__ void word_put(unsigned long long p, unsigned long long w) {
+  if constexpr (COMM == GRP_GRID)
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(w) : "memory");
+  else
+    asm volatile("st.relaxed.cluster.shared::cluster.u64 [%0], %1;" ::"r"((unsigned)p), "l"(w) : "memory");
+}
+template <int COMM>
+__device__ __forceinline__ unsigned long long word_get(unsigned long long p) {
+  unsigned long long w;
+  if constexpr (COMM == GRP_GRID)
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(p) : "memory");
+  else
+    asm volatile("ld.relaxed.cluster.shared::cta.u64 %0, [%1];" : "=l"(w) : "r"((unsigned)p) : "memory");
+  return w;
+}
+template <int COMM>
+__device__ __forceinline__ void slot_put(unsigned long long p, double x, unsigned tag) {
+  const unsigned long long u = (unsigned long long)__double_as_longlong(x), t = (unsigned long long)tag << 32;
+  word_put<COMM>(p, (u & 0xffffffffull) | t);
+  word_put<COMM>(p + 8, (u >> 32) | t);
+}
+template <int COMM>
+__device__ __forceinline__ bool slot_get(unsigned long long p, unsigned tag, double &x) {
+  const unsigned long long a = word_get<COMM>(p), b = word_get<COMM>(p + 8);
+  x = __longlong_as_double((long long)((a & 0xffffffffull) | (b << 32)));
+  return (unsigned)(a >> 32) == tag && (unsigned)(b >> 32) == tag;
+}
+// this CTA's shared-memory address p (32 bits) in CTA `rank` of the cluster
+__device__ __forceinline__ unsigned cluster_map(unsigned p, int rank) {
+  unsigned q;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(q) : "r"(p), "r"(rank));
+  return q;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <int CT, typename R, int K, int COMM>
+struct GroupSys {
+  static constexpr bool MIXED = !std::is_same<R, double>::value;
+  static constexpr int RN = 4;   // neighbours kept in registers where a thread has one element
+  typedef StepCtl<double> SC;
+  const PoolView<R> &P;
+  int s, nc, ncell, ncomp, off, cell0;
+  int G, cta, bw, t;           // CTAs of the group, this CTA, threads a CTA, this thread
+  int chunk0, rows, e0, L;     // this CTA's chunks, its first element, its element places
+  int r0, nrecv;               // its received values
+  const GroupTab *tab;
+  int ld;                      // places of the row tables (rows of the fullest CTA)
+  // shared memory
+  double *u;                   // [2][ld + most received]: the stage vector, own places then received ones
+  double *lg, *linv, *lG;      // [maxdeg][ld] conductances, [ld] 1/Cm; mixed: g/Cm, and its row sums
+  int *lcol, *lcnt;            // [maxdeg][ld] places of the neighbours, [ld] counts
+  double *wp, *res;
+  unsigned halo, red;          // cluster: [2][most received][2] and [2][chunks][2] words, shared-memory addresses
+  int *s_abort;                // [0] a wait gave up, [1] the same as of the last sum, alike for the CTA's threads
+  // registers
+  double y[K], yn[K], fn[K], v1[K], v2[K];
+  double b[K];                 // the current; mixed precision: -b / Cm
+  int slot[K];                 // grid: publishing slot, or -1
+  int send0, send1;            // cluster: the thread's hand-overs (P.grp_send)
+  int rc[RN];                  // K = 1: the row's first columns
+  double rg[RN];               //        and conductances
+  SC c;
+  Recip rnc;                   // 1 / nc
+  unsigned tag, rtag;          // evaluations and sums so far
+  double t0;
+  int k_iv, n_iv, iv0;
+  long long attempts0;
+
+  // cta_, G_: this CTA's place in its group and the group's CTAs
+  __device__ GroupSys(const PoolView<R> &P_, double *smem, double *wp_, double *res_, int *ab, int cta_, int G_)
+      : P(P_), wp(wp_), res(res_), s_abort(ab) {
+    t = threadIdx.x;
+    bw = P.grid_bw;
+    G = G_;
+    cta = cta_;
+    ld = P.grp_ld;
+    const int md = P.grid_maxdeg, rm = P.grp_recv_max;
+    u = smem;
+    lg = u + 2 * (ld + rm);
+    linv = lg + (long)md * ld;
+    lG = linv + ld;
+    lcol = (int *)(lG + ld);
+    lcnt = lcol + (long)md * ld;
+    tag = rtag = 0;
+    if constexpr (COMM == GRP_CLUSTER) {
+      // slots behind the rows, numbered 0 before any hand-over
+      unsigned long long *w = (unsigned long long *)(((unsigned long long)(lcnt + ld) + 15) & ~15ull);
+      const int n = 4 * rm + 4 * GRID_MAX_ROWS * G;
+      for (int i = t; i < n; i += bw) w[i] = 0ull;
+      halo = (unsigned)__cvta_generic_to_shared(w);
+      red = halo + 32 * rm;
+      cluster_sync_all();
+    }
+  }
+  // no CTA leaves while a peer may still store into its shared memory
+  __device__ __forceinline__ void leave() const {
+    if constexpr (COMM == GRP_CLUSTER) cluster_sync_all();
+  }
+
+  __device__ __forceinline__ int at(int k) const { return e0 + k * bw + t; }
+  __device__ __forceinline__ bool has(int k) const { return k < rows && at(k) < nc; }
+  __device__ __forceinline__ int ustride() const { return ld + P.grp_recv_max; }
+  __device__ __forceinline__ const double *ucur() const { return u + (tag & 1u) * ustride(); }
+
+  // Take the system: its operator rows into shared memory, its vectors into
+  // registers.
+  __device__ __forceinline__ void bind(int s_) {
+    s = s_;
+    nc = P.sys_nc[s];
+    ncell = P.sys_ncell[s];
+    ncomp = P.sys_ncomp[s];
+    off = P.sys_off[s];
+    cell0 = P.sys_cell0[s];
+    tab = P.grp_tab + s;
+    if constexpr (COMM == GRP_CTA) {
+      chunk0 = 0;
+      rows = (nc + bw - 1) / bw;
+      r0 = nrecv = 0;
+    } else {
+      chunk0 = P.grp_chunk0[tab->chunk0 + cta];
+      rows = P.grp_chunk0[tab->chunk0 + cta + 1] - chunk0;
+      r0 = P.grp_rptr[tab->rptr + cta];
+      nrecv = P.grp_rptr[tab->rptr + cta + 1] - r0;
+    }
+    e0 = chunk0 * bw;
+    L = rows * bw;
+    send0 = send1 = 0;
+    const int k = P.sys_csr[s], tm = P.sys_tmpl[s];
+    const bool csr = k >= 0;
+    const int *row = csr ? P.s_row + P.s_row0[k] : P.t_row + P.t_row0[tm];
+    const long nz0 = csr ? P.s_nz0[k] : P.t_nz0[tm], cm0 = csr ? P.s_cm0[k] : P.t_cm0[tm];
+    const double *g = (MIXED ? (csr ? P.s_gc : P.t_gc) : (csr ? P.s_g : P.t_g)) + nz0;
+    const double *inv = (csr ? P.s_invcm : P.t_invcm) + cm0, *Gc = (csr ? P.s_Gc : P.t_Gc) + cm0;
+    const int *map = P.ctl[s].map;
+    const long ncp = (nc + 1) & ~1;
+    const double *ws = P.ws + P.sys_ws[s];
+    const int *pcol = (csr ? P.s_col + P.s_nz0[k] : P.t_col + P.t_nz0[tm]);
+    if constexpr (COMM != GRP_CTA) pcol = P.grp_col + tab->col;
+    c.load(P.ctl[s]);
+    __syncthreads();               // the last system's readers of the tables are done
+#pragma unroll
+    for (int q = 0; q < RN; q++) {
+      rc[q] = 0;
+      rg[q] = 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < K; q++) {
+      y[q] = yn[q] = fn[q] = v1[q] = v2[q] = b[q] = 0.0;
+      slot[q] = -1;
+      if (!has(q)) continue;
+      // (cells of one template lie one after another)
+      const int i = at(q), lr = q * bw + t, base = csr ? 0 : i - i % ncomp, ri = i - base;
+      const int a = __ldg(row + ri), z = __ldg(row + ri + 1);
+      lcnt[lr] = z - a;
+      linv[lr] = __ldg(inv + ri);
+      if (MIXED) lG[lr] = __ldg(Gc + ri);
+      for (int j = a; j < z; j++) {
+        lg[(long)(j - a) * ld + lr] = __ldg(g + j);
+        lcol[(long)(j - a) * ld + lr] = (COMM == GRP_CTA ? base : 0) + __ldg(pcol + j);
+      }
+      if constexpr (K == 1) {
+#pragma unroll
+        for (int j = 0; j < RN; j++)
+          if (j < z - a) {
+            rc[j] = lcol[(long)j * ld + lr];
+            rg[j] = lg[(long)j * ld + lr];
+          }
+      }
+      if constexpr (COMM == GRP_GRID) slot[q] = P.grp_slot[tab->slot + i];
+      if constexpr (COMM == GRP_CLUSTER) {
+        // (a thread of several elements hands over in exchange's own loop)
+        if (q == 0) {
+          send0 = P.grp_sptr[tab->sptr + (cta * bw) + t];
+          send1 = P.grp_sptr[tab->sptr + (cta * bw) + t + 1];
+        }
+      }
+      y[q] = ws[map[LY] * ncp + i];
+      yn[q] = ws[map[LYN] * ncp + i];
+      fn[q] = ws[map[LFN] * ncp + i];
+      v1[q] = ws[map[LV1] * ncp + i];
+      v2[q] = ws[map[LV2] * ncp + i];
+      set_b(q, ws[WS_B * ncp + i]);
+    }
+    __syncthreads();
+  }
+
+  __device__ __forceinline__ void set_b(int q, double x) {
+    if constexpr (MIXED) b[q] = -x * linv[q * bw + t];
+    else b[q] = x;
+  }
+
+  // (b itself is written at each ion update)
+  __device__ __forceinline__ void store(bool init) const {
+    const int *map = P.ctl[s].map;
+    const long ncp = (nc + 1) & ~1;
+    double *ws = P.ws + P.sys_ws[s];
+#pragma unroll
+    for (int q = 0; q < K; q++)
+      if (has(q)) {
+        const int i = at(q);
+        ws[map[LY] * ncp + i] = y[q];
+        ws[map[LYN] * ncp + i] = yn[q];
+        ws[map[LFN] * ncp + i] = fn[q];
+        ws[map[LV1] * ncp + i] = v1[q];
+        ws[map[LV2] * ncp + i] = v2[q];
+      }
+    if (cta == 0 && t == 0) c.store(P.ctl[s], init);
+  }
+
+  // Poll a slot for evaluation or sum `want`.
+  __device__ __forceinline__ double wait(unsigned long long p, unsigned want) const {
+    double x;
+    long it = 0;
+    while (!slot_get<COMM>(p, want, x)) {
+      if ((++it & 255) == 0) {
+        volatile int *ab = P.grp_abort;
+        if (*ab || it > GRID_SPIN_LIMIT) {
+          *ab = 1;
+          *(volatile int *)s_abort = 1;
+          break;
+        }
+      }
+    }
+    return x;
+  }
+
+  // Hand the stage vector val to its readers: own values into shared memory,
+  // those other CTAs read into their slots, the received ones behind the own.
+  __device__ __forceinline__ void exchange(const double (&val)[K]) {
+    tag++;
+    const unsigned par = tag & 1u;
+    double *ub = u + par * ustride();
+    if constexpr (COMM == GRP_GRID) {
+      const unsigned long long h = (unsigned long long)(P.grp_halo + (long)par * P.grp_nslots * 2);
+#pragma unroll
+      for (int q = 0; q < K; q++)
+        if (has(q)) {
+          if (slot[q] >= 0) slot_put<COMM>(h + 16ull * slot[q], val[q], tag);
+          ub[q * bw + t] = val[q];
+        }
+      for (int j = t; j < nrecv; j += bw)
+        ub[L + j] = wait(h + 16ull * __ldg(P.grp_rslot + tab->rslot + r0 + j), tag);
+    } else {
+#pragma unroll
+      for (int q = 0; q < K; q++)
+        if (has(q)) ub[q * bw + t] = val[q];
+      if constexpr (COMM == GRP_CLUSTER) {
+        const unsigned h = halo + par * 16u * P.grp_recv_max;
+        for (int j = send0; j < send1; j++) {
+          // reading CTA, its slot, this thread's element
+          const int d = __ldg(P.grp_send + tab->send + j), q = (d >> 24) & 15;
+          double x = val[0];
+#pragma unroll
+          for (int k = 1; k < K; k++)
+            if (k == q) x = val[k];
+          slot_put<COMM>(cluster_map(h + 16u * (d & 0xffff), (d >> 16) & 255), x, tag);
+        }
+        for (int j = t; j < nrecv; j += bw) ub[L + j] = wait(h + 16u * j, tag);
+      }
+    }
+    __syncthreads();
+  }
+
+  // dydt at the thread's q-th element, whose stage value is ui (Sys::rhs)
+  __device__ __forceinline__ double rhs(int q, double ui) const {
+    const int lr = q * bw + t, n = lcnt[lr];
+    const double *ub = ucur();
+    if constexpr (K == 1) {
+      // the row's first entries from registers: one shared-memory latency
+      double x[RN];
+#pragma unroll
+      for (int j = 0; j < RN; j++) x[j] = ub[rc[j]];
+      double d = MIXED ? b[q] : -b[q];
+#pragma unroll
+      for (int j = 0; j < RN; j++)
+        if (j < n) d = fma(rg[j], MIXED ? x[j] : x[j] - ui, d);
+      for (int j = RN; j < n; j++) {
+        const double v = ub[lcol[(long)j * ld + lr]];
+        d = fma(lg[(long)j * ld + lr], MIXED ? v : v - ui, d);
+      }
+      if constexpr (MIXED) return fma(-lG[lr], ui, d);
+      else return d * linv[lr];
+    } else if constexpr (MIXED) {
+      double d = b[q];
+      for (int j = 0; j < n; j++) d = fma(lg[(long)j * ld + lr], ub[lcol[(long)j * ld + lr]], d);
+      return fma(-lG[lr], ui, d);
+    } else {
+      double d = -b[q];
+      for (int j = 0; j < n; j++) d = fma(lg[(long)j * ld + lr], ub[lcol[(long)j * ld + lr]] - ui, d);
+      return d * linv[lr];
+    }
+  }
+
+  // the pairwise tree over the system's elements of x, the same in every thread
+  __device__ __forceinline__ double sum(const double (&x)[K]) {
+    const int lane = t & 31, warp = t >> 5, nw = bw >> 5;
+#pragma unroll
+    for (int q = 0; q < K; q++) {
+      if (q >= rows) break;
+      const int i = at(q);
+      double a = i < nc ? x[q] : 0.0;
+#pragma unroll
+      for (int st = 1; st < 32; st *= 2) {
+        const double o = __shfl_down_sync(0xffffffffu, a, st);
+        if ((lane & (2 * st - 1)) == 0 && i + st < nc) a = a + o;
+      }
+      if (lane == 0) wp[q * nw + warp] = a;
+    }
+    rtag++;
+    __syncthreads();
+    if (warp == 0) {
+      // the parts that the tree goes on with: the CTA's 32-element parts (one
+      // CTA), or every chunk's sum
+      constexpr int VM = COMM == GRP_GRID ? GRID_MAX_BLOCKS / 32 : COMM == GRP_CLUSTER ? 4 : 2;
+      int nb, rr;
+      double v[VM];
+      if constexpr (COMM == GRP_CTA) {
+        nb = (nc + 31) >> 5;
+        rr = nb <= 32 ? 1 : 2;
+#pragma unroll
+        for (int j = 0; j < VM; j++) v[j] = (j < rr && lane * rr + j < nb) ? wp[lane * rr + j] : 0.0;
+      } else {
+        unsigned long long rd;
+        if constexpr (COMM == GRP_GRID) rd = (unsigned long long)(P.grp_red + (long)(rtag & 1u) * GRID_MAX_BLOCKS * 2);
+        else rd = red + (rtag & 1u) * 16u * GRID_MAX_ROWS * G;
+        if (lane < rows) {
+          const int i0 = (chunk0 + lane) * bw;
+          double w[8];
+#pragma unroll
+          for (int j = 0; j < 8; j++) w[j] = j < nw ? wp[lane * nw + j] : 0.0;
+#pragma unroll
+          for (int st = 1; st < 8; st *= 2)
+#pragma unroll
+            for (int j = 0; j + st < 8; j += 2 * st)
+              if (j + st < nw && i0 + (j + st) * 32 < nc) w[j] = w[j] + w[j + st];
+          if constexpr (COMM == GRP_GRID) slot_put<COMM>(rd + 16ull * (chunk0 + lane), w[0], rtag);
+          else wp[lane * nw] = w[0];
+        }
+        if constexpr (COMM == GRP_CLUSTER) {
+          __syncwarp();
+          // one lane a CTA
+          if (lane < G)
+            for (int k = 0; k < rows; k++)
+              slot_put<COMM>(cluster_map((unsigned)rd + 16u * (chunk0 + k), lane), wp[k * nw], rtag);
+        }
+        // each lane takes rr consecutive chunk sums
+        nb = (nc + bw - 1) / bw;
+        rr = nb <= 32 ? 1 : nb <= 64 ? 2 : nb <= 128 ? 4 : 8;
+#pragma unroll
+        for (int j = 0; j < VM; j++) {
+          const int k = lane * rr + j;
+          v[j] = (j < rr && k < nb) ? wait(rd + 16ull * k, rtag) : 0.0;
+        }
+      }
+#pragma unroll
+      for (int st = 1; st < VM; st *= 2) {
+        if (st >= rr) break;
+#pragma unroll
+        for (int j = 0; j + st < VM; j += 2 * st)
+          if (j + st < rr && lane * rr + j + st < nb) v[j] = v[j] + v[j + st];
+      }
+#pragma unroll
+      for (int st = 1; st < 32; st *= 2) {
+        if (st * rr >= nb) break;
+        const double o = __shfl_down_sync(0xffffffffu, v[0], st);
+        if ((lane & (2 * st - 1)) == 0 && (lane + st) * rr < nb) v[0] = v[0] + o;
+      }
+      if (lane == 0) {
+        *res = v[0];
+        s_abort[1] = *(volatile int *)s_abort;
+      }
+    }
+    __syncthreads();
+    return *res;
+  }
+
+  __device__ __forceinline__ double sumsq(const double (&x)[K]) {
+    double q[K];
+#pragma unroll
+    for (int j = 0; j < K; j++) q[j] = x[j] * x[j];
+    return sum(q);
+  }
+
+  // Sys::rkcrho
+  __device__ __forceinline__ void rkcrho() {
+    const double uround = UROUND, sqrtu = sqrt(UROUND);
+    double e[K];
+#pragma unroll
+    for (int q = 0; q < K; q++) e[q] = has(q) ? P.ede[off + at(q)] : 0.0;
+    c.n_rho++;
+    const double ynrm = sqrt(sumsq(yn));
+    const double vnrm = sqrt(sumsq(e));
+    double dynrm, al = 0.0;
+    const bool zy = fpi_is_zero(ynrm), zv = fpi_is_zero(vnrm);
+    dynrm = zy ? uround : ynrm * sqrtu;
+    if (!zv) al = mdiv(dynrm, vnrm);
+#pragma unroll
+    for (int q = 0; q < K; q++)
+      v1[q] = !zy ? (!zv ? fma(al, e[q], yn[q]) : fma(sqrtu, yn[q], yn[q])) : (!zv ? al * e[q] : dynrm);
+    RhoCtl rc;
+    rc.begin(dynrm);
+    for (int iter = 0; iter < RHO_ITMAX; iter++) {
+      c.n_rho_iter++;
+      exchange(v1);
+      double d[K];
+#pragma unroll
+      for (int q = 0; q < K; q++) {
+        d[q] = 0.0;
+        if (has(q)) {
+          v2[q] = rhs(q, v1[q]);
+          const double dm = -1.0 * fn[q] + v2[q];
+          d[q] = dm * dm;
+        }
+      }
+      const double dfnrm = sqrt(sum(d));
+      if (rc.next(iter, dfnrm, c.sprad) == RhoCtl::DONE) {
+#pragma unroll
+        for (int q = 0; q < K; q++)
+          if (has(q)) P.ede[off + at(q)] = -1.0 * yn[q] + v1[q];
+        return;
+      }
+      if (!fpi_is_zero(dfnrm)) {
+        const double a2 = mdiv(dynrm, dfnrm);
+#pragma unroll
+        for (int q = 0; q < K; q++) v1[q] = fma(a2, fn[q] - v2[q], yn[q]);
+      } else {
+        const int idx = iter % nc;
+#pragma unroll
+        for (int q = 0; q < K; q++)
+          if (has(q) && at(q) == idx) v1[q] = 2.0 * yn[q] - v1[q];
+      }
+    }
+    c.idid = 6;
+  }
+
+  // Sys::step, the buffer rotations as moves
+  __device__ __forceinline__ bool step(double h, int m) {
+    if (m > P.coef_mmax) {
+      c.status |= ST_COEF_TABLE;
+      return false;
+    }
+    const double *T = P.coef + P.coef_off[m];
+    const double hm1 = h * __ldg(T);
+#pragma unroll
+    for (int q = 0; q < K; q++) {
+      v2[q] = yn[q];
+      v1[q] = fma(hm1, fn[q], yn[q]);
+    }
+    for (int j = 1; j < m; j++) {
+      const double *p = T + 1 + 5 * (j - 1);
+      const double mu = __ldg(p), nu = __ldg(p + 1), omn = __ldg(p + 2), mus = __ldg(p + 3), ajm1 = __ldg(p + 4);
+      exchange(v1);
+      const double hm = h * mus;
+#pragma unroll
+      for (int q = 0; q < K; q++) {
+        if (q >= rows) break;
+        double out = 0.0;
+        if (has(q)) {
+          const double f = rhs(q, v1[q]);
+          double w = mu * v1[q];
+          w = fma(nu, v2[q], w);
+          w = fma(omn, yn[q], w);
+          out = fma(hm, fma(-ajm1, fn[q], f), w);
+        }
+        // written to y, then (v2, v1, y) <- (v1, y, v2)
+        y[q] = v2[q];
+        v2[q] = v1[q];
+        v1[q] = out;
+      }
+    }
+    // (y, v1, v2) <- (v1, v2, y)
+#pragma unroll
+    for (int q = 0; q < K; q++) {
+      const double w = y[q];
+      y[q] = v1[q];
+      v1[q] = v2[q];
+      v2[q] = w;
+    }
+    c.n_stage += m;
+    return true;
+  }
+
+  // Sys::attempt
+  __device__ __forceinline__ int attempt() {
+    if (c.newspc) {
+      rkcrho();
+      c.jacatt = 1;
+    }
+    double h;
+    int m;
+    if (!c.plan(h, m) || !step(h, m)) return SC::ATT_FAIL;
+    c.n_steps++;
+    exchange(y);
+    const double h04 = 0.4 * h;
+    double d[K];
+#pragma unroll
+    for (int q = 0; q < K; q++) {
+      d[q] = 0.0;
+      if (q >= rows) break;
+      if (has(q)) {
+        const double f = rhs(q, y[q]);
+        v1[q] = f;
+        const double wt = fma(c.tol, abs_max(y[q], yn[q]), c.tol);
+        const double est = fma(h04, fn[q] + f, 0.8 * (yn[q] - y[q]));
+        const double qv = mdiv(est, wt);
+        d[q] = qv * qv;
+      }
+    }
+    const int a = c.judge(norm(sum(d)), h);
+    if (a == SC::ATT_ACCEPT) {
+      // (v2, fn, v1, yn, y) <- (fn, v1, yn, y, v2)
+#pragma unroll
+      for (int q = 0; q < K; q++) {
+        const double w = v2[q];
+        v2[q] = fn[q];
+        fn[q] = v1[q];
+        v1[q] = yn[q];
+        yn[q] = y[q];
+        y[q] = w;
+      }
+    }
+    return a;
+  }
+
+  // sqrt(e / nc); a division by a power of two is an exact scaling
+  __device__ __forceinline__ double norm(double e) const {
+    if ((nc & (nc - 1)) == 0) return sqrt(e * __longlong_as_double((long long)(1023 - (__ffs(nc) - 1)) << 52));
+    return sqrt(div_by(e, rnc));
+  }
+
+  // Sys::ion_and_b.  The elements go through shared memory so that the ion
+  // update's code stands once, not K times.  (Every reader of both stage
+  // buffers is done: a sum's barriers, or bind's, lie between.)
+  __device__ __forceinline__ void ion_and_b(double sum_dt, bool update_ion, bool with_gap) {
+    const bool gap = CT == IO && with_gap && P.sys_ngap[s] > 0;
+    if (gap) {
+      // the gap currents read the receiving and sending dendrites' elem v,
+      // which this update sets to y
+      exchange(y);
+    } else {
+      double *ub = u + ((tag + 1u) & 1u) * ustride();
+#pragma unroll
+      for (int q = 0; q < K; q++)
+        if (has(q)) ub[q * bw + t] = y[q];
+    }
+    const double *yb = gap ? ucur() : u + ((tag + 1u) & 1u) * ustride();
+    double *bb = u + (gap ? (tag + 1u) & 1u : tag & 1u) * ustride();
+    const long ncp = (nc + 1) & ~1;
+    double *wsb = P.ws + P.sys_ws[s] + WS_B * ncp;
+#pragma unroll 1
+    for (int q = 0; q < K; q++) {
+      if (!has(q)) break;
+      const int lr = q * bw + t, i = at(q);
+      double x = comp_ion_b<CT, R>(P, off + i, yb[lr], sum_dt, update_ion);
+      const int cell = i / ncomp, e0g = P.sys_gap0[s] + 4 * cell;
+      if (gap && i == P.gap_post[e0g]) {
+        // per receiving dendrite its four edges in order (io_gap_update +
+        // add_io_gap_val)
+        for (int k = 0; k < 4; k++) {
+          int pre;
+          if constexpr (COMM == GRP_CTA) pre = P.gap_pre[e0g + k];
+          else pre = P.grp_gap[e0g + k];
+          const double diff = pre >= 0 ? yb[lr] - yb[pre] : 0.0;
+          x += io_gap_current(P.gap_g[e0g + k], diff);
+        }
+      }
+      bb[lr] = x;
+      wsb[i] = x;
+    }
+#pragma unroll
+    for (int q = 0; q < K; q++)
+      if (has(q)) set_b(q, bb[q * bw + t]);
+    if (update_ion) c.n_ion++;
+  }
+
+  // Sys::initialize
+  __device__ __forceinline__ void initialize() {
+#pragma unroll
+    for (int q = 0; q < K; q++) {
+      v1[q] = v2[q] = 0.0;
+      if (has(q)) {
+        const double v0 = P.v[off + at(q)];
+        P.vnew[off + at(q)] = v0;
+        y[q] = yn[q] = v0;
+      }
+    }
+    ion_and_b(0.0, false, false);
+    exchange(yn);
+#pragma unroll
+    for (int q = 0; q < K; q++)
+      if (has(q)) {
+        fn[q] = rhs(q, yn[q]);
+        P.ede[off + at(q)] = fn[q];
+      }
+    rkcrho();
+    // set_initial_absh (solve_rkc.cu:493-560)
+    double absh = H_MAX;
+    if (c.sprad * absh > 1.0) absh = 1.0 / c.sprad;
+    absh = (absh > c.hmin) ? absh : c.hmin;
+#pragma unroll
+    for (int q = 0; q < K; q++) v1[q] = fma(absh, fn[q], yn[q]);
+    exchange(v1);
+    double d[K];
+#pragma unroll
+    for (int q = 0; q < K; q++) {
+      d[q] = 0.0;
+      if (has(q)) {
+        v2[q] = rhs(q, v1[q]);
+        const double wt = fma(c.tol, fabs(yn[q]), c.tol);
+        const double dm = (v2[q] - fn[q]) * (1.0 / wt);
+        d[q] = dm * dm;
+      }
+    }
+    double est = sum(d);
+    est = absh * sqrt(est / nc);
+    if (0.1 * absh < H_MAX * sqrt(est)) {
+      const double a2 = 0.1 * absh / sqrt(est);
+      absh = (a2 > c.hmin) ? a2 : c.hmin;
+    } else {
+      absh = H_MAX;
+    }
+    c.absh = absh;
+    const double x = sqrt(c.tol / (10.0 * UROUND));
+    c.mmax = (x - (double)(int)x < 0.5) ? (int)x : (int)(x + 0.9);
+  }
+
+  // Sys::begin_interval; every thread sees to its own elements
+  __device__ __forceinline__ int begin_interval(double tb) {
+    if (P.stim_on) {
+#pragma unroll
+      for (int q = 0; q < K; q++)
+        if (has(q)) {
+          const int i = at(q), cell = i / ncomp, pc = cell0 + cell;
+          if (P.stim_comp[pc] == i - cell * ncomp) {
+            P.iext[off + i] = 0;
+            if (P.stim_t0[pc] <= tb && tb < P.stim_t1[pc]) P.iext[off + i] = P.stim_amp[pc];
+          }
+        }
+    }
+    if (P.syn_mode == SYN_BUFFERED || P.syn_mode == SYN_BUFFERED_DECAY) {
+#pragma unroll
+      for (int q = 0; q < K; q++)
+        if (has(q)) {
+          const long gi = off + at(q);
+          double acc = 0.0;
+          for (int k = P.syn_row[gi]; k < P.syn_row[gi + 1]; k++) {
+            const int sid = P.syn_idx[k];
+            acc = acc + P.syn_val[sid] * (y[q] - P.syn_e[sid]);
+          }
+          P.syn_buf[gi] = acc;
+        }
+    }
+    attempts0 = c.n_steps;
+    c.rej_run = 0;
+    return fpi_is_zero(c.sum_dt) ? TICK_MORE : TICK_ION;
+  }
+
+  // rkcint at the interval's end, the soma record and the raster, each by the
+  // thread that owns the element
+  __device__ __forceinline__ void end_interval() {
+    double a1, a2, b1, b2;
+    c.dense(a1, a2, b1, b2);
+    const double tend = t0 + (k_iv + 1) * H_MAX;
+#pragma unroll
+    for (int q = 0; q < K; q++)
+      if (has(q)) {
+        const int i = at(q), gi = off + i, pc = cell0 + i / ncomp;
+        const double x = fma(b2, fn[q], fma(b1, v2[q], fma(a2, yn[q], a1 * v1[q])));
+        P.vnew[gi] = x;
+        if (P.soma_out) {
+          const int k = gi - P.cell_soma[pc];
+          if (k >= 0 && k < P.rec_w) P.soma_out[((long)(iv0 + k_iv) * P.ncell_pool + pc) * P.rec_w + k] = x;
+        }
+        if (P.spk_prev && gi == P.cell_spk[pc]) log_spike(P, pc, tend);
+      }
+    c.tend += H_MAX;
+    if (c.iv_left > 0) c.iv_left--;
+  }
+
+  __device__ __forceinline__ int start(double tb, int n, int iv0_global) {
+    if (c.iv_left >= 0 && n > c.iv_left) n = c.iv_left;
+    t0 = tb;
+    n_iv = n;
+    iv0 = iv0_global;
+    k_iv = 0;
+    rnc = recip((double)nc);
+    if (c.status != 0 || n <= 0) return TICK_DONE;
+    return begin_interval(t0);
+  }
+
+  // Sys::tick
+  __device__ __forceinline__ int tick() {
+    const int a = attempt();
+    if (a == SC::ATT_REJECT) return TICK_MORE;
+    if (a == SC::ATT_FAIL) return TICK_DONE;
+    if (c.n_steps - attempts0 > STEPS_PER_INTERVAL_CAP) {
+      c.status |= ST_LOOP_CAP;
+      return TICK_DONE;
+    }
+    const bool due = c.clock(CT == GO || CT == PKJ);
+    if (!c.last) return due ? TICK_ION : TICK_MORE;
+    end_interval();
+    if (++k_iv >= n_iv) return TICK_DONE;
+    return begin_interval(t0 + k_iv * H_MAX);
+  }
+
+  // Advance the system by n intervals from tb, or initialise it.
+  __device__ __forceinline__ void run(int s_, double tb, int n, int iv0_global, bool init) {
+    if (!system_selected(P.ctl[s_], init, n)) return;
+    if (t == 0) s_abort[0] = s_abort[1] = 0;
+    bind(s_);
+    if (init) {
+      initialize();
+      c.status &= ~ST_INIT;
+      if (s_abort[1]) c.status |= ST_BARRIER;
+    } else {
+      int r = start(tb, n, iv0_global);
+      if (r == TICK_DONE) return;
+      while (r != TICK_DONE) {
+        if (r == TICK_ION) {
+          ion_and_b(c.sum_dt, true, true);
+          c.sum_dt = 0.0;
+          r = TICK_MORE;
+        } else {
+          r = tick();
+          if (s_abort[1]) {
+            c.status |= ST_BARRIER;
+            break;
+          }
+        }
+      }
+    }
+    store(init);
+  }
+};
+
+}  // namespace gbrkc

@@ -45,7 +45,7 @@ struct WVec {
 // a slot offset (vec_at) and gives the slot length for ncp elements
 // (vstride).  CLUSTER > 0 marks a team spread over a thread-block cluster.
 struct BlockTeam {
-  static constexpr int LS = 1, NCF = 0, CLUSTER = 0, GRID = 0;
+  static constexpr int LS = 1, NCF = 0, CLUSTER = 0;
   typedef WVec<1> Vec;
   __device__ __forceinline__ Vec vec_at(double *W, long off) const { return Vec{W + off}; }
   __device__ __forceinline__ static long vstride(int ncp) { return ncp; }
@@ -56,7 +56,7 @@ struct BlockTeam {
 
 template <int T>
 struct TileTeam {
-  static constexpr int LS = 1, NCF = 0, CLUSTER = 0, GRID = 0;
+  static constexpr int LS = 1, NCF = 0, CLUSTER = 0;
   typedef WVec<1> Vec;
   __device__ __forceinline__ Vec vec_at(double *W, long off) const { return Vec{W + off}; }
   __device__ __forceinline__ static long vstride(int ncp) { return ncp; }
@@ -76,7 +76,7 @@ struct TileTeam {
 // would otherwise serialise the loop) and the pairwise sums run in registers.
 template <int BLOCK, int NCF_ = 0>
 struct LaneTeam {
-  static constexpr int LS = BLOCK, NCF = NCF_, CLUSTER = 0, GRID = 0;
+  static constexpr int LS = BLOCK, NCF = NCF_, CLUSTER = 0;
   typedef WVec<BLOCK> Vec;
   __device__ __forceinline__ Vec vec_at(double *W, long off) const { return Vec{W + off * BLOCK}; }
   __device__ __forceinline__ static long vstride(int ncp) { return ncp; }
@@ -108,7 +108,7 @@ struct CVec {
 template <int C>
 struct ClusterTeam {
   static_assert((C & (C - 1)) == 0 && C <= 16, "cluster size must be a power of two up to 16");
-  static constexpr int LS = 1, NCF = 0, CLUSTER = C, GRID = 0;
+  static constexpr int LS = 1, NCF = 0, CLUSTER = C;
   typedef CVec<C> Vec;
   int crank;                   // this CTA's rank in the cluster
   double *const *bases;        // [C] workspace bases (distributed shared memory)
@@ -123,132 +123,6 @@ struct ClusterTeam {
   __device__ __forceinline__ void sync() const {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   }
-};
-
-// One system over every CTA of a cooperative launch (GridTeam): the
-// workspace stays in global memory (the L2 holds it), element i is owned by
-// thread i mod (gridDim * grid_bw) among each CTA's first grid_bw threads,
-// and the team barrier is a software grid barrier: every CTA adds one to a
-// counter (a reduction, no reply awaited) and polls it with acquire loads
-// until it reaches gridDim times the CTA's own barrier count.  The wait is
-// bounded: a CTA that waits more than GRID_SPIN_LIMIT polls raises the abort
-// flag, after which no barrier waits and every CTA leaves its system at the
-// next tick (status ST_BARRIER); the host reads the flag after the launch.
-// A cooperative launch makes every CTA co-resident, so the bound is a guard,
-// not a schedule.
-constexpr long GRID_SPIN_LIMIT = 1L << 22;
-
-__device__ __forceinline__ unsigned long long ld_acquire_gpu(const unsigned long long *p) {
-  unsigned long long v;
-  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
-}
-
-// epoch: this CTA's barrier count (shared memory, only thread 0 uses it).
-// light: order the arrival with fence.acq_rel.gpu and rely on the acquire
-// polls (the CTA's barrier carries both to its other threads); else
-// fence.sc.gpu (__threadfence) before the arrival and after the wait.
-__device__ __forceinline__ void grid_barrier(GridBarrier *b, unsigned long long *epoch, int light) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    volatile GridBarrier *vb = b;
-    if (!vb->abort) {
-      const unsigned long long target = (*epoch += 1) * gridDim.x;
-      if (light)
-        asm volatile("fence.acq_rel.gpu;" ::: "memory");
-      else
-        __threadfence();
-      asm volatile("red.relaxed.gpu.global.add.u64 [%0], 1;" ::"l"(&b->count) : "memory");
-      long it = 0;
-      while (ld_acquire_gpu(&b->count) < target) {
-        if (++it > GRID_SPIN_LIMIT || vb->abort) {
-          atomicExch(&b->abort, 1);
-          break;
-        }
-        if (it > 64) __nanosleep(32);
-      }
-      if (!light) __threadfence();
-    }
-  }
-  __syncthreads();
-}
-
-// The grid team's stage barrier (grid_local_barrier): between the stages of
-// one step a CTA reads only the elements of the CTAs that own its rows'
-// neighbours (the operator is symmetric, so those are also the CTAs that
-// read its elements), so it waits for those alone.  Each CTA publishes its
-// stage count in its own flag (a release store on a 128-byte line) and warp
-// 0's lanes poll the neighbours' flags with acquire loads, one flag a lane.
-// nbr[b * (GRID_MAX_NBR + 1)] is CTA b's neighbour count, followed by the
-// neighbours.  The wait is bounded like grid_barrier's and raises the same
-// abort flag.
-__device__ __forceinline__ void grid_local_barrier(GridBarrier *b, unsigned long long *flags, const int *nbr,
-                                                   unsigned long long *lepoch) {
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    volatile GridBarrier *vb = b;
-    if (!vb->abort) {
-      const int lane = threadIdx.x;
-      unsigned long long k = 0;
-      if (lane == 0) {
-        k = (*lepoch += 1);
-        asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(flags + (long)blockIdx.x * 16), "l"(k)
-                     : "memory");
-      }
-      k = __shfl_sync(0xffffffffu, k, 0);
-      const int *my = nbr + (long)blockIdx.x * (GRID_MAX_NBR + 1);
-      if (lane < my[0]) {
-        const unsigned long long *f = flags + (long)my[1 + lane] * 16;
-        long it = 0;
-        while (ld_acquire_gpu(f) < k) {
-          if (++it > GRID_SPIN_LIMIT || vb->abort) {
-            atomicExch(&b->abort, 1);
-            break;
-          }
-          if (it > 64) __nanosleep(32);
-        }
-      }
-      __syncwarp();
-    }
-  }
-  __syncthreads();
-}
-
-struct GridTeam {
-  static constexpr int LS = 1, NCF = 0, CLUSTER = 0, GRID = 1;
-  typedef WVec<1> Vec;
-  GridBarrier *bar;
-  double *red;                 // [2][GRID_MAX_BLOCKS] chunk sums (global)
-  double *wp;                  // [GRID_MAX_ROWS][8] warp partials (shared)
-  double *res;                 // the reduction's result (shared)
-  unsigned long long *epoch;   // this CTA's barrier count (shared)
-  int bw;                      // threads of each CTA that own elements
-  int light;                   // the barrier's fences (grid_barrier)
-  // the CTA's operator rows in shared memory (maxdeg 0: none): row slot
-  // k * bw + t holds thread t's k-th element's entries
-  int maxdeg;
-  double *linv, *lg;           // [rl] 1/Cm, [rl * maxdeg] conductances
-  int *lcnt, *lcol;            // [rl] entry counts, [rl * maxdeg] columns (system-wide)
-  // stage barriers with the neighbouring CTAs only (nbr null: the grid barrier)
-  const int *nbr;
-  unsigned long long *flags;   // [gridDim * 16] stage counts, one 128-byte line a CTA
-  unsigned long long *lepoch;  // this CTA's stage-barrier count (shared)
-  __device__ __forceinline__ Vec vec_at(double *W, long off) const { return Vec{W + off}; }
-  __device__ __forceinline__ static long vstride(int ncp) { return ncp; }
-  // (the CTA has bw threads; a thread past bw would own nothing: a rank no
-  // loop over the elements reaches)
-  __device__ __forceinline__ int rank() const {
-    return (int)threadIdx.x < bw ? (int)blockIdx.x * bw + (int)threadIdx.x : 0x3fffffff;
-  }
-  __device__ __forceinline__ int size() const { return (int)gridDim.x * bw; }
-  __device__ __forceinline__ void sync() const { grid_barrier(bar, epoch, light); }
-  __device__ __forceinline__ void sync_stage() const {
-    if (nbr)
-      grid_local_barrier(bar, flags, nbr, lepoch);
-    else
-      grid_barrier(bar, epoch, light);
-  }
-  __device__ __forceinline__ bool aborted() const { return ((volatile GridBarrier *)bar)->abort != 0; }
 };
 
 // pairwise tree over a[0..N) in registers, the same order as Sys::tree_sum
@@ -441,48 +315,8 @@ struct Sys {
   __device__ __forceinline__ V bvec() const { return tm.vec_at(W, (long)WS_B * Team::vstride(ncp)); }
   __device__ __forceinline__ V scratch() const { return tm.vec_at(W, (long)WS_SCRATCH * Team::vstride(ncp)); }
 
-  // Grid team: copy this CTA's rows of the operator (the rows of the
-  // elements its threads own, each thread its own) into shared memory, so
-  // that a stage's dydt reads only the neighbours' values from L2.
-  __device__ __forceinline__ void grid_rows_in() const {
-    if constexpr (Team::GRID > 0) {
-      if (tm.maxdeg == 0) return;
-      const int md = tm.maxdeg;
-      for (int i = tm.rank(), k = 0; i < nc; i += tm.size(), k++) {
-        int j = i, base = 0;
-        if (!(csr || ncell == 1)) {
-          const int cidx = i / ncomp;
-          j = i - cidx * ncomp;
-          base = cidx * ncomp;
-        }
-        const int lr = k * tm.bw + (int)threadIdx.x;
-        const int r0 = __ldg(row + j), r1 = __ldg(row + j + 1);
-        tm.lcnt[lr] = r1 - r0;
-        tm.linv[lr] = __ldg(invcm + j);
-        for (int q = 0; q < r1 - r0; q++) {
-          tm.lcol[lr * md + q] = base + __ldg(col + r0 + q);
-          tm.lg[lr * md + q] = __ldg(g + r0 + q);
-        }
-      }
-    }
-  }
-
   // dydt at compartment i (solve_rkc.cu:178-196): (-b + sum g (y_j - y_i)) / Cm
   __device__ __forceinline__ double rhs(const V y, int i) const {
-    if constexpr (Team::GRID > 0) {
-      if (tm.maxdeg > 0) {
-        // i is the calling thread's element: i = k * size + blockIdx * bw + t
-        const int size = tm.size(), k = i / size;
-        const int lr = k * tm.bw + (i - k * size - (int)blockIdx.x * tm.bw);
-        double d = -(bvec()[i]);
-        const double yi = y[i];
-        const int n = tm.lcnt[lr];
-        const int *cc = tm.lcol + lr * tm.maxdeg;
-        const double *gg = tm.lg + lr * tm.maxdeg;
-        for (int q = 0; q < n; q++) d = fma(gg[q], y[cc[q]] - yi, d);
-        return d * tm.linv[lr];
-      }
-    }
     if constexpr (!std::is_same<R, double>::value) {
       // mixed precision: -b / Cm + sum (g / Cm) y_j - (sum g / Cm) y_i, the
       // same operator with one FP64 operation fewer per entry (the rounding
@@ -518,7 +352,6 @@ struct Sys {
   // pairwise tree over a[0..n): stride doubling, identical to the oracle
   __device__ __forceinline__ double tree_sum(const V a, int n) const {
     if constexpr (Team::CLUSTER > 0) return cluster_tree_sum(a, n);
-    if constexpr (Team::GRID > 0) return grid_tree_sum(a, n);
     tm.sync();
     for (int stride = 1; stride < n; stride *= 2) {
       const int step = 2 * stride;
@@ -601,85 +434,6 @@ struct Sys {
     }
     __syncthreads();
     return *res;
-  }
-
-  // tree_sum on a grid team: the pairwise tree's additions in the same order.
-  // Element i is owned by the thread that writes it in the team loops, so the
-  // aligned chunk of bw elements (a power of two) starting at row k, CTA b
-  // (chunk index k * gridDim + b) lies in CTA b, one element per thread:
-  // levels 0-4 are warp shuffles, the next combine the chunk's bw / 32 warp
-  // partials, the chunk sum goes to global memory, and after one grid barrier
-  // warp 0 of every CTA combines all chunk sums (the remaining levels), every
-  // CTA computing the same value.  The chunk sums are double-buffered, as on
-  // a cluster.
-  __device__ __forceinline__ double grid_tree_sum(const V a, int n) const {
-    if constexpr (Team::GRID > 0) {
-      constexpr int RR = GRID_MAX_BLOCKS / 32;
-      const int t = threadIdx.x, lane = t & 31, warp = t >> 5, b = blockIdx.x, G = gridDim.x;
-      const int B = tm.bw, nw = B >> 5;
-      const int size = G * B;
-      const int rows = (n + size - 1) / size;
-      double *red = tm.red, *wp = tm.wp;
-      const int buf = red_buf;
-      red_buf ^= 1;
-      if (t < B) {
-        for (int k = 0; k < rows; k++) {
-          const int i0 = k * size + b * B;
-          if (i0 >= n) break;
-          const int i = i0 + t;
-          double x = (i < n) ? a[i] : 0.0;
-#pragma unroll
-          for (int st = 1; st < 32; st *= 2) {
-            const double y = __shfl_down_sync(0xffffffffu, x, st);
-            if ((lane & (2 * st - 1)) == 0 && i + st < n) x = x + y;
-          }
-          if (lane == 0) wp[k * 8 + warp] = x;
-        }
-      }
-      __syncthreads();
-      if (t < rows) {
-        const int i0 = t * size + b * B;
-        if (i0 < n) {
-          double w[8];
-#pragma unroll
-          for (int j = 0; j < 8; j++) w[j] = (j < nw) ? wp[t * 8 + j] : 0.0;
-#pragma unroll
-          for (int st = 1; st < 8; st *= 2)
-#pragma unroll
-            for (int j = 0; j + st < 8; j += 2 * st)
-              if (j + st < nw && i0 + (j + st) * 32 < n) w[j] = w[j] + w[j + st];
-          red[buf * GRID_MAX_BLOCKS + t * G + b] = w[0];
-        }
-      }
-      tm.sync();
-      if (warp == 0) {
-        const int nb = (n + B - 1) / B;
-        double v[RR];
-#pragma unroll
-        for (int r = 0; r < RR; r++) {
-          const int j = lane + 32 * r;
-          v[r] = (j < nb) ? __ldcg(red + buf * GRID_MAX_BLOCKS + j) : 0.0;
-        }
-#pragma unroll
-        for (int st = 1; st < 32; st *= 2)
-#pragma unroll
-          for (int r = 0; r < RR; r++) {
-            if (32 * r >= nb) break;
-            const double y = __shfl_down_sync(0xffffffffu, v[r], st);
-            if ((lane & (2 * st - 1)) == 0 && lane + 32 * r + st < nb) v[r] = v[r] + y;
-          }
-#pragma unroll
-        for (int st = 1; st < RR; st *= 2)
-#pragma unroll
-          for (int r = 0; r + st < RR; r += 2 * st)
-            if (32 * (r + st) < nb) v[r] = v[r] + v[r + st];
-        if (lane == 0) *tm.res = v[0];
-      }
-      __syncthreads();
-      return *tm.res;
-    } else {
-      return 0.0;
-    }
   }
 
   template <class A>
@@ -787,15 +541,6 @@ struct Sys {
     c.idid = 6;
   }
 
-  // the barrier between a step's stages: a stage reads its rows'
-  // neighbours only, so a grid team waits for the CTAs that own them
-  __device__ __forceinline__ void stage_sync() const {
-    if constexpr (Team::GRID > 0)
-      tm.sync_stage();
-    else
-      tm.sync();
-  }
-
   // ----------------------------------------------------------------- step
   __device__ __forceinline__ bool step(double h, int m) {
     if (m > P.coef_mmax) {
@@ -825,7 +570,7 @@ struct Sys {
         }
       }
     }
-    stage_sync();
+    tm.sync();
     for (int j = 1; j < m; j++) {
       const double *q = T + 1 + 5 * (j - 1);
       const double mu = __ldg(q), nu = __ldg(q + 1), omn = __ldg(q + 2), mus = __ldg(q + 3), ajm1 = __ldg(q + 4);
@@ -858,7 +603,7 @@ struct Sys {
       c.map[LV2] = c.map[LV1];
       c.map[LV1] = c.map[LY];
       c.map[LY] = t2;
-      stage_sync();
+      tm.sync();
     }
     const int t3 = c.map[LY];
     c.map[LY] = c.map[LV1];
@@ -993,11 +738,7 @@ struct Sys {
     c.errold = err;
     c.hold = h;
     c.idid = c.last ? 1 : 2;
-    // A grid team skips this barrier: every thread reads and writes only its
-    // own elements until the next step's first barrier, the error norm's
-    // grid barrier has already ordered every neighbour read of this attempt,
-    // and its chunk sums are double-buffered.
-    if constexpr (Team::GRID == 0) tm.sync();
+    tm.sync();
     return ATT_ACCEPT;
   }
 
@@ -1235,21 +976,12 @@ __device__ __forceinline__ void run_system(const PoolView<R> &P, const Team &tm,
   if (P.ws_in_smem) ws_in(tm, W, gws, wsn);
   Sys<CT, R, Team> S(P, tm, s, W);
   S.c = P.ctl[s];
-  S.grid_rows_in();
   if (init) {
     S.initialize();
     S.c.status &= ~ST_INIT;
-    if constexpr (Team::GRID > 0)
-      if (tm.aborted()) S.c.status |= ST_BARRIER;
   } else {
     int r = S.start(t0, n_iv, iv0_global);
     while (r != TICK_DONE) {
-      if constexpr (Team::GRID > 0) {
-        if (tm.aborted()) {
-          S.c.status |= ST_BARRIER;
-          break;
-        }
-      }
       if (r == TICK_ION) {
         S.ion_due();
         r = TICK_MORE;

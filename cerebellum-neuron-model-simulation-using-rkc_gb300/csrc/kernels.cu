@@ -1,97 +1,17 @@
 #include <type_traits>
-// The advance kernels.  k_advance: one launch advances every system of one
-// pool by n_iv output intervals (or initialises them), entirely on the
-// device.  Single lanes take the tiniest systems (one system per thread),
-// teams of 4 or 32 lanes small ones; a whole block takes one large system at
-// a time and loops over its share of systems.  k_mega: one persistent launch
-// for all pools, every CTA a role pulling systems from its role's queue.
+// k_mega: one persistent launch for all pools, every CTA a role pulling
+// systems from its role's queue; and the launches of it and of the per-pool
+// kernels (kernels_pool.cu).
 //
 // Built with -fmad=false (see integrator.cuh).  R selects FP64 or FP32
 // gating; the instantiations live in kernels_fp64.cu / kernels_fp32.cu.
 #include <algorithm>
-#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include "integrator.cuh"
 #include "quad_sys.cuh"
 
 namespace gbrkc {
-
-template <int CT, typename R, int TS>
-__global__ void __launch_bounds__(256, 1) k_advance(const __grid_constant__ PoolView<R> P, double t0, int n_iv,
-                                                 int iv0, int init) {
-  extern __shared__ __align__(16) double smem[];
-  if (TS == TEAM_THREAD || TS == TEAM_LANE4) {
-    // the first `per` systems of warp w of block b start at system
-    // per (w * grid + b): the first warps of every block are filled before
-    // any block's later warps
-    const bool quads = TS == TEAM_LANE4 && !init && n_iv > 0;
-    const int per = quads ? P.per_warp : P.lanes, lane = (int)threadIdx.x & 31;
-    const int first = (((int)threadIdx.x >> 5) * (int)gridDim.x + (int)blockIdx.x) * per + (quads ? lane >> 2 : lane);
-    const int stride = (int)gridDim.x * (MEGA_BLOCK / 32) * per;
-    if constexpr (TS == TEAM_LANE4) {
-      if (quads)
-        run_quads<CT, R>(P, nullptr, first, stride, per, t0, n_iv, iv0);
-      else
-        run_lanes<CT, R, MEGA_BLOCK, 4>(P, nullptr, first, stride, smem, t0, n_iv, iv0, init != 0);
-    } else {
-      run_lanes<CT, R, MEGA_BLOCK>(P, nullptr, first, stride, smem, t0, n_iv, iv0, init != 0);
-    }
-  } else if (TS == TEAM_BLOCK) {
-    BlockTeam tm;
-    for (int s = blockIdx.x; s < P.nsys; s += gridDim.x) {
-      run_system<CT, R, BlockTeam>(P, tm, s, smem, t0, n_iv, iv0, init != 0);
-      __syncthreads();
-    }
-  } else {
-    constexpr int T = TS > 0 ? TS : 1;
-    const int tiles = blockDim.x / T, tile = threadIdx.x / T;
-    TileTeam<TS> tm;
-    tm.r = threadIdx.x % T;
-    tm.mask = (T == 32) ? 0xffffffffu : (((1u << T) - 1u) << ((threadIdx.x & 31) / T * T));
-    double *my = smem + (long)tile * P.ws_tile_doubles;
-    for (int s = blockIdx.x * tiles + tile; s < P.nsys; s += gridDim.x * tiles)
-      run_system<CT, R, TileTeam<TS>>(P, tm, s, my, t0, n_iv, iv0, init != 0);
-  }
-}
-
-// One large system per thread-block cluster of C CTAs (ClusterTeam): the
-// cluster takes systems cid, cid + nclusters, ...
-template <int CT, typename R, int C>
-__global__ void __launch_bounds__(CLUSTER_BLOCK, 1) k_advance_cluster(const __grid_constant__ PoolView<R> P, double t0,
-                                                                       int n_iv, int iv0, int init) {
-  namespace cg = cooperative_groups;
-  extern __shared__ __align__(16) double smem[];
-  __shared__ double *s_bases[C];
-  cg::cluster_group cl = cg::this_cluster();
-  if (threadIdx.x < C) s_bases[threadIdx.x] = cl.map_shared_rank(smem, (int)threadIdx.x);
-  cl.sync();
-  const ClusterTeam<C> tm{(int)cl.block_rank(), s_bases, P.ws_tile_doubles};
-  const int ncl = gridDim.x / C, cid = blockIdx.x / C;
-  for (int s = cid; s < P.nsys; s += ncl) run_system<CT, R, ClusterTeam<C>>(P, tm, s, smem, t0, n_iv, iv0, init != 0);
-  // no CTA leaves while a peer may still reach its shared memory
-  cl.sync();
-}
-
-// One large system over every CTA of a cooperative launch (GridTeam): all
-// CTAs take the pool's systems one after another.
-template <int CT, typename R>
-__global__ void __launch_bounds__(GRID_BLOCK, 1) k_advance_grid(const __grid_constant__ PoolView<R> P, double t0,
-                                                                 int n_iv, int iv0, int init) {
-  extern __shared__ __align__(16) double grid_smem[];
-  __shared__ double s_wp[GRID_MAX_ROWS * 8];
-  __shared__ double s_res;
-  __shared__ unsigned long long s_epoch, s_lepoch;
-  if (threadIdx.x == 0) s_epoch = s_lepoch = 0;     // counter and flags are zeroed before every launch
-  __syncthreads();
-  // the operator rows' copy: [rl] 1/Cm, [rl * maxdeg] g, [rl] counts, [rl * maxdeg] columns
-  const long rl = P.grid_rl, md = P.grid_maxdeg;
-  double *linv = grid_smem, *lg = grid_smem + rl;
-  int *lcnt = (int *)(lg + rl * md), *lcol = lcnt + rl;
-  const GridTeam tm{(GridBarrier *)P.grid_bar, P.grid_red, s_wp, &s_res, &s_epoch, P.grid_bw, P.grid_light,
-                    P.grid_maxdeg, linv, lg, lcnt, lcol, P.grid_nbr, P.grid_flags, &s_lepoch};
-  for (int s = 0; s < P.nsys; s++) run_system<CT, R, GridTeam>(P, tm, s, nullptr, t0, n_iv, iv0, init != 0);
-}
 
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;
@@ -191,30 +111,13 @@ int launch_mega(const MegaView<R> &M, int grid, size_t smem, void *stream, doubl
   return (int)e;
 }
 
-template <int CT, typename R>
-static const void *kernel_for(int team) {
-  switch (team) {
-    case TEAM_GRID: return (const void *)k_advance_grid<CT, R>;
-    case TEAM_CLUSTER8: return (const void *)k_advance_cluster<CT, R, 8>;
-    case TEAM_CLUSTER16: return (const void *)k_advance_cluster<CT, R, 16>;
-    case TEAM_LANE4:
-      // instantiated for granule pools only (the others never have it)
-      if constexpr (CT == GR) return (const void *)k_advance<CT, R, TEAM_LANE4>;
-      return (const void *)k_advance<CT, R, TEAM_THREAD>;
-    case TEAM_THREAD: return (const void *)k_advance<CT, R, TEAM_THREAD>;
-    case TEAM_TILE4: return (const void *)k_advance<CT, R, TEAM_TILE4>;
-    case TEAM_WARP: return (const void *)k_advance<CT, R, TEAM_WARP>;
-    default: return (const void *)k_advance<CT, R, TEAM_BLOCK>;
-  }
-}
-
 template <typename R>
 static const void *kernel_ptr(int type, int team) {
   switch (type) {
-    case GR: return kernel_for<GR, R>(team);
-    case GO: return kernel_for<GO, R>(team);
-    case PKJ: return kernel_for<PKJ, R>(team);
-    default: return kernel_for<IO, R>(team);
+    case GR: return pool_kernel<GR, R>(team);
+    case GO: return pool_kernel<GO, R>(team);
+    case PKJ: return pool_kernel<PKJ, R>(team);
+    default: return pool_kernel<IO, R>(team);
   }
 }
 
@@ -225,22 +128,22 @@ int prepare_pool_kernel(int type, int team, size_t smem) {
     cudaError_t e = raise_smem_limit(k, smem);
     if (e != cudaSuccess) return (int)e;
   }
-  if (team_cluster_size(team) > 8) {
+  if (team_cluster_size(team) > 8 || team_is_clu(team)) {
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return (int)e;
   }
   return 0;
 }
 
-static cudaLaunchConfig_t cluster_config(int team, int grid, size_t smem, cudaStream_t stream,
+static cudaLaunchConfig_t cluster_config(int size, int grid, int block, size_t smem, cudaStream_t stream,
                                          cudaLaunchAttribute *attr) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(CLUSTER_BLOCK);
+  cfg.blockDim = dim3(block);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = team_cluster_size(team);
+  attr[0].val.clusterDim.x = size;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
@@ -257,7 +160,7 @@ int grid_capacity(int type) {
   cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (!coop) return 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kernel_ptr<R>(type, TEAM_GRID), GRID_BLOCK, 0) !=
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kernel_ptr<R>(type, TEAM_GRID8), GRID_BLOCK, 0) !=
       cudaSuccess) {
     cudaGetLastError();
     return 0;
@@ -271,8 +174,25 @@ int cluster_capacity(int type, int team, size_t smem) {
     cudaGetLastError();
     return 0;
   }
+  const int size = team_cluster_size(team);
   cudaLaunchAttribute attr[1];
-  const cudaLaunchConfig_t cfg = cluster_config(team, team_cluster_size(team), smem, 0, attr);
+  const cudaLaunchConfig_t cfg = cluster_config(size, size, CLUSTER_BLOCK, smem, 0, attr);
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kernel_ptr<R>(type, team), &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return n;
+}
+
+template <typename R>
+int group_capacity(int type, int team, int ctas, int block, size_t smem) {
+  if (prepare_pool_kernel<R>(type, team, smem) != 0) {
+    cudaGetLastError();
+    return 0;
+  }
+  cudaLaunchAttribute attr[1];
+  const cudaLaunchConfig_t cfg = cluster_config(ctas, ctas, block, smem, 0, attr);
   int n = 0;
   if (cudaOccupancyMaxActiveClusters(&n, kernel_ptr<R>(type, team), &cfg) != cudaSuccess) {
     cudaGetLastError();
@@ -287,7 +207,7 @@ int launch_pool(int type, const PoolView<R> &P, int team, int grid, int block, s
   const void *k = kernel_ptr<R>(type, team);
   PoolView<R> Pc = P;
   void *args[] = {(void *)&Pc, (void *)&t0, (void *)&n_iv, (void *)&iv0, (void *)&init};
-  if (team == TEAM_GRID) {
+  if (team_is_grid(team)) {
     if (block < 32 || block > GRID_BLOCK || (block & (block - 1)) != 0 || block != P.grid_bw)
       return (int)cudaErrorInvalidConfiguration;
     return (int)cudaLaunchCooperativeKernel(k, dim3(grid), dim3(block), args, smem, (cudaStream_t)stream);
@@ -295,7 +215,14 @@ int launch_pool(int type, const PoolView<R> &P, int team, int grid, int block, s
   if (team_cluster_size(team) > 0) {
     if (block != CLUSTER_BLOCK || grid % team_cluster_size(team) != 0) return (int)cudaErrorInvalidConfiguration;
     cudaLaunchAttribute attr[1];
-    const cudaLaunchConfig_t cfg = cluster_config(team, grid, smem, (cudaStream_t)stream, attr);
+    const cudaLaunchConfig_t cfg =
+        cluster_config(team_cluster_size(team), grid, block, smem, (cudaStream_t)stream, attr);
+    return (int)cudaLaunchKernelExC(&cfg, k, args);
+  }
+  if (team_is_clu(team)) {
+    if (block != P.grid_bw || P.grp_ctas < 1 || grid % P.grp_ctas != 0) return (int)cudaErrorInvalidConfiguration;
+    cudaLaunchAttribute attr[1];
+    const cudaLaunchConfig_t cfg = cluster_config(P.grp_ctas, grid, block, smem, (cudaStream_t)stream, attr);
     return (int)cudaLaunchKernelExC(&cfg, k, args);
   }
   cudaError_t e = cudaLaunchKernel(k, dim3(grid), dim3(block), args, smem, (cudaStream_t)stream);
