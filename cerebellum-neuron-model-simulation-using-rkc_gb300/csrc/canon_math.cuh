@@ -55,15 +55,17 @@ GB_HD double cm_from_bits(uint64_t u) {
 }
 
 GB_HD double cm_exp(double x) {
-  /* range checks on the bits: |x| < 704 (0x40860000...) needs none */
-  if ((uint32_t)(cm_bits(x) >> 32 & 0x7fffffff) >= 0x40860000u) {
+  /* |x| < 704 by its bits: no special case, and a normal result */
+  const int plain = (uint32_t)(cm_bits(x) >> 32 & 0x7fffffff) < 0x40860000u;
+  if (!plain) {
     if (x != x) return x;
     if (x > 709.782712893384) return HUGE_VAL;
     if (x < -745.1332191019412) return 0.0;
   }
-  /* rint and its integer by adding and subtracting 1.5 2^52 (|x / ln2| < 2^11) */
+  /* rint by adding 1.5 2^52 (|x / ln2| < 2^11), its low bits the integer */
   const double sh = x * CM_INV_LN2 + 0x1.8p52;
-  const double kd = sh - 0x1.8p52;
+  int k = (int)(uint32_t)cm_bits(sh);
+  const double kd = gbrkc::f2d((float)k);
   double r = fma(-kd, CM_LN2_HI, x);
   r = fma(-kd, CM_LN2_LO, r);
   double p = 0x1.6124613a86d09p-33;          /* 1/13! */
@@ -80,7 +82,7 @@ GB_HD double cm_exp(double x) {
   p = fma(p, r, 0x1.0000000000000p-1);       /* 1/2!  */
   p = fma(p, r, 1.0);
   p = fma(p, r, 1.0);
-  int k = (int)(uint32_t)cm_bits(sh);
+  if (plain) return cm_from_bits(cm_bits(p) + ((uint64_t)(int64_t)k << 52));   /* p 2^k, exact */
   if (k > 1023) { p *= 2.0; k -= 1; }
   if (k < -1022) { p *= 0x1p-54; k += 54; }
   return p * cm_from_bits((uint64_t)(k + 1023) << 52);

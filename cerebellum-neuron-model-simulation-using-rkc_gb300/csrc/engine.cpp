@@ -416,7 +416,10 @@ struct PoolHost {
   // grid team (engine.h, PoolView): the longest row, the fullest CTA's
   // elements, the most values a CTA receives, and the hand-over tables
   int grid_maxdeg = 0, grp_ld = 0, grp_recv_max = 0, grp_nslots = 0;
-  int grp_ctas = 1;
+  int grp_ctas = 1, grp_fast = 0;
+  long grp_stride = 0;                     // persistent launch: doubles of shared memory a team
+  int *d_line = nullptr;                   // persistent launch: abort flag, counters and line of a register role
+  bool pieces = false;                     // the last launch left systems in the line
   std::vector<GroupTab> grp_tab;
   std::vector<int> grp_chunk0, grp_col, grp_slot, grp_sptr, grp_send, grp_rptr, grp_rslot, grp_gap;
   unsigned long long *d_grp_words = nullptr;   // published values, chunk sums and the abort flag
@@ -842,10 +845,10 @@ bool group_tables(PoolHost &P, int bw, int ctas, bool grid) {
     for (int e = g0; e < g0 + ng; e++)
       if (P.gap_pre[e] >= 0) t_gap[e] = place(cta_of(P.gap_post[e]), P.gap_pre[e]);
   }
-  if (rows > (grid ? GRID_MAX_ROWS : 2)) return false;
+  if (rows > (grid ? GRID_MAX_ROWS : 2) || (rows > 1 && maxdeg > 15)) return false;   // (row lengths: four bits each)
   const int ld = rows * bw;
   const size_t smem = grid_smem(ld, most, maxdeg, (grid || ctas == 1) ? 0 : ctas);
-  if (smem > GRID_SMEM_MAX) return false;
+  if (smem > GRID_SMEM_MAX || ld + most + 2 > GRID_PLACES) return false;
   P.grp_tab = tab;
   for (auto *v : {&t_chunk0, &t_col, &t_slot, &t_sptr, &t_send, &t_rptr, &t_rslot})
     if (v->empty()) v->push_back(0);
@@ -868,20 +871,20 @@ bool group_tables(PoolHost &P, int bw, int ctas, bool grid) {
 
 // A group team (group_sys.cuh) for a pool alone in its engine, where it
 // shortens the launch: the shape is the one of least estimated time, and the
-// pool keeps its other teams (a warp, a block or an old-style cluster per
-// system, inside the persistent launch) where theirs is less.  The estimate
+// pool keeps its other teams (in the persistent launch, or an old-style
+// cluster) where theirs is less.  The estimate
 // counts FP64 warp instructions of a step attempt, 64 cycles each on an SM
 // with up to three warps and 19 per warp beyond (measured): 17 stages of 12
 // per element row, 22 for the error norm, the row's share of the ion updates
 // (FP64 gating: 0.15 to 0.5 updates of 1200 to 2300 an attempt), and 90 of the
 // controller, which every warp repeats; and the latency of handing over the
 // stage vector and the sums (CTA 60 and 500 cycles, cluster 400 and 1200,
-// grid 1400 and 4000).  A warp per system thus stays the better team once a
-// pool fills the GPU (77 Golgi cells: one CTA of 160 threads each; 2048: a
-// warp each).  A lone system of GRID_MIN_NC compartments always takes the
-// grid.  GBRKC_GROUP=0 and GBRKC_GRID=0 switch the teams off, a forced cluster
-// size (GBRKC_CLUSTER_SIZE) too; GBRKC_GRID_MIN_NC sends a lone system of that
-// size to the grid.
+// grid 1400 and 4000).  A pool that fills the GPU thus stays in the persistent
+// launch, whose teams take systems in turn (77 Golgi cells: clusters of five
+// CTAs of a warp; 2048: five warps each).  A lone system of GRID_MIN_NC
+// compartments always takes the grid.  GBRKC_GROUP=0 and GBRKC_GRID=0 switch
+// the teams off, a forced cluster size (GBRKC_CLUSTER_SIZE) too;
+// GBRKC_GRID_MIN_NC sends a lone system of that size to the grid.
 constexpr long GRID_MIN_NC = 8192;
 bool group_team(const gbrkc_engine *E, PoolHost &P) {
   const char *cs = getenv("GBRKC_CLUSTER_SIZE"), *gr = getenv("GBRKC_GROUP"), *gd = getenv("GBRKC_GRID");
@@ -910,10 +913,12 @@ bool group_team(const gbrkc_engine *E, PoolHost &P) {
     return rounds * ((rows * row + ctl) * std::max(64.0, 19.0 * warps) + (stages + 1) * hand + 1.3 * sum);
   };
   auto up = [](long a, long b) { return (a + b - 1) / b; };
-  // the persistent launch's teams: Golgi cells a warp each, others a block each
-  const double other = (P.type == GO && nc <= 320)
-                           ? time((double)up(nc, 32), (double)std::min(8L, up(nsys, sms)), (double)up(nsys, 8L * sms), 30, 700)
-                           : time((double)up(nc, 256), 8, (double)up(nsys, sms), 150, 1000);
+  // the persistent launch's teams: one element a thread on as many warps as
+  // that takes, or the whole block; systems beyond the places take turns
+  const bool one = P.type != PKJ && nc <= MEGA_BLOCK;
+  const long warps = one ? up(nc, 32) : 8, per = 8 / warps;
+  const double other = time((double)up(nc, 32 * warps), (double)(warps * std::min(per, up(nsys, sms))),
+                            std::max(1.0, nsys / (double)(per * sms)), one ? 60 : 150, 500);
   double best = 0.9 * other;
   int kind = 0, bbw = 0, bctas = 1;
   for (int bw = 32; bw <= GRID_BLOCK; bw += 32) {
@@ -1177,6 +1182,21 @@ int upload_pool(gbrkc_engine *E, PoolHost &P, PoolView<R> &V) {
     V.grp_halo = P.d_grp_words + 2;
     V.grp_red = V.grp_halo + 4 * (size_t)P.grp_nslots;
   }
+  V.grp_fast = 0;
+  if (!team_is_group(P.team) && P.grp_fast) {
+    V.grp_fast = P.grp_fast;
+    V.grid_maxdeg = P.grid_maxdeg;
+    V.grp_ld = P.grp_ld;
+    V.grp_stride = P.grp_stride;
+    V.grid_bw = P.grid_bw;
+    V.tiles = MEGA_BLOCK / P.grid_bw;
+    V.ivc = 1;
+    // abort flag and padding, counters, next intervals, the line
+    const std::vector<int> line(4 + (1 + LINE_PIECES) * P.systems.size(), 0);
+    UP(line, P.d_line);
+    V.grp_abort = P.d_line;
+    V.grp_line = P.d_line + 2;
+  }
   std::vector<double> zws(P.ws_total, 0.0);
   UP(zws, V.ws);
   std::vector<double> zero(P.nc, 0.0);
@@ -1315,23 +1335,48 @@ void fit_granule_warps(gbrkc_engine *E) {
 }
 
 // The persistent launch's pool views and role boundaries; returns the CTA
-// count.
+// count.  A register role's line (kernels.cu) is zeroed, and where its systems
+// exceed its teams they take turns.
 template <typename R>
-int mega_pools(gbrkc_engine *E, MegaView<R> &M) {
+int mega_pools(gbrkc_engine *E, MegaView<R> &M, int n_iv, int init) {
   int end = 0;
   for (int t = 0; t < NTYPES; t++) {
     PoolHost &P = E->pools[t];
     M.pool[t] = P.systems.empty() ? PoolView<R>{} : pool_view<R>(P);
+    if (P.grp_fast && !P.systems.empty() && !init) {
+      const int nsys = (int)P.systems.size(), ctas = std::max(1, E->role_ctas[t]);
+      M.pool[t].tiles = std::min(MEGA_BLOCK / P.grid_bw, (nsys + ctas - 1) / ctas);
+      const long places = (long)ctas * M.pool[t].tiles;
+      P.pieces = nsys > places && n_iv > 1;
+      M.pool[t].ivc = P.pieces ? std::max(1, (n_iv + LINE_PIECES - 1) / LINE_PIECES) : std::max(1, n_iv);
+      CUDA_TRY(cudaMemsetAsync(P.d_line, 0, (4 + (1 + (P.pieces ? LINE_PIECES : 0)) * (size_t)nsys) * sizeof(int),
+                               E->streams[0]));
+    }
     end += E->role_ctas[t];
     M.role_end[t] = end;
   }
   return end;
 }
 
+// After a persistent launch: whether a team gave up waiting for a place of the
+// line to be written.
+int check_pieces(gbrkc_engine *E) {
+  for (int t = 0; t < NTYPES; t++) {
+    PoolHost &P = E->pools[t];
+    if (!P.pieces) continue;
+    P.pieces = false;
+    int gave_up = 0;
+    CUDA_TRY(cudaMemcpy(&gave_up, P.d_line, sizeof gave_up, cudaMemcpyDeviceToHost));
+    if (gave_up) return fail(GBRKC_ECUDA, "persistent launch (type %d): a wait gave up", t);
+  }
+  return 0;
+}
+
 template <typename R>
 int launch_mega_all(gbrkc_engine *E, double t0, int n_iv, int iv0, int init) {
   MegaView<R> M{};
-  const int end = mega_pools<R>(E, M);
+  const int end = mega_pools<R>(E, M, n_iv, init);
+  if (end < 0) return end;
   if (end > E->mega_grid || end <= 0)
     return fail(GBRKC_ESTATE, "persistent launch: %d role CTAs for a grid of %d", end, E->mega_grid);
   M.gr_nc4 = E->pools[GR].team == TEAM_LANE4;
@@ -1364,6 +1409,7 @@ int launch_mega_all(gbrkc_engine *E, double t0, int n_iv, int iv0, int init) {
   CUDA_TRY(cudaEventRecord(E->ev_end, st));
   CUDA_TRY(cudaEventSynchronize(E->ev_end));
   CUDA_TRY(cudaEventElapsedTime(&E->last_ms, E->ev_start, E->ev_end));
+  if ((rc = check_pieces(E))) return rc;
   // per-role makespans from the CTAs' device timestamps
   std::vector<unsigned long long> ts(end), te(end);
   CUDA_TRY(cudaMemcpy(ts.data(), E->d_tstart, end * sizeof(unsigned long long), cudaMemcpyDeviceToHost));
@@ -1521,6 +1567,35 @@ void rebalance_roles(gbrkc_engine *E, const double *role_ms, bool tune_gr) {
     if (t != GR) E->role_ctas[t] = want[t];
 }
 
+// Whether a role of the persistent launch keeps its systems' vectors in
+// registers (PoolHost::grp_fast: 1 one element a thread, teams of as many warps
+// as that takes; 2 several, a CTA per system), raising the launch's shared
+// memory to what that takes.  GBRKC_GROUP=0 switches it off.
+bool register_role(PoolHost &P, size_t &smem) {
+  const char *gr = getenv("GBRKC_GROUP");
+  if (gr && gr[0] == '0') return false;
+  int maxdeg = 0;
+  for (size_t k = 0; k < P.systems.size(); k++) {
+    const bool own = P.sys_csr[k] >= 0;
+    const int *r = own ? P.s_row.data() + P.s_row0[P.sys_csr[k]] : P.t_row.data() + P.t_row0[P.sys_tmpl[k]];
+    for (int i = 0; i < (own ? P.sys_nc[k] : P.sys_ncomp[k]); i++) maxdeg = std::max(maxdeg, r[i + 1] - r[i]);
+  }
+  if (maxdeg > 15) return false;      // (row lengths: four bits each)
+  const bool one = P.type != PKJ && P.max_nc <= MEGA_BLOCK;
+  if (!one && (P.type == GO || P.max_nc > MEGA_BLOCK * GRP_CTA_ROWS)) return false;
+  const int bw = one ? (P.max_nc + 31) / 32 * 32 : MEGA_BLOCK, ld = (P.max_nc + bw - 1) / bw * bw;
+  const size_t bytes = grid_smem(ld, 0, maxdeg, 0) + GRP_COEF_M_DOUBLES * sizeof(double);
+  const size_t need = bytes * (MEGA_BLOCK / bw);
+  if (need > GRID_SMEM_MAX) return false;
+  smem = std::max(smem, need);
+  P.grp_fast = one ? 1 : 2;
+  P.grp_ld = ld;
+  P.grid_bw = bw;
+  P.grid_maxdeg = maxdeg;
+  P.grp_stride = (long)(bytes / sizeof(double));
+  return true;
+}
+
 // Decide whether all pools fit the persistent launch's team shapes and size
 // its shared memory; sets each pool's team / workspace placement.
 int setup_mega(gbrkc_engine *E) {
@@ -1539,7 +1614,7 @@ int setup_mega(gbrkc_engine *E) {
   if (!O.systems.empty() && O.max_nc > 320) return 0;
   // granule CTAs run up to MEGA_BLOCK single-lane systems (capped below at one
   // warp per CTA); Golgi 8 warps; Purkinje / olive one system per CTA
-  const int teams[NTYPES] = {32, MEGA_BLOCK / TEAM_WARP, 1, 1};
+  int teams[NTYPES] = {32, MEGA_BLOCK / TEAM_WARP, 1, 1};
   const int team_kind[NTYPES] = {(G.min_nc == 4 && G.max_nc == 4 && G.max_ncell == 1) ? TEAM_LANE4 : TEAM_THREAD, TEAM_WARP,
                                  TEAM_BLOCK, TEAM_BLOCK};
   size_t smem = 0;
@@ -1557,6 +1632,9 @@ int setup_mega(gbrkc_engine *E) {
     if (P.ws_in_smem) smem = std::max(smem, need);
     const int nsys = (int)P.systems.size();
     E->role_cap[t] = (nsys + teams[t] - 1) / teams[t];
+    // vectors in registers where they fit
+    P.grp_fast = 0;
+    if (t != GR && register_role(P, smem) && P.grp_fast == 1) E->role_cap[t] = nsys;
   }
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
@@ -2587,7 +2665,8 @@ namespace {
 template <typename R>
 int launch_mega_static(gbrkc_engine *E, double t0, int n_iv, int iv0, int init, unsigned long long *scratch) {
   MegaView<R> M{};
-  const int end = mega_pools<R>(E, M);
+  const int end = mega_pools<R>(E, M, n_iv, init);
+  if (end < 0) return end;
   if (end > NOALLOC_MAX_CTAS)
     return fail(GBRKC_EINVAL, "persistent launch of %d CTAs exceeds the static scratch (%d CTAs)", end,
                 NOALLOC_MAX_CTAS);
@@ -2623,6 +2702,7 @@ int launch_mega_static(gbrkc_engine *E, double t0, int n_iv, int iv0, int init, 
   CUDA_TRY(cudaEventSynchronize(E->ev_end));
   CUDA_TRY(cudaEventElapsedTime(&E->last_ms, E->ev_start, E->ev_end));
   if (init) return 0;
+  if ((rc = check_pieces(E))) return rc;
   unsigned long long ts[NOALLOC_MAX_CTAS], te[NOALLOC_MAX_CTAS];
   CUDA_TRY(cudaMemcpy(ts, M.t_start, end * sizeof(unsigned long long), cudaMemcpyDeviceToHost));
   CUDA_TRY(cudaMemcpy(te, M.t_end, end * sizeof(unsigned long long), cudaMemcpyDeviceToHost));

@@ -143,6 +143,13 @@ struct PoolView {
   unsigned long long *grp_halo;       // grid: [2][nslots][2] published values
   unsigned long long *grp_red;        // grid: [2][GRID_MAX_BLOCKS][2] published chunk sums
   int *grp_abort;                     // a wait gave up
+  // persistent launch: systems of one (1) or several (2) elements a thread,
+  // vectors in registers; 0: the teams with their vectors in memory
+  int grp_fast;
+  int tiles;                          // teams of a CTA that take systems
+  long grp_stride;                    // doubles of shared memory a team
+  int ivc;                            // intervals a team goes on with one system while others wait
+  int *grp_line;                      // [2] counters, [nsys] next intervals, [16 nsys] the line (kernels.cu, line_take)
 };
 
 // How a pool takes its synaptic current (solve_rkc.cu): granule cells add
@@ -234,12 +241,21 @@ constexpr bool team_is_group(int team) { return team > 200; }
 constexpr int GRID_BLOCK = 256;
 constexpr int GRID_MAX_BLOCKS = 256;
 constexpr int GRID_MAX_ROWS = 8;
+// In the persistent launch a team of a CTA's warps integrates systems of up to
+// MEGA_BLOCK compartments, one a thread, or, as the whole CTA, of up to
+// GRP_CTA_ROWS a thread; shared memory holds the coefficients of stage counts
+// up to GRP_COEF_M.
+constexpr int GRP_CTA_ROWS = 7, GRP_COEF_M = 96;
+constexpr int GRP_COEF_M_DOUBLES = (5 * (GRP_COEF_M - 1) + 1) & ~1;
+constexpr int LINE_PIECES = 16;   // most pieces of a system's launch
 constexpr size_t GRID_SMEM_MAX = 200 * 1024;   // shared memory of a CTA
-// bytes of it: two stage buffers, per element its row (conductances, columns,
-// count, 1/Cm, row sum), and in a cluster of `ctas` the slots of hand-overs
-// and sums
+// bytes of it: two stage buffers, per element its row (pairs of conductances
+// and columns, 1/Cm or the row sum), and in a cluster of `ctas` the slots of
+// hand-overs and sums.  Columns are byte offsets of 16 bits: at most
+// GRID_PLACES places in a stage buffer.
+constexpr long GRID_PLACES = 8191;
 constexpr size_t grid_smem(long ld, long recv, long maxdeg, int ctas) {
-  return 16 * (size_t)(ld + recv) + (size_t)ld * (20 + 12 * (size_t)maxdeg) +
+  return 16 * (size_t)(ld + recv + 2) + (size_t)ld * (8 + 20 * (size_t)((maxdeg + 1) / 2)) +
          (ctas > 0 ? 16 + 32 * (size_t)recv + 32 * (size_t)GRID_MAX_ROWS * ctas : 0);
 }
 

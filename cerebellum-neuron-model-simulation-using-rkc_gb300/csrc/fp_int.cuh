@@ -196,8 +196,29 @@ struct RecipF {
 GB_HD Recip mrecip(double b) { return recip(b); }
 GB_HD RecipF mrecip(float b) { return RecipF{b}; }
 GB_HD float div_by(float a, const RecipF &r) { return a / r.b; }
-// division by a constant, whose rounded reciprocal the compiler folds
-GB_HD double cdiv(double a, double b) { return div_by(a, Recip{b, 1.0 / b, true}); }
+// Division by a constant b = B 2^e, B odd; everything but the operations on a
+// folds at compile time.  B = 1: the exact product with 1 / b.  B < 2^21: the
+// product with 1 / b in two parts, ch + cl, rounded once (Brisebarre & Muller,
+// IEEE Trans. Comput. 57(2), 2008): it is within 2^-50 of a last place of
+// a / b before its rounding, and a / b, a multiple of 2^j / B that is no
+// midpoint of two doubles (A / B has no more bits than A), lies at least
+// 1 / (2 B) of a last place from every midpoint.  Else the corrected product.
+// The two-part product's range of a is div_by's.
+GB_HD double cdiv(double a, double b) {
+  const uint64_t m = fpi_bits(b) & 0x000fffffffffffffULL;
+  const uint32_t h = (uint32_t)(fpi_bits(a) >> 32) & 0x7fffffffu;
+  if (m == 0) return a * (1.0 / b);
+  if ((m & 0xffffffffULL) == 0) {            // at most 20 bits behind the leading one: B < 2^21
+    const double ch = 1.0 / b, cl = fma(-ch, b, 1.0) / b;
+    const bool zero = (fpi_bits(a) << 1) == 0;
+    if (zero || h - ((1023u - 400u) << 20) < (800u << 20)) {
+      const double q = fma(a, ch, a * cl);
+      return zero ? a * ch : q;
+    }
+    return a / b;
+  }
+  return div_by(a, Recip{b, 1.0 / b, true});
+}
 GB_HD float cdiv(float a, float b) { return a / b; }
 // to<R>(x): an FP64 value in R; up(x): a value of R in FP64
 template <typename R> GB_HD R to(double x);

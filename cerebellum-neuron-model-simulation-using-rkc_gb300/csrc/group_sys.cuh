@@ -1,5 +1,5 @@
-// RKC integrator for one system spread over the threads of a CTA, of a
-// cluster of CTAs, or (the grid team: a system alone in its engine, too large
+// RKC integrator for one system spread over some warps of a CTA, of a cluster
+// of CTAs, or (the grid team: a system alone in its engine, too large
 // for a cluster) of every CTA of a cooperative launch; its five RKC vectors
 // and its current b in registers, at most K elements a thread.
 //
@@ -92,29 +92,37 @@ __device__ __forceinline__ void cluster_sync_all() {
 template <int CT, typename R, int K, int COMM>
 struct GroupSys {
   static constexpr bool MIXED = !std::is_same<R, double>::value;
-  static constexpr int RN = 4;   // neighbours kept in registers where a thread has one element
+  static constexpr bool ALONE = COMM == GRP_CTA;   // no other CTA takes part
   typedef StepCtl<double> SC;
   const PoolView<R> &P;
   int s, nc, ncell, ncomp, off, cell0;
-  int G, cta, bw, t;           // CTAs of the group, this CTA, threads a CTA, this thread
+  int G, cta, bw, t, bar;      // CTAs of the group, this CTA, threads a CTA, this thread, the CTA team's barrier
   int chunk0, rows, e0, L;     // this CTA's chunks, its first element, its element places
   int r0, nrecv;               // its received values
   const GroupTab *tab;
-  int ld;                      // places of the row tables (rows of the fullest CTA)
+  int ld, pairs, us;           // places of the row tables (the fullest CTA's elements), neighbour pairs, places of a stage buffer
   // shared memory
-  double *u;                   // [2][ld + most received]: the stage vector, own places then received ones
-  double *lg, *linv, *lG;      // [maxdeg][ld] conductances, [ld] 1/Cm; mixed: g/Cm, and its row sums
-  int *lcol, *lcnt;            // [maxdeg][ld] places of the neighbours, [ld] counts
-  double *wp, *res;
+  double *u;                   // [2][us]: the stage vector, own places, received ones behind them, and a zero
+  // the row tables: pairs of neighbours, [pairs][ld] (conductance, conductance)
+  // -- mixed precision: g / Cm -- and [pairs][ld] their places in the stage
+  // buffer, as byte offsets of 16 bits each; [ld] 1/Cm (mixed: the row sums)
+  double2 *lg;
+  unsigned *lcol;
+  double *linv;
+  double *wp, *res, *coef;     // warp partials, a sum's result, the step's stage coefficients
   unsigned halo, red;          // cluster: [2][most received][2] and [2][chunks][2] words, shared-memory addresses
+  int coef_m;                  // stage counts whose coefficients it holds
   int *s_abort;                // [0] a wait gave up, [1] the same as of the last sum, alike for the CTA's threads
   // registers
   double y[K], yn[K], fn[K], v1[K], v2[K];
   double b[K];                 // the current; mixed precision: -b / Cm
   int slot[K];                 // grid: publishing slot, or -1
   int send0, send1;            // cluster: the thread's hand-overs (P.grp_send)
-  int rc[RN];                  // K = 1: the row's first columns
-  double rg[RN];               //        and conductances
+  unsigned dst;                // its first hand-over's slot in the reading CTA (evaluations of even number)
+  int dstq;                    // and its element
+  unsigned pc[K][2];           // the row's first two pairs of places
+  int wdeg;                    // the longest row of the warp at each of its elements (four bits each; K = 1: whole)
+  double2 rg[2];               // K = 1: the row's first two pairs of conductances
   SC c;
   Recip rnc;                   // 1 / nc
   unsigned tag, rtag;          // evaluations and sums so far
@@ -122,31 +130,40 @@ struct GroupSys {
   int k_iv, n_iv, iv0;
   long long attempts0;
 
-  // cta_, G_: this CTA's place in its group and the group's CTAs
-  __device__ GroupSys(const PoolView<R> &P_, double *smem, double *wp_, double *res_, int *ab, int cta_, int G_)
-      : P(P_), wp(wp_), res(res_), s_abort(ab) {
-    t = threadIdx.x;
-    bw = P.grid_bw;
+  // The team is the bw_ threads from first_ on, meeting at barrier bar_ (0 the
+  // whole CTA's); smem: grid_smem bytes; coef_: 5 (coef_m - 1) values; wp_,
+  // res_, ab: reduction words; cta_, G_: this CTA's place in its group and the
+  // group's CTAs.
+  __device__ GroupSys(const PoolView<R> &P_, double *smem, double *wp_, double *res_, double *coef_, int coef_m_,
+                      int *ab, int first_, int bw_, int bar_, int cta_, int G_)
+      : P(P_), wp(wp_), res(res_), coef(coef_), coef_m(coef_m_), s_abort(ab) {
+    t = (int)threadIdx.x - first_;
+    bw = bw_;
+    bar = bar_;
     G = G_;
     cta = cta_;
     ld = P.grp_ld;
-    const int md = P.grid_maxdeg, rm = P.grp_recv_max;
+    pairs = (P.grid_maxdeg + 1) >> 1;
+    us = ld + 1 + (ALONE ? 0 : P.grp_recv_max);
+    us += us & 1;
     u = smem;
-    lg = u + 2 * (ld + rm);
-    linv = lg + (long)md * ld;
-    lG = linv + ld;
-    lcol = (int *)(lG + ld);
-    lcnt = lcol + (long)md * ld;
+    lg = (double2 *)(u + 2 * us);
+    linv = (double *)(lg + pairs * ld);
+    lcol = (unsigned *)(linv + ld);
     tag = rtag = 0;
     if constexpr (COMM == GRP_CLUSTER) {
       // slots behind the rows, numbered 0 before any hand-over
-      unsigned long long *w = (unsigned long long *)(((unsigned long long)(lcnt + ld) + 15) & ~15ull);
-      const int n = 4 * rm + 4 * GRID_MAX_ROWS * G;
+      unsigned long long *w = (unsigned long long *)(((unsigned long long)(lcol + pairs * ld) + 15) & ~15ull);
+      const int rm = P.grp_recv_max, n = 4 * rm + 4 * GRID_MAX_ROWS * G;
       for (int i = t; i < n; i += bw) w[i] = 0ull;
       halo = (unsigned)__cvta_generic_to_shared(w);
       red = halo + 32 * rm;
       cluster_sync_all();
     }
+  }
+  __device__ __forceinline__ void sync() const {
+    if constexpr (COMM == GRP_CTA) asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(bw) : "memory");
+    else __syncthreads();
   }
   // no CTA leaves while a peer may still store into its shared memory
   __device__ __forceinline__ void leave() const {
@@ -155,8 +172,7 @@ struct GroupSys {
 
   __device__ __forceinline__ int at(int k) const { return e0 + k * bw + t; }
   __device__ __forceinline__ bool has(int k) const { return k < rows && at(k) < nc; }
-  __device__ __forceinline__ int ustride() const { return ld + P.grp_recv_max; }
-  __device__ __forceinline__ const double *ucur() const { return u + (tag & 1u) * ustride(); }
+  __device__ __forceinline__ const double *ucur() const { return u + (tag & 1u) * us; }
 
   // Take the system: its operator rows into shared memory, its vectors into
   // registers.
@@ -167,12 +183,12 @@ struct GroupSys {
     ncomp = P.sys_ncomp[s];
     off = P.sys_off[s];
     cell0 = P.sys_cell0[s];
-    tab = P.grp_tab + s;
-    if constexpr (COMM == GRP_CTA) {
+    if constexpr (ALONE) {
       chunk0 = 0;
       rows = (nc + bw - 1) / bw;
       r0 = nrecv = 0;
     } else {
+      tab = P.grp_tab + s;
       chunk0 = P.grp_chunk0[tab->chunk0 + cta];
       rows = P.grp_chunk0[tab->chunk0 + cta + 1] - chunk0;
       r0 = P.grp_rptr[tab->rptr + cta];
@@ -180,7 +196,8 @@ struct GroupSys {
     }
     e0 = chunk0 * bw;
     L = rows * bw;
-    send0 = send1 = 0;
+    send0 = send1 = dstq = 0;
+    dst = 0u;
     const int k = P.sys_csr[s], tm = P.sys_tmpl[s];
     const bool csr = k >= 0;
     const int *row = csr ? P.s_row + P.s_row0[k] : P.t_row + P.t_row0[tm];
@@ -191,58 +208,90 @@ struct GroupSys {
     const long ncp = (nc + 1) & ~1;
     const double *ws = P.ws + P.sys_ws[s];
     const int *pcol = (csr ? P.s_col + P.s_nz0[k] : P.t_col + P.t_nz0[tm]);
-    if constexpr (COMM != GRP_CTA) pcol = P.grp_col + tab->col;
+    if constexpr (!ALONE) pcol = P.grp_col + tab->col;
     c.load(P.ctl[s]);
-    __syncthreads();               // the last system's readers of the tables are done
-#pragma unroll
-    for (int q = 0; q < RN; q++) {
-      rc[q] = 0;
-      rg[q] = 0.0;
-    }
+    sync();               // the last system's readers of the tables are done
+    if (t < 2) u[t * us + us - 1] = 0.0;      // the zero
+    wdeg = 0;
 #pragma unroll
     for (int q = 0; q < K; q++) {
       y[q] = yn[q] = fn[q] = v1[q] = v2[q] = b[q] = 0.0;
       slot[q] = -1;
-      if (!has(q)) continue;
-      // (cells of one template lie one after another)
-      const int i = at(q), lr = q * bw + t, base = csr ? 0 : i - i % ncomp, ri = i - base;
-      const int a = __ldg(row + ri), z = __ldg(row + ri + 1);
-      lcnt[lr] = z - a;
-      linv[lr] = __ldg(inv + ri);
-      if (MIXED) lG[lr] = __ldg(Gc + ri);
-      for (int j = a; j < z; j++) {
-        lg[(long)(j - a) * ld + lr] = __ldg(g + j);
-        lcol[(long)(j - a) * ld + lr] = (COMM == GRP_CTA ? base : 0) + __ldg(pcol + j);
+      // a row's surplus entries: conductance -0 at the zero (mixed precision)
+      // or at the element itself, so that they add -0, which changes nothing
+      const int lr = q * bw + t;
+      const unsigned none = 8u * (unsigned)(MIXED ? us - 1 : lr);
+      if (lr < ld) {
+        linv[lr] = 0.0;
+        for (int j = 0; j < pairs; j++) {
+          lg[j * ld + lr] = make_double2(-0.0, -0.0);
+          lcol[j * ld + lr] = none | none << 16;
+        }
+        u[lr] = u[us + lr] = 0.0;
       }
-      if constexpr (K == 1) {
-#pragma unroll
-        for (int j = 0; j < RN; j++)
-          if (j < z - a) {
-            rc[j] = lcol[(long)j * ld + lr];
-            rg[j] = lg[(long)j * ld + lr];
+      pc[q][0] = pc[q][1] = none | none << 16;
+      int cnt = 0;
+      if (has(q)) {
+        // (cells of one template lie one after another)
+        const int i = at(q), base = csr ? 0 : i - i % ncomp, ri = i - base;
+        const int a = __ldg(row + ri), z = __ldg(row + ri + 1);
+        cnt = z - a;
+        linv[lr] = MIXED ? __ldg(Gc + ri) : __ldg(inv + ri);
+        for (int j = 0; j < cnt; j++) {
+          const unsigned place = 8u * (unsigned)((ALONE ? base : 0) + __ldg(pcol + a + j));
+          double2 &gp = lg[(j >> 1) * ld + lr];
+          unsigned &cp = lcol[(j >> 1) * ld + lr];
+          if (j & 1) {
+            gp.y = __ldg(g + a + j);
+            cp = (cp & 0xffffu) | place << 16;
+          } else {
+            gp.x = __ldg(g + a + j);
+            cp = (cp & 0xffff0000u) | place;
           }
-      }
+        }
+        pc[q][0] = pairs > 0 ? lcol[lr] : pc[q][0];
+        pc[q][1] = pairs > 1 ? lcol[ld + lr] : pc[q][1];
+        y[q] = ws[map[LY] * ncp + i];
+        yn[q] = ws[map[LYN] * ncp + i];
+        fn[q] = ws[map[LFN] * ncp + i];
+        v1[q] = ws[map[LV1] * ncp + i];
+        v2[q] = ws[map[LV2] * ncp + i];
+        b[q] = ws[WS_B * ncp + i];
+        if constexpr (MIXED) b[q] = -b[q] * __ldg(inv + ri);
       if constexpr (COMM == GRP_GRID) slot[q] = P.grp_slot[tab->slot + i];
       if constexpr (COMM == GRP_CLUSTER) {
         // (a thread of several elements hands over in exchange's own loop)
         if (q == 0) {
           send0 = P.grp_sptr[tab->sptr + (cta * bw) + t];
           send1 = P.grp_sptr[tab->sptr + (cta * bw) + t + 1];
+          if (send0 < send1) {
+            const int d = __ldg(P.grp_send + tab->send + send0);
+            dst = cluster_map(halo + 16u * (d & 0xffff), (d >> 16) & 255);
+            dstq = d >> 24;
+          }
         }
       }
-      y[q] = ws[map[LY] * ncp + i];
-      yn[q] = ws[map[LYN] * ncp + i];
-      fn[q] = ws[map[LFN] * ncp + i];
-      v1[q] = ws[map[LV1] * ncp + i];
-      v2[q] = ws[map[LV2] * ncp + i];
-      set_b(q, ws[WS_B * ncp + i]);
+      }
+      // the warp's longest row here
+#pragma unroll
+      for (int st = 16; st > 0; st /= 2) cnt = max(cnt, __shfl_xor_sync(0xffffffffu, cnt, st));
+      wdeg |= cnt << (4 * q);
     }
-    __syncthreads();
+    if constexpr (K == 1) {
+      rg[0] = pairs > 0 && t < ld ? lg[t] : make_double2(-0.0, -0.0);
+      rg[1] = pairs > 1 && t < ld ? lg[ld + t] : make_double2(-0.0, -0.0);
+    }
+    sync();
   }
 
   __device__ __forceinline__ void set_b(int q, double x) {
-    if constexpr (MIXED) b[q] = -x * linv[q * bw + t];
-    else b[q] = x;
+    if constexpr (MIXED) {
+      // -b / Cm; 1/Cm is read here only
+      const int k = P.sys_csr[s], i = at(q);
+      b[q] = -x * (k >= 0 ? __ldg(P.s_invcm + P.s_cm0[k] + i) : __ldg(P.t_invcm + P.t_cm0[P.sys_tmpl[s]] + i % ncomp));
+    } else {
+      b[q] = x;
+    }
   }
 
   // (b itself is written at each ion update)
@@ -285,7 +334,7 @@ struct GroupSys {
   __device__ __forceinline__ void exchange(const double (&val)[K]) {
     tag++;
     const unsigned par = tag & 1u;
-    double *ub = u + par * ustride();
+    double *ub = u + par * us;
     if constexpr (COMM == GRP_GRID) {
       const unsigned long long h = (unsigned long long)(P.grp_halo + (long)par * P.grp_nslots * 2);
 #pragma unroll
@@ -302,53 +351,125 @@ struct GroupSys {
         if (has(q)) ub[q * bw + t] = val[q];
       if constexpr (COMM == GRP_CLUSTER) {
         const unsigned h = halo + par * 16u * P.grp_recv_max;
-        for (int j = send0; j < send1; j++) {
-          // reading CTA, its slot, this thread's element
-          const int d = __ldg(P.grp_send + tab->send + j), q = (d >> 24) & 15;
+        auto pick = [&](int q) {
           double x = val[0];
 #pragma unroll
           for (int k = 1; k < K; k++)
             if (k == q) x = val[k];
-          slot_put<COMM>(cluster_map(h + 16u * (d & 0xffff), (d >> 16) & 255), x, tag);
+          return x;
+        };
+        if (send0 < send1) slot_put<COMM>(dst + par * 16u * P.grp_recv_max, pick(dstq), tag);
+        for (int j = send0 + 1; j < send1; j++) {
+          // this thread's element, reading CTA, its slot
+          const int d = __ldg(P.grp_send + tab->send + j);
+          slot_put<COMM>(cluster_map(h + 16u * (d & 0xffff), (d >> 16) & 255), pick(d >> 24), tag);
         }
         for (int j = t; j < nrecv; j += bw) ub[L + j] = wait(h + 16u * j, tag);
       }
     }
-    __syncthreads();
+    sync();
   }
 
-  // dydt at the thread's q-th element, whose stage value is ui (Sys::rhs)
-  __device__ __forceinline__ double rhs(int q, double ui) const {
-    const int lr = q * bw + t, n = lcnt[lr];
-    const double *ub = ucur();
-    if constexpr (K == 1) {
-      // the row's first entries from registers: one shared-memory latency
-      double x[RN];
+  // dydt at the thread's elements, whose stage values are ui (Sys::rhs).  A
+  // row of a warp runs to its longest row, in pairs of neighbours.
+  __device__ __forceinline__ void rhs(const double (&ui)[K], double (&f)[K]) const {
+    const char *ub = (const char *)ucur();
+    auto term = [&](double g, unsigned o, double v, double d) {
+      const double x = *(const double *)(ub + o);
+      return fma(g, MIXED ? x : x - v, d);
+    };
 #pragma unroll
-      for (int j = 0; j < RN; j++) x[j] = ub[rc[j]];
+    for (int q = 0; q < K; q++) {
+      f[q] = 0.0;
+      if (K > 1 && q >= rows) break;
+      const int lr = q * bw + t, n = deg(wdeg, q);
       double d = MIXED ? b[q] : -b[q];
-#pragma unroll
-      for (int j = 0; j < RN; j++)
-        if (j < n) d = fma(rg[j], MIXED ? x[j] : x[j] - ui, d);
-      for (int j = RN; j < n; j++) {
-        const double v = ub[lcol[(long)j * ld + lr]];
-        d = fma(lg[(long)j * ld + lr], MIXED ? v : v - ui, d);
+      if (n > 0) {
+        const double2 g = K == 1 ? rg[0] : lg[lr];
+        d = term(g.x, pc[q][0] & 0xffffu, ui[q], d);
+        if (n > 1) d = term(g.y, pc[q][0] >> 16, ui[q], d);
       }
-      if constexpr (MIXED) return fma(-lG[lr], ui, d);
-      else return d * linv[lr];
-    } else if constexpr (MIXED) {
-      double d = b[q];
-      for (int j = 0; j < n; j++) d = fma(lg[(long)j * ld + lr], ub[lcol[(long)j * ld + lr]], d);
-      return fma(-lG[lr], ui, d);
-    } else {
-      double d = -b[q];
-      for (int j = 0; j < n; j++) d = fma(lg[(long)j * ld + lr], ub[lcol[(long)j * ld + lr]] - ui, d);
-      return d * linv[lr];
+      if (n > 2) {
+        const double2 g = K == 1 ? rg[1] : lg[ld + lr];
+        d = term(g.x, pc[q][1] & 0xffffu, ui[q], d);
+        if (n > 3) d = term(g.y, pc[q][1] >> 16, ui[q], d);
+      }
+      for (int j = 4; j < n; j += 2) {
+        const double2 g = lg[(j >> 1) * ld + lr];
+        const unsigned p = lcol[(j >> 1) * ld + lr];
+        d = term(g.x, p & 0xffffu, ui[q], d);
+        if (n > j + 1) d = term(g.y, p >> 16, ui[q], d);
+      }
+      if constexpr (MIXED) f[q] = fma(-linv[lr], ui[q], d);
+      else f[q] = d * linv[lr];
     }
+  }
+  static __device__ __forceinline__ int deg(int packed, int q) {
+    return K == 1 ? packed : (int)((unsigned)packed >> (4 * q)) & 15;
+  }
+
+  // the pairwise tree over a[0..8) of which n are there
+  static __device__ __forceinline__ double tree8(double (&w)[8], int n) {
+#pragma unroll
+    for (int st = 1; st < 8; st *= 2)
+#pragma unroll
+      for (int j = 0; j + st < 8; j += 2 * st) {
+        const double x = w[j] + w[j + st];
+        w[j] = j + st < n ? x : w[j];
+      }
+    return w[0];
   }
 
   // the pairwise tree over the system's elements of x, the same in every thread
   __device__ __forceinline__ double sum(const double (&x)[K]) {
+    if constexpr (ALONE && K > 2) return sum8(x);
+    else return sum_rows(x);
+  }
+
+  // Many elements a thread: through shared memory, a thread eight consecutive
+  // values at a time, then a warp eight such sums a lane (systems of up to
+  // 2048 elements): 61 FP64 additions for 1600 elements where a shuffle tree
+  // per row takes 280.
+  __device__ __forceinline__ double sum8(const double (&x)[K]) {
+    double *sc = u + ((tag + 1u) & 1u) * us;    // the next evaluation's buffer
+#pragma unroll
+    for (int q = 0; q < K; q++)
+      if (has(q)) sc[q * bw + t] = x[q];
+    sync();
+    const int n8 = (nc + 7) >> 3;
+    double a = 0.0;
+    for (int k = t; k < n8; k += bw) {
+      double w[8];
+#pragma unroll
+      for (int j = 0; j < 8; j++) w[j] = 8 * k + j < nc ? sc[8 * k + j] : 0.0;
+      a = tree8(w, nc - 8 * k);
+      if (n8 > 32) sc[8 * k] = a;
+    }
+    int nb = n8;
+    if (n8 > 32) {
+      sync();
+      nb = (n8 + 7) >> 3;
+      if (t < 32) {
+        double w[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) w[j] = 8 * t + j < n8 ? sc[64 * t + 8 * j] : 0.0;
+        a = tree8(w, n8 - 8 * t);
+      }
+    }
+    if (t < 32) {
+#pragma unroll
+      for (int st = 1; st < 32; st *= 2) {
+        if (st >= nb) break;
+        const double o = __shfl_down_sync(0xffffffffu, a, st);
+        if ((t & (2 * st - 1)) == 0 && t + st < nb) a = a + o;
+      }
+    }
+    if (t == 0) *res = a;
+    sync();
+    return *res;
+  }
+
+  __device__ __forceinline__ double sum_rows(const double (&x)[K]) {
     const int lane = t & 31, warp = t >> 5, nw = bw >> 5;
 #pragma unroll
     for (int q = 0; q < K; q++) {
@@ -363,14 +484,14 @@ struct GroupSys {
       if (lane == 0) wp[q * nw + warp] = a;
     }
     rtag++;
-    __syncthreads();
+    sync();
     if (warp == 0) {
       // the parts that the tree goes on with: the CTA's 32-element parts (one
       // CTA), or every chunk's sum
-      constexpr int VM = COMM == GRP_GRID ? GRID_MAX_BLOCKS / 32 : COMM == GRP_CLUSTER ? 4 : 2;
+      constexpr int VM = COMM == GRP_GRID ? GRID_MAX_BLOCKS / 32 : COMM == GRP_CLUSTER ? 4 : 2;   // (one CTA: 64 parts)
       int nb, rr;
       double v[VM];
-      if constexpr (COMM == GRP_CTA) {
+      if constexpr (ALONE) {
         nb = (nc + 31) >> 5;
         rr = nb <= 32 ? 1 : 2;
 #pragma unroll
@@ -423,10 +544,10 @@ struct GroupSys {
       }
       if (lane == 0) {
         *res = v[0];
-        s_abort[1] = *(volatile int *)s_abort;
+        if constexpr (!ALONE) s_abort[1] = *(volatile int *)s_abort;
       }
     }
-    __syncthreads();
+    sync();
     return *res;
   }
 
@@ -459,14 +580,11 @@ struct GroupSys {
       c.n_rho_iter++;
       exchange(v1);
       double d[K];
+      rhs(v1, v2);
 #pragma unroll
       for (int q = 0; q < K; q++) {
-        d[q] = 0.0;
-        if (has(q)) {
-          v2[q] = rhs(q, v1[q]);
-          const double dm = -1.0 * fn[q] + v2[q];
-          d[q] = dm * dm;
-        }
+        const double dm = -1.0 * fn[q] + v2[q];
+        d[q] = dm * dm;
       }
       const double dfnrm = sqrt(sum(d));
       if (rc.next(iter, dfnrm, c.sprad) == RhoCtl::DONE) {
@@ -496,6 +614,11 @@ struct GroupSys {
       return false;
     }
     const double *T = P.coef + P.coef_off[m];
+    // the stages' coefficients into shared memory (the first evaluation's
+    // barrier publishes them): one trip to the L2 a step, not one a stage
+    const bool near = m <= coef_m;
+    if (near)
+      for (int i = t; i < 5 * (m - 1); i += bw) coef[i] = __ldg(T + 1 + i);
     const double hm1 = h * __ldg(T);
 #pragma unroll
     for (int q = 0; q < K; q++) {
@@ -503,21 +626,25 @@ struct GroupSys {
       v1[q] = fma(hm1, fn[q], yn[q]);
     }
     for (int j = 1; j < m; j++) {
-      const double *p = T + 1 + 5 * (j - 1);
-      const double mu = __ldg(p), nu = __ldg(p + 1), omn = __ldg(p + 2), mus = __ldg(p + 3), ajm1 = __ldg(p + 4);
       exchange(v1);
+      double mu, nu, omn, mus, ajm1;
+      if (near) {
+        const double *p = coef + 5 * (j - 1);
+        mu = p[0]; nu = p[1]; omn = p[2]; mus = p[3]; ajm1 = p[4];
+      } else {
+        const double *p = T + 1 + 5 * (j - 1);
+        mu = __ldg(p); nu = __ldg(p + 1); omn = __ldg(p + 2); mus = __ldg(p + 3); ajm1 = __ldg(p + 4);
+      }
       const double hm = h * mus;
+      double f[K];
+      rhs(v1, f);
 #pragma unroll
       for (int q = 0; q < K; q++) {
         if (q >= rows) break;
-        double out = 0.0;
-        if (has(q)) {
-          const double f = rhs(q, v1[q]);
-          double w = mu * v1[q];
-          w = fma(nu, v2[q], w);
-          w = fma(omn, yn[q], w);
-          out = fma(hm, fma(-ajm1, fn[q], f), w);
-        }
+        double w = mu * v1[q];
+        w = fma(nu, v2[q], w);
+        w = fma(omn, yn[q], w);
+        const double out = fma(hm, fma(-ajm1, fn[q], f[q]), w);
         // written to y, then (v2, v1, y) <- (v1, y, v2)
         y[q] = v2[q];
         v2[q] = v1[q];
@@ -548,16 +675,15 @@ struct GroupSys {
     c.n_steps++;
     exchange(y);
     const double h04 = 0.4 * h;
-    double d[K];
+    double d[K], f[K];
+    rhs(y, f);
 #pragma unroll
     for (int q = 0; q < K; q++) {
       d[q] = 0.0;
-      if (q >= rows) break;
-      if (has(q)) {
-        const double f = rhs(q, y[q]);
-        v1[q] = f;
+      if (q < rows) {
+        v1[q] = f[q];
         const double wt = fma(c.tol, abs_max(y[q], yn[q]), c.tol);
-        const double est = fma(h04, fn[q] + f, 0.8 * (yn[q] - y[q]));
+        const double est = fma(h04, fn[q] + f[q], 0.8 * (yn[q] - y[q]));
         const double qv = mdiv(est, wt);
         d[q] = qv * qv;
       }
@@ -594,13 +720,13 @@ struct GroupSys {
       // which this update sets to y
       exchange(y);
     } else {
-      double *ub = u + ((tag + 1u) & 1u) * ustride();
+      double *ub = u + ((tag + 1u) & 1u) * us;
 #pragma unroll
       for (int q = 0; q < K; q++)
         if (has(q)) ub[q * bw + t] = y[q];
     }
-    const double *yb = gap ? ucur() : u + ((tag + 1u) & 1u) * ustride();
-    double *bb = u + (gap ? (tag + 1u) & 1u : tag & 1u) * ustride();
+    const double *yb = gap ? ucur() : u + ((tag + 1u) & 1u) * us;
+    double *bb = u + (gap ? (tag + 1u) & 1u : tag & 1u) * us;
     const long ncp = (nc + 1) & ~1;
     double *wsb = P.ws + P.sys_ws[s] + WS_B * ncp;
 #pragma unroll 1
@@ -614,7 +740,7 @@ struct GroupSys {
         // add_io_gap_val)
         for (int k = 0; k < 4; k++) {
           int pre;
-          if constexpr (COMM == GRP_CTA) pre = P.gap_pre[e0g + k];
+          if constexpr (ALONE) pre = P.gap_pre[e0g + k];
           else pre = P.grp_gap[e0g + k];
           const double diff = pre >= 0 ? yb[lr] - yb[pre] : 0.0;
           x += io_gap_current(P.gap_g[e0g + k], diff);
@@ -642,12 +768,10 @@ struct GroupSys {
     }
     ion_and_b(0.0, false, false);
     exchange(yn);
+    rhs(yn, fn);
 #pragma unroll
     for (int q = 0; q < K; q++)
-      if (has(q)) {
-        fn[q] = rhs(q, yn[q]);
-        P.ede[off + at(q)] = fn[q];
-      }
+      if (has(q)) P.ede[off + at(q)] = fn[q];
     rkcrho();
     // set_initial_absh (solve_rkc.cu:493-560)
     double absh = H_MAX;
@@ -657,11 +781,11 @@ struct GroupSys {
     for (int q = 0; q < K; q++) v1[q] = fma(absh, fn[q], yn[q]);
     exchange(v1);
     double d[K];
+    rhs(v1, v2);
 #pragma unroll
     for (int q = 0; q < K; q++) {
       d[q] = 0.0;
       if (has(q)) {
-        v2[q] = rhs(q, v1[q]);
         const double wt = fma(c.tol, fabs(yn[q]), c.tol);
         const double dm = (v2[q] - fn[q]) * (1.0 / wt);
         d[q] = dm * dm;
@@ -733,15 +857,15 @@ struct GroupSys {
     if (c.iv_left > 0) c.iv_left--;
   }
 
-  __device__ __forceinline__ int start(double tb, int n, int iv0_global) {
+  __device__ __forceinline__ int start(double tb, int k0, int n, int iv0_global) {
     if (c.iv_left >= 0 && n > c.iv_left) n = c.iv_left;
     t0 = tb;
-    n_iv = n;
+    n_iv = k0 + n;
     iv0 = iv0_global;
-    k_iv = 0;
+    k_iv = k0;
     rnc = recip((double)nc);
     if (c.status != 0 || n <= 0) return TICK_DONE;
-    return begin_interval(t0);
+    return begin_interval(t0 + k0 * H_MAX);
   }
 
   // Sys::tick
@@ -760,17 +884,25 @@ struct GroupSys {
     return begin_interval(t0 + k_iv * H_MAX);
   }
 
-  // Advance the system by n intervals from tb, or initialise it.
-  __device__ __forceinline__ void run(int s_, double tb, int n, int iv0_global, bool init) {
+  __device__ __forceinline__ bool gave_up() const {
+    if constexpr (ALONE) return false;
+    else return s_abort[1] != 0;
+  }
+
+  // Advance the system by n intervals, the launch's k0-th and on (the launch
+  // begins at tb), or initialise it.
+  template <bool INIT = true>
+  __device__ __forceinline__ void run(int s_, double tb, int k0, int n, int iv0_global, bool init) {
     if (!system_selected(P.ctl[s_], init, n)) return;
-    if (t == 0) s_abort[0] = s_abort[1] = 0;
+    if constexpr (!ALONE)
+      if (t == 0) s_abort[0] = s_abort[1] = 0;
     bind(s_);
-    if (init) {
+    if (INIT && init) {
       initialize();
       c.status &= ~ST_INIT;
-      if (s_abort[1]) c.status |= ST_BARRIER;
+      if (gave_up()) c.status |= ST_BARRIER;
     } else {
-      int r = start(tb, n, iv0_global);
+      int r = start(tb, k0, n, iv0_global);
       if (r == TICK_DONE) return;
       while (r != TICK_DONE) {
         if (r == TICK_ION) {
@@ -779,7 +911,7 @@ struct GroupSys {
           r = TICK_MORE;
         } else {
           r = tick();
-          if (s_abort[1]) {
+          if (gave_up()) {
             c.status |= ST_BARRIER;
             break;
           }

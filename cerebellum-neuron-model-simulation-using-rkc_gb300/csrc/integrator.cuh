@@ -150,22 +150,32 @@ constexpr int ION_WAIT_MAX = 12;             // warp iterations a due ion update
 template <int CT, typename R>
 __device__ __forceinline__ double comp_ion_b_cell(const PoolView<R> &P, long gi, double vyi, double sum_dt,
                                                  bool update_ion) {
-  const Slots<R> sl{P.ion, P.cond, P.stride, gi};
-  if (CT == PKJ) {
+  if constexpr (CT == PKJ) {
+    Slots<R, PK_NION> sl(P.ion, P.cond, P.stride, gi);
+    double rv = P.rev[gi];
+    const double iext = P.iext[gi];
     if (update_ion) {
-      double ve = P.v[gi], ca = P.ca[gi], rv = P.rev[gi];
+      double ve = P.v[gi], ca = P.ca[gi];
       Pkj<R>::ion(sl, ve, ca, rv, P.shell[gi], (P.flags[gi] & 1) != 0, vyi, sum_dt);
       P.v[gi] = ve; P.ca[gi] = ca; P.rev[gi] = rv;
     }
-    return (double)Pkj<R>::b(sl, vyi, P.iext[gi], P.rev[gi]);
-  } else if (CT == IO) {
+    const R b = Pkj<R>::b(sl, vyi, iext, rv);
+    if (update_ion) sl.store();
+    return up(b);
+  } else if constexpr (CT == IO) {
+    Slots<R, IO_NION> sl(P.ion, P.cond, P.stride, gi);
+    const double iext = P.iext[gi];
     if (update_ion) {
       double ve = P.v[gi], ca = P.ca[gi];
       Io<R>::ion(sl, ve, ca, P.ctype[gi], vyi, sum_dt);
       P.v[gi] = ve; P.ca[gi] = ca;
     }
-    return (double)Io<R>::b(sl, vyi, P.iext[gi]);
-  } else if (CT == GR) {
+    const R b = Io<R>::b(sl, vyi, iext);
+    if (update_ion) sl.store();
+    return up(b);
+  } else if constexpr (CT == GR) {
+    Slots<R, GR_NION> sl(P.ion, P.cond, P.stride, gi);
+    const double iext = P.iext[gi];
     if (update_ion) {
       const int t = P.ctype[gi];
       double ve = P.v[gi];
@@ -173,15 +183,22 @@ __device__ __forceinline__ double comp_ion_b_cell(const PoolView<R> &P, long gi,
       Gr<R>::ion(sl, ve, P.ca[gi], vyi, sum_dt);
       P.v[gi] = ve;
     }
-    return (double)Gr<R>::b(sl, vyi, P.iext[gi]);
+    const R b = Gr<R>::b(sl, vyi, iext);
+    if (update_ion) sl.store();
+    return up(b);
   } else {  // GO
+    Slots<R, GO_NION> sl(P.ion, P.cond, P.stride, gi);
+    double rv = P.rev[gi];
+    const double iext = P.iext[gi];
     if (update_ion) {
-      double ve = P.v[gi], ca = P.ca[gi], ca2 = P.ca2[gi], rv = P.rev[gi], cao = P.ca_old[gi];
+      double ve = P.v[gi], ca = P.ca[gi], ca2 = P.ca2[gi], cao = P.ca_old[gi];
       Go<R>::ion(sl, ve, ca, ca2, rv, P.area[gi], vyi, sum_dt);
       Go<R>::kahp(sl, ca, cao, sum_dt);
       P.v[gi] = ve; P.ca[gi] = ca; P.ca2[gi] = ca2; P.rev[gi] = rv; P.ca_old[gi] = cao;
     }
-    return (double)Go<R>::b(sl, vyi, P.iext[gi], P.rev[gi]);
+    const R b = Go<R>::b(sl, vyi, iext, rv);
+    if (update_ion) sl.store();
+    return up(b);
   }
 }
 

@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 
 #include "integrator.cuh"
+#include "group_sys.cuh"
 #include "quad_sys.cuh"
 
 namespace gbrkc {
@@ -54,6 +55,94 @@ __device__ __forceinline__ void role_block(const PoolView<R> &P, int *q, double 
   }
 }
 
+// The systems of a role whose teams (warps or CTAs) keep them in registers.
+// With more systems than teams a launch in whole systems ends with most teams
+// idle (200 Purkinje cells on 152 CTAs take two cells' time).  So a team goes
+// on with another system after P.ivc intervals of one, as long as systems
+// wait: it takes the longest-waiting one and leaves its own at the end of the
+// line, and goes on with its own when none waits.  Every unfinished system is
+// thus in the line or with a running team, nothing waits for a particular
+// one, and the line only shortens.  Counters (zeroed per launch): [0] taken,
+// [1] left; place i of the line is system i for i < nsys, else line[i - nsys]
+// - 1 once it is written; at[s] is the system's next interval.
+template <typename R>
+__device__ __forceinline__ int line_take(const PoolView<R> &P) {
+  int *head = P.grp_line;
+  const int *tail = P.grp_line + 1;
+  int h = *(volatile int *)head;
+  for (;;) {
+    if (h >= P.nsys + *(volatile const int *)tail) return -1;
+    const int got = atomicCAS(head, h, h + 1);
+    if (got == h) break;
+    h = got;
+  }
+  if (h < P.nsys) return h;
+  // (its writer has counted it already: the store follows at once)
+  int v = 0;
+  for (long it = 0; it < GRID_SPIN_LIMIT && v == 0; it++)
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(P.grp_line + 2 + h) : "memory");
+  if (v == 0) *(volatile int *)P.grp_abort = 1;
+  return v - 1;
+}
+template <typename R>
+__device__ __forceinline__ void line_leave(const PoolView<R> &P, int s, int next_iv) {
+  P.grp_line[2 + s] = next_iv;
+  const int i = atomicAdd(P.grp_line + 1, 1);
+  __threadfence();
+  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(P.grp_line + 2 + P.nsys + i), "r"(s + 1) : "memory");
+}
+// (one thread of the team) the next system and its first interval: after a
+// finished system (s < 0) or after a piece of s up to interval k; s -1: none
+template <typename R>
+__device__ __forceinline__ void line_next(const PoolView<R> &P, int &s, int &k) {
+  const int mine = s, at = k;
+  const int got = line_take(P);
+  if (got >= 0) {
+    s = got;
+    k = *(volatile int *)(P.grp_line + 2 + got);
+    if (mine >= 0) line_leave(P, mine, at);
+  } else if (mine < 0) {
+    s = -1;
+  }
+}
+
+// A role of teams with their system's vectors in registers (group_sys.cuh), at
+// most K elements a thread: P.tiles teams of P.grid_bw threads a CTA.  A
+// Golgi cell takes five warps: alone on its SM each issues an FP64 instruction
+// in 95 cycles, so that the cells whose step size is at its floor (up to 1024
+// attempts a ms where the median cell takes 115), whose serial chains set the
+// launch's time, run five times as fast as on a warp of eight systems' warps;
+// and the warps of a team run the same instructions at the same time, where
+// eight systems' warps each fetched their own (40% of their cycles).
+template <int CT, typename R, int K>
+__device__ __forceinline__ void role_teams(const PoolView<R> &P, double *smem, double t0, int n_iv, int iv0) {
+  __shared__ int s_next[MEGA_BLOCK / 32], s_at[MEGA_BLOCK / 32];
+  __shared__ double s_wp[K == 1 ? MEGA_BLOCK / 32 : K * MEGA_BLOCK / 32], s_res[MEGA_BLOCK / 32];
+  const int bw = P.grid_bw, team = (int)threadIdx.x / bw, first = team * bw;
+  if (team >= P.tiles) return;
+  double *my = smem + (long)team * P.grp_stride;
+  GroupSys<CT, R, K, GRP_CTA> S(P, my + GRP_COEF_M_DOUBLES, s_wp + first / 32, s_res + team, my, GRP_COEF_M, nullptr,
+                                first, bw, 1 + team, 0, 1);
+  int s = -1, k = 0;
+  for (;;) {
+    if (S.t == 0) {
+      line_next(P, s, k);
+      s_next[team] = s;
+      s_at[team] = k;
+    }
+    S.sync();
+    s = s_next[team];
+    k = s_at[team];
+    if (s < 0) break;
+    const int n = min(P.ivc, n_iv - k);
+    S.template run<false>(s, t0, k, n, iv0, false);
+    S.sync();
+    k += n;
+    if (k >= n_iv) s = -1;
+    else if (S.t == 0) __threadfence();
+  }
+}
+
 template <typename R>
 __global__ void __launch_bounds__(MEGA_BLOCK, 1) k_mega(const __grid_constant__ MegaView<R> M, double t0,
                                                          int n_iv, int iv0, int init) {
@@ -73,9 +162,28 @@ __global__ void __launch_bounds__(MEGA_BLOCK, 1) k_mega(const __grid_constant__ 
           run_lanes<GR, R, MEGA_BLOCK>(M.pool[GR], M.queue + GR, 0, 0, smem, t0, n_iv, iv0, init != 0);
       }
       break;
-    case GO: role_tiles<GO, R, TEAM_WARP>(M.pool[GO], M.queue + GO, smem, t0, n_iv, iv0, init); break;
-    case PKJ: role_block<PKJ, R>(M.pool[PKJ], M.queue + PKJ, smem, t0, n_iv, iv0, init); break;
-    default: role_block<IO, R>(M.pool[IO], M.queue + IO, smem, t0, n_iv, iv0, init); break;
+    // (initialisation, and systems of more compartments than a team's
+    // registers take, go through the teams with their vectors in memory)
+    case GO:
+      if (M.pool[GO].grp_fast && !init)
+        role_teams<GO, R, 1>(M.pool[GO], smem, t0, n_iv, iv0);
+      else
+        role_tiles<GO, R, TEAM_WARP>(M.pool[GO], M.queue + GO, smem, t0, n_iv, iv0, init);
+      break;
+    case PKJ:
+      if (M.pool[PKJ].grp_fast && !init)
+        role_teams<PKJ, R, GRP_CTA_ROWS>(M.pool[PKJ], smem, t0, n_iv, iv0);
+      else
+        role_block<PKJ, R>(M.pool[PKJ], M.queue + PKJ, smem, t0, n_iv, iv0, init);
+      break;
+    default:
+      if (M.pool[IO].grp_fast == 1 && !init)
+        role_teams<IO, R, 1>(M.pool[IO], smem, t0, n_iv, iv0);
+      else if (M.pool[IO].grp_fast && !init)
+        role_teams<IO, R, GRP_CTA_ROWS>(M.pool[IO], smem, t0, n_iv, iv0);
+      else
+        role_block<IO, R>(M.pool[IO], M.queue + IO, smem, t0, n_iv, iv0, init);
+      break;
   }
   __syncthreads();
   if (threadIdx.x == 0) M.t_end[blockIdx.x] = global_ns();

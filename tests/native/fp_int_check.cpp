@@ -43,6 +43,17 @@ static void check(double a, double b) {
   if (!same(abs_max(a, b), p > q ? p : q)) fail("abs_max", a, b);
 }
 
+// quotients by the kinds of constant that the gating uses: a power of two, a
+// short mantissa, a full one
+static void constants(double a) {
+#define GB_C(b) \
+  if (!same(cdiv(a, b), a / (b))) fail("cdiv " #b, a, b);
+  GB_C(8.0) GB_C(-16.0) GB_C(0.25) GB_C(3.0) GB_C(6.0) GB_C(7.0) GB_C(10.0) GB_C(-10.0) GB_C(12.5) GB_C(14.5) GB_C(20.0)
+  GB_C(30.0) GB_C(17.0) GB_C(62.5) GB_C(83.0) GB_C(900.0) GB_C(-12.0) GB_C(14.9) GB_C(23.32708) GB_C(0.85) GB_C(0.099986667)
+  GB_C(4.2) GB_C(-5.8) GB_C(1.9297e-1) GB_C(1048577.0) GB_C(2097151.0)
+#undef GB_C
+}
+
 int main() {
   std::vector<double> v = {0.0, -0.0, 1.0, -1.0, 0.1, 1e-9, 65.0, -65.3, 1e300, -1e300, INFINITY, -INFINITY, NAN,
                            0x1p-1074, 0x1p-1022, 0x1p-149, 0x1p-150, 0x1.8p-150, 0x1p-126, 0x1.fffffffffffffp-127,
@@ -56,12 +67,16 @@ int main() {
                    0x1.6a09e667f3bccp+0, 0x1.6a09e667f3bcdp+0, 0x1.6a09e667f3bcep+0}) v.push_back(x);
   for (double a : v) {
     canon(a);
+    constants(a);
     for (double b : v) check(a, b);
   }
   std::mt19937_64 rng(7);
   for (int i = 0; i < 500000; i++) {
     uint64_t u = rng(), w = rng();
     canon(fpi_double(u));
+    constants(fpi_double(u));
+    constants(1.0 + (double)(u >> 12) * 0x1p-52);
+    constants(-100.0 + (double)(w >> 11) * 0x1p-45);
     canon((double)(int64_t)w * 0x1p-63 * 800);
     canon(1.0 + (double)(int64_t)u * 0x1p-64);
     check(fpi_double(u), fpi_double(w));
