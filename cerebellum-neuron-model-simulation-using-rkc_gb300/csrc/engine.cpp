@@ -20,6 +20,7 @@
 #include <map>
 #include <type_traits>
 #include <memory>
+#include <numeric>
 #include <string>
 #include <vector>
 
@@ -384,7 +385,25 @@ struct DeviceMem {
   }
 };
 
-struct PoolHost {
+// A pool's team and launch shape, and the tables of a group team
+// (group_sys.cuh; engine.h, PoolView) with their device copies.
+struct GroupCfg {
+  int team = TEAM_BLOCK, block = 256, grid = 1;
+  size_t smem = 0;
+  int ws_in_smem = 0;
+  long ws_tile = 0;
+  int grid_bw = GRID_BLOCK;                 // elements of a chunk, threads of a CTA
+  int grid_maxdeg = 0, grp_ld = 0, grp_recv_max = 0, grp_nslots = 0, grp_ctas = 1;
+  std::vector<GroupTab> grp_tab;
+  std::vector<int> grp_chunk0, grp_col, grp_slot, grp_sptr, grp_send, grp_rptr, grp_rslot, grp_gap;
+  GroupTab *d_tab = nullptr;
+  int *d_chunk0 = nullptr, *d_col = nullptr, *d_slot = nullptr, *d_sptr = nullptr, *d_send = nullptr, *d_rptr = nullptr,
+      *d_rslot = nullptr, *d_gap = nullptr;
+  unsigned long long *d_grp_words = nullptr;   // the abort flag, published values and chunk sums
+  size_t grp_bytes = 0;
+};
+
+struct PoolHost : GroupCfg {
   int type;
   bool f64 = false;                    // the pool's gating arithmetic: FP64 (vd) or FP32 (vf)
   std::vector<int> systems;            // engine system ids
@@ -410,23 +429,18 @@ struct PoolHost {
   std::vector<double> stim_amp, stim_t0, stim_t1;
   long ws_total = 0;
   int max_nc = 0, min_nc = 1 << 30, max_ncell = 0;
-  // launch configuration
-  int team = TEAM_BLOCK, block = 256, grid = 1;
-  int grid_bw = GRID_BLOCK;                 // grid team: threads of each CTA that own elements
-  // grid team (engine.h, PoolView): the longest row, the fullest CTA's
-  // elements, the most values a CTA receives, and the hand-over tables
-  int grid_maxdeg = 0, grp_ld = 0, grp_recv_max = 0, grp_nslots = 0;
-  int grp_ctas = 1, grp_fast = 0;
-  long grp_stride = 0;                     // persistent launch: doubles of shared memory a team
-  int *d_line = nullptr;                   // persistent launch: abort flag, counters and line of a register role
+  // persistent launch
+  int grp_fast = 0;
+  long grp_stride = 0;                     // doubles of shared memory a team
+  int *d_line = nullptr;                   // abort flag, counters and line of the pool's teams
   bool pieces = false;                     // the last launch left systems in the line
-  std::vector<GroupTab> grp_tab;
-  std::vector<int> grp_chunk0, grp_col, grp_slot, grp_sptr, grp_send, grp_rptr, grp_rslot, grp_gap;
-  unsigned long long *d_grp_words = nullptr;   // published values, chunk sums and the abort flag
-  size_t grp_bytes = 0;
-  size_t smem = 0;
-  int ws_in_smem = 0;
-  long ws_tile = 0;
+  // cluster teams for the launches of a persistent engine whose systems'
+  // chains are uneven, and the one the next launch takes (plan_launch)
+  std::vector<GroupCfg> alt;
+  int use_alt = -1;
+  int *d_order = nullptr;                  // the order of its line
+  bool ordered = false;                    // ... is not 0, 1, 2, ...
+  std::vector<long long> steps, stages;    // counters after the last advance
   // device views
   PoolView<double> vd{};
   PoolView<float> vf{};
@@ -845,7 +859,7 @@ bool group_tables(PoolHost &P, int bw, int ctas, bool grid) {
     for (int e = g0; e < g0 + ng; e++)
       if (P.gap_pre[e] >= 0) t_gap[e] = place(cta_of(P.gap_post[e]), P.gap_pre[e]);
   }
-  if (rows > (grid ? GRID_MAX_ROWS : 2) || (rows > 1 && maxdeg > 15)) return false;   // (row lengths: four bits each)
+  if (rows > (grid ? GRID_MAX_ROWS : ctas > 1 && P.type == PKJ ? 4 : 2) || (rows > 1 && maxdeg > 15)) return false;   // (row lengths: four bits each)
   const int ld = rows * bw;
   const size_t smem = grid_smem(ld, most, maxdeg, (grid || ctas == 1) ? 0 : ctas);
   if (smem > GRID_SMEM_MAX || ld + most + 2 > GRID_PLACES) return false;
@@ -859,7 +873,7 @@ bool group_tables(PoolHost &P, int bw, int ctas, bool grid) {
   P.grp_ld = ld;
   P.grp_recv_max = most;
   P.grp_nslots = nslots;
-  P.team = (grid ? TEAM_GRID1 : ctas > 1 ? TEAM_CLU1 : TEAM_CTA1) + (rows == 1 ? 0 : rows == 2 ? 1 : 7);
+  P.team = (grid ? TEAM_GRID1 : ctas > 1 ? TEAM_CLU1 : TEAM_CTA1) + (rows == 1 ? 0 : rows == 2 ? 1 : grid ? 7 : 3);
   P.block = bw;
   P.grid = ctas;
   P.grid_bw = bw;
@@ -869,17 +883,31 @@ bool group_tables(PoolHost &P, int bw, int ctas, bool grid) {
   return true;
 }
 
+// Estimated cycles of step attempts and stages of one system on a team of
+// `rows` elements a thread, with `warps` warps sharing its SM: comm 0 within a
+// CTA, 1 a cluster, 2 the grid.
+struct TeamCost {
+  double attempt, stage;
+  double of(double attempts, double stages) const { return attempts * attempt + stages * stage; }
+};
+TeamCost team_cost(const PoolHost &P, double rows, double warps, int comm) {
+  static const double ion[NTYPES] = {350.0, 860.0, 840.0, 170.0};
+  static const double hand[3] = {300.0, 900.0, 2500.0}, sum[3] = {600.0, 2500.0, 5000.0};
+  const double rate = std::max(64.0, 19.0 * warps);
+  return TeamCost{(rows * (22.0 + (P.f64 ? ion[P.type] : 60.0)) + 90.0) * rate + hand[comm] + 1.3 * sum[comm],
+                  rows * 12.0 * rate + hand[comm]};
+}
+
 // A group team (group_sys.cuh) for a pool alone in its engine, where it
 // shortens the launch: the shape is the one of least estimated time, and the
 // pool keeps its other teams (in the persistent launch, or an old-style
-// cluster) where theirs is less.  The estimate
-// counts FP64 warp instructions of a step attempt, 64 cycles each on an SM
-// with up to three warps and 19 per warp beyond (measured): 17 stages of 12
-// per element row, 22 for the error norm, the row's share of the ion updates
-// (FP64 gating: 0.15 to 0.5 updates of 1200 to 2300 an attempt), and 90 of the
-// controller, which every warp repeats; and the latency of handing over the
-// stage vector and the sums (CTA 60 and 500 cycles, cluster 400 and 1200,
-// grid 1400 and 4000).  A pool that fills the GPU thus stays in the persistent
+// cluster) where theirs is less.  The estimate counts FP64 warp instructions
+// of a step attempt, 64 cycles each on an SM with up to three warps and 19 per
+// warp beyond (measured): 12 a stage and element row, 22 for the error norm,
+// the row's share of the ion updates (FP64 gating: 0.15 to 0.5 updates of
+// 1200 to 2300 an attempt), and 90 of the controller, which every warp
+// repeats; and the measured latency of handing over the stage vector and the
+// sums.  A pool that fills the GPU thus stays in the persistent
 // launch, whose teams take systems in turn (77 Golgi cells: clusters of five
 // CTAs of a warp; 2048: five warps each).  A lone system of GRID_MIN_NC
 // compartments always takes the grid.  GBRKC_GROUP=0 and GBRKC_GRID=0 switch
@@ -907,53 +935,77 @@ bool group_team(const gbrkc_engine *E, PoolHost &P) {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (sms < 1) return false;
-  static const double ion[NTYPES] = {350.0, 860.0, 840.0, 170.0};
-  const double stages = 17.0, row = stages * 12.0 + 22.0 + (P.f64 ? ion[P.type] : 40.0), ctl = 90.0;
-  auto time = [&](double rows, double warps, double rounds, double hand, double sum) {
-    return rounds * ((rows * row + ctl) * std::max(64.0, 19.0 * warps) + (stages + 1) * hand + 1.3 * sum);
-  };
   auto up = [](long a, long b) { return (a + b - 1) / b; };
+  auto time = [&](double rows, double warps, double rounds, int comm) {
+    return rounds * team_cost(P, rows, warps, comm).of(1.0, 17.0);
+  };
   // the persistent launch's teams: one element a thread on as many warps as
   // that takes, or the whole block; systems beyond the places take turns
   const bool one = P.type != PKJ && nc <= MEGA_BLOCK;
   const long warps = one ? up(nc, 32) : 8, per = 8 / warps;
-  const double other = time((double)up(nc, 32 * warps), (double)(warps * std::min(per, up(nsys, sms))),
-                            std::max(1.0, nsys / (double)(per * sms)), one ? 60 : 150, 500);
+  const double mega_warps = (double)(warps * std::min(per, up(nsys, sms))), mega_rows = (double)up(nc, 32 * warps);
+  const double other = time(mega_rows, mega_warps, std::max(1.0, nsys / (double)(per * sms)), 0);
   double best = 0.9 * other;
   int kind = 0, bbw = 0, bctas = 1;
+  struct Wide { double time; int bw, ctas, cap; };
+  std::map<int, Wide> wide;                // per CTAs of a cluster: the best shape with one long system
   for (int bw = 32; bw <= GRID_BLOCK; bw += 32) {
     const long rows = up(nc, bw), fit = std::max(1, 65536 / (256 * bw));   // CTAs an SM's registers hold
     if (rows <= 2) {
       const long per = std::min(fit, up(nsys, sms));
-      const double t = time((double)rows, (double)(per * (bw / 32)), (double)up(nsys, per * sms), 60, 500);
+      const double t = time((double)rows, (double)(per * (bw / 32)), std::max(1.0, nsys / (double)(per * sms)), 0);
       if (t < best) { best = t; kind = 1; bbw = bw; bctas = 1; }
     }
     if (bw & (bw - 1)) continue;
-    for (long r = 1; r <= 2; r++) {
+    for (long r = 1; r <= (P.type == PKJ ? 4 : 2); r++) {
       const long ctas = up(rows, r);
       if (ctas < 2 || ctas > 16 || up(rows, ctas) != r) continue;
-      const long per = std::min(fit, up((long)nsys * ctas, sms));
-      const long at_once = std::max(1L, per * sms / ctas);
-      const double t = time((double)r, (double)(per * (bw / 32)), (double)up(nsys, at_once), 400, 1200);
+      const int team = r == 1 ? TEAM_CLU1 : r == 2 ? TEAM_CLU2 : TEAM_CLU4;
+      const size_t smem = grid_smem(r * bw, 2 * bw, 6, (int)ctas);
+      const int cap = P.f64 ? group_capacity<double>(P.type, team, (int)ctas, bw, smem)
+                            : group_capacity<float>(P.type, team, (int)ctas, bw, smem);
+      if (cap < 1) continue;
+      const long at_once = std::min<long>(nsys, cap);
+      const double w = (double)(up(at_once * ctas, sms) * (bw / 32));
+      const double t = time((double)r, w, std::max(1.0, nsys / (double)at_once), 1);
       if (t < best) { best = t; kind = 2; bbw = bw; bctas = (int)ctas; }
+      // the same with one system six times as long as the mean
+      const double th = time((double)r, w, std::max(6.0, nsys / (double)at_once), 1);
+      const auto it = wide.find((int)ctas);
+      if (it == wide.end() || th < it->second.time) wide[(int)ctas] = Wide{th, bw, (int)ctas, cap};
     }
   }
   if (grid_ok) {
     int bw = 0, ctas = 0;
     if (grid_shape(nc, sms, &bw, &ctas)) {
-      const double t = time((double)up(nc, (long)bw * ctas), bw / 32.0, 1, 1400, 4000);
+      const double t = time((double)up(nc, (long)bw * ctas), bw / 32.0, 1, 2);
       if (t < best && to_grid()) return true;
     }
   }
-  if (kind == 0) return false;
-  PoolHost before = P;
+  if (kind == 0) {
+    // the persistent launch; a cluster team beside it where that would be
+    // shorter with one system six times as long as the mean (200 Purkinje
+    // cells: 24 attempts a ms each at rest, up to 470 in a spiking one)
+    const double at = time(mega_rows, mega_warps, std::max(6.0, nsys / (double)(per * sms)), 0);
+    for (const auto &w : wide) {
+      if (w.second.time > 0.9 * at) continue;
+      const GroupCfg before = P;
+      if (group_tables(P, w.second.bw, w.second.ctas, false)) {
+        P.alt.push_back(P);
+        P.alt.back().grid = std::min(nsys, w.second.cap) * w.second.ctas;
+      }
+      static_cast<GroupCfg &>(P) = before;
+    }
+    return false;
+  }
+  const GroupCfg before = P;
   if (!group_tables(P, bbw, bctas, false)) return false;
   int groups = nsys;
   if (kind == 2) {
     const int cap = P.f64 ? group_capacity<double>(P.type, P.team, bctas, bbw, P.smem)
                           : group_capacity<float>(P.type, P.team, bctas, bbw, P.smem);
     if (cap < 1) {
-      P = before;
+      static_cast<GroupCfg &>(P) = before;
       return false;
     }
     groups = std::min(nsys, cap);
@@ -1143,6 +1195,41 @@ int assemble_pool(gbrkc_engine *E, PoolHost &P) {
   return 0;
 }
 
+// A group team's tables onto the device.
+int upload_group(gbrkc_engine *E, GroupCfg &C) {
+  DeviceMem &M = E->mem;
+  int rc = 0;
+  if ((rc = M.upload(C.grp_tab, &C.d_tab)) || (rc = M.upload(C.grp_chunk0, &C.d_chunk0)) ||
+      (rc = M.upload(C.grp_col, &C.d_col)) || (rc = M.upload(C.grp_slot, &C.d_slot)) ||
+      (rc = M.upload(C.grp_sptr, &C.d_sptr)) || (rc = M.upload(C.grp_send, &C.d_send)) ||
+      (rc = M.upload(C.grp_rptr, &C.d_rptr)) || (rc = M.upload(C.grp_rslot, &C.d_rslot)) ||
+      (rc = M.upload(C.grp_gap, &C.d_gap)))
+    return rc;
+  // one block, zeroed before each launch: the abort flag, and in the grid
+  // team the published values and chunk sums
+  const size_t n = team_is_grid(C.team) ? 4 * (size_t)C.grp_nslots + 4 * GRID_MAX_BLOCKS : 0;
+  const std::vector<unsigned long long> words(2 + n, 0ull);
+  C.grp_bytes = words.size() * sizeof(unsigned long long);
+  return M.upload(words, &C.d_grp_words);
+}
+
+// The view's group fields for that team.
+template <typename R>
+void apply_group(const GroupCfg &C, PoolView<R> &V) {
+  V.grid_bw = C.grid_bw;
+  V.grid_maxdeg = C.grid_maxdeg;
+  V.grp_ctas = C.grp_ctas;
+  V.grp_ld = C.grp_ld;
+  V.grp_recv_max = C.grp_recv_max;
+  V.grp_nslots = C.grp_nslots;
+  V.grp_tab = C.d_tab;
+  V.grp_chunk0 = C.d_chunk0; V.grp_col = C.d_col; V.grp_slot = C.d_slot; V.grp_sptr = C.d_sptr; V.grp_send = C.d_send;
+  V.grp_rptr = C.d_rptr; V.grp_rslot = C.d_rslot; V.grp_gap = C.d_gap;
+  V.grp_abort = (int *)C.d_grp_words;
+  V.grp_halo = C.d_grp_words + 2;
+  V.grp_red = V.grp_halo + 4 * (size_t)C.grp_nslots;
+}
+
 template <typename R>
 int upload_pool(gbrkc_engine *E, PoolHost &P, PoolView<R> &V) {
   DeviceMem &M = E->mem;
@@ -1163,24 +1250,21 @@ int upload_pool(gbrkc_engine *E, PoolHost &P, PoolView<R> &V) {
   UP(P.sys_cell0, V.sys_cell0); UP(P.sys_gap0, V.sys_gap0); UP(P.sys_ngap, V.sys_ngap);
   UP(P.sys_ws, V.sys_ws); UP(P.ctl, V.ctl);
   if (team_is_group(P.team)) {
-    V.grid_bw = P.grid_bw;
-    V.grid_maxdeg = P.grid_maxdeg;
-    V.grp_ctas = P.grp_ctas;
-    V.grp_ld = P.grp_ld;
-    V.grp_recv_max = P.grp_recv_max;
-    V.grp_nslots = P.grp_nslots;
-    UP(P.grp_tab, V.grp_tab); UP(P.grp_chunk0, V.grp_chunk0); UP(P.grp_col, V.grp_col); UP(P.grp_slot, V.grp_slot);
-    UP(P.grp_sptr, V.grp_sptr); UP(P.grp_send, V.grp_send);
-    UP(P.grp_rptr, V.grp_rptr); UP(P.grp_rslot, V.grp_rslot); UP(P.grp_gap, V.grp_gap);
-    // one block, zeroed before each launch: the abort flag, and in the grid
-    // team the published values and chunk sums
-    const size_t n = team_is_grid(P.team) ? 4 * (size_t)P.grp_nslots + 4 * GRID_MAX_BLOCKS : 0;
-    const std::vector<unsigned long long> words(2 + n, 0ull);
-    UP(words, P.d_grp_words);
-    P.grp_bytes = words.size() * sizeof(unsigned long long);
-    V.grp_abort = (int *)P.d_grp_words;
-    V.grp_halo = P.d_grp_words + 2;
-    V.grp_red = V.grp_halo + 4 * (size_t)P.grp_nslots;
+    if ((rc = upload_group(E, P))) return rc;
+    apply_group(P, V);
+  }
+  for (GroupCfg &C : P.alt)
+    if ((rc = upload_group(E, C))) return rc;
+  if (team_is_group(P.team) || P.grp_fast) {
+    // abort flag and padding, counters, next intervals, the line
+    const std::vector<int> line(4 + (1 + LINE_PIECES) * P.systems.size(), 0);
+    UP(line, P.d_line);
+    V.grp_line = P.d_line + 2;
+    V.ivc = 1;
+    std::vector<int> order(P.systems.size());
+    std::iota(order.begin(), order.end(), 0);
+    UP(order, P.d_order);
+    V.grp_order = P.d_order;
   }
   V.grp_fast = 0;
   if (!team_is_group(P.team) && P.grp_fast) {
@@ -1190,12 +1274,7 @@ int upload_pool(gbrkc_engine *E, PoolHost &P, PoolView<R> &V) {
     V.grp_stride = P.grp_stride;
     V.grid_bw = P.grid_bw;
     V.tiles = MEGA_BLOCK / P.grid_bw;
-    V.ivc = 1;
-    // abort flag and padding, counters, next intervals, the line
-    const std::vector<int> line(4 + (1 + LINE_PIECES) * P.systems.size(), 0);
-    UP(line, P.d_line);
     V.grp_abort = P.d_line;
-    V.grp_line = P.d_line + 2;
   }
   std::vector<double> zws(P.ws_total, 0.0);
   UP(zws, V.ws);
@@ -1428,8 +1507,27 @@ int launch_mega_all(gbrkc_engine *E, double t0, int n_iv, int iv0, int init) {
   return 0;
 }
 
+// One pool's kernel with the team C.
+template <typename R>
+int launch_cfg(gbrkc_engine *E, PoolHost &P, const GroupCfg &C, cudaStream_t st, double t0, int n_iv, int iv0, int init) {
+  if (!team_is_group(C.team))
+    return launch_pool<R>(P.type, pool_view<R>(P), C.team, C.grid, C.block, C.smem, st, t0, n_iv, iv0, init);
+  CUDA_TRY(cudaMemsetAsync(C.d_grp_words, 0, C.grp_bytes, st));
+  PoolView<R> V = pool_view<R>(P);
+  apply_group(C, V);
+  const int nsys = (int)P.systems.size(), groups = C.grid / C.grp_ctas;
+  const bool pieces = nsys > groups && n_iv > 1;
+  V.ivc = pieces ? std::max(1, (n_iv + LINE_PIECES - 1) / LINE_PIECES) : std::max(1, n_iv);
+  if (!init && !team_is_grid(C.team))
+    CUDA_TRY(cudaMemsetAsync(P.d_line, 0, (4 + (1 + (pieces ? LINE_PIECES : 0)) * (size_t)nsys) * sizeof(int), st));
+  return launch_pool<R>(P.type, V, C.team, C.grid, C.block, C.smem, st, t0, n_iv, iv0, init);
+}
+
 int launch_all(gbrkc_engine *E, double t0, int n_iv, int iv0, int init) {
-  if (E->mega)
+  // an engine of one type whose last launch showed uneven chains
+  bool alt = false;
+  for (const PoolHost &P : E->pools) alt |= P.use_alt >= 0 && !init;
+  if (E->mega && !alt)
     return (E->precision == GBRKC_FP64) ? launch_mega_all<double>(E, t0, n_iv, iv0, init)
                                         : launch_mega_all<float>(E, t0, n_iv, iv0, init);
   CUDA_TRY(cudaEventRecord(E->ev_start, E->streams[0]));
@@ -1442,12 +1540,10 @@ int launch_all(gbrkc_engine *E, double t0, int n_iv, int iv0, int init) {
         (P.block != MEGA_BLOCK || !P.ws_in_smem ||
          P.smem < (size_t)MEGA_BLOCK * (size_t)P.ws_tile * sizeof(double)))
       return fail(GBRKC_ESTATE, "single-lane pool %d: launch shape does not cover its workspaces", t);
-    if (team_is_group(P.team)) CUDA_TRY(cudaMemsetAsync(P.d_grp_words, 0, P.grp_bytes, E->streams[t]));
+    const GroupCfg &C = alt ? P.alt[P.use_alt] : P;
     CUDA_TRY(cudaEventRecord(E->ev_k0[t], E->streams[t]));
-    if (P.f64)
-      rc = launch_pool<double>(t, P.vd, P.team, P.grid, P.block, P.smem, E->streams[t], t0, n_iv, iv0, init);
-    else
-      rc = launch_pool<float>(t, P.vf, P.team, P.grid, P.block, P.smem, E->streams[t], t0, n_iv, iv0, init);
+    rc = P.f64 ? launch_cfg<double>(E, P, C, E->streams[t], t0, n_iv, iv0, init)
+               : launch_cfg<float>(E, P, C, E->streams[t], t0, n_iv, iv0, init);
     if (rc) return fail(GBRKC_ECUDA, "launch (type %d): %s", t, cudaGetErrorString((cudaError_t)rc));
     CUDA_TRY(cudaEventRecord(E->ev_k1[t], E->streams[t]));
     if (t != 0) CUDA_TRY(cudaStreamWaitEvent(E->streams[0], E->ev_k1[t], 0));
@@ -1459,9 +1555,11 @@ int launch_all(gbrkc_engine *E, double t0, int n_iv, int iv0, int init) {
   for (int t = 0; t < NTYPES; t++) {
     E->last_kernel_ms[t] = 0.0f;
     if (!E->pools[t].systems.empty()) CUDA_TRY(cudaEventElapsedTime(&E->last_kernel_ms[t], E->ev_k0[t], E->ev_k1[t]));
-    if (team_is_group(E->pools[t].team) && E->pools[t].grp_ctas > 1 && !E->pools[t].systems.empty()) {
+    if (E->pools[t].systems.empty()) continue;
+    const GroupCfg &C = alt ? E->pools[t].alt[E->pools[t].use_alt] : E->pools[t];
+    if (team_is_group(C.team)) {
       int gave_up = 0;
-      CUDA_TRY(cudaMemcpy(&gave_up, E->pools[t].d_grp_words, sizeof gave_up, cudaMemcpyDeviceToHost));
+      CUDA_TRY(cudaMemcpy(&gave_up, C.d_grp_words, sizeof gave_up, cudaMemcpyDeviceToHost));
       if (gave_up)
         return fail(GBRKC_ECUDA, "group team (type %d): a wait gave up; the system is stopped", t);
     }
@@ -1929,6 +2027,84 @@ static int build_impl(gbrkc_engine *E) {
 
 extern "C" int gbrkc_build(gbrkc_engine *E) { return no_throw([&] { return build_impl(E); }); }
 
+// The next launch of a pool whose systems outnumber its teams, from the
+// attempts and stages that each system took in the last one.  A launch takes
+// about the larger of its longest system's time and the systems' time over
+// the teams; where a system is long, (1) the longest systems come first in
+// the line and are held, and (2) a pool with cluster teams beside the
+// persistent launch takes the team for which that is least: wider teams
+// shorten the longest system and do less in all.  The estimates are within a
+// third of the measured times, so a cluster team has to promise a quarter.
+// (200 Purkinje cells, mixed, a ms: at rest 7.0 ms in the persistent launch,
+// 7.6 in clusters of two CTAs, 9.5 of thirteen; with some spiking at the
+// step floor 42.9 to 53.6 against 20.7 to 28.8.)
+static int plan_launch(gbrkc_engine *E, PoolHost &P, const std::vector<Ctl> &c) {
+  const int n = (int)c.size();
+  if (!P.d_order || !(E->mega ? P.grp_fast != 0 : team_is_group(P.team))) return 0;
+  auto up = [](long a, long b) { return (a + b - 1) / b; };
+  const long ctas = std::max(1, E->role_ctas[P.type]);
+  const long tiles = E->mega ? std::min<long>(MEGA_BLOCK / P.grid_bw, up(n, ctas)) : 1;
+  const long teams = E->mega ? ctas * tiles : P.grid / P.grp_ctas;
+  if (n <= teams && P.alt.empty()) return 0;
+  if ((int)P.steps.size() != n) {
+    P.steps.assign(n, 0);
+    P.stages.assign(n, 0);
+  }
+  std::vector<double> att(n), stg(n), len(n);
+  for (int i = 0; i < n; i++) {
+    // (a system refilled since counts from 0 again)
+    att[i] = (double)(c[i].n_steps - (c[i].n_steps >= P.steps[i] ? P.steps[i] : 0));
+    stg[i] = (double)(c[i].n_stage - (c[i].n_stage >= P.stages[i] ? P.stages[i] : 0));
+    P.steps[i] = c[i].n_steps;
+    P.stages[i] = c[i].n_stage;
+  }
+  auto length = [&](const TeamCost &T, long places) {
+    double longest = 0.0, sum = 0.0;
+    for (int i = 0; i < n; i++) {
+      const double t = T.of(att[i], stg[i]);
+      longest = std::max(longest, t);
+      sum += t;
+    }
+    return std::max(longest, sum / (double)places);
+  };
+  const int comm = E->mega || P.grp_ctas == 1 ? 0 : team_is_grid(P.team) ? 2 : 1;
+  TeamCost T = team_cost(P, (double)(P.grp_ld / P.grid_bw), (double)(tiles * P.grid_bw / 32), comm);
+  long places = teams;
+  double best = 0.75 * length(T, teams);
+  P.use_alt = -1;
+  for (size_t j = 0; j < P.alt.size(); j++) {
+    const GroupCfg &C = P.alt[j];
+    const TeamCost A = team_cost(P, (double)(C.grp_ld / C.grid_bw),
+                                 (double)(up(C.grid, E->mega_grid) * C.grid_bw / 32), 1);
+    const double t = length(A, C.grid / C.grp_ctas);
+    if (t < best) {
+      best = t;
+      P.use_alt = (int)j;
+      T = A;
+      places = C.grid / C.grp_ctas;
+    }
+  }
+  double sum = 0.0, longest = 0.0;
+  for (int i = 0; i < n; i++) {
+    len[i] = T.of(att[i], stg[i]);
+    sum += len[i];
+    longest = std::max(longest, len[i]);
+  }
+  const double share = sum / (double)places;
+  const bool order = n > places && longest > 0.7 * share;
+  if (!order && !P.ordered) return 0;
+  std::vector<int> line(n);
+  std::iota(line.begin(), line.end(), 0);
+  if (order) {
+    std::stable_sort(line.begin(), line.end(), [&](int a, int b) { return len[a] > len[b]; });
+    for (int &i : line)
+      if (len[i] > std::max(0.5 * std::max(longest, share), 1.5 * sum / n)) i |= 1 << 30;
+  }
+  CUDA_TRY(cudaMemcpy(P.d_order, line.data(), n * sizeof(int), cudaMemcpyHostToDevice));
+  P.ordered = order;
+  return 0;
+}
+
 extern "C" int gbrkc_advance(gbrkc_engine *E, double t0, int n_iv) {
   if (!E || n_iv < 0) return fail(GBRKC_EINVAL, "bad arguments");
   if (!E->built) return fail(GBRKC_ESTATE, "engine not built");
@@ -1972,6 +2148,7 @@ extern "C" int gbrkc_advance(gbrkc_engine *E, double t0, int n_iv) {
     std::vector<Ctl> c(P.systems.size());
     CUDA_TRY(cudaMemcpy(c.data(), P.d_ctl, c.size() * sizeof(Ctl), cudaMemcpyDeviceToHost));
     if (P.retired.size() != c.size()) P.retired.assign(c.size(), 0);
+    if ((rc = plan_launch(E, P, c))) return rc;
     if (t == GR) {
       long active = 0;
       for (const Ctl &x : c) active += (x.status == 0 && x.iv_left != 0);
@@ -2285,6 +2462,7 @@ extern "C" int gbrkc_type_team(gbrkc_engine *E, int type) {
   if (!E->built) return fail(GBRKC_ESTATE, "engine not built");
   const PoolHost &P = E->pools[type];
   if (P.systems.empty()) return 0;
+  if (P.use_alt >= 0) return GBRKC_TEAM_CLUSTER;
   if (E->mega) return GBRKC_TEAM_MEGA;
   if (team_is_grid(P.team)) return GBRKC_TEAM_GRID;
   if (team_cluster_size(P.team) > 0 || team_is_clu(P.team)) return GBRKC_TEAM_CLUSTER;

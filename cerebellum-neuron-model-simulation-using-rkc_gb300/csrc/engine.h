@@ -149,7 +149,8 @@ struct PoolView {
   int tiles;                          // teams of a CTA that take systems
   long grp_stride;                    // doubles of shared memory a team
   int ivc;                            // intervals a team goes on with one system while others wait
-  int *grp_line;                      // [2] counters, [nsys] next intervals, [16 nsys] the line (kernels.cu, line_take)
+  int *grp_line;                      // [2] counters, [nsys] next intervals, [16 nsys] the line (group_sys.cuh, line_take)
+  const int *grp_order;               // [nsys] the line's first systems; bit 30: taken to its end without a turn
 };
 
 // How a pool takes its synaptic current (solve_rkc.cu): granule cells add
@@ -198,7 +199,8 @@ int launch_syn_update(const SynView &S, void *stream, double t, long long interv
 // cooperative launch (a system that is alone in its engine).
 enum TeamKind {
   TEAM_THREAD = 1, TEAM_LANE4 = 2, TEAM_TILE4 = 4, TEAM_WARP = 32, TEAM_BLOCK = 0,
-  TEAM_CLUSTER8 = 108, TEAM_CLUSTER16 = 116, TEAM_CTA1 = 201, TEAM_CTA2 = 202, TEAM_CLU1 = 301, TEAM_CLU2 = 302,
+  TEAM_CLUSTER8 = 108, TEAM_CLUSTER16 = 116, TEAM_CTA1 = 201, TEAM_CTA2 = 202,
+  TEAM_CLU1 = 301, TEAM_CLU2 = 302, TEAM_CLU4 = 304,
   TEAM_GRID1 = 401, TEAM_GRID2 = 402, TEAM_GRID8 = 408
 };
 // systems a warp takes when `lanes` of its lanes are in use, four lanes each

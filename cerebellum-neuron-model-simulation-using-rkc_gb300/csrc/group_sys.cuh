@@ -165,6 +165,11 @@ struct GroupSys {
     if constexpr (COMM == GRP_CTA) asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(bw) : "memory");
     else __syncthreads();
   }
+  // every CTA of the group
+  __device__ __forceinline__ void group_sync() const {
+    if constexpr (COMM == GRP_CLUSTER) cluster_sync_all();
+    else sync();
+  }
   // no CTA leaves while a peer may still store into its shared memory
   __device__ __forceinline__ void leave() const {
     if constexpr (COMM == GRP_CLUSTER) cluster_sync_all();
@@ -921,5 +926,61 @@ struct GroupSys {
     store(init);
   }
 };
+
+// The line of systems that teams take turns with.  With more systems than
+// teams a launch in whole systems ends with most teams idle (200 Purkinje
+// cells on 152 CTAs take two cells' time).  So a team goes on with another
+// system after P.ivc intervals of one, as long as systems wait: it takes the
+// longest-waiting one and leaves its own at the end of the line, and goes on
+// with its own when none waits.  Every unfinished system is thus in the line
+// or with a running team, nothing waits for a particular one, and the line
+// only shortens.  Counters (zeroed per launch): [0] taken, [1] left; place i
+// of the line is order[i] for i < nsys, else line[i - nsys] - 1 once it is
+// written; at[s] is the system's next interval.  Systems that took much longer
+// than the others in the launch before come first in order, and those that
+// may decide the launch's length are held: no other is taken for them.
+template <typename R>
+__device__ __forceinline__ int line_take(const PoolView<R> &P) {
+  int *head = P.grp_line;
+  const int *tail = P.grp_line + 1;
+  int h = *(volatile int *)head;
+  for (;;) {
+    if (h >= P.nsys + *(volatile const int *)tail) return -1;
+    const int got = atomicCAS(head, h, h + 1);
+    if (got == h) break;
+    h = got;
+  }
+  if (h < P.nsys) return P.grp_order[h];
+  // (its writer has counted it already: the store follows at once)
+  int v = 0;
+  for (long it = 0; it < GRID_SPIN_LIMIT && v == 0; it++)
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(P.grp_line + 2 + h) : "memory");
+  if (v == 0) *(volatile int *)P.grp_abort = 1;
+  return v - 1;
+}
+template <typename R>
+__device__ __forceinline__ void line_leave(const PoolView<R> &P, int s, int next_iv) {
+  P.grp_line[2 + s] = next_iv;
+  const int i = atomicAdd(P.grp_line + 1, 1);
+  __threadfence();
+  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(P.grp_line + 2 + P.nsys + i), "r"(s + 1) : "memory");
+}
+// (one thread of the team) the next system and its first interval: after a
+// finished system (s < 0) or after a piece of s up to interval k; s -1: none
+template <typename R>
+__device__ __forceinline__ void line_next(const PoolView<R> &P, int &s, int &k, bool &hold) {
+  const int mine = s, at = k;
+  if (mine >= 0 && hold) return;
+  int got = line_take(P);
+  if (got >= 0) {
+    hold = (got >> 30) != 0;
+    got &= (1 << 30) - 1;
+    s = got;
+    k = *(volatile int *)(P.grp_line + 2 + got);
+    if (mine >= 0) line_leave(P, mine, at);
+  } else if (mine < 0) {
+    s = -1;
+  }
+}
 
 }  // namespace gbrkc

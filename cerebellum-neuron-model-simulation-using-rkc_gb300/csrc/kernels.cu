@@ -55,57 +55,6 @@ __device__ __forceinline__ void role_block(const PoolView<R> &P, int *q, double 
   }
 }
 
-// The systems of a role whose teams (warps or CTAs) keep them in registers.
-// With more systems than teams a launch in whole systems ends with most teams
-// idle (200 Purkinje cells on 152 CTAs take two cells' time).  So a team goes
-// on with another system after P.ivc intervals of one, as long as systems
-// wait: it takes the longest-waiting one and leaves its own at the end of the
-// line, and goes on with its own when none waits.  Every unfinished system is
-// thus in the line or with a running team, nothing waits for a particular
-// one, and the line only shortens.  Counters (zeroed per launch): [0] taken,
-// [1] left; place i of the line is system i for i < nsys, else line[i - nsys]
-// - 1 once it is written; at[s] is the system's next interval.
-template <typename R>
-__device__ __forceinline__ int line_take(const PoolView<R> &P) {
-  int *head = P.grp_line;
-  const int *tail = P.grp_line + 1;
-  int h = *(volatile int *)head;
-  for (;;) {
-    if (h >= P.nsys + *(volatile const int *)tail) return -1;
-    const int got = atomicCAS(head, h, h + 1);
-    if (got == h) break;
-    h = got;
-  }
-  if (h < P.nsys) return h;
-  // (its writer has counted it already: the store follows at once)
-  int v = 0;
-  for (long it = 0; it < GRID_SPIN_LIMIT && v == 0; it++)
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(P.grp_line + 2 + h) : "memory");
-  if (v == 0) *(volatile int *)P.grp_abort = 1;
-  return v - 1;
-}
-template <typename R>
-__device__ __forceinline__ void line_leave(const PoolView<R> &P, int s, int next_iv) {
-  P.grp_line[2 + s] = next_iv;
-  const int i = atomicAdd(P.grp_line + 1, 1);
-  __threadfence();
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(P.grp_line + 2 + P.nsys + i), "r"(s + 1) : "memory");
-}
-// (one thread of the team) the next system and its first interval: after a
-// finished system (s < 0) or after a piece of s up to interval k; s -1: none
-template <typename R>
-__device__ __forceinline__ void line_next(const PoolView<R> &P, int &s, int &k) {
-  const int mine = s, at = k;
-  const int got = line_take(P);
-  if (got >= 0) {
-    s = got;
-    k = *(volatile int *)(P.grp_line + 2 + got);
-    if (mine >= 0) line_leave(P, mine, at);
-  } else if (mine < 0) {
-    s = -1;
-  }
-}
-
 // A role of teams with their system's vectors in registers (group_sys.cuh), at
 // most K elements a thread: P.tiles teams of P.grid_bw threads a CTA.  A
 // Golgi cell takes five warps: alone on its SM each issues an FP64 instruction
@@ -124,9 +73,10 @@ __device__ __forceinline__ void role_teams(const PoolView<R> &P, double *smem, d
   GroupSys<CT, R, K, GRP_CTA> S(P, my + GRP_COEF_M_DOUBLES, s_wp + first / 32, s_res + team, my, GRP_COEF_M, nullptr,
                                 first, bw, 1 + team, 0, 1);
   int s = -1, k = 0;
+  bool hold = false;
   for (;;) {
     if (S.t == 0) {
-      line_next(P, s, k);
+      line_next(P, s, k, hold);
       s_next[team] = s;
       s_at[team] = k;
     }

@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(CLUSTER_BLOCK, 1) k_advance_cluster(const __gr
 
 // Group teams (group_sys.cuh), at most K elements a thread: one system per
 // CTA, per cluster of P.grp_ctas CTAs, or over the whole (cooperative) grid;
-// group g takes systems g, g + groups, ...
+// the groups take systems from the line (group_sys.cuh).
 template <int CT, typename R, int K, int COMM>
 __global__ void __launch_bounds__(GRID_BLOCK, 1) k_advance_group(const __grid_constant__ PoolView<R> P, double t0,
                                                                   int n_iv, int iv0, int init) {
@@ -83,7 +83,38 @@ __global__ void __launch_bounds__(GRID_BLOCK, 1) k_advance_group(const __grid_co
   const int G = COMM == GRP_CTA ? 1 : P.grp_ctas, groups = (int)gridDim.x / G, group = (int)blockIdx.x / G;
   GroupSys<CT, R, K, COMM> S(P, smem, s_wp, &s_res, s_coef, GRP_COEF_M, s_abort, 0, P.grid_bw, 0,
                              (int)blockIdx.x - group * G, G);
-  for (int s = group; s < P.nsys; s += groups) S.run(s, t0, 0, n_iv, iv0, init != 0);
+  if (COMM == GRP_GRID || init) {
+    for (int s = group; s < P.nsys; s += groups) S.run(s, t0, 0, n_iv, iv0, init != 0);
+  } else {
+    // the group's first CTA takes systems from the line
+    __shared__ __align__(8) int s_item[2];
+    int s = -1, k = 0;
+    bool hold = false;
+    for (;;) {
+      if (S.cta == 0 && S.t == 0) {
+        line_next(P, s, k, hold);
+        s_item[0] = s;
+        s_item[1] = k;
+        if (COMM == GRP_CLUSTER)
+          for (int c = 1; c < G; c++) {
+            const unsigned a = cluster_map((unsigned)__cvta_generic_to_shared(s_item), c);
+            asm volatile("st.relaxed.cluster.shared::cluster.v2.u32 [%0], {%1, %2};" ::"r"(a), "r"(s), "r"(k) : "memory");
+          }
+      }
+      S.group_sync();
+      // (a system's state may come from another SM)
+      __threadfence();
+      s = s_item[0];
+      k = s_item[1];
+      if (s < 0) break;
+      const int n = min(P.ivc, n_iv - k);
+      S.run(s, t0, k, n, iv0, false);
+      S.group_sync();
+      k += n;
+      if (k >= n_iv) s = -1;
+      else if (S.cta == 0 && S.t == 0) __threadfence();
+    }
+  }
   S.leave();
 }
 
@@ -94,6 +125,10 @@ const void *pool_kernel(int team) {
     case TEAM_CTA2: return (const void *)k_advance_group<CT, R, 2, GRP_CTA>;
     case TEAM_CLU1: return (const void *)k_advance_group<CT, R, 1, GRP_CLUSTER>;
     case TEAM_CLU2: return (const void *)k_advance_group<CT, R, 2, GRP_CLUSTER>;
+    case TEAM_CLU4:
+      // instantiated for Purkinje pools only (the others never have it)
+      if constexpr (CT == PKJ) return (const void *)k_advance_group<CT, R, 4, GRP_CLUSTER>;
+      return (const void *)k_advance_group<CT, R, 2, GRP_CLUSTER>;
     case TEAM_GRID1: return (const void *)k_advance_group<CT, R, 1, GRP_GRID>;
     case TEAM_GRID2: return (const void *)k_advance_group<CT, R, 2, GRP_GRID>;
     case TEAM_GRID8: return (const void *)k_advance_group<CT, R, GRID_MAX_ROWS, GRP_GRID>;

@@ -83,3 +83,42 @@ def test_group_team_same_bits(oracle, monkeypatch, shape, precision):
     for a, b in zip(got, want):
         np.testing.assert_array_equal(a, b)
     assert stats == wstats
+
+
+def _uneven(precision, n=170):
+    """Rounds of 2 and 20 intervals with few and with all of the slots at work."""
+    rng = np.random.default_rng(8)
+    eng = G.Engine(precision)
+    for k in range(n):
+        r = M.pkj_synthetic(2 + k % 2, 1599 if k % 2 else 801)
+        stim = ([r.shape[0] - 1], [rng.uniform(0, 0.4e-3)], [0.0], [1e9])
+        eng.add_system(M.PKJ, 1, 1, r, rng.uniform(-0.5, 0.5, 1), stim=stim)
+    eng.build()
+    eng.record_spikes(1 << 16)
+    at, teams = 0.0, []
+    for busy, intervals in ((n, 2), (3, 2), (3, 2), (n, 20), (n, 2), (70, 2), (70, 2)):
+        eng.set_budget(0, n, 0)
+        eng.set_budget(0, busy, -1)
+        teams.append(eng.type_team(M.PKJ))
+        eng.advance(at, intervals)
+        at += intervals * G.H_MAX
+    out = [eng.read(i, f) for i in range(n) for f in (G.F_V, G.F_B)] + [eng.read_spikes(M.PKJ)[0]]
+    stats = [eng.ctl(i) for i in range(n)]
+    eng.close()
+    return teams, out, stats
+
+
+@pytest.mark.parametrize("precision", [G.FP64, G.MIXED])
+def test_wide_teams_same_bits(monkeypatch, precision):
+    """A pool whose chains were uneven in the last launch goes on in cluster
+    teams that take systems from the line, and back; the same bits as in the
+    persistent launch alone."""
+    monkeypatch.delenv("GBRKC_GROUP", raising=False)
+    teams, got, stats = _uneven(precision)
+    assert teams[0] == "mega" and teams[3] == "cluster" and teams[4] == "mega"
+    monkeypatch.setenv("GBRKC_GROUP", "0")
+    other, want, wstats = _uneven(precision)
+    assert set(other) == {"mega"}
+    for a, b in zip(got, want):
+        np.testing.assert_array_equal(a, b)
+    assert stats == wstats
