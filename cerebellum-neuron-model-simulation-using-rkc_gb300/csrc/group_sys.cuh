@@ -109,7 +109,8 @@ struct GroupSys {
   double2 *lg;
   unsigned *lcol;
   double *linv;
-  double *wp, *res, *coef;     // warp partials, a sum's result, the step's stage coefficients
+  double *wp, *res, *coef;     // warp partials, a sum's result or a verdict (4), the step's stage coefficients
+  bool due;                    // an ion update follows the accepted step
   unsigned halo, red;          // cluster: [2][most received][2] and [2][chunks][2] words, shared-memory addresses
   int coef_m;                  // stage counts whose coefficients it holds
   int *s_abort;                // [0] a wait gave up, [1] the same as of the last sum, alike for the CTA's threads
@@ -427,15 +428,24 @@ struct GroupSys {
 
   // the pairwise tree over the system's elements of x, the same in every thread
   __device__ __forceinline__ double sum(const double (&x)[K]) {
-    if constexpr (ALONE && K > 2) return sum8(x);
-    else return sum_rows(x);
+    total(x, [&](double e) {
+      if (t == 0) *res = e;
+    });
+    return *res;
+  }
+  // ... or what its first warp makes of it, between the sum and the barrier
+  template <class F>
+  __device__ __forceinline__ void total(const double (&x)[K], F fin) {
+    if constexpr (ALONE && K > 2) sum8(x, fin);
+    else sum_rows(x, fin);
   }
 
   // Many elements a thread: through shared memory, a thread eight consecutive
   // values at a time, then a warp eight such sums a lane (systems of up to
   // 2048 elements): 61 FP64 additions for 1600 elements where a shuffle tree
   // per row takes 280.
-  __device__ __forceinline__ double sum8(const double (&x)[K]) {
+  template <class F>
+  __device__ __forceinline__ void sum8(const double (&x)[K], F fin) {
     double *sc = u + ((tag + 1u) & 1u) * us;    // the next evaluation's buffer
 #pragma unroll
     for (int q = 0; q < K; q++)
@@ -468,13 +478,13 @@ struct GroupSys {
         const double o = __shfl_down_sync(0xffffffffu, a, st);
         if ((t & (2 * st - 1)) == 0 && t + st < nb) a = a + o;
       }
+      fin(__shfl_sync(0xffffffffu, a, 0));
     }
-    if (t == 0) *res = a;
     sync();
-    return *res;
   }
 
-  __device__ __forceinline__ double sum_rows(const double (&x)[K]) {
+  template <class F>
+  __device__ __forceinline__ void sum_rows(const double (&x)[K], F fin) {
     const int lane = t & 31, warp = t >> 5, nw = bw >> 5;
 #pragma unroll
     for (int q = 0; q < K; q++) {
@@ -547,13 +557,50 @@ struct GroupSys {
         const double o = __shfl_down_sync(0xffffffffu, v[0], st);
         if ((lane & (2 * st - 1)) == 0 && (lane + st) * rr < nb) v[0] = v[0] + o;
       }
-      if (lane == 0) {
-        *res = v[0];
-        if constexpr (!ALONE) s_abort[1] = *(volatile int *)s_abort;
-      }
+      fin(__shfl_sync(0xffffffffu, v[0], 0));
+      if constexpr (!ALONE)
+        if (lane == 0) s_abort[1] = *(volatile int *)s_abort;
     }
     sync();
-    return *res;
+  }
+
+  // The error norm and the controller's verdict.  In a CTA of its own they are
+  // the work of the warp that ends the sum, and the others take what they
+  // need of it: the controller's 60 FP64 instructions took 7200 cycles an
+  // attempt in each of eight warps, 4000 in one (Golgi cells, five warps:
+  // 37.4 -> 36.7 ms for 2048 cells).  The warps of a cluster or grid team
+  // have their SM's FP64 pipe nearly to themselves, and each repeats them
+  // (handing the verdict over took 16 x 16 olives from 9.5 to 10.1 ms).
+  __device__ __forceinline__ int verdict(const double (&d)[K], double h) {
+    if constexpr (!ALONE) {
+      const int a = c.judge(norm(sum(d)), h);
+      due = a == SC::ATT_ACCEPT && c.clock(CT == GO || CT == PKJ);
+      return a;
+    }
+    total(d, [&](double e) {
+      const int a = c.judge(norm(e), h);
+      due = a == SC::ATT_ACCEPT && c.clock(CT == GO || CT == PKJ);
+      if (t == 0) {
+        res[0] = c.absh; res[1] = c.lt; res[2] = c.sum_dt;
+        int *r = (int *)(res + 3);
+        r[0] = c.status;
+        r[1] = (a + 1) * 2 + (due ? 1 : 0);
+      }
+    });
+    const int *r = (const int *)(res + 3);
+    const int a = (r[1] >> 1) - 1;
+    due = (r[1] & 1) != 0;
+    c.absh = res[0];
+    c.status = r[0];
+    if (a == SC::ATT_ACCEPT) {
+      c.lt = c.gt_old = c.hw1 = res[1];
+      c.hw0 = h;
+      c.sum_dt = res[2];
+      c.jacatt = c.newspc = 0;
+    } else if (a == SC::ATT_REJECT) {
+      c.newspc = !c.jacatt;
+    }
+    return a;
   }
 
   __device__ __forceinline__ double sumsq(const double (&x)[K]) {
@@ -693,7 +740,7 @@ struct GroupSys {
         d[q] = qv * qv;
       }
     }
-    const int a = c.judge(norm(sum(d)), h);
+    const int a = verdict(d, h);
     if (a == SC::ATT_ACCEPT) {
       // (v2, fn, v1, yn, y) <- (fn, v1, yn, y, v2)
 #pragma unroll
@@ -882,7 +929,6 @@ struct GroupSys {
       c.status |= ST_LOOP_CAP;
       return TICK_DONE;
     }
-    const bool due = c.clock(CT == GO || CT == PKJ);
     if (!c.last) return due ? TICK_ION : TICK_MORE;
     end_interval();
     if (++k_iv >= n_iv) return TICK_DONE;

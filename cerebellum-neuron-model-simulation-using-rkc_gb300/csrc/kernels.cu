@@ -66,11 +66,11 @@ __device__ __forceinline__ void role_block(const PoolView<R> &P, int *q, double 
 template <int CT, typename R, int K>
 __device__ __forceinline__ void role_teams(const PoolView<R> &P, double *smem, double t0, int n_iv, int iv0) {
   __shared__ int s_next[MEGA_BLOCK / 32], s_at[MEGA_BLOCK / 32];
-  __shared__ double s_wp[K == 1 ? MEGA_BLOCK / 32 : K * MEGA_BLOCK / 32], s_res[MEGA_BLOCK / 32];
+  __shared__ double s_wp[K == 1 ? MEGA_BLOCK / 32 : K * MEGA_BLOCK / 32], s_res[4 * MEGA_BLOCK / 32];
   const int bw = P.grid_bw, team = (int)threadIdx.x / bw, first = team * bw;
   if (team >= P.tiles) return;
   double *my = smem + (long)team * P.grp_stride;
-  GroupSys<CT, R, K, GRP_CTA> S(P, my + GRP_COEF_M_DOUBLES, s_wp + first / 32, s_res + team, my, GRP_COEF_M, nullptr,
+  GroupSys<CT, R, K, GRP_CTA> S(P, my + GRP_COEF_M_DOUBLES, s_wp + first / 32, s_res + 4 * team, my, GRP_COEF_M, nullptr,
                                 first, bw, 1 + team, 0, 1);
   int s = -1, k = 0;
   bool hold = false;

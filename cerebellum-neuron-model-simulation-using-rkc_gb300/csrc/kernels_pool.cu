@@ -78,10 +78,10 @@ __global__ void __launch_bounds__(GRID_BLOCK, 1) k_advance_group(const __grid_co
                                                                   int n_iv, int iv0, int init) {
   extern __shared__ __align__(16) double smem[];
   __shared__ double s_wp[GRID_MAX_ROWS * 8];
-  __shared__ double s_res, s_coef[5 * (GRP_COEF_M - 1)];
+  __shared__ double s_res[4], s_coef[5 * (GRP_COEF_M - 1)];
   __shared__ int s_abort[2];
   const int G = COMM == GRP_CTA ? 1 : P.grp_ctas, groups = (int)gridDim.x / G, group = (int)blockIdx.x / G;
-  GroupSys<CT, R, K, COMM> S(P, smem, s_wp, &s_res, s_coef, GRP_COEF_M, s_abort, 0, P.grid_bw, 0,
+  GroupSys<CT, R, K, COMM> S(P, smem, s_wp, s_res, s_coef, GRP_COEF_M, s_abort, 0, P.grid_bw, 0,
                              (int)blockIdx.x - group * G, G);
   if (COMM == GRP_GRID || init) {
     for (int s = group; s < P.nsys; s += groups) S.run(s, t0, 0, n_iv, iv0, init != 0);
