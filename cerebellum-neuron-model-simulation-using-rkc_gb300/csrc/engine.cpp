@@ -1988,10 +1988,22 @@ static int build_impl(gbrkc_engine *E) {
     int rc = assemble_pool(E, P);
     if (rc) return rc;
   }
-  // granule cells of four compartments start from two to a warp (8 lanes): the
+  // Granule cells of four compartments start from two to a warp (8 lanes): the
   // fewer share a warp the less it diverges, and fit_granule_warps doubles
-  // the count while the warps would not fit
-  if (E->pools[GR].team == TEAM_LANE4 && !getenv("GBRKC_LANES")) E->lanes = 8;
+  // the count while the warps would not fit.  Alone in their engine they
+  // start from as many as leave an SM one warp: its warps share the
+  // instruction cache (mixed, 512 cells, 8 / 16 / 32 lanes: 18.9 / 16.6 /
+  // 17.3 ms; FP64, 999: 29.4 / 29.4 / 27.9; beside 64 Golgi and 48 Purkinje
+  // cells, 512 in a network: 11.0 / 12.7 / 13.8).
+  if (E->pools[GR].team == TEAM_LANE4 && !getenv("GBRKC_LANES")) {
+    const long n = (long)E->pools[GR].systems.size();
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    E->lanes = 8;
+    if (n == (long)E->systems.size())
+      while (E->lanes < 32 && (n + E->lanes / 4 - 1) / (E->lanes / 4) > sms) E->lanes *= 2;
+  }
   {
     int rc = setup_mega(E);
     if (rc) return rc;
