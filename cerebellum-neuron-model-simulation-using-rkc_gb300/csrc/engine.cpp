@@ -1390,6 +1390,15 @@ void fit_granule_warps(gbrkc_engine *E) {
   const bool all_in = granules_all_in_flight(E, need);
   const int want = all_in ? (int)need : (int)std::min(need, (long)per * E->role_ctas[GR]);
   E->gr_warps = want;
+  bool alone = true;
+  for (int t = 0; t < NTYPES; t++) alone &= t == GR || E->role_ctas[t] == 0;
+  if (alone) {
+    // no other role to leave CTAs to: a warp a CTA as far as they go (512
+    // cells, mixed, 256 warps: 18.9 ms on 64 CTAs, 15.5 on 152)
+    E->gr_warps = (int)need;
+    E->role_ctas[GR] = (int)std::min(need, (long)E->mega_grid);
+    return;
+  }
   const int c = all_in ? std::max((want + per - 1) / per, std::min(want, E->role_ctas[GR]))
                        : std::min(want, E->role_ctas[GR]);
   while (c > E->role_ctas[GR]) {  // take from the other role with the most CTAs
@@ -1990,18 +1999,19 @@ static int build_impl(gbrkc_engine *E) {
   }
   // Granule cells of four compartments start from two to a warp (8 lanes): the
   // fewer share a warp the less it diverges, and fit_granule_warps doubles
-  // the count while the warps would not fit.  Alone in their engine they
-  // start from as many as leave an SM one warp: its warps share the
-  // instruction cache (mixed, 512 cells, 8 / 16 / 32 lanes: 18.9 / 16.6 /
-  // 17.3 ms; FP64, 999: 29.4 / 29.4 / 27.9; beside 64 Golgi and 48 Purkinje
-  // cells, 512 in a network: 11.0 / 12.7 / 13.8).
+  // the count while the warps would not fit.  With FP64 gating and alone in
+  // their engine they start from as many as leave an SM one warp: the ion
+  // update's code is long, and two warps of an SM share its instruction cache
+  // (999 cells, 8 / 16 / 32 lanes: 29.1 / 29.0 / 27.8 ms; mixed precision, 512
+  // cells: 15.5 / 16.4 / 17.2; in a network beside 64 Golgi and 48 Purkinje
+  // cells, mixed: 11.0 / 12.7 / 13.8).
   if (E->pools[GR].team == TEAM_LANE4 && !getenv("GBRKC_LANES")) {
     const long n = (long)E->pools[GR].systems.size();
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     E->lanes = 8;
-    if (n == (long)E->systems.size())
+    if (E->pools[GR].f64 && n == (long)E->systems.size())
       while (E->lanes < 32 && (n + E->lanes / 4 - 1) / (E->lanes / 4) > sms) E->lanes *= 2;
   }
   {
