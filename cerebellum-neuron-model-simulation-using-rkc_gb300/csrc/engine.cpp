@@ -962,6 +962,9 @@ bool group_team(const gbrkc_engine *E, PoolHost &P) {
       if (ctas < 2 || ctas > 16 || up(rows, ctas) != r) continue;
       const int team = r == 1 ? TEAM_CLU1 : r == 2 ? TEAM_CLU2 : TEAM_CLU4;
       const size_t smem = grid_smem(r * bw, 2 * bw, 6, (int)ctas);
+      // (asking what the device holds takes 0.1 ms: not for a lone system on a
+      // shape that is no better)
+      if (nsys == 1 && time((double)r, up(ctas, sms) * bw / 32.0, 1, 1) >= best) continue;
       const int cap = P.f64 ? group_capacity<double>(P.type, team, (int)ctas, bw, smem)
                             : group_capacity<float>(P.type, team, (int)ctas, bw, smem);
       if (cap < 1) continue;

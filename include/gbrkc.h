@@ -166,8 +166,8 @@ int gbrkc_type_team(gbrkc_engine *e, int cell_type);
 
 /* The grid team's launch shape for a lone system of nc compartments on at
  * most max_ctas co-resident CTAs (the engine uses the device's SM count):
- * CTAs of threads_per_cta threads (a power of two, 32..256), each thread
- * owning elements i with i mod (ctas * threads_per_cta) its index.  The rule
+ * CTAs of threads_per_cta threads (a power of two, 32..256), each CTA owning
+ * a run of chunks of threads_per_cta consecutive elements.  The rule
  * minimises the busiest CTA's elements, then the CTA count, within 256
  * chunks of threads_per_cta elements and 8 elements a thread.  Host only
  * (no device needed); GBRKC_EINVAL when no shape holds nc. */
