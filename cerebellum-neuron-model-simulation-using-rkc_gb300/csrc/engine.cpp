@@ -1258,12 +1258,13 @@ int upload_pool(gbrkc_engine *E, PoolHost &P, PoolView<R> &V) {
   }
   for (GroupCfg &C : P.alt)
     if ((rc = upload_group(E, C))) return rc;
-  if (team_is_group(P.team) || P.grp_fast) {
+  if (team_is_group(P.team) || P.grp_fast || P.team == TEAM_LANE4) {
     // abort flag and padding, counters, next intervals, the line
     const std::vector<int> line(4 + (1 + LINE_PIECES) * P.systems.size(), 0);
     UP(line, P.d_line);
     V.grp_line = P.d_line + 2;
-    V.ivc = 1;
+    V.ivc = 1 << 30;
+    if (!team_is_group(P.team)) V.grp_abort = P.d_line;
     std::vector<int> order(P.systems.size());
     std::iota(order.begin(), order.end(), 0);
     UP(order, P.d_order);
@@ -1277,7 +1278,6 @@ int upload_pool(gbrkc_engine *E, PoolHost &P, PoolView<R> &V) {
     V.grp_stride = P.grp_stride;
     V.grid_bw = P.grid_bw;
     V.tiles = MEGA_BLOCK / P.grid_bw;
-    V.grp_abort = P.d_line;
   }
   std::vector<double> zws(P.ws_total, 0.0);
   UP(zws, V.ws);
@@ -1356,14 +1356,14 @@ template <typename R> PoolView<R> &pool_view(PoolHost &P);
 template <> PoolView<double> &pool_view<double>(PoolHost &P) { return P.vd; }
 template <> PoolView<float> &pool_view<float>(PoolHost &P) { return P.vf; }
 
-// Whether the warps that give every granule system with work its own lane
-// fit in half the CTAs the other roles leave (8 warps a CTA): then every
-// system is in flight, the latency a request server needs; else lanes run
-// several systems in turn and the role split decides the granule CTAs.
+// Whether the warps that give every granule system with work its own place
+// fit in a quarter of the CTAs the other roles leave (8 warps a CTA): then every
+// system is in flight, which shortens a request server's rounds; else quads
+// take systems in turns and the role split decides the granule CTAs.
 bool granules_all_in_flight(const gbrkc_engine *E, long warps) {
   int nother = 0;
   for (int t = 0; t < NTYPES; t++) nother += (t != GR && E->role_ctas[t] > 0);
-  return (warps + MEGA_BLOCK / 32 - 1) / (MEGA_BLOCK / 32) <= (E->mega_grid - nother) / 2;
+  return (warps + MEGA_BLOCK / 32 - 1) / (MEGA_BLOCK / 32) <= (E->mega_grid - nother) / 4;
 }
 
 // Granule warps for the next persistent launch: a place (one lane, or four)
@@ -1442,6 +1442,13 @@ int mega_pools(gbrkc_engine *E, MegaView<R> &M, int n_iv, int init) {
       M.pool[t].ivc = P.pieces ? std::max(1, (n_iv + LINE_PIECES - 1) / LINE_PIECES) : std::max(1, n_iv);
       CUDA_TRY(cudaMemsetAsync(P.d_line, 0, (4 + (1 + (P.pieces ? LINE_PIECES : 0)) * (size_t)nsys) * sizeof(int),
                                E->streams[0]));
+    }
+    if (P.team == TEAM_LANE4 && !P.systems.empty() && !init) {
+      const long nsys = (long)P.systems.size(), active = E->gr_active >= 0 ? E->gr_active : nsys;
+      P.pieces = n_iv > 1 && active > (long)E->gr_warps * systems_per_warp(P, P.vd.lanes);
+      M.pool[t].ivc = P.pieces ? (n_iv + LINE_PIECES - 1) / LINE_PIECES : n_iv;
+      if (P.pieces)
+        CUDA_TRY(cudaMemsetAsync(P.d_line, 0, (4 + (1 + LINE_PIECES) * (size_t)nsys) * sizeof(int), E->streams[0]));
     }
     end += E->role_ctas[t];
     M.role_end[t] = end;

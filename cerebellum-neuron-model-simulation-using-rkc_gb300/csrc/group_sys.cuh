@@ -984,23 +984,25 @@ struct GroupSys {
 // of the line is order[i] for i < nsys, else line[i - nsys] - 1 once it is
 // written; at[s] is the system's next interval.  Systems that took much longer
 // than the others in the launch before come first in order, and those that
-// may decide the launch's length are held: no other is taken for them.
+// may decide the launch's length are held: no other is taken for them.  Granule
+// quads take the first round from their queue (first 0), then from the line.
 template <typename R>
-__device__ __forceinline__ int line_take(const PoolView<R> &P) {
+__device__ __forceinline__ int line_take(const PoolView<R> &P, int first) {
   int *head = P.grp_line;
   const int *tail = P.grp_line + 1;
   int h = *(volatile int *)head;
   for (;;) {
-    if (h >= P.nsys + *(volatile const int *)tail) return -1;
+    if (h >= first + *(volatile const int *)tail) return -1;
     const int got = atomicCAS(head, h, h + 1);
     if (got == h) break;
     h = got;
   }
-  if (h < P.nsys) return P.grp_order[h];
+  if (h < first) return P.grp_order[h];
+  const int *place = P.grp_line + 2 + P.nsys + (h - first);
   // (its writer has counted it already: the store follows at once)
   int v = 0;
   for (long it = 0; it < GRID_SPIN_LIMIT && v == 0; it++)
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(P.grp_line + 2 + h) : "memory");
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(place) : "memory");
   if (v == 0) *(volatile int *)P.grp_abort = 1;
   return v - 1;
 }
@@ -1017,7 +1019,7 @@ template <typename R>
 __device__ __forceinline__ void line_next(const PoolView<R> &P, int &s, int &k, bool &hold) {
   const int mine = s, at = k;
   if (mine >= 0 && hold) return;
-  int got = line_take(P);
+  int got = line_take(P, P.nsys);
   if (got >= 0) {
     hold = (got >> 30) != 0;
     got &= (1 << 30) - 1;

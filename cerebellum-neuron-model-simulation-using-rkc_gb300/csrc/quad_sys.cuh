@@ -256,14 +256,15 @@ struct QuadSys {
     if (c.iv_left > 0) c.iv_left--;
   }
 
-  __device__ __forceinline__ int start(double t, int n, int iv0_global) {
+  // intervals k0 .. k0 + n - 1 of a launch that begins at t
+  __device__ __forceinline__ int start(double t, int k0, int n, int iv0_global) {
     if (c.iv_left >= 0 && n > c.iv_left) n = c.iv_left;
     t0 = t;
-    n_iv = n;
+    n_iv = k0 + n;
     iv0 = iv0_global;
-    k_iv = 0;
+    k_iv = k0;
     if (c.status != 0 || n <= 0) return TICK_DONE;
-    return begin_interval(t0);
+    return begin_interval(t0 + k0 * H_MAX);
   }
 
   // Sys::tick
@@ -284,7 +285,14 @@ struct QuadSys {
 };
 
 // The systems of a warp, four lanes each on its first `quads` groups of four:
-// systems from *q or (q null) the static sequence first, first + stride, ...
+// the static sequence first, first + stride, ... (q null), or systems from
+// *q, and while P.ivc is less than the launch's intervals the line's (group_sys.cuh):
+// with more systems than places a quad goes on with another system after
+// P.ivc intervals of one.  (Whole systems in turn, 1.4 systems a place take
+// the time of two, so the granule role of the mixed batch had to hold every
+// cell at once, on 64 CTAs: 4.9 s a step beside 7.6 s of the other roles on
+// the rest.  In turns on 42 CTAs: 6.2 s each, 16.7e9 -> 20.3e9
+// compartment-updates/s.)
 // A system whose ion update is due parks; the warp runs the parked systems'
 // updates together once every live one is parked or the oldest has waited
 // ION_WAIT_MAX iterations (run_lanes, integrator.cuh).
@@ -292,24 +300,53 @@ template <int CT, typename R>
 __device__ __forceinline__ void run_quads(const PoolView<R> &P, int *q, int first, int stride, int quads, double t0,
                                           int n_iv, int iv0_global) {
   QuadSys<CT, R> S(P);
+  const bool turns = q && P.ivc < n_iv;
+  const int piece = turns ? P.ivc : n_iv;
+  int s = -1, k = 0, r = TICK_DONE;       // the system and its next interval
+  bool more = ((int)(threadIdx.x & 31) >> 2) < quads;
+  // the next system, after s up to interval k (s -1: after a finished one)
   auto next = [&]() {
-    int k = 0;
-    if (S.r == 0) k = atomicAdd(q, 1);
-    return __shfl_sync(S.mask, k, 0, 4);
+    if (!q) {
+      s = first < P.nsys ? first : -1;
+      first += stride;
+      k = 0;
+      return;
+    }
+    if (S.r == 0) {
+      int got = -1, at = 0;
+      if (*(volatile int *)q < P.nsys) {
+        got = atomicAdd(q, 1);
+        if (got >= P.nsys) got = -1;
+      }
+      if (got < 0 && turns) {
+        got = line_take(P, 0);
+        if (got >= 0) at = *(volatile int *)(P.grp_line + 2 + got);
+      }
+      if (got >= 0) {
+        if (s >= 0) line_leave(P, s, k);
+        s = got;
+        k = at;
+      }
+    }
+    s = __shfl_sync(S.mask, s, 0, 4);
+    k = __shfl_sync(S.mask, k, 0, 4);
+    if (turns) __threadfence();           // (a system's state may come from another SM)
   };
-  int s = ((int)(threadIdx.x & 31) >> 2) >= quads ? P.nsys : (q ? next() : first);
-  int r = TICK_DONE;
   auto acquire = [&]() {
-    while (s < P.nsys) {
+    while (more) {
+      next();
+      if (s < 0) break;
       if (system_selected(P.ctl[s], false, n_iv)) {
         S.load(s);
-        r = S.start(t0, n_iv, iv0_global);
+        r = S.start(t0, k, min(piece, n_iv - k), iv0_global);
         if (r != TICK_DONE) return;
         __syncwarp(S.mask);
         S.store();
+        __syncwarp(S.mask);
       }
-      s = q ? next() : s + stride;
+      s = -1;
     }
+    more = false;
     r = TICK_DONE;
   };
   acquire();
@@ -332,7 +369,12 @@ __device__ __forceinline__ void run_quads(const PoolView<R> &P, int *q, int firs
       if (r == TICK_DONE) {
         __syncwarp(S.mask);
         S.store();
-        s = q ? next() : s + stride;
+        k += piece;
+        if (k >= n_iv || S.c.status != 0) s = -1;
+        if (turns) {
+          __threadfence();
+          __syncwarp(S.mask);
+        }
         acquire();
       }
     }

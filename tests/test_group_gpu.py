@@ -122,3 +122,39 @@ def test_wide_teams_same_bits(monkeypatch, precision):
     for a, b in zip(got, want):
         np.testing.assert_array_equal(a, b)
     assert stats == wstats
+
+
+@pytest.mark.parametrize("precision", [G.FP64, G.MIXED])
+def test_granule_turns_same_bits(monkeypatch, precision):
+    """More granule cells than the persistent launch's quads (8 warps of 8 on
+    each SM): quads take turns between intervals; the same bits as cells run to
+    their end one after another in the type's own launch."""
+    n, intervals = 9900, 3
+    rng = np.random.default_rng(5)
+    jit, amp = rng.uniform(-0.5, 0.5, (n, 1)), rng.uniform(0, 0.012e-3, n)
+    ids = np.arange(0, n, 37)
+
+    def run():
+        eng = G.Engine(precision)
+        for k in range(n):
+            eng.add_system(M.GR, 1, 1, M.gr_reduced4(), jit[k], stim=([1], [amp[k]], [0.0], [1e9]))
+        eng.build()
+        team = eng.type_team(M.GR)
+        eng.set_budget(50, 400, 2)       # budgets that end within the launch
+        eng.record_soma(intervals)
+        eng.advance(0.0, intervals)
+        soma = np.empty((intervals, eng.type_cells(M.GR)))
+        out = [eng.read_soma_type(M.GR, intervals, soma)] + [eng.read(i, f) for i in ids for f in (G.F_V, G.F_B)]
+        stats = [eng.ctl(i) for i in ids]
+        eng.close()
+        return team, out, stats
+
+    monkeypatch.delenv("GBRKC_NO_MEGA", raising=False)
+    team, got, stats = run()
+    assert team == "mega"
+    monkeypatch.setenv("GBRKC_NO_MEGA", "1")
+    other, want, wstats = run()
+    assert other == "pool"
+    for a, b in zip(got, want):
+        np.testing.assert_array_equal(a, b)
+    assert stats == wstats
