@@ -1377,14 +1377,19 @@ void fit_granule_warps(gbrkc_engine *E) {
   if (!E->mega || E->role_ctas[GR] == 0) return;
   PoolHost &G = E->pools[GR];
   const long active = (E->gr_active >= 0) ? E->gr_active : (long)G.systems.size();
-  // the preferred lanes per warp, doubled while the warps would need more
-  // than half of the CTAs' warp slots (the other roles need the rest)
+  // the preferred lanes per warp, doubled while the warps would need more than
+  // a quarter of the CTAs' warp slots, where the other roles need the rest
+  // and a warp's FP64 instructions had better serve eight cells (a stream of
+  // requests of up to 4096 granule cells: 5.5 s at a half, 5.0 s at a quarter), or
+  // than half of them alone
+  bool alone = true;
+  for (int t = 0; t < NTYPES; t++) alone &= t == GR || E->role_ctas[t] == 0;
   int lanes = E->lanes;
   auto warps_for = [&](int l) {
     const int k = systems_per_warp(G, l);
     return (active + k - 1) / k;
   };
-  while (lanes < 32 && warps_for(lanes) > E->gr_warps_max / 2) lanes = std::min(32, 2 * lanes);
+  while (lanes < 32 && warps_for(lanes) > E->gr_warps_max / (alone ? 2 : 4)) lanes = std::min(32, 2 * lanes);
   G.vd.lanes = G.vf.lanes = lanes;
   G.vd.per_warp = G.vf.per_warp = systems_per_warp(G, lanes);
   const int per = MEGA_BLOCK / 32;
@@ -1393,8 +1398,6 @@ void fit_granule_warps(gbrkc_engine *E) {
   const bool all_in = granules_all_in_flight(E, need);
   const int want = all_in ? (int)need : (int)std::min(need, (long)per * E->role_ctas[GR]);
   E->gr_warps = want;
-  bool alone = true;
-  for (int t = 0; t < NTYPES; t++) alone &= t == GR || E->role_ctas[t] == 0;
   if (alone) {
     // no other role to leave CTAs to: a warp a CTA as far as they go (512
     // cells, mixed, 256 warps: 18.9 ms on 64 CTAs, 15.5 on 152)
@@ -2021,8 +2024,11 @@ static int build_impl(gbrkc_engine *E) {
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     E->lanes = 8;
-    if (E->pools[GR].f64 && n == (long)E->systems.size())
-      while (E->lanes < 32 && (n + E->lanes / 4 - 1) / (E->lanes / 4) > sms) E->lanes *= 2;
+    // (beside other types at most a quarter of the GPU's warps, as in
+    // fit_granule_warps, so that the first split knows)
+    const bool alone = n == (long)E->systems.size();
+    const long most = !alone ? 2L * sms : E->pools[GR].f64 ? sms : LONG_MAX;
+    while (E->lanes < 32 && (n + E->lanes / 4 - 1) / (E->lanes / 4) > most) E->lanes *= 2;
   }
   {
     int rc = setup_mega(E);
