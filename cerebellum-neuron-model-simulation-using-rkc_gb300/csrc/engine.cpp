@@ -947,7 +947,7 @@ bool group_team(const gbrkc_engine *E, PoolHost &P) {
   const double other = time(mega_rows, mega_warps, std::max(1.0, nsys / (double)(per * sms)), 0);
   double best = 0.9 * other;
   int kind = 0, bbw = 0, bctas = 1;
-  struct Wide { double time; int bw, ctas, cap; };
+  struct Wide { double time; int bw, ctas; };
   std::map<int, Wide> wide;                // per CTAs of a cluster: the best shape with one long system
   for (int bw = 32; bw <= GRID_BLOCK; bw += 32) {
     const long rows = up(nc, bw), fit = std::max(1, 65536 / (256 * bw));   // CTAs an SM's registers hold
@@ -975,7 +975,7 @@ bool group_team(const gbrkc_engine *E, PoolHost &P) {
       // the same with one system six times as long as the mean
       const double th = time((double)r, w, std::max(6.0, nsys / (double)at_once), 1);
       const auto it = wide.find((int)ctas);
-      if (it == wide.end() || th < it->second.time) wide[(int)ctas] = Wide{th, bw, (int)ctas, cap};
+      if (it == wide.end() || th < it->second.time) wide[(int)ctas] = Wide{th, bw, (int)ctas};
     }
   }
   if (grid_ok) {
@@ -994,8 +994,14 @@ bool group_team(const gbrkc_engine *E, PoolHost &P) {
       if (w.second.time > 0.9 * at) continue;
       const GroupCfg before = P;
       if (group_tables(P, w.second.bw, w.second.ctas, false)) {
-        P.alt.push_back(P);
-        P.alt.back().grid = std::min(nsys, w.second.cap) * w.second.ctas;
+        // (the tables' own shared memory, not the estimate's; this also sets
+        // the kernel's limit to it)
+        const int cap = P.f64 ? group_capacity<double>(P.type, P.team, P.grp_ctas, P.grid_bw, P.smem)
+                              : group_capacity<float>(P.type, P.team, P.grp_ctas, P.grid_bw, P.smem);
+        if (cap > 0) {
+          P.alt.push_back(P);
+          P.alt.back().grid = std::min(nsys, cap) * w.second.ctas;
+        }
       }
       static_cast<GroupCfg &>(P) = before;
     }

@@ -1,0 +1,82 @@
+"""How the next launch of a pool is planned (csrc/engine.cpp): the teams it may
+take, the systems it counts, and what idle slots cost it."""
+import os
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+
+import gbrkc as G
+import morph as M
+
+pytestmark = pytest.mark.gpu
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+def comb_purkinje(teeth=700, soma_dendrites=9):
+    """A Purkinje cell of 2 * teeth compartments: a trunk whose every
+    compartment carries one tooth, the teeth numbered before the trunk, so that
+    on two CTAs nearly every tooth reads and is read across them; and a soma
+    with several dendrites of one compartment beside the trunk."""
+    n = 2 * teeth
+    rows = np.zeros((n, 7))
+    rng = np.random.default_rng(1)
+    for i in range(n):
+        along = rng.standard_normal(3)
+        length = rng.uniform(5.0, 20.0) / np.linalg.norm(along)
+        parent = i + teeth if i < teeth else i + 1
+        rows[i] = [i, parent, *(length * along), 3.0 if i < teeth else 6.0, 3 if i < teeth else 2]
+    soma = n - 1
+    for i in range(soma_dendrites - 2):       # (the trunk's end and the soma's own tooth are two)
+        rows[i, 1] = soma
+    rows[soma] = [soma, -1, 0.0, 0.0, 0.0, 29.8, 0]
+    return rows
+
+
+def uneven_comb(others):
+    """170 comb cells, of which one has 20 intervals to do in the second launch
+    and the others fewer; the third launch's team and the last voltages."""
+    n, r = 170, comb_purkinje()
+    eng = G.Engine(G.MIXED)
+    for k in range(n):
+        eng.add_system(M.PKJ, 1, 1, r, [0.0])
+    eng.build()
+    eng.advance(0.0, 4)
+    eng.set_budget(0, n, others)
+    eng.set_budget(0, 1, -1)
+    eng.advance(4 * G.H_MAX, 20)
+    team = eng.type_team(M.PKJ)
+    eng.set_budget(0, n, -1)
+    eng.advance(24 * G.H_MAX, 2)
+    out = np.concatenate([eng.vnew(i) for i in range(n)])
+    eng.close()
+    return team, out
+
+
+def _alone(others, group):
+    """uneven_comb in a process of its own: a kernel's shared-memory limit is the
+    process's, and other tests raise it."""
+    env = dict(os.environ)
+    env.pop("GBRKC_GROUP", None)
+    if group is not None:
+        env["GBRKC_GROUP"] = group
+    code = ("import sys; sys.path[:0] = %r; import numpy as np, test_launch_plan_gpu as t; team, v = t.uneven_comb(%d); "
+            "print('TEAM', team); print('BITS', v.tobytes().hex())" % ([p for p in sys.path if p] + [HERE], others))
+    p = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=600)
+    assert p.returncode == 0, p.stderr[-2000:]
+    line = {w.split(" ", 1)[0]: w.split(" ", 1)[1] for w in p.stdout.splitlines() if w.startswith(("TEAM", "BITS"))}
+    return line["TEAM"], np.frombuffer(bytes.fromhex(line["BITS"]))
+
+
+@pytest.mark.parametrize("others", [6, 7])
+def test_wide_rows_on_a_cluster(others):
+    """A cluster team whose rows and hand-overs take more shared memory than
+    the estimate's (rows of nine neighbours, 640 received values) is
+    launched with what it needs: the same bits as in the persistent launch."""
+    team, got = _alone(others, None)
+    assert team == "cluster"
+    other, want = _alone(others, "0")
+    assert other == "mega"
+    np.testing.assert_array_equal(got, want)
