@@ -456,6 +456,13 @@ struct PoolHost : GroupCfg {
   int *d_spk_count = nullptr;
   int spk_cap = 0;
   std::vector<char> retired;
+  // systems with work, as far as the host knows: not stopped, intervals left in their budget
+  std::vector<char> work;
+  int n_work = 0;
+  void set_work(int i, bool w) {
+    n_work += (int)w - (int)work[i];
+    work[i] = w;
+  }
 };
 
 }  // namespace gbrkc
@@ -494,7 +501,6 @@ struct gbrkc_engine {
   int gr_warps_need = 0;        // granule warps that would give every granule system with work its own lane
   int gr_warps_max = 0;         // granule warps the CTAs can hold beside the other roles
   int lanes = 16;               // lanes of a warp in use by granule systems (one each, or four: TEAM_LANE4)
-  long gr_active = -1;          // granule systems with work (-1: not known yet)
   double role_work[NTYPES] = {};  // smoothed CTA-ms per role
   int *d_queue = nullptr;
   unsigned long long *d_tstart = nullptr, *d_tend = nullptr;
@@ -1142,6 +1148,8 @@ int assemble_pool(gbrkc_engine *E, PoolHost &P) {
       P.cell_local.push_back(c);
     }
     P.ctl.push_back(initial_ctl(S, S.idle ? 0 : -1));
+    P.work.push_back(!S.idle);
+    P.n_work += !S.idle;
     off += S.nc;
     cell0 += S.n;
   }
@@ -1382,7 +1390,7 @@ bool granules_all_in_flight(const gbrkc_engine *E, long warps) {
 void fit_granule_warps(gbrkc_engine *E) {
   if (!E->mega || E->role_ctas[GR] == 0) return;
   PoolHost &G = E->pools[GR];
-  const long active = (E->gr_active >= 0) ? E->gr_active : (long)G.systems.size();
+  const long active = G.n_work;
   // the preferred lanes per warp, doubled while the warps would need more than
   // a quarter of the CTAs' warp slots, where the other roles need the rest
   // and a warp's FP64 instructions had better serve eight cells (a stream of
@@ -1453,8 +1461,8 @@ int mega_pools(gbrkc_engine *E, MegaView<R> &M, int n_iv, int init) {
                                E->streams[0]));
     }
     if (P.team == TEAM_LANE4 && !P.systems.empty() && !init) {
-      const long nsys = (long)P.systems.size(), active = E->gr_active >= 0 ? E->gr_active : nsys;
-      P.pieces = n_iv > 1 && active > (long)E->gr_warps * systems_per_warp(P, P.vd.lanes);
+      const long nsys = (long)P.systems.size();
+      P.pieces = n_iv > 1 && P.n_work > (long)E->gr_warps * systems_per_warp(P, P.vd.lanes);
       M.pool[t].ivc = P.pieces ? (n_iv + LINE_PIECES - 1) / LINE_PIECES : n_iv;
       if (P.pieces)
         CUDA_TRY(cudaMemsetAsync(P.d_line, 0, (4 + (1 + LINE_PIECES) * (size_t)nsys) * sizeof(int), E->streams[0]));
@@ -2193,17 +2201,14 @@ extern "C" int gbrkc_advance(gbrkc_engine *E, double t0, int n_iv) {
     CUDA_TRY(cudaMemcpy(c.data(), P.d_ctl, c.size() * sizeof(Ctl), cudaMemcpyDeviceToHost));
     if (P.retired.size() != c.size()) P.retired.assign(c.size(), 0);
     if ((rc = plan_launch(E, P, c))) return rc;
-    if (t == GR) {
-      long active = 0;
-      for (const Ctl &x : c) active += (x.status == 0 && x.iv_left != 0);
-      E->gr_active = active;
-    }
-    for (size_t i = 0; i < c.size(); i++)
+    for (size_t i = 0; i < c.size(); i++) {
+      P.set_work((int)i, c[i].status == 0 && c[i].iv_left != 0);
       if (c[i].status && !P.retired[i]) {
         P.retired[i] = 1;
         E->n_retired++;
         if (!newly++) { first_id = P.systems[i]; first_status = c[i].status; }
       }
+    }
   }
   if (newly)
     return fail(GBRKC_ESOLVER, "%d system(s) stopped (first: system %d, status %d); the others advanced", newly,
@@ -2273,12 +2278,10 @@ int autotune_impl(gbrkc_engine *E, double t0, int n_iv, int *lanes_out) {
   int ctas[NTYPES], warps = E->gr_warps, warps_need = E->gr_warps_need, lanes0 = E->lanes;
   double work[NTYPES];
   for (int t = 0; t < NTYPES; t++) { ctas[t] = E->role_ctas[t]; work[t] = E->role_work[t]; }
-  const long active = E->gr_active;
   auto restore_host = [&]() {
     for (int t = 0; t < NTYPES; t++) { E->role_ctas[t] = ctas[t]; E->role_work[t] = work[t]; }
     E->gr_warps = warps;
     E->gr_warps_need = warps_need;
-    E->gr_active = active;
   };
   for (int t = 0; t < NTYPES; t++) {
     E->pools[t].vd.soma_out = nullptr;     // the records are not written while tuning
@@ -2736,12 +2739,12 @@ static int systems_reset_impl(gbrkc_engine *E, int first_id, int n, const gbrkc_
     fill_state(E, *P, S, P->sys_off[pi], P->sys_cell0[pi]);
     P->ctl[pi] = initial_ctl(S, d->n_intervals);
     if ((int)P->retired.size() > pi) P->retired[pi] = 0;
+    P->set_work(pi, d->n_intervals != 0);
     cells += S.n;
   }
   rc = P->f64 ? upload_run<double>(E, *P, pi0, pi0 + n) : upload_run<float>(E, *P, pi0, pi0 + n);
   if (rc) return rc;
   E->pending_init = true;
-  if (P->type == GR && E->gr_active >= 0) E->gr_active += n;
   return 0;
 }
 
@@ -2791,7 +2794,11 @@ extern "C" int gbrkc_set_budget(gbrkc_engine *E, int first_id, int n, int n_inte
   std::vector<int> v(n, n_intervals);
   CUDA_TRY(cudaMemcpy2D((char *)(P->d_ctl + pi0) + offsetof(Ctl, iv_left), sizeof(Ctl), v.data(), sizeof(int),
                         sizeof(int), n, cudaMemcpyHostToDevice));
-  for (int k = 0; k < n; k++) P->ctl[pi0 + k].iv_left = n_intervals;
+  for (int k = 0; k < n; k++) {
+    const int pi = pi0 + k;
+    P->ctl[pi].iv_left = n_intervals;
+    P->set_work(pi, n_intervals != 0 && !((int)P->retired.size() > pi && P->retired[pi]));
+  }
   return 0;
 }
 
@@ -2974,9 +2981,8 @@ extern "C" int gbrkc_advance_noalloc(gbrkc_engine *E, double t0, int n_iv) {
   }
   if (E->soma_cap > 0) E->soma_iv += n_iv;
   // stopped systems: their status words and interval budgets (adjacent in
-  // Ctl), read in chunks with a strided copy; the granule systems with work
-  // left are counted as gbrkc_advance counts them, for the next launch's
-  // granule warps
+  // Ctl), read in chunks with a strided copy; the systems with work left are
+  // noted as gbrkc_advance notes them, for the next launch
   static_assert(offsetof(Ctl, iv_left) == offsetof(Ctl, status) + sizeof(int), "status and iv_left adjacent");
   int stopped = 0, first_id = -1, first_status = 0;
   constexpr int CHUNK = 512;
@@ -2984,20 +2990,18 @@ extern "C" int gbrkc_advance_noalloc(gbrkc_engine *E, double t0, int n_iv) {
   for (int t = 0; t < NTYPES; t++) {
     PoolHost &P = E->pools[t];
     const int nsys = (int)P.systems.size();
-    long active = 0;
     for (int i0 = 0; i0 < nsys; i0 += CHUNK) {
       const int cnt = std::min(CHUNK, nsys - i0);
       CUDA_TRY(cudaMemcpy2D(word, 2 * sizeof(int), (const char *)(P.d_ctl + i0) + offsetof(Ctl, status),
                             sizeof(Ctl), 2 * sizeof(int), cnt, cudaMemcpyDeviceToHost));
       for (int i = 0; i < cnt; i++) {
         const int status = word[2 * i], iv_left = word[2 * i + 1];
-        active += (status == 0 && iv_left != 0);
+        P.set_work(i0 + i, status == 0 && iv_left != 0);
         if (status) {
           if (!stopped++) { first_id = P.systems[i0 + i]; first_status = status; }
         }
       }
     }
-    if (t == GR && nsys > 0) E->gr_active = active;
   }
   if (stopped)
     return fail(GBRKC_ESOLVER, "%d system(s) are stopped (first: system %d, status %d); the others advanced", stopped,

@@ -80,3 +80,27 @@ def test_wide_rows_on_a_cluster(others):
     other, want = _alone(others, "0")
     assert other == "mega"
     np.testing.assert_array_equal(got, want)
+
+
+def test_granule_places_follow_the_work():
+    """Granule cells alone take a place each: as many CTAs after all of them
+    were refilled as before (999 cells, FP64: 8 to a warp, a warp a CTA), and
+    as many as there are cells with work after budgets ended and were raised."""
+    n = 999
+    eng = G.Engine(G.FP64)
+    for k in range(n):
+        eng.add_system(M.GR, 1, 1, M.gr_reduced4(), [0.0])
+    eng.build()
+    eng.advance(0.0, 1)
+    first = eng.launch_layout()
+    eng.reset_systems(0, n, np.zeros(n))
+    eng.advance(G.H_MAX, 1)
+    assert eng.launch_layout() == first
+    eng.set_budget(0, 900, 0)
+    eng.advance(2 * G.H_MAX, 1)
+    few = eng.launch_layout()
+    assert few[1][M.GR] < first[1][M.GR] / 4
+    eng.set_budget(0, 900, -1)
+    eng.advance(3 * G.H_MAX, 1)
+    assert eng.launch_layout() == first
+    eng.close()
