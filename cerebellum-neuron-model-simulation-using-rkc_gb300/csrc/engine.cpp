@@ -438,8 +438,12 @@ struct PoolHost : GroupCfg {
   // chains are uneven, and the one the next launch takes (plan_launch)
   std::vector<GroupCfg> alt;
   int use_alt = -1;
-  int *d_order = nullptr;                  // the order of its line
-  bool ordered = false;                    // ... is not 0, 1, 2, ...
+  // the line's first systems: those with work, in the planned order (bit 30:
+  // held), and whether the device's copy is out of date
+  std::vector<int> order, line;
+  int *d_order = nullptr;
+  bool ordered = false;                    // order is not 0, 1, 2, ...
+  bool line_stale = true;
   std::vector<long long> steps, stages;    // counters after the last advance
   // device views
   PoolView<double> vd{};
@@ -460,8 +464,10 @@ struct PoolHost : GroupCfg {
   std::vector<char> work;
   int n_work = 0;
   void set_work(int i, bool w) {
-    n_work += (int)w - (int)work[i];
+    if (w == (bool)work[i]) return;
+    n_work += w ? 1 : -1;
     work[i] = w;
+    line_stale = true;
   }
 };
 
@@ -1279,9 +1285,10 @@ int upload_pool(gbrkc_engine *E, PoolHost &P, PoolView<R> &V) {
     V.grp_line = P.d_line + 2;
     V.ivc = 1 << 30;
     if (!team_is_group(P.team)) V.grp_abort = P.d_line;
-    std::vector<int> order(P.systems.size());
-    std::iota(order.begin(), order.end(), 0);
-    UP(order, P.d_order);
+    P.order.resize(P.systems.size());
+    std::iota(P.order.begin(), P.order.end(), 0);
+    P.line = P.order;
+    UP(P.order, P.d_order);
     V.grp_order = P.d_order;
   }
   V.grp_fast = 0;
@@ -1442,6 +1449,19 @@ void fit_granule_warps(gbrkc_engine *E) {
   }
 }
 
+// The line's first systems for the next launch, on the stream it runs on: a
+// system without work would cost its team a turn for every piece (4608 Golgi
+// slots of a server, 2 CTAs, none with work: 39 ms a launch).
+int send_line(PoolHost &P, cudaStream_t st) {
+  if (!P.line_stale) return 0;
+  int n = 0;
+  for (int i : P.order)
+    if (P.work[i & ((1 << 30) - 1)]) P.line[n++] = i;
+  if (n > 0) CUDA_TRY(cudaMemcpyAsync(P.d_order, P.line.data(), n * sizeof(int), cudaMemcpyHostToDevice, st));
+  P.line_stale = false;
+  return 0;
+}
+
 // The persistent launch's pool views and role boundaries; returns the CTA
 // count.  A register role's line (kernels.cu) is zeroed, and where its systems
 // exceed its teams they take turns.
@@ -1453,9 +1473,12 @@ int mega_pools(gbrkc_engine *E, MegaView<R> &M, int n_iv, int init) {
     M.pool[t] = P.systems.empty() ? PoolView<R>{} : pool_view<R>(P);
     if (P.grp_fast && !P.systems.empty() && !init) {
       const int nsys = (int)P.systems.size(), ctas = std::max(1, E->role_ctas[t]);
-      M.pool[t].tiles = std::min(MEGA_BLOCK / P.grid_bw, (nsys + ctas - 1) / ctas);
+      M.pool[t].tiles = std::max(1, std::min(MEGA_BLOCK / P.grid_bw, (P.n_work + ctas - 1) / ctas));
       const long places = (long)ctas * M.pool[t].tiles;
-      P.pieces = nsys > places && n_iv > 1;
+      P.pieces = P.n_work > places && n_iv > 1;
+      M.pool[t].grp_first = P.n_work;
+      int rc = send_line(P, E->streams[0]);
+      if (rc) return rc;
       M.pool[t].ivc = P.pieces ? std::max(1, (n_iv + LINE_PIECES - 1) / LINE_PIECES) : std::max(1, n_iv);
       CUDA_TRY(cudaMemsetAsync(P.d_line, 0, (4 + (1 + (P.pieces ? LINE_PIECES : 0)) * (size_t)nsys) * sizeof(int),
                                E->streams[0]));
@@ -1552,10 +1575,14 @@ int launch_cfg(gbrkc_engine *E, PoolHost &P, const GroupCfg &C, cudaStream_t st,
   PoolView<R> V = pool_view<R>(P);
   apply_group(C, V);
   const int nsys = (int)P.systems.size(), groups = C.grid / C.grp_ctas;
-  const bool pieces = nsys > groups && n_iv > 1;
+  const bool pieces = P.n_work > groups && n_iv > 1;
+  V.grp_first = P.n_work;
   V.ivc = pieces ? std::max(1, (n_iv + LINE_PIECES - 1) / LINE_PIECES) : std::max(1, n_iv);
-  if (!init && !team_is_grid(C.team))
+  if (!init && !team_is_grid(C.team)) {
+    int rc = send_line(P, st);
+    if (rc) return rc;
     CUDA_TRY(cudaMemsetAsync(P.d_line, 0, (4 + (1 + (pieces ? LINE_PIECES : 0)) * (size_t)nsys) * sizeof(int), st));
+  }
   return launch_pool<R>(P.type, V, C.team, C.grid, C.block, C.smem, st, t0, n_iv, iv0, init);
 }
 
@@ -2095,9 +2122,8 @@ static int plan_launch(gbrkc_engine *E, PoolHost &P, const std::vector<Ctl> &c) 
   if (!P.d_order || !(E->mega ? P.grp_fast != 0 : team_is_group(P.team))) return 0;
   auto up = [](long a, long b) { return (a + b - 1) / b; };
   const long ctas = std::max(1, E->role_ctas[P.type]);
-  const long tiles = E->mega ? std::min<long>(MEGA_BLOCK / P.grid_bw, up(n, ctas)) : 1;
+  const long tiles = E->mega ? std::max(1L, std::min<long>(MEGA_BLOCK / P.grid_bw, up(P.n_work, ctas))) : 1;
   const long teams = E->mega ? ctas * tiles : P.grid / P.grp_ctas;
-  if (n <= teams && P.alt.empty()) return 0;
   if ((int)P.steps.size() != n) {
     P.steps.assign(n, 0);
     P.stages.assign(n, 0);
@@ -2143,17 +2169,17 @@ static int plan_launch(gbrkc_engine *E, PoolHost &P, const std::vector<Ctl> &c) 
     longest = std::max(longest, len[i]);
   }
   const double share = sum / (double)places;
-  const bool order = n > places && longest > 0.7 * share;
+  const bool order = P.n_work > places && longest > 0.7 * share;
   if (!order && !P.ordered) return 0;
-  std::vector<int> line(n);
-  std::iota(line.begin(), line.end(), 0);
+  std::iota(P.order.begin(), P.order.end(), 0);
   if (order) {
-    std::stable_sort(line.begin(), line.end(), [&](int a, int b) { return len[a] > len[b]; });
-    for (int &i : line)
-      if (len[i] > std::max(0.5 * std::max(longest, share), 1.5 * sum / n)) i |= 1 << 30;
+    const double mean = sum / std::max(1, P.n_work);
+    std::stable_sort(P.order.begin(), P.order.end(), [&](int a, int b) { return len[a] > len[b]; });
+    for (int &i : P.order)
+      if (len[i] > std::max(0.5 * std::max(longest, share), 1.5 * mean)) i |= 1 << 30;
   }
-  CUDA_TRY(cudaMemcpy(P.d_order, line.data(), n * sizeof(int), cudaMemcpyHostToDevice));
   P.ordered = order;
+  P.line_stale = true;
   return 0;
 }
 
@@ -2200,7 +2226,6 @@ extern "C" int gbrkc_advance(gbrkc_engine *E, double t0, int n_iv) {
     std::vector<Ctl> c(P.systems.size());
     CUDA_TRY(cudaMemcpy(c.data(), P.d_ctl, c.size() * sizeof(Ctl), cudaMemcpyDeviceToHost));
     if (P.retired.size() != c.size()) P.retired.assign(c.size(), 0);
-    if ((rc = plan_launch(E, P, c))) return rc;
     for (size_t i = 0; i < c.size(); i++) {
       P.set_work((int)i, c[i].status == 0 && c[i].iv_left != 0);
       if (c[i].status && !P.retired[i]) {
@@ -2209,6 +2234,7 @@ extern "C" int gbrkc_advance(gbrkc_engine *E, double t0, int n_iv) {
         if (!newly++) { first_id = P.systems[i]; first_status = c[i].status; }
       }
     }
+    if ((rc = plan_launch(E, P, c))) return rc;
   }
   if (newly)
     return fail(GBRKC_ESOLVER, "%d system(s) stopped (first: system %d, status %d); the others advanced", newly,
@@ -2282,6 +2308,7 @@ int autotune_impl(gbrkc_engine *E, double t0, int n_iv, int *lanes_out) {
     for (int t = 0; t < NTYPES; t++) { E->role_ctas[t] = ctas[t]; E->role_work[t] = work[t]; }
     E->gr_warps = warps;
     E->gr_warps_need = warps_need;
+    for (PoolHost &P : E->pools) P.line_stale = true;   // (its device copy is restored to an older one)
   };
   for (int t = 0; t < NTYPES; t++) {
     E->pools[t].vd.soma_out = nullptr;     // the records are not written while tuning

@@ -150,7 +150,8 @@ struct PoolView {
   long grp_stride;                    // doubles of shared memory a team
   int ivc;                            // intervals a team goes on with one system while others wait
   int *grp_line;                      // [2] counters, [nsys] next intervals, [16 nsys] the line (group_sys.cuh, line_take)
-  const int *grp_order;               // [nsys] the line's first systems; bit 30: taken to its end without a turn
+  const int *grp_order;               // the line's first systems, those with work; bit 30: taken to its end without a turn
+  int grp_first;                      // their number
 };
 
 // How a pool takes its synaptic current (solve_rkc.cu): granule cells add

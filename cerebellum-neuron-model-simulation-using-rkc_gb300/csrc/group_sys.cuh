@@ -941,10 +941,11 @@ struct GroupSys {
   }
 
   // Advance the system by n intervals, the launch's k0-th and on (the launch
-  // begins at tb), or initialise it.
+  // begins at tb), or initialise it.  Whether it may go on after them: not
+  // stopped, and intervals left in its budget.
   template <bool INIT = true>
-  __device__ __forceinline__ void run(int s_, double tb, int k0, int n, int iv0_global, bool init) {
-    if (!system_selected(P.ctl[s_], init, n)) return;
+  __device__ __forceinline__ bool run(int s_, double tb, int k0, int n, int iv0_global, bool init) {
+    if (!system_selected(P.ctl[s_], init, n)) return false;
     if constexpr (!ALONE)
       if (t == 0) s_abort[0] = s_abort[1] = 0;
     bind(s_);
@@ -954,7 +955,7 @@ struct GroupSys {
       if (gave_up()) c.status |= ST_BARRIER;
     } else {
       int r = start(tb, k0, n, iv0_global);
-      if (r == TICK_DONE) return;
+      if (r == TICK_DONE) return false;
       while (r != TICK_DONE) {
         if (r == TICK_ION) {
           ion_and_b(c.sum_dt, true, true);
@@ -970,6 +971,7 @@ struct GroupSys {
       }
     }
     store(init);
+    return c.status == 0 && c.iv_left != 0;
   }
 };
 
@@ -984,8 +986,9 @@ struct GroupSys {
 // round, [0] taken, [1] left, by additions only (with compare and swap, 9700
 // quads that ended an interval together took 47 million tries: 26000 granule
 // cells 107 to 171 ms, 75 without turns).  Place i of the line is order[i] for
-// i < nsys, else line[i - nsys] - 1 once it is written; at[s] is the system's
-// next interval.  Systems that took much longer than the others in the launch
+// i < first (the systems with work), else line[i - first] - 1 once it is
+// written; at[s] is the system's next interval.  A system that stops, or whose
+// budget ends, leaves the line.  Systems that took much longer than the others in the launch
 // before come first in order, and those that may decide the launch's length
 // are held: no other is taken for them.  Granule quads take the first round
 // from their queue (first 0), then from the line.
@@ -1021,7 +1024,7 @@ template <typename R>
 __device__ __forceinline__ void line_next(const PoolView<R> &P, int &s, int &k, bool &hold) {
   const int mine = s, at = k;
   if (mine >= 0 && hold) return;
-  int got = line_take(P, P.nsys);
+  int got = line_take(P, P.grp_first);
   if (got >= 0) {
     hold = (got >> 30) != 0;
     got &= (1 << 30) - 1;

@@ -85,10 +85,10 @@ __device__ __forceinline__ void role_teams(const PoolView<R> &P, double *smem, d
     k = s_at[team];
     if (s < 0) break;
     const int n = min(P.ivc, n_iv - k);
-    S.template run<false>(s, t0, k, n, iv0, false);
+    const bool goes_on = S.template run<false>(s, t0, k, n, iv0, false);
     S.sync();
     k += n;
-    if (k >= n_iv) s = -1;
+    if (k >= n_iv || !goes_on) s = -1;
     else if (S.t == 0) __threadfence();
   }
 }

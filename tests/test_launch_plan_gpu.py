@@ -104,3 +104,46 @@ def test_granule_places_follow_the_work():
     eng.advance(3 * G.H_MAX, 1)
     assert eng.launch_layout() == first
     eng.close()
+
+
+def test_idle_slots_cost_a_role_nothing():
+    """A role of the persistent launch whose slots have no work ends at once: the
+    systems without work are not in the line that its teams take systems from.
+    (Within half a millisecond, where the granule cells beside them take 14 or
+    more; the split leaves such a role one CTA or two after a few launches.)"""
+    eng = G.Engine(G.MIXED)
+    for k in range(3000):
+        eng.add_system(M.GR, 1, 1, M.gr_reduced4(), [1e-4 * k])
+    go = [eng.add_system(M.GO, 1, 1, M.go_synthetic(2000), [0.0], idle=k > 0) for k in range(2000)]
+    eng.build()
+    for k in range(12):
+        if k == 2:
+            eng.set_budget(go[0], 1, 0)
+        eng.advance(8 * k * G.H_MAX, 8)
+    assert eng.type_team(M.GO) == "mega"
+    assert eng.last_kernel_ms(M.GO) < 0.5 < eng.last_kernel_ms(M.GR)
+    eng.close()
+
+
+def test_autotune_keeps_the_line():
+    """Budgets change between an advance and autotune, which restores the
+    device's state: the next launch still takes the systems with work."""
+    def run(tune):
+        eng = G.Engine(G.MIXED)
+        for k in range(64):
+            eng.add_system(M.GR, 1, 1, M.gr_reduced4(), [0.0])
+        go = [eng.add_system(M.GO, 1, 1, M.go_synthetic(2000), [0.0]) for k in range(40)]
+        eng.build()
+        eng.advance(0.0, 2)
+        eng.set_budget(go[0], 30, 0)
+        eng.advance(2 * G.H_MAX, 2)
+        eng.set_budget(go[0], 40, -1)
+        if tune:
+            eng.autotune(4 * G.H_MAX, 2)
+        eng.advance(4 * G.H_MAX, 2)
+        out = [eng.vnew(i) for i in go] + [eng.ctl(i) for i in go]
+        eng.close()
+        return out
+
+    for a, b in zip(run(True), run(False)):
+        np.testing.assert_equal(a, b)
