@@ -508,6 +508,8 @@ struct gbrkc_engine {
   int gr_warps_max = 0;         // granule warps the CTAs can hold beside the other roles
   int lanes = 16;               // lanes of a warp in use by granule systems (one each, or four: TEAM_LANE4)
   double role_work[NTYPES] = {};  // smoothed CTA-ms per role
+  int split_n[NTYPES] = {};     // systems with work in the last launch, and its intervals (follow_work)
+  int split_iv = 8;
   int *d_queue = nullptr;
   unsigned long long *d_tstart = nullptr, *d_tend = nullptr;
   // device address of noalloc.cu's static launch scratch, looked up at build
@@ -1642,6 +1644,38 @@ int system_loc(gbrkc_engine *E, int id, PoolHost **P, HostSystem **S) {
 
 namespace {
 
+// The CTAs of the roles other than the granule cells': `avail` in proportion to
+// their work, each within its cap (a role cannot use more CTAs than it has
+// teams of work).
+void split_rest(gbrkc_engine *E, const double *work, int avail) {
+  double total = 0.0;
+  for (int t = 0; t < NTYPES; t++)
+    if (t != GR && E->role_ctas[t] > 0) total += work[t];
+  int want[NTYPES] = {}, used = 0;
+  for (int t = 0; t < NTYPES; t++) {
+    if (t == GR || E->role_ctas[t] == 0) continue;
+    const int n = total > 0.0 ? (int)std::lround(avail * work[t] / total) : 1;
+    want[t] = std::max(1, std::min(E->role_cap[t], n));
+    used += want[t];
+  }
+  // fix the total by moving CTAs to / from the role with the largest work per CTA
+  while (used != avail) {
+    int best = -1;
+    double bv = used < avail ? -1.0 : 1e300;
+    for (int t = 0; t < NTYPES; t++) {
+      if (t == GR || want[t] == 0) continue;
+      const double v = work[t] / want[t];
+      if (used < avail && want[t] < E->role_cap[t] && v > bv) { bv = v; best = t; }
+      if (used > avail && want[t] > 1 && v < bv) { bv = v; best = t; }
+    }
+    if (best < 0) break;
+    want[best] += used < avail ? 1 : -1;
+    used += used < avail ? 1 : -1;
+  }
+  for (int t = 0; t < NTYPES; t++)
+    if (t != GR) E->role_ctas[t] = want[t];
+}
+
 // Re-split the persistent launch's CTAs between roles so that they finish
 // together.  Granule warps are latency-bound (a lone warp runs one dependent
 // FP64 chain per system at ~64 cycles an operation): spreading them over more
@@ -1650,8 +1684,7 @@ namespace {
 // inversely proportional to the CTAs they get.  The granule CTA count moves
 // halfway to where the two models cross; the other roles then split the
 // remaining CTAs in proportion to their measured work (CTAs x makespan,
-// smoothed over launches), each within its cap (a role cannot use more CTAs
-// than it has teams of work).
+// smoothed over launches).
 void rebalance_roles(gbrkc_engine *E, const double *role_ms, bool tune_gr) {
   int avail = E->mega_grid;
   if (E->role_ctas[GR] > 0) {
@@ -1693,39 +1726,57 @@ void rebalance_roles(gbrkc_engine *E, const double *role_ms, bool tune_gr) {
     E->role_ctas[GR] = std::max(lo, std::min(hi, c));
     avail -= E->role_ctas[GR];
   }
-  // work per role (CTA-ms), smoothed over launches
-  double work[NTYPES] = {}, total = 0.0;
+  // work per role (CTA-ms), smoothed over launches; a role has no more CTAs at
+  // work than systems
+  double work[NTYPES] = {};
   for (int t = 0; t < NTYPES; t++) {
-    if (t == GR || E->role_ctas[t] == 0) continue;
-    const double w = std::max(role_ms[t], 1e-3) * E->role_ctas[t];
+    if (E->role_ctas[t] == 0) continue;
+    const double w = std::max(role_ms[t], 1e-3) * std::min(E->role_ctas[t], std::max(1, E->pools[t].n_work));
     E->role_work[t] = (E->role_work[t] > 0.0) ? 0.5 * E->role_work[t] + 0.5 * w : w;
     work[t] = E->role_work[t];
-    total += work[t];
   }
-  if (total <= 0.0) return;
-  int want[NTYPES] = {}, used = 0;
+  split_rest(E, work, avail);
+}
+
+// Called before a launch: where the systems with work have changed since the
+// last one -- a type has more than twice as many, or none left -- the CTAs are
+// split anew, by the roles' work: what was measured, and for such a type an
+// estimate.  rebalance_roles alone takes several launches to follow: it
+// moves half way, and where one granule cell had left its role one CTA the 3433
+// that came next took 1050 ms on it, 19 on the 88 of this split (a stream of
+// 48 requests to a server: p50 3.6 -> 2.3 s, p99 4.7 -> 3.4 s).  The estimates
+// are CTA-ms per compartment and interval of pools that fill their CTAs: 2048
+// Golgi cells 36 ms on 152 CTAs for 8 intervals, 200 Purkinje cells 7 ms,
+// granule cells 0.13 to 0.5 CTA-ms a cell by their currents, olive networks of
+// 64 compartments 3 ms on a quarter of a CTA.
+void follow_work(gbrkc_engine *E, int n_iv) {
+  if (!E->mega) return;
+  static const double est[NTYPES] = {0.0094, 0.0026, 0.0004, 0.0013};
+  double work[NTYPES] = {}, total = 0.0;
+  bool changed = false;
+  int others = 0;
   for (int t = 0; t < NTYPES; t++) {
-    if (t == GR || E->role_ctas[t] == 0) continue;
-    const int n = (int)std::lround(avail * work[t] / total);
-    want[t] = std::max(1, std::min(E->role_cap[t], n));
-    used += want[t];
+    if (E->role_ctas[t] == 0) continue;
+    const PoolHost &P = E->pools[t];
+    const bool grown = P.n_work > 2 * E->split_n[t], ended = P.n_work == 0 && E->split_n[t] > 0;
+    if (grown || ended) E->role_work[t] = 0.0;
+    changed |= grown || ended;
+    if (P.n_work > 0)
+      work[t] = E->role_work[t] > 0.0
+                    ? E->role_work[t] * n_iv / std::max(1, E->split_iv)
+                    : est[t] * n_iv * (double)P.nc * P.n_work / (double)P.systems.size();
+    total += work[t];
+    others += t != GR;
+    E->split_n[t] = P.n_work;
   }
-  // fix the total by moving CTAs to / from the role with the largest work per CTA
-  while (used != avail) {
-    int best = -1;
-    double bv = used < avail ? -1.0 : 1e300;
-    for (int t = 0; t < NTYPES; t++) {
-      if (t == GR || want[t] == 0) continue;
-      const double v = work[t] / want[t];
-      if (used < avail && want[t] < E->role_cap[t] && v > bv) { bv = v; best = t; }
-      if (used > avail && want[t] > 1 && v < bv) { bv = v; best = t; }
-    }
-    if (best < 0) break;
-    want[best] += used < avail ? 1 : -1;
-    used += used < avail ? 1 : -1;
+  E->split_iv = n_iv;
+  if (!changed || total <= 0.0) return;
+  int avail = E->mega_grid;
+  if (E->role_ctas[GR] > 0) {
+    E->role_ctas[GR] = std::max(1, std::min(avail - others, (int)std::lround(avail * work[GR] / total)));
+    avail -= E->role_ctas[GR];
   }
-  for (int t = 0; t < NTYPES; t++)
-    if (t != GR) E->role_ctas[t] = want[t];
+  split_rest(E, work, avail);
 }
 
 // Whether a role of the persistent launch keeps its systems' vectors in
@@ -1848,7 +1899,10 @@ int setup_mega(gbrkc_engine *E) {
   // the first launch's granule warps fit the granule CTAs (lanes take
   // further systems in turn)
   E->gr_warps = std::min(E->gr_warps, (MEGA_BLOCK / 32) * E->role_ctas[GR]);
-  for (int t = 0; t < NTYPES; t++) E->role_work[t] = 0.0;
+  for (int t = 0; t < NTYPES; t++) {
+    E->role_work[t] = 0.0;
+    E->split_n[t] = E->pools[t].n_work;
+  }
   return 0;
 }
 
@@ -2194,6 +2248,7 @@ extern "C" int gbrkc_advance(gbrkc_engine *E, double t0, int n_iv) {
     P.vf.soma_out = so;
   }
   int rc = 0;
+  follow_work(E, std::max(1, E->sv.n > 0 ? 1 : n_iv));
   fit_granule_warps(E);
   if (E->pending_init) {
     // systems reset since the last call: initialise them (only them) first
@@ -2982,6 +3037,7 @@ extern "C" int gbrkc_advance_noalloc(gbrkc_engine *E, double t0, int n_iv) {
   if (!E || n_iv < 0) return fail(GBRKC_EINVAL, "bad arguments");
   if (!E->built) return fail(GBRKC_ESTATE, "engine not built");
   if (E->sv.n > 0) return fail(GBRKC_EINVAL, "engines with synapses step through gbrkc_advance");
+  follow_work(E, std::max(1, n_iv));
   fit_granule_warps(E);
   const int iv0 = E->soma_iv;
   for (int t = 0; t < NTYPES; t++) {

@@ -147,3 +147,38 @@ def test_autotune_keeps_the_line():
 
     for a, b in zip(run(True), run(False)):
         np.testing.assert_equal(a, b)
+
+
+def test_split_follows_the_work():
+    """Granule cells that come beside other types get the CTAs they need in
+    their first launch, not after the split has crept there: it takes less
+    than three times the launch of the same cells eight launches later."""
+    eng = G.Engine(G.MIXED)
+    n = 3400
+    for k in range(n):
+        eng.add_system(M.GR, 1, 1, M.gr_reduced4(), [1e-4 * k])
+    for k in range(40):
+        eng.add_system(M.GO, 1, 1, M.go_synthetic(2000), [0.0])
+    eng.build()
+    at = 0.0
+
+    def advance():
+        nonlocal at
+        eng.advance(at, 8)
+        at += 8 * G.H_MAX
+        return eng.last_advance_ms()
+
+    eng.set_budget(1, n - 1, 0)
+    for _ in range(6):
+        advance()
+    assert eng.launch_layout()[1][M.GR] == 1
+    eng.set_budget(1, n - 1, -1)
+    first = advance()
+    for _ in range(8):
+        later = advance()
+    assert first < 3.0 * later, (first, later)
+    eng.set_budget(n, 40, 0)
+    advance()
+    advance()
+    assert eng.launch_layout()[1][M.GO] == 1      # (and of a type with no work left they go to the others)
+    eng.close()
