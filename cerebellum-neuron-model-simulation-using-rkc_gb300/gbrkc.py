@@ -83,6 +83,7 @@ class SynapseDesc(C.Structure):
 
 
 SYN_MFGR, SYN_GRGO, SYN_GOGR, SYN_GRPKJ = 0, 1, 2, 3
+NCOND = (10, 13, 11, 8)          # channel densities of a cell, by type
 SYNF_VAL, SYNF_S0, SYNF_S1, SYNF_S2, SYNF_OLD_V = 0, 1, 2, 3, 4
 
 _LIB = None
@@ -179,6 +180,18 @@ def _ip(a):
     return a.ctypes.data_as(C.POINTER(C.c_int))
 
 
+def _channel_factors(factors, cell_type, systems, cells):
+    """Channel-density factors as the C ABI reads them, one row per cell, from
+    one row per cell or one per system (all of its cells alike)."""
+    f = np.ascontiguousarray(factors, dtype=np.float64).reshape(-1)
+    k = NCOND[cell_type] if 0 <= cell_type < len(NCOND) else 0
+    if f.size < cells * k:
+        if f.size != systems * k:
+            raise ValueError(f"{f.size} channel factors for {cells} cells of {k} channels in {systems} systems")
+        f = np.repeat(f.reshape(systems, k), cells // systems, axis=0).reshape(-1)
+    return f
+
+
 class Engine:
     """A set of RKC systems advanced together on the GPU."""
 
@@ -232,7 +245,7 @@ class Engine:
             keep.append(cs)
         d.idle = int(idle)
         if cond_scale_ch is not None:
-            cc = np.ascontiguousarray(cond_scale_ch, dtype=np.float64).reshape(-1)
+            cc = _channel_factors(cond_scale_ch, cell_type, 1, n)
             d.cond_scale_ch = _dp(cc)
             keep.append(cc)
         sid = C.c_int()
@@ -264,7 +277,7 @@ class Engine:
             d.io_gap_g = _dp(gg)
             keep.append(gg)
         if cond_scale_ch is not None:
-            cc = np.ascontiguousarray(cond_scale_ch, dtype=np.float64).reshape(-1)
+            cc = _channel_factors(cond_scale_ch, self.ncomp[first][0] if first in self.ncomp else 0, n, cells)
             d.cond_scale_ch = _dp(cc)
             keep.append(cc)
         d.n_intervals = n_intervals
