@@ -873,7 +873,8 @@ bool group_tables(PoolHost &P, int bw, int ctas, bool grid) {
     for (int e = g0; e < g0 + ng; e++)
       if (P.gap_pre[e] >= 0) t_gap[e] = place(cta_of(P.gap_post[e]), P.gap_pre[e]);
   }
-  if (rows > (grid ? GRID_MAX_ROWS : ctas > 1 && P.type == PKJ ? 4 : 2) || (rows > 1 && maxdeg > 15)) return false;   // (row lengths: four bits each)
+  if (rows > (grid ? GRID_MAX_ROWS : ctas > 1 && P.type == PKJ ? 4 : 2)) return false;
+  if (!grid && rows > 1 && maxdeg > 15) return false;   // (row lengths: four bits each; GroupSys::deg)
   const int ld = rows * bw;
   const size_t smem = grid_smem(ld, most, maxdeg, (grid || ctas == 1) ? 0 : ctas);
   if (smem > GRID_SMEM_MAX || ld + most + 2 > GRID_PLACES) return false;

@@ -281,6 +281,7 @@ struct GroupSys {
       // the warp's longest row here
 #pragma unroll
       for (int st = 16; st > 0; st /= 2) cnt = max(cnt, __shfl_xor_sync(0xffffffffu, cnt, st));
+      if constexpr (K > 1 && COMM == GRP_GRID) cnt = min(cnt, 15);
       wdeg |= cnt << (4 * q);
     }
     if constexpr (K == 1) {
@@ -388,7 +389,7 @@ struct GroupSys {
     for (int q = 0; q < K; q++) {
       f[q] = 0.0;
       if (K > 1 && q >= rows) break;
-      const int lr = q * bw + t, n = deg(wdeg, q);
+      const int lr = q * bw + t, n = deg(q);
       double d = MIXED ? b[q] : -b[q];
       if (n > 0) {
         const double2 g = K == 1 ? rg[0] : lg[lr];
@@ -410,8 +411,12 @@ struct GroupSys {
       else f[q] = d * linv[lr];
     }
   }
-  static __device__ __forceinline__ int deg(int packed, int q) {
-    return K == 1 ? packed : (int)((unsigned)packed >> (4 * q)) & 15;
+  __device__ __forceinline__ int deg(int q) const {
+    if constexpr (K == 1) return wdeg;
+    const int n = (int)((unsigned)wdeg >> (4 * q)) & 15;
+    // (grid: 15 stands for 15 and more, a row run to the longest row's end)
+    if constexpr (COMM == GRP_GRID) return n < 15 ? n : 2 * pairs;
+    return n;
   }
 
   // the pairwise tree over a[0..8) of which n are there
