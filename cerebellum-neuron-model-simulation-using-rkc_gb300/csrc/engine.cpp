@@ -774,8 +774,8 @@ void fill_state(gbrkc_engine *E, PoolHost &P, const HostSystem &S, long off, int
 }
 
 // The group team's tables for the pool's systems on groups of `ctas` CTAs of
-// bw threads (group_sys.cuh); ctas 1 is the one-CTA team, which needs none.
-// CTA c owns the chunks of bw elements from c chunks / ctas on; every operator
+// bw threads (group_sys.cuh); the one-CTA team (ctas 1, not the grid) needs
+// none.  CTA c owns the chunks of bw elements from c chunks / ctas on; every operator
 // entry's column becomes its place in the row's CTA, among the CTA's own
 // elements or behind them among the values it receives.  In the grid team an
 // element that another CTA reads gets a publishing slot; in a cluster its
@@ -796,7 +796,7 @@ bool group_tables(PoolHost &P, int bw, int ctas, bool grid) {
     const int *cl = own ? P.s_col.data() + P.s_nz0[P.sys_csr[k]] : P.t_col.data() + P.t_nz0[P.sys_tmpl[k]];
     const int chunks = (nc + bw - 1) / bw;
     for (int i = 0; i < (own ? nc : ncomp); i++) maxdeg = std::max(maxdeg, r[i + 1] - r[i]);
-    if (ctas == 1) {
+    if (ctas == 1 && !grid) {
       rows = std::max(rows, chunks);
       continue;
     }

@@ -49,6 +49,31 @@ def test_long_rows_several_a_thread(oracle, monkeypatch, branches, bw, ctas):
     eng.close()
 
 
+@pytest.mark.parametrize("ncomp,bw", [(9, 0), (32, 0), (250, 32), (700, 128), (700, 256)])
+def test_grid_of_one_cta(oracle, monkeypatch, ncomp, bw):
+    """The grid team on one CTA -- a system of a warp at most, or a forced shape
+    -- has its tables like any other, with nothing to receive."""
+    monkeypatch.setenv("GBRKC_GRID_MIN_NC", "9")
+    if bw:
+        monkeypatch.setenv("GBRKC_GRID_BW", str(bw))
+        monkeypatch.setenv("GBRKC_GRID_CTAS", "1")
+    t, rows, stim = M.PKJ, M.pkj_synthetic(2, ncomp), (ncomp - 1, 0.02e-3, 0.0, 1e9)
+    jit = jitter_for(oracle, t, 1)
+    s = oracle.System(t, 1, 1, rows, jit, stim=stim, canon=True)
+    assert s.init() == 0
+    eng = G.Engine(G.FP64)
+    sid = eng.add_system(t, 1, 1, rows, jit, stim=stim)
+    eng.build()
+    assert eng.type_team(t) == "grid" and eng.launch_layout()[1][t] == 1
+    for k in range(4):
+        eng.advance(k * G.H_MAX, 1)
+        assert s.advance(k * G.H_MAX) == 0
+        np.testing.assert_array_equal(eng.vnew(sid), s.vnew())
+    ctl, st, status = eng.ctl(sid)
+    assert status == 0 and st == s.stats()
+    eng.close()
+
+
 def test_large_system_with_a_long_row_takes_the_grid():
     """5 x 5 Purkinje cells of 1600 compartments whose somas have 17 dendrites and
     more (two elements a thread on every SM)."""
