@@ -927,7 +927,9 @@ TeamCost team_cost(const PoolHost &P, double rows, double warps, int comm) {
 // CTAs of a warp; 2048: five warps each).  A lone system of GRID_MIN_NC
 // compartments always takes the grid.  GBRKC_GROUP=0 and GBRKC_GRID=0 switch
 // the teams off, a forced cluster size (GBRKC_CLUSTER_SIZE) too;
-// GBRKC_GRID_MIN_NC sends a lone system of that size to the grid.
+// GBRKC_GRID_MIN_NC sends a lone system of that size to the grid, and
+// GBRKC_GROUP=cta:THREADS or cluster:THREADSxCTAS forces a shape where the
+// pool's systems fit it.
 constexpr long GRID_MIN_NC = 8192;
 bool group_team(const gbrkc_engine *E, PoolHost &P) {
   const char *cs = getenv("GBRKC_CLUSTER_SIZE"), *gr = getenv("GBRKC_GROUP"), *gd = getenv("GBRKC_GRID");
@@ -944,7 +946,12 @@ bool group_team(const gbrkc_engine *E, PoolHost &P) {
     return g > 0 && grid_shape(nc, g, &bw, &ctas) &&
            group_tables(P, bw, (int)std::min<long>(ctas, (nc + bw - 1) / bw), true);
   };
-  if (grid_ok && nc >= grid_nc) return to_grid();
+  int want_bw = 0, want_ctas = 1;
+  if (gr && sscanf(gr, "cta:%d", &want_bw) != 1 && sscanf(gr, "cluster:%dx%d", &want_bw, &want_ctas) != 2) want_bw = 0;
+  if (want_bw > 0 && (want_bw > GRID_BLOCK || want_bw % 32 != 0 || want_ctas < 1 || want_ctas > 16 ||
+                      (want_ctas > 1 && (want_bw & (want_bw - 1)) != 0)))
+    return false;
+  if (want_bw == 0 && grid_ok && nc >= grid_nc) return to_grid();
   if (nc >= GRID_MIN_NC) return false;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
@@ -964,7 +971,12 @@ bool group_team(const gbrkc_engine *E, PoolHost &P) {
   int kind = 0, bbw = 0, bctas = 1;
   struct Wide { double time; int bw, ctas; };
   std::map<int, Wide> wide;                // per CTAs of a cluster: the best shape with one long system
-  for (int bw = 32; bw <= GRID_BLOCK; bw += 32) {
+  if (want_bw > 0) {
+    kind = want_ctas > 1 ? 2 : 1;
+    bbw = want_bw;
+    bctas = want_ctas;
+  }
+  for (int bw = 32; bw <= GRID_BLOCK && want_bw == 0; bw += 32) {
     const long rows = up(nc, bw), fit = std::max(1, 65536 / (256 * bw));   // CTAs an SM's registers hold
     if (rows <= 2) {
       const long per = std::min(fit, up(nsys, sms));
@@ -993,7 +1005,7 @@ bool group_team(const gbrkc_engine *E, PoolHost &P) {
       if (it == wide.end() || th < it->second.time) wide[(int)ctas] = Wide{th, bw, (int)ctas};
     }
   }
-  if (grid_ok) {
+  if (grid_ok && want_bw == 0) {
     int bw = 0, ctas = 0;
     if (grid_shape(nc, sms, &bw, &ctas)) {
       const double t = time((double)up(nc, (long)bw * ctas), bw / 32.0, 1, 2);
