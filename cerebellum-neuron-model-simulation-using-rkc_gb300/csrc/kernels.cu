@@ -141,13 +141,16 @@ __global__ void __launch_bounds__(MEGA_BLOCK, 1) k_mega(const __grid_constant__ 
 
 // The dynamic shared-memory limit is a per-kernel attribute shared by every
 // engine in the process: only ever raise it, so that a later engine with
-// smaller needs cannot break an earlier one's launches.
+// smaller needs cannot break an earlier one's launches.  Unless it is set, a
+// launch may have 48 KB in all, the kernel's own variables (4.4 KB in the group
+// teams) among them.
 static cudaError_t raise_smem_limit(const void *k, size_t smem) {
   cudaFuncAttributes a;
   cudaError_t e = cudaFuncGetAttributes(&a, k);
   if (e != cudaSuccess) return e;
-  if ((size_t)a.maxDynamicSharedSizeBytes >= smem) return cudaSuccess;
-  return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const size_t limit = (size_t)a.maxDynamicSharedSizeBytes, unset = 48 * 1024;
+  if (smem <= limit && (limit > unset || smem + a.sharedSizeBytes <= unset)) return cudaSuccess;
+  return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(smem, limit));
 }
 
 template <typename R>
@@ -182,12 +185,12 @@ static const void *kernel_ptr(int type, int team) {
 template <typename R>
 int prepare_pool_kernel(int type, int team, size_t smem) {
   const void *k = kernel_ptr<R>(type, team);
-  if (smem > 48 * 1024) {
-    cudaError_t e = raise_smem_limit(k, smem);
-    if (e != cudaSuccess) return (int)e;
-  }
+  cudaError_t e = cudaSuccess;
+  // (no kernel has 16 KB of its own; asking loads it)
+  if (smem > 32 * 1024) e = raise_smem_limit(k, smem);
+  if (e != cudaSuccess) return (int)e;
   if (team_cluster_size(team) > 8 || team_is_clu(team)) {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return (int)e;
   }
   return 0;

@@ -10,6 +10,7 @@ import pytest
 import gbrkc as G
 import morph as M
 import test_group_gpu as T
+from test_grid_rows_gpu import star_purkinje
 
 pytestmark = pytest.mark.gpu
 
@@ -34,6 +35,8 @@ FORMS = [
     ((M.IO, 1, 16, 16, io), "cluster:64x12", "cluster", 1),
     ((M.PKJ, 3, 1, 1, pkj(977)), "cluster:64x16", "cluster", 1),
     ((M.PKJ, 3, 1, 1, pkj(977)), "cluster:128x4", "cluster", 2),
+    ((M.PKJ, 3, 1, 1, pkj(977)), "cluster:256x2", "cluster", 2),     # 46 KB of shared memory beside the kernel's own 4
+    ((M.PKJ, 2, 1, 1, lambda k: star_purkinje(440, 6, 2 + k)), "cta:224", "pool", 2),      # the same
     ((M.PKJ, 3, 1, 1, pkj(977)), "cluster:128x3", "cluster", 4),     # three and two chunks a CTA
     ((M.PKJ, 3, 1, 1, pkj(977)), "cluster:64x4", "cluster", 4),
     ((M.PKJ, 20, 1, 1, pkj(1599)), "cluster:128x13", "cluster", 1),
