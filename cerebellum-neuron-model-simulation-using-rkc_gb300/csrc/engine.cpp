@@ -1763,7 +1763,7 @@ void rebalance_roles(gbrkc_engine *E, const double *role_ms, bool tune_gr) {
 // granule cells 0.13 to 0.5 CTA-ms a cell by their currents, olive networks of
 // 64 compartments 3 ms on a quarter of a CTA.
 void follow_work(gbrkc_engine *E, int n_iv) {
-  if (!E->mega) return;
+  if (!E->mega || n_iv < 1) return;
   static const double est[NTYPES] = {0.0094, 0.0026, 0.0004, 0.0013};
   double work[NTYPES] = {}, total = 0.0;
   bool changed = false;
@@ -2261,7 +2261,7 @@ extern "C" int gbrkc_advance(gbrkc_engine *E, double t0, int n_iv) {
     P.vf.soma_out = so;
   }
   int rc = 0;
-  follow_work(E, std::max(1, E->sv.n > 0 ? 1 : n_iv));
+  follow_work(E, E->sv.n > 0 ? std::min(1, n_iv) : n_iv);
   fit_granule_warps(E);
   if (E->pending_init) {
     // systems reset since the last call: initialise them (only them) first
@@ -3050,7 +3050,7 @@ extern "C" int gbrkc_advance_noalloc(gbrkc_engine *E, double t0, int n_iv) {
   if (!E || n_iv < 0) return fail(GBRKC_EINVAL, "bad arguments");
   if (!E->built) return fail(GBRKC_ESTATE, "engine not built");
   if (E->sv.n > 0) return fail(GBRKC_EINVAL, "engines with synapses step through gbrkc_advance");
-  follow_work(E, std::max(1, n_iv));
+  follow_work(E, n_iv);
   fit_granule_warps(E);
   const int iv0 = E->soma_iv;
   for (int t = 0; t < NTYPES; t++) {
