@@ -510,6 +510,7 @@ struct gbrkc_engine {
   double role_work[NTYPES] = {};  // smoothed CTA-ms per role
   int split_n[NTYPES] = {};     // systems with work in the last launch, and its intervals (follow_work)
   int split_iv = 8;
+  bool copies_pending = true;   // copies or fills on the default stream since the last launch (settle)
   int *d_queue = nullptr;
   unsigned long long *d_tstart = nullptr, *d_tend = nullptr;
   // device address of noalloc.cu's static launch scratch, looked up at build
@@ -1477,6 +1478,17 @@ int send_line(PoolHost &P, cudaStream_t st) {
   return 0;
 }
 
+// The engine's streams do not wait for the default stream, on which state is
+// copied and cleared between launches (a device-to-device copy or a fill, and
+// a small copy from the host, may still run when the call returns): called
+// before a launch.
+int settle(gbrkc_engine *E) {
+  if (!E->copies_pending) return 0;
+  CUDA_TRY(cudaStreamSynchronize(0));
+  E->copies_pending = false;
+  return 0;
+}
+
 // The persistent launch's pool views and role boundaries; returns the CTA
 // count.  A register role's line (kernels.cu) is zeroed, and where its systems
 // exceed its teams they take turns.
@@ -1528,6 +1540,7 @@ int check_pieces(gbrkc_engine *E) {
 template <typename R>
 int launch_mega_all(gbrkc_engine *E, double t0, int n_iv, int iv0, int init) {
   MegaView<R> M{};
+  if (int rc = settle(E)) return rc;
   const int end = mega_pools<R>(E, M, n_iv, init);
   if (end < 0) return end;
   if (end > E->mega_grid || end <= 0)
@@ -1608,6 +1621,7 @@ int launch_all(gbrkc_engine *E, double t0, int n_iv, int iv0, int init) {
   if (E->mega && !alt)
     return (E->precision == GBRKC_FP64) ? launch_mega_all<double>(E, t0, n_iv, iv0, init)
                                         : launch_mega_all<float>(E, t0, n_iv, iv0, init);
+  if (int rc = settle(E)) return rc;
   CUDA_TRY(cudaEventRecord(E->ev_start, E->streams[0]));
   for (int t = 1; t < NTYPES; t++) CUDA_TRY(cudaStreamWaitEvent(E->streams[t], E->ev_start, 0));
   for (int t = 0; t < NTYPES; t++) {
@@ -2339,6 +2353,7 @@ struct Snapshot {
     dev.push_back(q);
     src.push_back({p, n});
     e = cudaMemcpy(q, p, n, cudaMemcpyDeviceToDevice);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(0);
     if (e != cudaSuccess) return fail(GBRKC_ECUDA, "autotune snapshot: %s", cudaGetErrorString(e));
     return 0;
   }
@@ -2347,6 +2362,7 @@ struct Snapshot {
       cudaError_t e = cudaMemcpy(src[k].first, dev[k], src[k].second, cudaMemcpyDeviceToDevice);
       if (e != cudaSuccess) return fail(GBRKC_ECUDA, "autotune restore: %s", cudaGetErrorString(e));
     }
+    CUDA_TRY(cudaStreamSynchronize(0));       // (the copies: device-to-device ones return at once)
     return 0;
   }
 };
@@ -2631,6 +2647,7 @@ static int record_soma_impl(gbrkc_engine *E, int n_max) {
   if (!E->built) return fail(GBRKC_ESTATE, "engine not built");
   E->soma_cap = n_max;
   E->soma_iv = 0;
+  E->copies_pending = true;
   for (int t = 0; t < NTYPES; t++) {
     PoolHost &P = E->pools[t];
     if (P.systems.empty() || n_max == 0) { P.d_soma = nullptr; continue; }
@@ -2661,6 +2678,7 @@ extern "C" int gbrkc_record_width(gbrkc_engine *E, int type, int width) {
     }
   }
   CUDA_TRY(cudaMemcpy(P.d_cell_soma, first.data(), first.size() * sizeof(int), cudaMemcpyHostToDevice));
+  E->copies_pending = true;
   P.cell_soma = first;
   P.rec_w = width;
   P.vd.rec_w = P.vf.rec_w = width;
@@ -2889,6 +2907,7 @@ extern "C" int gbrkc_set_budget(gbrkc_engine *E, int first_id, int n, int n_inte
   std::vector<int> v(n, n_intervals);
   CUDA_TRY(cudaMemcpy2D((char *)(P->d_ctl + pi0) + offsetof(Ctl, iv_left), sizeof(Ctl), v.data(), sizeof(int),
                         sizeof(int), n, cudaMemcpyHostToDevice));
+  E->copies_pending = true;
   for (int k = 0; k < n; k++) {
     const int pi = pi0 + k;
     P->ctl[pi].iv_left = n_intervals;
@@ -2912,6 +2931,7 @@ static int record_spikes_impl(gbrkc_engine *E, long capacity) {
       P.spk_cap = (int)capacity;
     }
     CUDA_TRY(cudaMemset(P.d_spk_count, 0, sizeof(int)));
+    E->copies_pending = true;
     P.vd.spk_log = P.vf.spk_log = P.d_spk_log;
     P.vd.spk_cap = P.vf.spk_cap = P.spk_cap;
   }
@@ -2935,6 +2955,7 @@ static int read_spikes_impl(gbrkc_engine *E, int type, long cap, double *t, int 
   std::vector<SpikeRec> r(avail);
   if (avail > 0) CUDA_TRY(cudaMemcpy(r.data(), P.d_spk_log, avail * sizeof(SpikeRec), cudaMemcpyDeviceToHost));
   CUDA_TRY(cudaMemset(P.d_spk_count, 0, sizeof(int)));
+  E->copies_pending = true;
   // the device appends in completion order: sort by time, then pool cell
   std::sort(r.begin(), r.end(), [](const SpikeRec &a, const SpikeRec &b) {
     return a.t < b.t || (a.t == b.t && a.cell < b.cell);
@@ -2989,6 +3010,7 @@ namespace {
 template <typename R>
 int launch_mega_static(gbrkc_engine *E, double t0, int n_iv, int iv0, int init, unsigned long long *scratch) {
   MegaView<R> M{};
+  if (int rc = settle(E)) return rc;
   const int end = mega_pools<R>(E, M, n_iv, init);
   if (end < 0) return end;
   if (end > NOALLOC_MAX_CTAS)

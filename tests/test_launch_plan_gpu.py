@@ -7,6 +7,7 @@ import sys
 import numpy as np
 import pytest
 
+import configs
 import gbrkc as G
 import morph as M
 
@@ -182,3 +183,24 @@ def test_split_follows_the_work():
     advance()
     assert eng.launch_layout()[1][M.GO] == 1      # (and of a type with no work left they go to the others)
     eng.close()
+
+
+def test_autotune_restores_before_the_next_launch():
+    """A batch whose state takes longer to copy back than a launch to begin:
+    every launch of the tuning, and the advance after it, starts from the
+    restored state -- the same bits as without the tuning."""
+    def run(tune):
+        eng = G.Engine(G.MIXED)
+        specs = configs.scaled_stated_batch(0.5)
+        ids = configs.add_to(eng, specs)
+        eng.build()
+        eng.advance(0.0, 2, tolerate_retire=True)
+        for _ in range(2 if tune else 0):
+            eng.autotune(2 * G.H_MAX, 8)
+        eng.advance(2 * G.H_MAX, 8, tolerate_retire=True)
+        out = [eng.vnew(i) for i in ids[::7]] + [eng.ctl(i) for i in ids[::7]]
+        eng.close()
+        return out
+
+    for a, b in zip(run(True), run(False)):
+        np.testing.assert_equal(a, b)
