@@ -3,17 +3,18 @@
 // for a cluster) of every CTA of a cooperative launch; its five RKC vectors
 // and its current b in registers, at most K elements a thread.
 //
-// What bounds it: an FP64 warp instruction costs 64 cycles on its SM
-// sub-partition whatever its lanes do, so a stage is about 12 of them per
-// element row, and the rest of a stage is the latency of handing the stage
-// vector's values to the threads that read them.  So:
+// What bounds it: a warp issues an FP64 instruction every 64 cycles whatever
+// its lanes do, an SM one every 19 for all of its warps, so a stage is about
+// 12 of them per element row, and the rest of a stage is the latency of handing
+// the stage vector's values to the threads that read them.  So:
 //  * Elements go to CTAs in runs of whole chunks of bw consecutive elements
 //    (a power of two where there are several CTAs): in a tree numbered along
 //    its branches most neighbours are then in the same CTA, read from shared
 //    memory.
 //  * A value that another CTA reads is handed over as two 64-bit words, each
-//    half of the value beside the evaluation's number: one store and one load
-//    that polls for that number, no fence, no flag, no barrier over the CTAs.
+//    half of the value beside the evaluation's number: two stores, and two
+//    loads that poll for that number, no fence, no flag, no barrier over the
+//    CTAs.
 //    In a cluster the writer stores into the reader's shared memory (about
 //    200 cycles), in the grid team into a slot of global memory that its
 //    readers poll in the L2 (about 1500).  Slots are double-buffered.  A CTA
@@ -36,8 +37,9 @@
 // ms): full granule cell, FP64, one interval 39.5 -> 12.2 (a cluster of
 // 10 CTAs of 64 threads; one CTA before); 77 Golgi cells, FP64, five
 // intervals 45.5 -> 10.7 (clusters of 5 x 32); 16x16 olive network, mixed, 16
-// intervals 26.9 -> 10.8 (12 x 64); Purkinje 3x3, FP64, eight intervals 23.6
-// -> 20.3 (grid, 113 x 128: two fifths of it the FP64 ion updates).
+// intervals 26.9 -> 9.7 (12 x 64); Purkinje 3x3, FP64, eight intervals
+// 3.7 -> 3.0 (from t = 5 ms, sums over the same windows; grid, 113 x 128: two
+// fifths of it the FP64 ion updates).
 //
 // The arithmetic is Sys's (integrator.cuh) operation for operation.
 #pragma once
@@ -946,11 +948,10 @@ struct GroupSys {
   }
 
   // Advance the system by n intervals, the launch's k0-th and on (the launch
-  // begins at tb), or initialise it.  Whether it may go on after them: not
-  // stopped, and intervals left in its budget.
+  // begins at tb), or initialise it.
   template <bool INIT = true>
-  __device__ __forceinline__ bool run(int s_, double tb, int k0, int n, int iv0_global, bool init) {
-    if (!system_selected(P.ctl[s_], init, n)) return false;
+  __device__ __forceinline__ void run(int s_, double tb, int k0, int n, int iv0_global, bool init) {
+    if (!system_selected(P.ctl[s_], init, n)) return;
     if constexpr (!ALONE)
       if (t == 0) s_abort[0] = s_abort[1] = 0;
     bind(s_);
@@ -960,7 +961,7 @@ struct GroupSys {
       if (gave_up()) c.status |= ST_BARRIER;
     } else {
       int r = start(tb, k0, n, iv0_global);
-      if (r == TICK_DONE) return false;
+      if (r == TICK_DONE) return;
       while (r != TICK_DONE) {
         if (r == TICK_ION) {
           ion_and_b(c.sum_dt, true, true);
@@ -976,7 +977,6 @@ struct GroupSys {
       }
     }
     store(init);
-    return c.status == 0 && c.iv_left != 0;
   }
 };
 

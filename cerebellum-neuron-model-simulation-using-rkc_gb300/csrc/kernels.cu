@@ -1,7 +1,8 @@
 #include <type_traits>
-// k_mega: one persistent launch for all pools, every CTA a role pulling
-// systems from its role's queue; and the launches of it and of the per-pool
-// kernels (kernels_pool.cu).
+// k_mega: one persistent launch for all pools, every CTA a role taking
+// systems from its role's queue or pieces of them from its line
+// (group_sys.cuh); and the launches of it and of the per-pool kernels
+// (kernels_pool.cu).
 //
 // Built with -fmad=false (see integrator.cuh).  R selects FP64 or FP32
 // gating; the instantiations live in kernels_fp64.cu / kernels_fp32.cu.
@@ -58,9 +59,10 @@ __device__ __forceinline__ void role_block(const PoolView<R> &P, int *q, double 
 // A role of teams with their system's vectors in registers (group_sys.cuh), at
 // most K elements a thread: P.tiles teams of P.grid_bw threads a CTA.  A
 // Golgi cell takes five warps: alone on its SM each issues an FP64 instruction
-// in 95 cycles, so that the cells whose step size is at its floor (up to 1024
-// attempts a ms where the median cell takes 115), whose serial chains set the
-// launch's time, run five times as fast as on a warp of eight systems' warps;
+// in 95 cycles (five at the SM's 19), so that the cells whose step size is at
+// its floor (up to 1024 attempts a ms where the median cell takes 115), whose
+// serial chains set the launch's time, run five times as fast as on a warp of
+// eight systems' warps;
 // and the warps of a team run the same instructions at the same time, where
 // eight systems' warps each fetched their own (40% of their cycles).
 template <int CT, typename R, int K>
@@ -85,10 +87,11 @@ __device__ __forceinline__ void role_teams(const PoolView<R> &P, double *smem, d
     k = s_at[team];
     if (s < 0) break;
     const int n = min(P.ivc, n_iv - k);
-    const bool goes_on = S.template run<false>(s, t0, k, n, iv0, false);
+    S.template run<false>(s, t0, k, n, iv0, false);
     S.sync();
     k += n;
-    if (k >= n_iv || !goes_on) s = -1;
+    // (thread 0 takes and leaves systems, and wrote this one's Ctl)
+    if (k >= n_iv || (S.t == 0 && !system_selected(P.ctl[s], false, 1))) s = -1;
     else if (S.t == 0) __threadfence();
   }
 }

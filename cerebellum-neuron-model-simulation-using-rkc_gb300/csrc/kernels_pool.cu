@@ -108,10 +108,11 @@ __global__ void __launch_bounds__(GRID_BLOCK, 1) k_advance_group(const __grid_co
       k = s_item[1];
       if (s < 0) break;
       const int n = min(P.ivc, n_iv - k);
-      const bool goes_on = S.run(s, t0, k, n, iv0, false);
+      S.run(s, t0, k, n, iv0, false);
       S.group_sync();
       k += n;
-      if (k >= n_iv || !goes_on) s = -1;
+      // (the group's first thread takes and leaves systems, and wrote this one's Ctl)
+      if (k >= n_iv || (S.cta == 0 && S.t == 0 && !system_selected(P.ctl[s], false, 1))) s = -1;
       else if (S.cta == 0 && S.t == 0) __threadfence();
     }
   }
