@@ -438,6 +438,7 @@ struct PoolHost : GroupCfg {
   // chains are uneven, and the one the next launch takes (plan_launch)
   std::vector<GroupCfg> alt;
   int use_alt = -1;
+  bool warps = false;                      // Golgi: the next launch takes a warp per cell (plan_launch)
   // the line's first systems: those with work, in the planned order (bit 30:
   // held), and whether the device's copy is out of date
   std::vector<int> order, line;
@@ -504,7 +505,7 @@ struct gbrkc_engine {
   int role_ctas[NTYPES] = {};
   int role_cap[NTYPES] = {};
   int gr_warps = 0;             // granule warps of the next launch (32 lanes each)
-  int gr_warps_need = 0;        // granule warps that would give every granule system with work its own lane
+  int gr_warps_need = 0;        // granule warps that would give every granule system with work its own place (a lane, or four)
   int gr_warps_max = 0;         // granule warps the CTAs can hold beside the other roles
   int lanes = 16;               // lanes of a warp in use by granule systems (one each, or four: TEAM_LANE4)
   double role_work[NTYPES] = {};  // smoothed CTA-ms per role
@@ -1498,7 +1499,16 @@ int mega_pools(gbrkc_engine *E, MegaView<R> &M, int n_iv, int init) {
   for (int t = 0; t < NTYPES; t++) {
     PoolHost &P = E->pools[t];
     M.pool[t] = P.systems.empty() ? PoolView<R>{} : pool_view<R>(P);
-    if (P.grp_fast && !P.systems.empty() && !init) {
+    if (P.warps) {
+      P.pieces = false;
+      M.pool[t].grp_fast = 0;
+      if (!init) {
+        int rc = send_line(P, E->streams[0]);
+        if (rc) return rc;
+        M.pool[t].in_order = 1;
+        M.pool[t].grp_first = P.n_work;
+      }
+    } else if (P.grp_fast && !P.systems.empty() && !init) {
       const int nsys = (int)P.systems.size(), ctas = std::max(1, E->role_ctas[t]);
       M.pool[t].tiles = std::max(1, std::min(MEGA_BLOCK / P.grid_bw, (P.n_work + ctas - 1) / ctas));
       const long places = (long)ctas * M.pool[t].tiles;
@@ -1704,10 +1714,11 @@ void split_rest(gbrkc_engine *E, const double *work, int avail) {
 }
 
 // Re-split the persistent launch's CTAs between roles so that they finish
-// together.  Granule warps are latency-bound (a lone warp runs one dependent
-// FP64 chain per system at ~64 cycles an operation): spreading them over more
-// CTAs shortens their time only through less sharing of each SM's FP64 pipe,
-// modelled as T ~ (warps per CTA)^0.5.  The other roles' time is taken as
+// together.  Granule warps are latency-bound (a warp runs its cells' dependent
+// FP64 chains at ~64 cycles an operation): spreading them over more CTAs
+// shortens their time only through less sharing of each SM's FP64 pipe,
+// modelled as T ~ (warps per CTA)^0.5; with more cells than places (quads in
+// turns) the time is the rounds' besides.  The other roles' time is taken as
 // inversely proportional to the CTAs they get.  The granule CTA count moves
 // halfway to where the two models cross; the other roles then split the
 // remaining CTAs in proportion to their measured work (CTAs x makespan,
@@ -1723,9 +1734,9 @@ void rebalance_roles(gbrkc_engine *E, const double *role_ms, bool tune_gr) {
         nother++;
         other_ctas += E->role_ctas[t];
       }
-    // granule role time on x CTAs, A warps giving every system a lane:
-    // each lane runs max(1, A / 8x) systems in turn, and a system's serial
-    // chain slows as sqrt(warps per CTA) (FP64 issue shared on the SM)
+    // granule role time on x CTAs, A warps giving every system a place (a lane,
+    // or four): each place serves max(1, A / 8x) systems in turn, and a system's
+    // serial chain slows as sqrt(warps per CTA) (FP64 issue shared on the SM)
     const double A = std::max(1, E->gr_warps_need > 0 ? E->gr_warps_need : E->gr_warps);
     auto gr_time = [&](double x) {
       const double per = MEGA_BLOCK / 32;
@@ -1930,6 +1941,11 @@ int setup_mega(gbrkc_engine *E) {
     E->role_work[t] = 0.0;
     E->split_n[t] = E->pools[t].n_work;
   }
+  // warps for the Golgi cells (plan_launch), as long as nothing is known of
+  // their chains, from twice the cells a team where they pay if some are at
+  // the step floor
+  PoolHost &Go = E->pools[GO];
+  Go.warps = Go.grp_fast == 1 && !Go.f64 && Go.n_work > 100 * E->role_ctas[GO];
   return 0;
 }
 
@@ -2197,7 +2213,12 @@ extern "C" int gbrkc_build(gbrkc_engine *E) { return no_throw([&] { return build
 // third of the measured times, so a cluster team has to promise a quarter.
 // (200 Purkinje cells, mixed, a ms: at rest 7.0 ms in the persistent launch,
 // 7.6 in clusters of two CTAs, 9.5 of thirteen; with some spiking at the
-// step floor 42.9 to 53.6 against 20.7 to 28.8.)
+// step floor 42.9 to 53.6 against 20.7 to 28.8.)  (3) Where Golgi cells outnumber
+// their teams some fifty times, no cell's chain counts and a warp per cell
+// does more: eight cells' warps fill the SM's FP64 pipe where a team's wait for
+// one another and for the controller.  The longest cells come first, each to
+// its end.  (32 768 Golgi beside as many granule cells, 5 ms: 3.9 s with teams, 3.2 with warps; 2048 alone,
+// a ms: 36 ms with teams, 77 with warps.)
 static int plan_launch(gbrkc_engine *E, PoolHost &P, const std::vector<Ctl> &c) {
   const int n = (int)c.size();
   if (!P.d_order || !(E->mega ? P.grp_fast != 0 : team_is_group(P.team))) return 0;
@@ -2249,8 +2270,19 @@ static int plan_launch(gbrkc_engine *E, PoolHost &P, const std::vector<Ctl> &c) 
     sum += len[i];
     longest = std::max(longest, len[i]);
   }
+  P.warps = false;
+  if (E->mega && P.type == GO && P.grp_fast == 1) {
+    const TeamCost W = team_cost(P, (double)up(P.max_nc, 32), MEGA_BLOCK / 32.0, 0);
+    double wsum = 0.0, wlong = 0.0;
+    for (int i = 0; i < n; i++) {
+      const double t = W.of(att[i], stg[i]);
+      wsum += t;
+      wlong = std::max(wlong, t);
+    }
+    P.warps = std::max(wlong, wsum / (double)(ctas * (MEGA_BLOCK / 32))) < 0.9 * std::max(longest, sum / (double)places);
+  }
   const double share = sum / (double)places;
-  const bool order = P.n_work > places && longest > 0.7 * share;
+  const bool order = P.warps || (P.n_work > places && longest > 0.7 * share);
   if (!order && !P.ordered) return 0;
   std::iota(P.order.begin(), P.order.end(), 0);
   if (order) {

@@ -152,6 +152,7 @@ struct PoolView {
   int *grp_line;                      // [2] counters, [nsys] next intervals, [16 nsys] the line (group_sys.cuh, line_take)
   const int *grp_order;               // the line's first systems, those with work; bit 30: taken to its end without a turn
   int grp_first;                      // their number
+  int in_order;                       // warps take whole systems in that order (else all of the pool's, 0, 1, 2, ...)
 };
 
 // How a pool takes its synaptic current (solve_rkc.cu): granule cells add
@@ -211,9 +212,12 @@ constexpr int team_cluster_size(int team) {
 }
 
 // All pools in one persistent launch: CTA b < role_end[0] integrates granule
-// systems (one per lane or per four, on the CTA's first warps), then Golgi
-// (32-lane warps), Purkinje and olive (whole blocks).  Each role pulls
-// systems from its own atomic queue.
+// systems (one per lane or per four, on the CTA's first warps), then Golgi,
+// Purkinje and olive ones.  Granule lanes take systems from an atomic queue,
+// quads with more systems than places then from the line; the other roles'
+// register teams take pieces of systems from the line (group_sys.cuh), and
+// where those do not hold a role's systems (grp_fast 0), and at initialisation,
+// warps (Golgi) and whole blocks take whole systems from the queue.
 template <typename R>
 struct MegaView {
   PoolView<R> pool[NTYPES];

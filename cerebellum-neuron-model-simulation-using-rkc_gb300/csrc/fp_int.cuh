@@ -1,17 +1,18 @@
 // FP64 comparisons, conversions and the stage count's square root in integer
 // and FP32 arithmetic, with the results of the FP64 instructions they stand
-// for, bit for bit.
+// for, bit for bit; and quotients, rounded as the divide rounds them but for
+// one operand pair in about 2^51 (recip, below).
 //
-// On GB300 every FP64 warp instruction holds its SM sub-partition's FP64 port
-// for 64 cycles, whatever the active lanes or the independent work beside it,
-// and the comparisons and conversions hold it longer (measured on one SM,
-// cycles per warp instruction: DFMA 64, DSETP 110, F2F.F32.F64 102,
+// On GB300 a warp issues an FP64 instruction every 64 cycles, whatever its
+// active lanes or the independent work beside it (an SM, from four warps on,
+// one every 19), and the comparisons and conversions take longer (one warp on
+// an SM, cycles per instruction: DFMA 64, DSETP 110, F2F.F32.F64 102,
 // F2F.F64.F32 99, F2I.F64 102, DSQRT 600), while the integer pipe takes an
 // instruction every cycle or two and is otherwise idle here.  A comparison of
 // non-negative values is two integer instructions.
 //
 // Host and device: tests/native/fp_int_check.cpp compares every function with
-// the host's FP64 arithmetic.
+// the host's FP64 arithmetic, tests/native/fp_int_gpu.cu with the GPU's.
 #ifndef GBRKC_FP_INT_CUH
 #define GBRKC_FP_INT_CUH
 
@@ -143,7 +144,8 @@ GB_HD int int_sqrt(double x, bool &ok) {
 // (Markstein, IBM J. Res. Dev. 34(1), 1990).  The correction's error is under
 // 2^-52 of q0's last place, so the result is the rounded quotient unless a / b
 // lies that close to the midpoint of two doubles (one operand pair in about
-// 2^51); none of 10^9 random pairs differs.  Three FP64 operations for the
+// 2^51); none of 4 10^8 random quotients differs from the GPU's own, and none
+// of the host check's.  Three FP64 operations for the
 // reciprocal and three for each quotient, where the divide takes 565 cycles
 // (nine FP64 operations' time).  Operands outside the ranges below
 // (subnormals, infinities, NaN and a zero divisor among them) take the divide.

@@ -32,7 +32,10 @@ __device__ __forceinline__ void role_tiles(const PoolView<R> &P, int *q, double 
   double *my = smem + (long)tile * P.ws_tile_doubles;
   for (;;) {
     int s = 0;
-    if (tm.r == 0) s = atomicAdd(q, 1);
+    if (tm.r == 0) {
+      s = atomicAdd(q, 1);
+      if (P.in_order) s = s < P.grp_first ? P.grp_order[s] & ((1 << 30) - 1) : P.nsys;
+    }
     s = __shfl_sync(tm.mask, s, 0, TS);
     if (s >= P.nsys) break;
     run_system<CT, R, TileTeam<TS>>(P, tm, s, my, t0, n_iv, iv0, init != 0);

@@ -4,7 +4,7 @@
 //
 // What bounds it: a granule system is one serial chain of FP64 instructions
 // (its controller's tolerance of 1e-9 keeps it at about 4000 step attempts
-// per ms), and an FP64 warp instruction costs 64 cycles whether one lane or
+// per ms), and a warp issues one in 64 cycles whether one lane or
 // all 32 are active and whatever its independence.  So the count of FP64 warp
 // instructions per attempt sets the pace, and a compartment a lane quarters
 // the vector part of it: about 40 instructions an attempt here (mixed

@@ -204,3 +204,41 @@ def test_autotune_restores_before_the_next_launch():
 
     for a, b in zip(run(True), run(False)):
         np.testing.assert_equal(a, b)
+
+
+def _many_golgi(n=5600):
+    """Golgi cells that outnumber the persistent launch's teams some 37 times,
+    alike but for a few currents: the third launch, planned from the second."""
+    rng = np.random.default_rng(6)
+    eng = G.Engine(G.MIXED)
+    rows = M.go_synthetic(2000)
+    for k in range(n):
+        eng.add_system(M.GO, 1, 1, rows, rng.uniform(-0.5, 0.5, 1), stim=([30], [1e-5 * (k % 7)], [0.0], [1e9]))
+    eng.build()
+    eng.set_budget(17, 9, 5)
+    eng.record_soma(6)
+    for k in range(3):
+        eng.advance(2 * k * G.H_MAX, 2)
+    team = eng.type_team(M.GO)
+    soma = np.empty((6, eng.type_cells(M.GO)))
+    out = [eng.read_soma_type(M.GO, 6, soma)] + [eng.read(i, f) for i in range(0, n, 41) for f in (G.F_V, G.F_B, G.F_YN)]
+    stats = [eng.ctl(i) for i in range(0, n, 41)]
+    ms = eng.last_advance_ms()
+    eng.close()
+    return team, out, stats, ms
+
+
+def test_golgi_cells_beyond_their_teams_take_warps(monkeypatch):
+    """The next launch takes a warp per cell where that does more: the same bits
+    as with warps alone (GBRKC_GROUP=0), and about their time (the launches of
+    two seeds of the same work differ by less than a sixth; a launch in teams
+    takes a third longer)."""
+    monkeypatch.delenv("GBRKC_GROUP", raising=False)
+    team, got, stats, ms = _many_golgi()
+    monkeypatch.setenv("GBRKC_GROUP", "0")
+    other, want, wstats, wms = _many_golgi()
+    assert team == other == "mega"
+    for a, b in zip(got, want):
+        np.testing.assert_array_equal(a, b)
+    assert stats == wstats
+    assert ms < 1.17 * wms, (ms, wms)
