@@ -1057,7 +1057,7 @@ def run_batch(args, G, configs, torch, specs, wl, precision, rank, world, dist):
     else:
         dom = max(range(4), key=lambda k: kern_ms[k])
         team = eng.type_team(dom)
-        base = {"grid": "k_advance_grid", "cluster": "k_advance_cluster"}.get(team, "k_advance")
+        base = "k_advance_group" if team in ("grid", "cluster") else "k_advance"
         kname, key = f"{base}<{names[dom]}>", names[dom]
         per_launch_units, per_launch_ms = units_t[dom] / args.steps, kern_ms[dom] / args.steps
     achieved = bpu * per_launch_units / (per_launch_ms * 1e-3) / 1e9 if per_launch_ms > 0 else 0.0
