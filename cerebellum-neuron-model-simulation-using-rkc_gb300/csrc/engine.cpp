@@ -2232,9 +2232,8 @@ static int plan_launch(gbrkc_engine *E, PoolHost &P, const std::vector<Ctl> &c) 
   }
   std::vector<double> att(n), stg(n), len(n);
   for (int i = 0; i < n; i++) {
-    // (a system refilled since counts from 0 again)
-    att[i] = (double)(c[i].n_steps - (c[i].n_steps >= P.steps[i] ? P.steps[i] : 0));
-    stg[i] = (double)(c[i].n_stage - (c[i].n_stage >= P.stages[i] ? P.stages[i] : 0));
+    att[i] = (double)(c[i].n_steps - P.steps[i]);
+    stg[i] = (double)(c[i].n_stage - P.stages[i]);
     P.steps[i] = c[i].n_steps;
     P.stages[i] = c[i].n_stage;
   }
@@ -2348,7 +2347,8 @@ extern "C" int gbrkc_advance(gbrkc_engine *E, double t0, int n_iv) {
         if (!newly++) { first_id = P.systems[i]; first_status = c[i].status; }
       }
     }
-    if ((rc = plan_launch(E, P, c))) return rc;
+    // (an advance of no intervals, as after a refill, says nothing of the next)
+    if (n_iv > 0 && (rc = plan_launch(E, P, c))) return rc;
   }
   if (newly)
     return fail(GBRKC_ESOLVER, "%d system(s) stopped (first: system %d, status %d); the others advanced", newly,
@@ -2885,6 +2885,7 @@ static int systems_reset_impl(gbrkc_engine *E, int first_id, int n, const gbrkc_
     P->ctl[pi] = initial_ctl(S, d->n_intervals);
     if ((int)P->retired.size() > pi) P->retired[pi] = 0;
     P->set_work(pi, d->n_intervals != 0);
+    if ((int)P->steps.size() > pi) P->steps[pi] = P->stages[pi] = 0;
     cells += S.n;
   }
   rc = P->f64 ? upload_run<double>(E, *P, pi0, pi0 + n) : upload_run<float>(E, *P, pi0, pi0 + n);

@@ -242,3 +242,22 @@ def test_golgi_cells_beyond_their_teams_take_warps(monkeypatch):
         np.testing.assert_array_equal(a, b)
     assert stats == wstats
     assert ms < 1.17 * wms, (ms, wms)
+
+
+def test_no_intervals_leave_the_plan():
+    """An advance of no intervals -- a refill's initialisation -- keeps what the
+    last launch said of the next one's teams."""
+    n = 170
+    eng = G.Engine(G.MIXED)
+    for k in range(n):
+        eng.add_system(M.PKJ, 1, 1, M.pkj_synthetic(2, 801), [0.0])
+    eng.build()
+    eng.set_budget(3, n - 3, 0)
+    eng.advance(0.0, 2)
+    assert eng.type_team(M.PKJ) == "cluster"
+    eng.reset_systems(0, 3, np.zeros(3))
+    eng.advance(0.0, 0)
+    assert eng.type_team(M.PKJ) == "cluster"
+    eng.advance(0.0, 2)
+    assert eng.type_team(M.PKJ) == "cluster"
+    eng.close()
