@@ -2218,7 +2218,7 @@ extern "C" int gbrkc_build(gbrkc_engine *E) { return no_throw([&] { return build
 // does more: eight cells' warps fill the SM's FP64 pipe where a team's wait for
 // one another and for the controller.  The longest cells come first, each to
 // its end.  (32 768 Golgi beside as many granule cells, 5 ms: 3.9 s with teams,
-// 3.2 with warps; 2048 alone, a ms: 36 ms with teams, 77 with warps.)
+// 3.0 with warps; 2048 alone, a ms: 36 ms with teams, 77 with warps.)
 static int plan_launch(gbrkc_engine *E, PoolHost &P, const std::vector<Ctl> &c) {
   const int n = (int)c.size();
   if (!P.d_order || !(E->mega ? P.grp_fast != 0 : team_is_group(P.team))) return 0;
